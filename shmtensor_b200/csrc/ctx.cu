@@ -2,7 +2,7 @@
 #include <stdarg.h>
 #include <string.h>
 
-#include "ctx.cuh"
+#include "relabel.cuh"
 
 namespace shmt {
 
@@ -226,9 +226,9 @@ int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, 
   DeviceGuard guard(ctx->device);
   if (int rc = ctx_reserve(ctx, (size_t)scratch_bytes)) return rc;
   if (relabel_ids > 0) {
-    uint64_t cap = 64;
-    while (cap < (uint64_t)relabel_ids * 2) cap <<= 1;
-    if (int rc = ctx_reserve_table(ctx, cap * 16, static_cast<cudaStream_t>(stream))) return rc;
+    if (int rc = ctx_reserve_table(ctx, relabel_capacity(relabel_ids) * sizeof(RelSlot),
+                                   static_cast<cudaStream_t>(stream)))
+      return rc;
   }
   return SHMT_OK;
 }

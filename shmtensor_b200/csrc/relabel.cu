@@ -7,16 +7,16 @@
 // scan: (1) claim a table slot per distinct id and take the minimum input
 // index per slot, remembering each element's slot in the output array;
 // (2) flag first occurrences, scan the flags with a decoupled look-back inside
-// the same kernel, emit unique ids and the slot -> new id table; (3) remap, and
-// put every slot that was used back to "empty", so the table needs no memset
-// between calls.  Every element probes the table once (the reference four times).
+// the same kernel, emit unique ids and the slot -> new id table, and put every slot
+// that was used back to "empty", so the table needs no memset between calls;
+// (3) remap the repeats.  Every element probes the table once (the reference four times).
 // The element counts may live on the device (written by an earlier kernel), so a
 // chain of hops can be queued without the host knowing any size.
 #include "relabel.cuh"
 
 namespace shmt {
 
-constexpr uint64_t kRelDirectMinTableBytes = 32ull << 20;
+constexpr uint64_t kRelSurveyMinTableBytes = 32ull << 20;
 
 __device__ __forceinline__ void resolve_sizes(Parts& ps, int64_t* numel) {
   if (ps.dev_n1) {  // |part 0| from the device if given there, else the host's start[1]
@@ -36,83 +36,139 @@ __device__ __forceinline__ int64_t part_elem(const Parts& ps, int64_t i) {
   return load_int(ps.ptr[p], ps.is64, i - ps.start[p]);
 }
 
-// Largest id of the input, read as an unsigned number (so that a negative id counts as huge).
+// One id in 2^shift is in the sample, picked by its hash, so that all its occurrences are or none
+// is; at most 2^(kRelSampleBits - 1) of the ids then are, and the bitmap stays sparse enough to
+// count them by the bits they set (linear counting, Whang et al. 1990).
+__device__ __forceinline__ int relabel_sample_shift(int64_t numel) {
+  int shift = 0;
+  while ((numel >> shift) > ((int64_t)1 << (kRelSampleBits - 1))) ++shift;
+  return shift;
+}
+
+// A look at a large input before any slot is claimed: its largest id (a negative id counts as
+// huge), and how many distinct ids it holds, from a sample.
 __global__ void __launch_bounds__(kRelThreads)
-relabel_range_kernel(Parts ps, unsigned long long* range) {
+relabel_survey_kernel(Parts ps, RelSurvey* survey) {
+  __shared__ unsigned s_marked[kRelThreads / 32];
   pdl_prologue();
   int64_t numel;
   resolve_sizes(ps, &numel);
+  const int shift = relabel_sample_shift(numel);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long m = 0;
-  int64_t done = 0;  // elements covered by the 16-byte loads below
-  if (ps.n == 1 && (reinterpret_cast<uintptr_t>(ps.ptr[0]) & 15) == 0) {
-    // one aligned array: 16-byte loads, four per thread in flight
-    const int per = ps.is64 ? 2 : 4;
-    const int64_t n_vec = numel / per;
-    const uint4* src = static_cast<const uint4*>(ps.ptr[0]);
-    for (int64_t v = gtid; v < n_vec; v += 4 * stride) {
-      uint4 x[4];
+  unsigned marked = 0;
+  auto take = [&](long long id) {
+    m = max(m, (unsigned long long)id);
+    const uint64_t h = mix64((uint64_t)id);
+    if (shift == 0 || (h >> (64 - shift)) == 0) {
+      const uint32_t at = (uint32_t)h & ((1u << kRelSampleBits) - 1u), bit = 1u << (at & 31);
+      if (!(__ldcg(survey->bitmap + (at >> 5)) & bit))
+        marked += (atomicOr(survey->bitmap + (at >> 5), bit) & bit) == 0;
+    }
+  };
+  for (int p = 0; p < ps.n; ++p) {
+    const int64_t n = ps.start[p + 1] - ps.start[p];
+    int64_t done = 0;  // elements covered by the 16-byte loads below
+    if ((reinterpret_cast<uintptr_t>(ps.ptr[p]) & 15) == 0) {
+      // an aligned part: 16-byte loads, four per thread in flight
+      const int per = ps.is64 ? 2 : 4;
+      const int64_t n_vec = n / per;
+      const uint4* src = static_cast<const uint4*>(ps.ptr[p]);
+      for (int64_t v = gtid; v < n_vec; v += 4 * stride) {
+        uint4 x[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        x[u] = v + u * stride < n_vec ? __ldg(src + v + u * stride) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < 4; ++u)
+          if (v + u * stride < n_vec) x[u] = __ldg(src + v + u * stride);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (ps.is64) {
-          m = max(m, ((unsigned long long)x[u].y << 32) | x[u].x);
-          m = max(m, ((unsigned long long)x[u].w << 32) | x[u].z);
-        } else {
-          m = max(m, (unsigned long long)(long long)(int)x[u].x);
-          m = max(m, (unsigned long long)(long long)(int)x[u].y);
-          m = max(m, (unsigned long long)(long long)(int)x[u].z);
-          m = max(m, (unsigned long long)(long long)(int)x[u].w);
+        for (int u = 0; u < 4; ++u) {
+          if (v + u * stride >= n_vec) continue;
+          if (ps.is64) {
+            take((long long)(((unsigned long long)x[u].y << 32) | x[u].x));
+            take((long long)(((unsigned long long)x[u].w << 32) | x[u].z));
+          } else {
+            take((int)x[u].x);
+            take((int)x[u].y);
+            take((int)x[u].z);
+            take((int)x[u].w);
+          }
         }
       }
+      done = n_vec * per;
     }
-    done = n_vec * per;
-  }
-  for (int64_t i = done + gtid; i < numel; i += 4 * stride) {
-    long long v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = i + u * stride < numel ? part_elem(ps, i + u * stride) : 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) m = max(m, (unsigned long long)v[u]);
+    for (int64_t i = done + gtid; i < n; i += stride) take(load_int(ps.ptr[p], ps.is64, i));
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(range, m);
+  for (int o = 16; o > 0; o >>= 1) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    marked += __shfl_xor_sync(0xffffffffu, marked, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_marked[threadIdx.x >> 5] = marked;
+    if (m) atomicMax(&survey->largest, m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    marked = 0;
+    for (int w = 0; w < kRelThreads / 32; ++w) marked += s_marked[w];
+    if (marked) atomicAdd(&survey->marked, (unsigned long long)marked);
+  }
 }
 
-__global__ void __launch_bounds__(kRelThreads)
+// How a call of `numel` ids uses the table.  Without a survey: at least two slots per id, as if all
+// were distinct.  With one: ids that all fit the table are their own slots (a frontier of densely
+// numbered nodes touches a compact part of the table); else kRelSlotsPerId slots per distinct id.
+constexpr double kRelSlotsPerId = 1.5;
+__device__ __forceinline__ RelRange relabel_range(const RelTable& t, int64_t numel, const RelSurvey* survey) {
+  RelRange r{t.slots, relabel_near((double)numel, relabel_slots_per_id((double)numel, 2.0), t.cap), t.cap, false};
+  if (survey) {
+    if (survey->largest < (unsigned long long)t.cap) {
+      r.near = t.cap;
+      r.direct = true;
+    } else {
+      const float bits = (float)(1 << kRelSampleBits), free_bits = bits - (float)survey->marked;
+      const float sampled = free_bits > 0.0f ? -bits * logf(free_bits / bits) : bits * 16.0f;
+      const double ids = (double)sampled * (double)(1ull << relabel_sample_shift(numel));
+      r.near = relabel_near(ids < (double)numel ? ids : (double)numel, kRelSlotsPerId, t.cap);
+    }
+  }
+  return r;
+}
+
+__global__ void __launch_bounds__(kRelThreads, 6)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
-                      const unsigned long long* __restrict__ range) {
+                      const RelSurvey* __restrict__ survey) {
   pdl_prologue();
   int64_t numel;
   resolve_sizes(ps, &numel);
-  // The table is provisioned for the largest input the caller allows; hash into only as
-  // much of it as this input needs (load <= 0.5), so a small input stays in a small,
-  // cache-resident part.  Only the inserting code hashes; the rest follows recorded slots.
-  const uint32_t mask = relabel_mask_for(numel, t.mask);
-  // ids that all fit the table are their own slots: a frontier of densely numbered nodes then
-  // touches a compact, cache-resident part of the table instead of one line per distinct id
-  const bool direct = range != nullptr && *range <= (unsigned long long)mask;
+  const RelRange range = relabel_range(t, numel, survey);
+  // One element per thread and step, its successor's id read ahead: six resident CTAs of 38
+  // registers claim 33.5 M ids in 690 us where two elements per thread (3 CTAs) took 1,150.
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += stride) {
-    bool maybe_first;
-    const uint32_t pos = relabel_insert_one(t.slots, mask, part_elem(ps, i), (unsigned)i, status, &maybe_first,
-                                            direct);
-    store_int(out, ps.is64, i, relabel_pack(pos, maybe_first, ps.is64, t.mask));
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  long long next = i < numel ? part_elem(ps, i) : 0;
+  for (; i < numel; i += stride) {
+    const long long key = next;
+    if (i + stride < numel) next = part_elem(ps, i + stride);
+    unsigned seen;
+    const uint32_t pos = relabel_claim(range, key, status, &seen);
+    store_int(out, ps.is64, i, relabel_pack(pos, relabel_settle(range, pos, seen, (unsigned)i), ps.is64));
   }
 }
 
+// Flags first occurrences, numbers them in input order (look-back over the tiles) and finishes
+// everything that can be finished for them: the unique id, the element's own result, and the slot,
+// which gets the new id and is emptied for the next call in the same 16-byte store (a later
+// candidate of the same id still finds an index that is not its own there).  What is left for the
+// remap kernel are the repeats alone, marked as such.  A warp takes 32 * ITEMS consecutive
+// elements, 32 at a time, so that every access to the streamed arrays is contiguous; all slot
+// reads of a thread are in flight together.
 template <int ITEMS>
-__global__ void __launch_bounds__(kRelThreads)
-relabel_compact_kernel(Parts ps, RelTable t, const void* __restrict__ slot_of,
-                       void* __restrict__ unique, TileStates st, int64_t* ticket, int64_t* status,
-                       int64_t* result, HostPost post) {
-  __shared__ int64_t warp_sums[32];
-  __shared__ int64_t s_total;
-  __shared__ int64_t s_prefix;
+__global__ void __launch_bounds__(kRelThreads, 4)
+relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique, TileStates st,
+                       int64_t* ticket, int64_t* status, int64_t* result, HostPost post) {
+  __shared__ int s_warp_firsts[kRelThreads / 32];
+  __shared__ LookbackShared s_look;
   __shared__ int s_tile;
   pdl_prologue();
   int64_t numel;
@@ -127,97 +183,104 @@ relabel_compact_kernel(Parts ps, RelTable t, const void* __restrict__ slot_of,
     }
     return;
   }
-  const int64_t base = (int64_t)tile * kTile + (int64_t)threadIdx.x * ITEMS;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = (int64_t)tile * kTile + (int64_t)warp * (32 * ITEMS) + lane;
   uint32_t pos[ITEMS];
+  unsigned first[ITEMS];
   unsigned maybe = 0, is_first = 0;  // one bit per element of this thread
-  // the thread's ITEMS slot numbers: 16-byte loads when the whole run lies inside the input
-  // and the array is aligned, else one by one
-  if (base + ITEMS <= numel && (reinterpret_cast<uintptr_t>(slot_of) & 15) == 0) {
-    if (ps.is64) {
-      const ulonglong2* src = reinterpret_cast<const ulonglong2*>(slot_of) + base / 2;
 #pragma unroll
-      for (int q = 0; q < ITEMS / 2; ++q) {
-        const ulonglong2 v = __ldg(src + q);
-        bool m0, m1;
-        pos[2 * q] = relabel_unpack64(v.x, &m0);
-        pos[2 * q + 1] = relabel_unpack64(v.y, &m1);
-        maybe |= ((unsigned)m0 << (2 * q)) | ((unsigned)m1 << (2 * q + 1));
-      }
-    } else {
-      const uint4* src = reinterpret_cast<const uint4*>(slot_of) + base / 4;
-#pragma unroll
-      for (int q = 0; q < ITEMS / 4; ++q) {
-        const uint4 v = __ldg(src + q);
-        const uint32_t raw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          bool m;
-          pos[4 * q + e] = relabel_unpack32(raw[e], t.mask, &m);
-          maybe |= (unsigned)m << (4 * q + e);
-        }
-      }
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      pos[j] = 0;
-      if (base + j < numel) {
-        bool m;
-        pos[j] = relabel_unpack(slot_of, ps.is64, base + j, t.mask, &m);
-        maybe |= (unsigned)m << j;
-      }
+  for (int j = 0; j < ITEMS; ++j) {
+    const int64_t i = base + 32 * j;
+    pos[j] = 0;
+    if (i < numel) {
+      bool m;
+      pos[j] = relabel_unpack(slot_of, ps.is64, i, &m);
+      maybe |= (unsigned)m << j;
     }
   }
   // only an element the inserting pass did not rule out has to look at its slot
 #pragma unroll
-  for (int j = 0; j < ITEMS; ++j)
-    if ((maybe >> j & 1u) && __ldcg(&t.slots[pos[j]].first) == (unsigned)(base + j)) is_first |= 1u << j;
-  const int64_t cnt = __popc(is_first);
-  const int64_t local = block_exclusive_scan(cnt, warp_sums, &s_total);
-  if (threadIdx.x < 32) {
-    const int64_t p = lookback_exclusive_prefix(st, tile, s_total, status);
-    if (threadIdx.x == 0) {
-      s_prefix = p;
-      if (tile == n_tiles - 1) st_relaxed64(result, p + s_total);
-    }
+  for (int j = 0; j < ITEMS; ++j) {
+    first[j] = 0xFFFFFFFFu;
+    if (maybe >> j & 1u) first[j] = __ldcg(&t.slots[pos[j]].first);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) post_when_last(post, n_tiles);
-  int64_t uid = s_prefix + local;
+  int before = 0, firsts = 0;  // first occurrences of earlier warps and of this one
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
+    if (first[j] == (unsigned)(base + 32 * j)) is_first |= 1u << j;
+    firsts += __popc(__ballot_sync(0xffffffffu, is_first >> j & 1u));
+  }
+  if (lane == 0) s_warp_firsts[warp] = firsts;
+  __syncthreads();
+  int64_t total = 0;
+#pragma unroll
+  for (int w = 0; w < kRelThreads / 32; ++w) {
+    if (w < (int)warp) before += s_warp_firsts[w];
+    total += s_warp_firsts[w];
+  }
+  if (threadIdx.x == 0) lookback_publish(st, tile, total);
+  const int64_t prefix = lookback_block(st, tile, total, &s_look, status);
+  if (threadIdx.x == 0 && tile == n_tiles - 1) st_relaxed64(result, prefix + total);
+  if (post.host) {
+    __syncthreads();  // every thread's look-back (which may flag a timeout) is over
+    if (threadIdx.x == 0) post_when_last(post, n_tiles);
+  }
+  int64_t row_uid = prefix + before;
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int64_t i = base + 32 * j;
+    const unsigned row = __ballot_sync(0xffffffffu, is_first >> j & 1u);
     if (is_first >> j & 1u) {
-      store_int(unique, ps.is64, uid, part_elem(ps, base + j));
-      t.slots[pos[j]].newid = (unsigned)uid;
-      ++uid;
+      const int64_t uid = row_uid + __popc(row & ((1u << lane) - 1u));
+      store_int(unique, ps.is64, uid, part_elem(ps, i));
+      store_int(slot_of, ps.is64, i, uid);
+      *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, ~0u, (unsigned)uid);
+    } else if (maybe >> j & 1u) {
+      store_int(slot_of, ps.is64, i, relabel_pack(pos[j], false, ps.is64));
     }
+    row_uid += __popc(row);
   }
 }
 
+// The repeats: slot -> new id.  First occurrences hold theirs already.
 __global__ void __launch_bounds__(kRelThreads)
 relabel_remap_kernel(Parts ps, RelTable t, void* out) {
   pdl_prologue();
   int64_t numel;
   resolve_sizes(ps, &numel);
+  constexpr int U = 4;  // independent slot reads per thread in flight
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += stride) {
-    bool maybe_first;
-    const uint32_t pos = relabel_unpack(out, ps.is64, i, t.mask, &maybe_first);
-    const uint4 slot = __ldcg(reinterpret_cast<const uint4*>(t.slots + pos));  // key lo, key hi, first, newid
-    store_int(out, ps.is64, i, (int64_t)slot.w);
-    // leave the slot empty for the next call: the id's first occurrence does it, once (the new id
-    // stays, because another element of the same id may not have read it yet)
-    if (maybe_first && slot.z == (unsigned)i)
-      *reinterpret_cast<uint4*>(t.slots + pos) = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, slot.w);
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < numel; i0 += U * stride) {
+    uint32_t pos[U];
+    unsigned newid[U];
+    bool repeat[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * stride;
+      repeat[u] = false;
+      if (i < numel) {
+        bool done;
+        pos[u] = relabel_unpack(out, ps.is64, i, &done);
+        repeat[u] = !done;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (repeat[u]) newid[u] = __ldcg(&t.slots[pos[u]].newid);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (repeat[u]) store_int(out, ps.is64, i0 + u * stride, (int64_t)newid[u]);
   }
 }
 
 // Table for up to `numel_bound` ids at load <= 0.5, in the context's block whose keys and
 // first-index words are all ones between calls (whatever the capacity, so regions of different
 // capacities may overlap freely); the new-id words need no initial value.
+// Small inputs get four times the room (see kRelRoomy).
 uint64_t relabel_capacity(int64_t numel_bound) {
   uint64_t cap = 64;
   while (cap < (uint64_t)numel_bound * 2) cap <<= 1;
+  while (cap < (uint64_t)numel_bound * 8 && cap < (uint64_t)kRelRoomy) cap <<= 1;
   return cap;
 }
 
@@ -225,13 +288,13 @@ int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t 
   const uint64_t cap = relabel_capacity(numel_bound);
   if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s)) return rc;
   t->slots = reinterpret_cast<RelSlot*>(ctx->table);
-  t->mask = (uint32_t)(cap - 1);
+  t->cap = (uint32_t)cap;
   return SHMT_OK;
 }
 
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
                    int64_t* status, int64_t* result, cudaStream_t s, bool inserted, bool pdl,
-                   const HostPost* post, int64_t* range) {
+                   const HostPost* post, RelSurvey* survey) {
   RelTable t;
   if (int rc = relabel_table(ctx, numel_bound, &t, s)) return rc;
   const int64_t n_tiles = (numel_bound + kRelTile - 1) / kRelTile;
@@ -239,19 +302,18 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
   const int64_t cap_blocks = (int64_t)sm_count() * 16;
   const unsigned grid = (unsigned)(blocks < cap_blocks ? blocks : cap_blocks);
   if (!inserted) {
-    unsigned long long* r = reinterpret_cast<unsigned long long*>(range);
-    if (r) SHMT_CUDA_TRY(launch_kernel(pdl, relabel_range_kernel, grid, kRelThreads, 0, s, ps, r));
+    if (survey) SHMT_CUDA_TRY(launch_kernel(pdl, relabel_survey_kernel, grid, kRelThreads, 0, s, ps, survey));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_insert_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel, status,
-                                (const unsigned long long*)r));
+                                (const RelSurvey*)survey));
   }
   if (numel_bound >= kRelLargeInput) {
     const int64_t big_tiles = (numel_bound + kRelThreads * kRelItemsLarge - 1) / (kRelThreads * kRelItemsLarge);
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItemsLarge>, (unsigned)big_tiles, kRelThreads, 0, s,
-                                ps, t, (const void*)out_relabel, out_unique, st, ticket, status, result,
+                                ps, t, out_relabel, out_unique, st, ticket, status, result,
                                 post ? *post : HostPost{}));
   } else {
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItems>, (unsigned)n_tiles, kRelThreads, 0, s, ps, t,
-                                (const void*)out_relabel, out_unique, st, ticket, status, result,
+                                out_relabel, out_unique, st, ticket, status, result,
                                 post ? *post : HostPost{}));
   }
   SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel));
@@ -293,20 +355,22 @@ extern "C" int shmt_relabel(shmt_ctx* ctx, const void* const* parts, const int64
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t n_tiles = (numel + kRelTile - 1) / kRelTile;
   const size_t states = (tile_state_bytes(n_tiles) + 255) & ~(size_t)255;
-  if (int rc = ctx_reserve(ctx, states)) return rc;
+  // a table that fits the L2 cache gains nothing from compact slots; a larger one may
+  const bool look = relabel_capacity(numel) * sizeof(RelSlot) > kRelSurveyMinTableBytes;
+  const size_t zeroed = look ? states + sizeof(RelSurvey) : tile_state_bytes(n_tiles);
+  if (int rc = ctx_reserve(ctx, zeroed)) return rc;
   TileStates st = carve_tile_states(ctx->region(), n_tiles);
-  // result words + tile descriptors to zero
-  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + tile_state_bytes(n_tiles), s));
+  RelSurvey* survey = look ? reinterpret_cast<RelSurvey*>(ctx->region() + states) : nullptr;
+  // result words, tile descriptors and the survey to zero
+  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + zeroed, s));
   int64_t* w = ctx->d_words();
   // with a count to return, the compact kernel posts it and the call returns while the remap
   // kernel runs; the next user of the context waits for that kernel first
   HostPost post{};
   if (n_unique_host) post = ctx_begin_post(ctx, w, 4, w + W_DONE);
-  // a table that fits the L2 cache gains nothing from compact slots; a larger one may
-  int64_t* range = relabel_capacity(numel) * sizeof(RelSlot) > kRelDirectMinTableBytes ? w + W_RANGE : nullptr;
   if (int rc = launch_relabel(ctx, ps, numel, out_unique, out_relabel, st, w + W_TICKET,
                               w + W_STATUS, w + W_RESULT, s, false, false,
-                              n_unique_host ? &post : nullptr, range))
+                              n_unique_host ? &post : nullptr, survey))
     return rc;
   if (n_unique_host) {
     if (int rc = ctx_mark_tail(ctx, s)) return rc;

@@ -8,10 +8,9 @@
 namespace shmt {
 
 constexpr int kRelThreads = 256;
-// Elements per thread of the compact kernel, and so per tile.  Its tiles hand their counts on
-// through a look-back that advances 32 tiles per round trip: for a large input the length of that
-// chain, not memory, is what small tiles cost, so inputs of kRelLargeInput elements and more use
-// kRelItemsLarge per thread; a small input is a few dependent reads long and wants many CTAs.
+// Elements per thread of the compact kernel, and so per tile.  Inputs of kRelLargeInput elements and
+// more use kRelItemsLarge per thread, whose slot reads are all in flight together (33.5 M ids: 505 us
+// with 16, 510 with 8, more with 4); a small input is a few dependent reads long and wants many CTAs.
 // Look-back state is always sized for the small tile.
 constexpr int kRelItems = 4;
 constexpr int kRelItemsLarge = 16;
@@ -40,85 +39,150 @@ struct __align__(16) RelSlot {
 
 struct RelTable {
   RelSlot* slots;  // cap entries
-  uint32_t mask;   // cap - 1
+  uint32_t cap;
+};
+
+// Slots per id.  A small input waits for its longest walk (at half load a few of 5,000 ids walk six
+// pairs, 1 us each), so it spreads out over up to kRelRoomy slots; a large one is bound by the
+// sectors it draws from HBM and stays compact.
+constexpr double kRelRoomy = (double)(1 << 21);  // 32 MB
+
+// What a first look at a large input says about it.
+constexpr int kRelSampleBits = 20;  // size of the bitmap that counts the distinct ids of the sample
+struct RelSurvey {
+  unsigned long long largest;  // largest id, read as an unsigned number
+  unsigned long long marked;   // bits set in the bitmap
+  uint32_t bitmap[1 << (kRelSampleBits - 5)];
 };
 
 #ifdef __CUDACC__
-// Hash mask for an input of at most `numel` ids: load <= 0.5, never beyond the table.
-__device__ __forceinline__ uint32_t relabel_mask_for(int64_t numel, uint32_t table_mask) {
-  if (numel <= 0) return table_mask < 63u ? table_mask : 63u;
-  const uint32_t want = numel * 2 <= 64 ? 63u : (0xFFFFFFFFu >> __clz((uint32_t)(numel * 2 - 1)));
-  return want < table_mask ? want : table_mask;
-}
-
 // What the inserting pass leaves per element in the output array: the element's slot, plus a mark
 // on the elements that are certainly NOT the first occurrence of their id (they met a smaller index
-// in the slot), so that the later passes need not look at the slot to know.  64-bit arrays always
-// have room for the mark; 32-bit ones as long as the table has fewer than 2^31 slots.
+// in the slot), so that the later passes need not look at the slot to know.  The compact kernel
+// turns this into: no mark = the element is a first occurrence and holds its new id already;
+// mark = a repeat, whose new id is in the slot.  A 32-bit array has room for the mark because the
+// table never has more than 2^31 slots (inputs stay below 2^30 ids).
 constexpr unsigned long long kRelNotFirst64 = 1ull << 40;
 constexpr uint32_t kRelNotFirst32 = 0x80000000u;
 
-__device__ __forceinline__ int64_t relabel_pack(uint32_t pos, bool maybe_first, bool is64, uint32_t table_mask) {
-  if (is64) return (int64_t)((unsigned long long)pos | (maybe_first ? 0ull : kRelNotFirst64));
-  if (table_mask < kRelNotFirst32 && !maybe_first) pos |= kRelNotFirst32;
-  return (int64_t)(int32_t)pos;
+__device__ __forceinline__ int64_t relabel_pack(uint32_t pos, bool unmarked, bool is64) {
+  if (is64) return (int64_t)((unsigned long long)pos | (unmarked ? 0ull : kRelNotFirst64));
+  return (int64_t)(int32_t)(unmarked ? pos : pos | kRelNotFirst32);
 }
 
-__device__ __forceinline__ uint32_t relabel_unpack64(unsigned long long raw, bool* maybe_first) {
-  *maybe_first = !(raw & kRelNotFirst64);
-  return (uint32_t)raw;
-}
-
-__device__ __forceinline__ uint32_t relabel_unpack32(uint32_t raw, uint32_t table_mask, bool* maybe_first) {
-  if (table_mask < kRelNotFirst32) {
-    *maybe_first = !(raw & kRelNotFirst32);
-    return raw & ~kRelNotFirst32;
+__device__ __forceinline__ uint32_t relabel_unpack(const void* slot_of, bool is64, int64_t i, bool* unmarked) {
+  if (is64) {
+    const unsigned long long raw = reinterpret_cast<const unsigned long long*>(slot_of)[i];
+    *unmarked = !(raw & kRelNotFirst64);
+    return (uint32_t)raw;
   }
-  *maybe_first = true;
-  return raw;
+  const uint32_t raw = reinterpret_cast<const uint32_t*>(slot_of)[i];
+  *unmarked = !(raw & kRelNotFirst32);
+  return raw & ~kRelNotFirst32;
 }
 
-__device__ __forceinline__ uint32_t relabel_unpack(const void* slot_of, bool is64, int64_t i, uint32_t table_mask,
-                                                   bool* maybe_first) {
-  if (is64) return relabel_unpack64(reinterpret_cast<const unsigned long long*>(slot_of)[i], maybe_first);
-  return relabel_unpack32(reinterpret_cast<const uint32_t*>(slot_of)[i], table_mask, maybe_first);
+// The part of the table one call uses.  A key is looked for in consecutive slots from its home in
+// [0, near) on, and after kRelNearProbes slots from a second home in [near, full); every element of
+// a call walks the same way, so `near` may be smaller than the distinct ids need: it decides how
+// compact the used slots lie (what fits the L2 cache is never read from HBM), not whether they fit.
+// Homes are even and slots are read in pairs, 32 bytes and one sector a time: at half load the home
+// pair is full of other keys for 1 id in 12, where a single slot is taken for 1 in 3, and a warp
+// waits for the lane that walks furthest.
+struct RelRange {
+  RelSlot* slots;
+  uint32_t near, full;  // even
+  bool direct;  // every id of the input lies in [0, near): the id itself is its slot, nothing collides
+};
+constexpr uint32_t kRelNearProbes = 128;
+
+// `near` for about `ids` distinct ids at `per_id` slots each.  What little the rest would hold if
+// `near` took most of the table is not worth a second region.
+__device__ __forceinline__ uint32_t relabel_near(double ids, double per_id, uint32_t full) {
+  double want = ids * per_id;
+  if (want < 8.0 * kRelNearProbes) want = 8.0 * kRelNearProbes;  // never a lap before the second region
+  if (want >= 0.5 * (double)full) return full;
+  return (uint32_t)want & ~1u;
 }
 
-// Claim (or find) the slot of `key`, record `i` as a candidate first occurrence, and return
-// the slot.  Linear probing from mix64(key) & mask; bounded by the table size.  *maybe_first is
-// false when the slot was seen to hold a smaller index (then `i` cannot be the first occurrence).
-// `direct`: every id of the input is known to lie in [0, mask], so the id itself is its slot:
-// neighbouring ids share cache lines and nothing collides.
-__device__ __forceinline__ uint32_t relabel_insert_one(RelSlot* slots, uint32_t mask, long long key,
-                                                       unsigned i, int64_t* status, bool* maybe_first,
-                                                       bool direct = false) {
-  uint32_t pos = direct ? (uint32_t)key : (uint32_t)mix64((uint64_t)key) & mask;
-  uint32_t steps = 0;
-  unsigned seen_first;
-  while (true) {
-    // key and first index come with one 16-byte load
-    const uint4 s = __ldcg(reinterpret_cast<const uint4*>(slots + pos));
-    long long cur = (long long)(((unsigned long long)s.y << 32) | s.x);
-    seen_first = s.z;
+__device__ __forceinline__ double relabel_slots_per_id(double ids, double least) {
+  return ids * least >= kRelRoomy ? least : (ids * 8.0 <= kRelRoomy ? 8.0 : kRelRoomy / ids);
+}
+
+struct RelPair {
+  long long key0, key1;
+  unsigned first0, first1;
+};
+// Slots at, at + 1 (`at` even), past L1: other CTAs' claims are made in L2.
+__device__ __forceinline__ RelPair relabel_load_pair(const RelSlot* slots, uint32_t at) {
+  unsigned long long k0, m0, k1, m1;
+  asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(k0), "=l"(m0), "=l"(k1), "=l"(m1)
+               : "l"(slots + at)
+               : "memory");
+  return RelPair{(long long)k0, (long long)k1, (unsigned)m0, (unsigned)m1};
+}
+
+__device__ __forceinline__ long long relabel_cas(RelSlot* slot, long long key) {
+  return (long long)atomicCAS(reinterpret_cast<unsigned long long*>(&slot->key), (unsigned long long)kEmptyKey,
+                              (unsigned long long)key);
+}
+
+__device__ __forceinline__ uint32_t relabel_home(const RelRange& t, long long key) {
+  if (t.direct) return (uint32_t)key;
+  return __umulhi((uint32_t)(mix64((uint64_t)key) >> 32), t.near) & ~1u;
+}
+
+// The slot behind `at` on the way of `key`.
+__device__ __forceinline__ uint32_t relabel_next(const RelRange& t, long long key, uint32_t at) {
+  ++at;
+  if (at & 1u) return at;  // the other slot of a pair
+  if (at <= t.near) {
+    if (t.near < t.full) {
+      const uint32_t home = relabel_home(t, key), walked = at > home ? at - home : at + t.near - home;
+      if (walked >= kRelNearProbes) return t.near + (__umulhi((uint32_t)mix64((uint64_t)key), t.full - t.near) & ~1u);
+    }
+    return at == t.near ? 0u : at;
+  }
+  return at == t.full ? t.near : at;
+}
+
+// Claim (or find) the slot of `key`.  What bounds a claim is latency: a read of the home, then a CAS
+// if it had room, 0.7 - 1 us each and more under load.  *seen is the first index the slot held (all
+// ones if it was claimed just now, by this element or by another one of the same id).
+__device__ __forceinline__ uint32_t relabel_claim(const RelRange& t, long long key, int64_t* status,
+                                                  unsigned* seen) {
+  uint32_t pos = relabel_home(t, key);
+  *seen = 0xFFFFFFFFu;
+  for (uint32_t round = 0;; ++round) {
+    const RelPair p = relabel_load_pair(t.slots, pos & ~1u);
+    const bool second = (pos & 1u) || (p.key0 != key && p.key0 != kEmptyKey);
+    const long long cur = second ? p.key1 : p.key0;
+    pos |= (uint32_t)second;
+    if (cur == key) {
+      *seen = second ? p.first1 : p.first0;
+      return pos;
+    }
     if (cur == kEmptyKey) {
-      cur = (long long)atomicCAS(reinterpret_cast<unsigned long long*>(&slots[pos].key),
-                                 (unsigned long long)kEmptyKey, (unsigned long long)key);
-      seen_first = 0xFFFFFFFFu;  // claimed just now, by this element or by another one of the same id
+      const long long old = relabel_cas(t.slots + pos, key);
+      if (old == kEmptyKey || old == key) return pos;
     }
-    if (cur == kEmptyKey || cur == key) break;
-    pos = (pos + 1) & mask;
-    if (++steps > mask) {  // cannot happen at load <= 0.5; bounded all the same
+    if (round > t.full) {  // the table holds twice the ids: cannot happen
       atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
-      break;
+      return pos;
     }
+    pos = relabel_next(t, key, pos);
   }
-  // `first` only ever goes down: when the index seen there is already smaller than this one the
-  // atomic would change nothing, and most elements of a frontier are such repeats.  Nothing waits
-  // for the atomic's result: an element that lowers the index, or loses to a still smaller one, is
-  // simply left among the candidates.
-  *maybe_first = seen_first > i;
-  if (*maybe_first) atomicMin(&slots[pos].first, i);
-  return pos;
+}
+
+// Enter index `i` for the slot as a candidate first occurrence; false if it certainly is not one.
+// `first` only ever goes down: when the index seen there is already smaller than this one the
+// atomic would change nothing, and most elements of a frontier are such repeats.  Nothing waits
+// for the atomic's result: an element that lowers the index, or loses to a still smaller one, is
+// simply left among the candidates.
+__device__ __forceinline__ bool relabel_settle(const RelRange& t, uint32_t pos, unsigned seen, unsigned i) {
+  if (seen <= i) return false;
+  atomicMin(&t.slots[pos].first, i);
+  return true;
 }
 #endif
 
@@ -132,11 +196,11 @@ uint64_t relabel_capacity(int64_t numel_bound);
 // of the ids (the fused sampling kernel), so only the compact and remap kernels run.
 // `post`: the compact kernel hands the result words to the host as soon as the unique count is
 // final, i.e. while the remap kernel is still to run (it produces neither sizes nor errors).
-// `range`: a zeroed device word; when given, a first kernel stores the largest id there and the
-// insert kernel uses ids as slots if they all fit the table (see relabel_insert_one).
+// `survey`: zeroed device memory; when given, a first kernel looks the ids over and the insert
+// kernel uses as much of the table as they need (see relabel_survey_kernel).
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
                    int64_t* status, int64_t* result, cudaStream_t s, bool inserted = false,
-                   bool pdl = false, const HostPost* post = nullptr, int64_t* range = nullptr);
+                   bool pdl = false, const HostPost* post = nullptr, RelSurvey* survey = nullptr);
 
 // The context's table for `numel_bound` ids (reserving it).
 int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s);

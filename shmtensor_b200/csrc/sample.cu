@@ -27,6 +27,10 @@
 namespace shmt {
 
 constexpr int kHopThreads = 256;
+// Relabel slots looked at first per possible edge of a hop (every row as long as the fan-out, no
+// repeats): a usual hop fills a third of them.  2.0 -> 1.25 took the compact kernel behind a hop of
+// 1.5 M edges from 80 to 65 us, for less of the table comes from HBM.
+constexpr double kHopSlotsPerEdge = 1.25;
 constexpr int kMaxSeedsPerTile = 1024;
 
 struct HopJob {
@@ -65,7 +69,7 @@ struct HopJob {
   // records the slot in rel_out -- the work of relabel's first kernel, done while this
   // kernel would otherwise wait on memory.  rel_slots == nullptr: off.
   RelSlot* rel_slots;
-  uint32_t rel_mask;
+  uint32_t rel_cap;
   void* rel_out;
   // Single-hop call with a host result: the CTA that finishes its bookkeeping last hands the
   // result words to the host, which returns while the rows are still being written.
@@ -115,7 +119,7 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
   __shared__ int64_t s_eshift[kMaxSeedsPerTile];  // edge id = position read from + this (edge ids only)
   __shared__ int64_t warp_sums[32];
   __shared__ int64_t s_total;
-  __shared__ int64_t s_prefix;
+  __shared__ LookbackShared s_look;
   __shared__ int s_tile;
 
   pdl_prologue();
@@ -219,6 +223,7 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
   }
 
   // ---- 3. offsets: scan inside the tile, look-back across tiles
+  int64_t prefix;
   {
     const int ch = (S + kHopThreads - 1) / kHopThreads;  // seeds per thread, 1..4
     int64_t c[kMaxSeedsPerTile / kHopThreads];
@@ -230,10 +235,8 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
       sum += c[q];
     }
     int64_t run = block_exclusive_scan(sum, warp_sums, &s_total);
-    if (tid < 32) {
-      const int64_t p = lookback_exclusive_prefix(job.st, tile, s_total, job.status);
-      if (tid == 0) s_prefix = p;
-    }
+    if (tid == 0) lookback_publish(job.st, tile, s_total);
+    prefix = lookback_block(job.st, tile, s_total, &s_look, job.status);
 #pragma unroll
     for (int q = 0; q < kMaxSeedsPerTile / kHopThreads; ++q) {
       const int j = (int)tid * ch + q;
@@ -242,20 +245,21 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
     }
     __syncthreads();
   }
-  const int64_t prefix = s_prefix;
   const bool relabel = job.rel_slots != nullptr;
-  // ids are hashed into as much of the table as n seeds with k picks each can need
-  const uint32_t rel_mask = relabel ? relabel_mask_for(n * (1 + k), job.rel_mask) : 0u;
+  const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
+  const RelRange range{job.rel_slots,
+                       relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
+                       job.rel_cap, false};
+  // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
+  auto enter = [&](int64_t i, IxT id) {
+    unsigned seen;
+    const uint32_t at = relabel_claim(range, (long long)id, job.status, &seen);
+    const bool maybe_first = relabel_settle(range, at, seen, (unsigned)i);
+    store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
+  };
   for (int j = (int)tid; j < rows; j += kHopThreads) {
     store_int(job.sub_indptr, job.indptr64, first + j, prefix + s_off[j]);
-    if (relabel) {
-      const int64_t i = first + j;
-      bool maybe_first;
-      const uint32_t pos = relabel_insert_one(job.rel_slots, rel_mask,
-                                              load_int(job.seeds, job.seeds64, i), (unsigned)i,
-                                              job.status, &maybe_first);
-      store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(pos, maybe_first, sizeof(IxT) == 8, job.rel_mask));
-    }
+    if (relabel) enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
   }
   if (tile == n_tiles - 1 && tid == 0) {
     store_int(job.sub_indptr, job.indptr64, n, prefix + s_total);
@@ -277,13 +281,7 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
         if (job.out_eids)
           store_int(job.out_eids, job.indptr64, o,
                     (src[u] - static_cast<const IxT*>(s_hit[j] ? job.gpu_indices : job.indices)) + s_eshift[j]);
-        if (relabel) {
-          bool maybe_first;
-          const uint32_t pos = relabel_insert_one(job.rel_slots, rel_mask, (long long)v[u],
-                                                  (unsigned)(n + o), job.status, &maybe_first);
-          store_int(job.rel_out, sizeof(IxT) == 8, n + o,
-                    relabel_pack(pos, maybe_first, sizeof(IxT) == 8, job.rel_mask));
-        }
+        if (relabel) enter(n + o, v[u]);
       }
     }
     return;
@@ -309,13 +307,7 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
       const IxT val = __ldg(in + pos);
       out_all[o] = val;
       if (job.out_eids) store_int(job.out_eids, job.indptr64, o, s_begin[j] + pos + s_eshift[j]);
-      if (relabel) {
-        bool maybe_first;
-        const uint32_t slot = relabel_insert_one(job.rel_slots, rel_mask, (long long)val,
-                                                 (unsigned)(n + o), job.status, &maybe_first);
-        store_int(job.rel_out, sizeof(IxT) == 8, n + o,
-                  relabel_pack(slot, maybe_first, sizeof(IxT) == 8, job.rel_mask));
-      }
+      if (relabel) enter(n + o, val);
     };
     if (job.weights && deg > 0 && (job.replace || deg > k)) {
       const float* w = (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j];
@@ -849,7 +841,7 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
       RelTable t;
       if (int rc = relabel_table(ctx, cap[h + 1], &t, s)) return rc;
       job.rel_slots = t.slots;
-      job.rel_mask = t.mask;
+      job.rel_cap = t.cap;
       job.rel_out = out_relabel[h];
     }
     SHMT_CUDA_TRY(indices_dtype == SHMT_I64 ? launch_hop<long long>(job, hop_tiles[h], s, /*pdl=*/h > 0)

@@ -42,7 +42,8 @@ scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStat
   constexpr int TILE = kScanTileBytes / (int)sizeof(T);
   constexpr int PER_LANE = kScanPartials / 32;
   __shared__ U partial[kScanPartials];  // [row][warp]
-  __shared__ int64_t s_prefix;
+  __shared__ LookbackShared s_look;
+  __shared__ int64_t s_total;
   __shared__ int s_tile;
   const unsigned full = 0xffffffffu;
   const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -103,13 +104,16 @@ scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStat
     }
     const U total = __shfl_sync(full, linc, 31);
     // zero-extended aggregate: tile sums add up in 64 bits, of which the low bits are used
-    const int64_t p = lookback_exclusive_prefix(st, tile, (int64_t)(uint64_t)total, words + W_STATUS);
-    // `carry`: this launch continues a scan whose first part another kernel did (its last
-    // descriptor holds the sum of everything before `data`)
-    if (lane == 0) s_prefix = p + (carry ? carry->value : 0);
+    if (lane == 0) {
+      s_total = (int64_t)(uint64_t)total;
+      lookback_publish(st, tile, s_total);
+    }
   }
   __syncthreads();
-  const U prefix = (U)(uint64_t)s_prefix;
+  // `carry`: this launch continues a scan whose first part another kernel did (its last
+  // descriptor holds the sum of everything before `data`)
+  const U prefix = (U)(uint64_t)(lookback_block(st, tile, s_total, &s_look, words + W_STATUS) +
+                                 (carry ? carry->value : 0));
 #pragma unroll
   for (int k = 0; k < kScanVecs; ++k) {
     const int64_t at = tile_base + ((int64_t)k * kScanThreads + tid) * VEC;
@@ -466,7 +470,9 @@ static int run_scan_large(void* data, int64_t n, int exclusive, char* state_base
 // of a scan whose tile 0 never runs, with a short spin limit.  It must record DEV_TIMEOUT and
 // return; nothing else is touched.
 __global__ void lookback_timeout_probe_kernel(TileStates st, int64_t* words, int spin_limit) {
-  lookback_exclusive_prefix(st, /*tile=*/1, /*aggregate=*/1, words + W_STATUS, spin_limit);
+  __shared__ LookbackShared look;
+  if (threadIdx.x == 0) lookback_publish(st, /*tile=*/1, /*aggregate=*/1);
+  lookback_block(st, /*tile=*/1, /*aggregate=*/1, &look, words + W_STATUS, spin_limit);
 }
 
 // Launch helper shared with relabel / sub-CSR: scans `n` items in place using

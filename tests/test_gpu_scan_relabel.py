@@ -167,6 +167,51 @@ def test_relabel_five_million_ids(capi, spread):
     capi.check_async()
 
 
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 1, (4 << 20) + 4095])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_relabel_around_the_survey_and_tile_limits(capi, n, dtype):
+    """More than 2^20 ids are surveyed first (largest id, sampled distinct count) and use a part of
+    the table; from 2^22 on tiles are larger.  Few, many and only distinct ids; parts of odd length,
+    the second off a 16-byte boundary."""
+    rng = np.random.default_rng(n)
+    for distinct in (7, n // 5, n):
+        ids = rng.permutation(distinct * 3)[:distinct] if distinct < n else rng.permutation(distinct)
+        x = ids[rng.integers(0, distinct, size=n)] if distinct < n else ids
+        x = x.astype(np.int32 if dtype == torch.int32 else np.int64)
+        if dtype == torch.int64 and distinct < n:
+            x = x * 0x100000001 + 5                              # hashed, not used as slots
+        cut = n // 3 | 1
+        whole = torch.from_numpy(x).cuda()
+        uniq, rel = capi.tensor_relabel([whole[:cut].clone(), whole[cut:]])
+        wu, (wr,) = oracle.tensor_relabel([x])
+        assert np.array_equal(uniq.cpu().numpy(), wu)
+        assert np.array_equal(torch.cat(rel).cpu().numpy(), wr)
+    capi.check_async()
+
+
+def test_relabel_when_the_survey_sees_far_too_few_ids(capi):
+    """Ids picked so that none of them falls into the survey's sample: the part of the table meant
+    for them holds almost none, and every id has to find its second home."""
+    def mix64(x):
+        x = x ^ (x >> np.uint64(33))
+        x = x * np.uint64(0xff51afd7ed558ccd)
+        x = x ^ (x >> np.uint64(33))
+        x = x * np.uint64(0xc4ceb9fe1a85ec53)
+        return x ^ (x >> np.uint64(33))
+    n = (1 << 20) + 300
+    x = np.random.default_rng(3).integers(1 << 30, 1 << 40, size=2 * n).astype(np.int64)
+    x = x[mix64(x.astype(np.uint64)) >> np.uint64(62) != 0][:n]   # one id in four is sampled at this size
+    assert x.size == n
+    for _ in range(2):                                            # the second call finds a clean table
+        uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(x).cuda()])
+        wu, (wr,) = oracle.tensor_relabel([x])
+        assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+    y = x[:5000]
+    uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(y).cuda()])
+    wu, (wr,) = oracle.tensor_relabel([y])
+    assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+
+
 def test_relabel_is_repeatable_and_idempotent(capi):
     g = torch.Generator(device="cuda").manual_seed(1)
     x = torch.randint(0, 100_000, (500_000,), generator=g, device="cuda")
