@@ -8,13 +8,16 @@
 // Here a CTA takes a tile of S seeds:
 //   1. one seed per thread: cooperative map probe, row bounds from the cached
 //      indptr (hit) or the host indptr over UVA (miss), picks = min(deg, k);
-//   2. block scan of the picks, decoupled look-back for the tile's offset ->
-//      sub_indptr, so no separate scan kernel and no host round trip;
-//   3. groups of G = 8/16/32 lanes (smallest power of two >= k) sample one seed
-//      each: deg <= k copies the row; otherwise each lane p < k draws
+//   2. block scan of the picks; the tile's sum is published at once;
+//   3. groups of G = 8/16/32 lanes (smallest power of two >= k) pick positions, one
+//      seed each: deg <= k takes the row; otherwise each lane p < k draws
 //      t_p ~ U[0, deg-k+p] with Philox4x32-10 and the group resolves Floyd's
 //      subset algorithm with k shuffle+ballot steps (O(k) work, exact uniform
-//      k-subset; the reference draws O(deg) numbers and uses global atomics).
+//      k-subset; the reference draws O(deg) numbers and uses global atomics);
+//   4. look-back for the tile's offset -> sub_indptr, so no separate scan kernel and
+//      no host round trip;
+//   5. all threads fetch and store the picked neighbours, one each, whatever the rows'
+//      lengths, and in a mini-batch claim their relabel slots.
 //      k > 32: one warp per seed draws positions into a shared-memory set until k distinct
 //      ones (or, for rows shorter than 2k, the deg-k to leave out) are held: O(k) draws, no
 //      global atomics.  Only beyond 1024 picks per seed does it fall back to the reference's
@@ -27,6 +30,14 @@
 namespace shmt {
 
 constexpr int kHopThreads = 256;
+// A hop is a chain of dependent reads per edge (row bounds, neighbour, relabel slot), so resident
+// threads count for more than reads in flight per thread: the third hop of 8,192 seeds x 5/10/15
+// took 118 us with four edges per thread (64 registers, 4 CTAs per SM), 99 with two (5 CTAs) and 94
+// with one (6 CTAs).
+constexpr int kHopCtasPerSm = 6;
+// Seeds of a tile come in steps of 8: a small hop is as long as its slowest CTA, and 1,024 seeds over
+// a host graph took 20 us in 32 CTAs of 32 seeds and 16 us in 128 CTAs of 8.
+constexpr int kHopSeedStep = 8;
 // Relabel slots looked at first per possible edge of a hop (every row as long as the fan-out, no
 // repeats): a usual hop fills a third of them.  2.0 -> 1.25 took the compact kernel behind a hop of
 // 1.5 M edges from 80 to 65 us, for less of the table comes from HBM.
@@ -110,13 +121,23 @@ __device__ __forceinline__ uint64_t draw_below(const Philox& rng, uint32_t seed_
   return bounded(r.x, r.y, range);
 }
 
+// A picked neighbour on its way through a tile: where it lies in the full or the cached index
+// array, and the seed of the tile it belongs to.
+struct HopEdge {
+  uint64_t bits;
+  __device__ __forceinline__ explicit HopEdge(uint64_t b) : bits(b) {}
+  static __device__ __forceinline__ uint64_t pack(int64_t at, int seed, bool hit) {
+    return (uint64_t)at | ((uint64_t)seed << 50) | ((uint64_t)hit << 63);
+  }
+  __device__ __forceinline__ int64_t at() const { return (int64_t)(bits & ((1ull << 50) - 1)); }
+  __device__ __forceinline__ int seed() const { return (int)(bits >> 50) & ((1 << 13) - 1); }
+  __device__ __forceinline__ bool hit() const { return bits >> 63; }
+};
+static_assert(kMaxSeedsPerTile <= 1 << 13, "a seed of the tile takes 13 bits");
+
 template <typename IxT, int G>
-__global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob job) {
-  __shared__ int64_t s_begin[kMaxSeedsPerTile];
-  __shared__ int64_t s_deg[kMaxSeedsPerTile];
-  __shared__ int64_t s_off[kMaxSeedsPerTile];
-  __shared__ uint8_t s_hit[kMaxSeedsPerTile];
-  __shared__ int64_t s_eshift[kMaxSeedsPerTile];  // edge id = position read from + this (edge ids only)
+__global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];  // hop_smem_bytes()
   __shared__ int64_t warp_sums[32];
   __shared__ int64_t s_total;
   __shared__ LookbackShared s_look;
@@ -126,6 +147,15 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
   const unsigned full = 0xffffffffu;
   const unsigned tid = threadIdx.x, lane = tid & 31;
   const int S = job.seeds_per_tile;
+  int64_t* s_begin = reinterpret_cast<int64_t*>(s_dyn);
+  int64_t* s_deg = s_begin + S;
+  int64_t* s_off = s_deg + S;
+  int64_t* s_eshift = s_off + S;  // edge id = position read from + this (edge ids only)
+  uint8_t* s_hit = reinterpret_cast<uint8_t*>(s_eshift + S);
+  // one of the two behind them: the picked neighbours of the tile in output order (k <= 32), or per
+  // warp a set of chosen positions (job.set_slots words)
+  uint64_t* s_list = reinterpret_cast<uint64_t*>(s_hit + S);
+  uint32_t* s_sets = reinterpret_cast<uint32_t*>(s_hit + S);
   const int64_t n = job.n_dev ? *job.n_dev : job.n;
   const int64_t n_tiles = (n + S - 1) / S;
   const int tile = take_tile(job.ticket, &s_tile);
@@ -167,26 +197,56 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
   }
   __syncthreads();
 
+  // ---- 2. offsets inside the tile.  The tile's sum goes out now: the tiles behind it then never
+  // wait for the neighbour loads and slot claims below.
+  {
+    const int ch = (S + kHopThreads - 1) / kHopThreads;  // seeds per thread, 1..4
+    int64_t c[kMaxSeedsPerTile / kHopThreads];
+    int64_t sum = 0;
+#pragma unroll
+    for (int q = 0; q < kMaxSeedsPerTile / kHopThreads; ++q) {
+      const int j = (int)tid * ch + q;
+      c[q] = (q < ch && j < S) ? s_off[j] : 0;
+      sum += c[q];
+    }
+    int64_t run = block_exclusive_scan(sum, warp_sums, &s_total);
+    if (tid == 0) lookback_publish(job.st, tile, s_total);
+#pragma unroll
+    for (int q = 0; q < kMaxSeedsPerTile / kHopThreads; ++q) {
+      const int j = (int)tid * ch + q;
+      if (q < ch && j < S) s_off[j] = run;
+      run += c[q];
+    }
+    __syncthreads();
+  }
+
   constexpr int kGroups = kHopThreads / G;
-  constexpr int U = 8;  // seeds per group; a tile never holds more than kGroups * U when k <= G
   const unsigned gl = tid & (G - 1);
   const unsigned gshift = lane & ~(unsigned)(G - 1);  // first lane of my group within the warp
   const unsigned gmask = G == 32 ? full : (((1u << G) - 1u) << gshift);
   const int group = (int)(tid / G);
   const Philox rng(job.rng_seed);
   IxT* out_all = static_cast<IxT*>(job.sub_indices);
+  const bool relabel = job.rel_slots != nullptr;
+  const bool listed = G < 32 || (k <= G && !job.weights);  // a smaller group is only launched for such calls
+  const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
+  const RelRange range{job.rel_slots,
+                       relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
+                       job.rel_cap, false};
+  // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
+  auto enter = [&](int64_t i, IxT id) {
+    unsigned seen;
+    const uint32_t at = relabel_claim(range, (long long)id, job.status, &seen);
+    const bool maybe_first = relabel_settle(range, at, seen, (unsigned)i);
+    store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
+  };
 
-  // ---- 2. (k <= G) pick positions and LOAD the neighbours now, before the tile's output
-  // offset is known: the loads (often over the host link) then overlap the look-back wait
-  // and the other tiles' row-bound reads.  One element per lane and seed; the U seeds of a
-  // group are resolved first (arithmetic and shuffles only), then their loads go out back
-  // to back.
-  const IxT* src[U];
-  IxT v[U];
-  if (k <= G && !job.weights) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = u * kGroups + group;
+  // ---- 3. (k <= 32) positions of the picked neighbours, a group of lanes per seed, into a list in
+  // output order.  Arithmetic and shuffles only: the memory work is left to step 5, where all
+  // threads of the tile share it evenly whatever the rows' lengths.
+  if (listed) {
+    for (int j0 = 0; j0 < rows; j0 += kGroups) {
+      const int j = j0 + group;
       const bool active = j < rows;
       const int64_t deg = active ? s_deg[j] : 0;
       const uint32_t seed_idx = (uint32_t)(first + j);
@@ -213,54 +273,25 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
           if (pick && (int64_t)gl < k) pos = res;
         }
       }
-      src[u] = nullptr;
-      if (pos >= 0)
-        src[u] = static_cast<const IxT*>(s_hit[j] ? job.gpu_indices : job.indices) + s_begin[j] + pos;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (src[u]) v[u] = __ldg(src[u]);
-  }
-
-  // ---- 3. offsets: scan inside the tile, look-back across tiles
-  int64_t prefix;
-  {
-    const int ch = (S + kHopThreads - 1) / kHopThreads;  // seeds per thread, 1..4
-    int64_t c[kMaxSeedsPerTile / kHopThreads];
-    int64_t sum = 0;
-#pragma unroll
-    for (int q = 0; q < kMaxSeedsPerTile / kHopThreads; ++q) {
-      const int j = (int)tid * ch + q;
-      c[q] = (q < ch && j < S) ? s_off[j] : 0;
-      sum += c[q];
-    }
-    int64_t run = block_exclusive_scan(sum, warp_sums, &s_total);
-    if (tid == 0) lookback_publish(job.st, tile, s_total);
-    prefix = lookback_block(job.st, tile, s_total, &s_look, job.status);
-#pragma unroll
-    for (int q = 0; q < kMaxSeedsPerTile / kHopThreads; ++q) {
-      const int j = (int)tid * ch + q;
-      if (q < ch && j < S) s_off[j] = run;
-      run += c[q];
+      if (pos >= 0) s_list[s_off[j] + gl] = HopEdge::pack(s_begin[j] + pos, j, s_hit[j]);
     }
     __syncthreads();
   }
-  const bool relabel = job.rel_slots != nullptr;
-  const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
-  const RelRange range{job.rel_slots,
-                       relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
-                       job.rel_cap, false};
-  // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
-  auto enter = [&](int64_t i, IxT id) {
-    unsigned seen;
-    const uint32_t at = relabel_claim(range, (long long)id, job.status, &seen);
-    const bool maybe_first = relabel_settle(range, at, seen, (unsigned)i);
-    store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
+
+  // ---- 4. the tile's place in the output.  The first neighbours are fetched ahead of the look-back,
+  // so that the two waits overlap.
+  const int lead = relabel ? rows : 0;  // the seeds come first: they are relabelled too
+  const int n_items = listed ? lead + (int)s_total : 0;
+  auto fetch = [&](int e) -> IxT {
+    if (e >= n_items) return IxT(0);
+    if (e < lead) return (IxT)load_int(job.seeds, job.seeds64, first + e);
+    const HopEdge x(s_list[e - lead]);
+    return __ldg(static_cast<const IxT*>(x.hit() ? job.gpu_indices : job.indices) + x.at());
   };
-  for (int j = (int)tid; j < rows; j += kHopThreads) {
+  IxT next = fetch((int)tid);
+  const int64_t prefix = lookback_block(job.st, tile, s_total, &s_look, job.status);
+  for (int j = (int)tid; j < rows; j += kHopThreads)
     store_int(job.sub_indptr, job.indptr64, first + j, prefix + s_off[j]);
-    if (relabel) enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
-  }
   if (tile == n_tiles - 1 && tid == 0) {
     store_int(job.sub_indptr, job.indptr64, n, prefix + s_total);
     st_relaxed64(job.result, prefix + s_total);
@@ -270,25 +301,30 @@ __global__ void __launch_bounds__(kHopThreads) sample_hop_kernel(const HopJob jo
     if (tid == 0) post_when_last(job.post, n_tiles);
   }
 
-  // ---- 4. output
-  if (k <= G && !job.weights) {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = u * kGroups + group;
-      if (src[u]) {
-        const int64_t o = prefix + s_off[j] + gl;
-        out_all[o] = v[u];
-        if (job.out_eids)
-          store_int(job.out_eids, job.indptr64, o,
-                    (src[u] - static_cast<const IxT*>(s_hit[j] ? job.gpu_indices : job.indices)) + s_eshift[j]);
-        if (relabel) enter(n + o, v[u]);
+  // ---- 5. output and relabel slots, one list element per thread and step
+  if (listed) {
+    for (int e = (int)tid; e < n_items; e += kHopThreads) {
+      const IxT v = next;
+      next = fetch(e + kHopThreads);
+      int64_t i = first + e;  // index in [seeds | neighbours]
+      if (e >= lead) {
+        const int64_t o = prefix + (e - lead);
+        i = n + o;
+        out_all[o] = v;
+        if (job.out_eids) {
+          const HopEdge x(s_list[e - lead]);
+          store_int(job.out_eids, job.indptr64, o, x.at() + s_eshift[x.seed()]);
+        }
       }
+      if (relabel) enter(i, v);
     }
     return;
   }
+  if (relabel)
+    for (int j = (int)tid; j < rows; j += kHopThreads)
+      enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
 
   // k > 32 (G == 32): one warp per seed
-  extern __shared__ uint32_t s_sets[];  // per warp: a set of chosen positions (job.set_slots words)
   const uint32_t set_slots = job.set_slots;
   uint32_t* set = s_sets + (size_t)(tid >> 5) * set_slots;
   for (int j0 = 0; j0 < rows; j0 += kGroups) {
@@ -547,10 +583,10 @@ size_t scan_scratch_bytes(int64_t n);
 
 static int pick_seeds_per_tile(int64_t n, int64_t k) {
   int64_t s = (n + (int64_t)sm_count() * 4 - 1) / ((int64_t)sm_count() * 4);
-  s = (s + 31) / 32 * 32;
-  if (s < 32) s = 32;
+  s = (s + kHopSeedStep - 1) / kHopSeedStep * kHopSeedStep;
+  if (s < kHopSeedStep) s = kHopSeedStep;
   if (s > kMaxSeedsPerTile) s = kMaxSeedsPerTile;
-  // with k <= 32 a tile is sampled in one pass of 8 seeds per lane group (see the kernel)
+  // with k <= 32 the list of a tile's neighbours takes at most 16 KB of shared memory
   const int64_t one_pass = k <= 8 ? 256 : (k <= 16 ? 128 : (k <= 32 ? 64 : kMaxSeedsPerTile));
   if (s > one_pass) s = one_pass;
   return (int)s;
@@ -567,22 +603,29 @@ static uint32_t set_slots_for(int64_t k) {
   return slots;
 }
 
+// The per-seed arrays of a tile and what lies behind them (see the kernel).
+static size_t hop_smem_bytes(int seeds_per_tile, int64_t k, uint32_t set_slots) {
+  const size_t list = k <= 32 ? (size_t)seeds_per_tile * (size_t)k * sizeof(uint64_t) : 0;
+  const size_t sets = (size_t)set_slots * sizeof(uint32_t) * (kHopThreads / 32);
+  return (size_t)seeds_per_tile * (4 * sizeof(int64_t) + 1) + (list > sets ? list : sets);
+}
+
 template <typename IxT>
 static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool pdl = false) {
   const unsigned grid = (unsigned)n_tiles;
   job.set_slots = set_slots_for(job.k);
+  const size_t smem = hop_smem_bytes(job.seeds_per_tile, job.weights ? 33 : job.k, job.set_slots);
   if (!job.weights) {
-    if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8>, grid, kHopThreads, 0, s, job);
-    if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16>, grid, kHopThreads, 0, s, job);
+    if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8>, grid, kHopThreads, smem, s, job);
+    if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16>, grid, kHopThreads, smem, s, job);
   }
-  const size_t smem = (size_t)job.set_slots * sizeof(uint32_t) * (kHopThreads / 32);
-  if (smem > 0) {
+  if (smem > (48 << 10)) {
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev]) {
-      const cudaError_t e = cudaFuncSetAttribute(sample_hop_kernel<IxT, 32>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)(2 * kMaxSetPicks * sizeof(uint32_t) * (kHopThreads / 32)));
+      const cudaError_t e =
+          cudaFuncSetAttribute(sample_hop_kernel<IxT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)hop_smem_bytes(kMaxSeedsPerTile, 33, 2 * kMaxSetPicks));
       if (e != cudaSuccess) return e;
       configured[dev] = true;
     }

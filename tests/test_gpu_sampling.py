@@ -360,3 +360,27 @@ def test_row_offsets_at_an_odd_element_offset(capi, ptr_dt):
         assert torch.equal(q0, q1) and torch.equal(y0, y1)
         oracle.check_sample(indptr_n, indices_n, seeds.cpu().numpy(), k, False, p1.cpu().numpy(),
                             x1.cpu().numpy())
+
+
+@pytest.mark.parametrize("n_seeds", [1, 7, 8, 9, 8 * 592 - 1, 8 * 592 + 1])
+@pytest.mark.parametrize("k", [8, 9, 32])
+def test_tiles_of_eight_seeds_fused_and_hop_by_hop(capi, n_seeds, k):
+    """Tiles hold a multiple of 8 seeds and share their picked neighbours between all threads:
+    seed counts at the edges of one tile and of the largest grid of smallest tiles, the first and
+    the last fan-out of a lane-group size; the fused call equals the hop plus relabel."""
+    rng = np.random.default_rng(n_seeds * 100 + k)
+    deg = np.minimum((rng.pareto(1.1, size=9000) * 6).astype(np.int64), 700)
+    indptr_n = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    indices_n = np.concatenate([(np.arange(d) * 7 + v) % 9000 for v, d in enumerate(deg)]).astype(np.int64)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    seeds_n = rng.permutation(9000)[:n_seeds].astype(np.int64)
+    seeds = torch.from_numpy(seeds_n).cuda()
+    capi.set_sampling_seed(99)
+    p, x, e = capi.csr_sampling_with_eids(indptr, indices, seeds, k, False)
+    oracle.check_sample_bulk(indptr_n, indices_n, seeds_n, k, False, p.cpu().numpy(), x.cpu().numpy(), distinct_rows=True)
+    assert torch.equal(indices[e], x)
+    capi.set_sampling_seed(99)
+    frontier, [(fp, fx, rel, _, fe)] = capi.sample_minibatch(indptr, indices, seeds, [k], False, return_eids=True)
+    assert torch.equal(fp, p) and torch.equal(fx, x) and torch.equal(fe, e)
+    wu, (_, wx) = oracle.tensor_relabel([seeds_n, x.cpu().numpy()])
+    assert np.array_equal(frontier.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
