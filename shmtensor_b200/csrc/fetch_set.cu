@@ -255,6 +255,166 @@ row_scatter_bulk_kernel(const RowJob job) {
   bulk_wait_read<0>();
 }
 
+// ---- rows that are not 16-byte units ----------------------------------------------------------
+// A row of 602 bytes starts on any even address, and its copy in the output on another one; with
+// accesses no wider than both allow, a warp instruction moved 64 bytes.  Here a row travels as the
+// 16-byte granules that hold it: one bulk copy per row brings them into a ring buffer like the one
+// of row_gather_bulk_kernel, and the warp then writes the tile's output, which is contiguous, in
+// aligned 16-byte chunks, each shifted together from two chunks of shared memory (from two rows
+// where the chunk holds a seam).  A granule is only read because it holds a byte of the row, so what
+// is read beside the row lies in the same 16 bytes, and page, as that byte.
+
+// 16 bytes from byte `sh` (0..15) of the 32 bytes lo | hi
+__device__ __forceinline__ uint4 shift_bytes(uint4 lo, uint4 hi, unsigned sh) {
+  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  const bool by2 = sh & 8u, by1 = sh & 4u;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) w[i] = by2 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) w[i] = by1 ? w[i + 1] : w[i];
+  const unsigned bits = (sh & 3u) * 8u;
+  return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits),
+                    __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
+}
+
+// 16 bytes of shared memory from byte `at` of `base` (16-byte aligned) on
+__device__ __forceinline__ uint4 shared_unaligned16(const unsigned char* base, int at) {
+  const uint4* a = reinterpret_cast<const uint4*>(base + (at & ~15));
+  return shift_bytes(a[0], a[1], (unsigned)at & 15u);
+}
+
+// the first `left` bytes of l, the others of r
+__device__ __forceinline__ uint4 join_bytes(uint4 l, uint4 r, int left) {
+  auto mix = [&](uint32_t x, uint32_t y, int w) {
+    const int n = left - 4 * w;  // bytes of this word that belong to l
+    const uint32_t keep = n <= 0 ? 0u : (n >= 4 ? 0xFFFFFFFFu : (1u << (8 * n)) - 1u);
+    return (x & keep) | (y & ~keep);
+  };
+  return make_uint4(mix(l.x, r.x, 0), mix(l.y, r.y, 1), mix(l.z, r.z, 2), mix(l.w, r.w, 3));
+}
+
+// bytes [from, to) of v to dst + from .. (a chunk whose other bytes are not this tile's to write)
+__device__ __forceinline__ void store_bytes(char* dst, uint4 v, int from, int to) {
+  for (int i = from; i < to; ++i) {
+    const uint32_t w = i < 8 ? (i < 4 ? v.x : v.y) : (i < 12 ? v.z : v.w);
+    dst[i] = (char)(w >> (8 * (i & 3)));
+  }
+}
+
+// Shared memory between two rows of a stage buffer: the granules of a row that starts on any byte.
+__host__ __device__ constexpr int64_t ragged_pitch(int64_t row_bytes) { return (row_bytes + 30) & ~(int64_t)15; }
+constexpr int kRaggedPad = 32;  // in front of and behind a warp's buffers: what seams read past a row is never used
+
+template <int STAGES>
+__global__ void __launch_bounds__(kRowThreads)
+row_gather_ragged_kernel(const RowJob job) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t s_bar[kRowWarps][STAGES];
+  const unsigned full = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int R = job.rows_per_tile;
+  const int rb = (int)job.row_bytes, pitch = (int)ragged_pitch(job.row_bytes);
+  const int stage_bytes = R * pitch;
+  unsigned char* wbase = smem_raw + (size_t)warp * (STAGES * stage_bytes + 2 * kRaggedPad) + kRaggedPad;
+  const int64_t n_tiles = (job.n + R - 1) / R;
+  const int64_t stride = (int64_t)gridDim.x * kRowWarps;
+  const int64_t slot_mask = ((int64_t)1 << job.owner_shift) - 1;
+  const int step_row = 512 / rb, step_off = 512 % rb;
+
+  if (lane == 0)
+    for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[warp][s], 1);
+  mbar_init_fence();
+  __syncwarp();
+
+  unsigned vmask[STAGES];  // lanes whose row is being loaded into the stage
+  int start[STAGES];       // byte of this lane's slot at which its row starts
+  uint32_t parity = 0;     // bit s: phase of stage s to wait for next
+
+  auto issue = [&](int64_t tile, int s) {
+    const int64_t first = tile * R;
+    const int rows = (int)min((int64_t)R, job.n - first);
+    const int64_t id = load_id(job, first, rows, lane);
+    const char* p = resolve_row(job, first, rows, lane, slot_mask, id);
+    const int sh = (int)((uintptr_t)p & 15);
+    const uint32_t bytes = p ? (uint32_t)(sh + rb + 15) & ~15u : 0u;
+    const uint32_t total = __reduce_add_sync(full, bytes);
+    if (lane == 0) mbar_arrive_expect_tx(&s_bar[warp][s], total);
+    __syncwarp();
+    if (p) bulk_load(wbase + s * stage_bytes + (int)lane * pitch, p - sh, bytes, &s_bar[warp][s]);
+    vmask[s] = __ballot_sync(full, p != nullptr);
+    start[s] = sh;
+  };
+
+  constexpr int D = STAGES - 1;
+  int64_t tile = (int64_t)blockIdx.x * kRowWarps + warp;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < D; ++j)
+    if (tile + j * stride < n_tiles) issue(tile + j * stride, j);
+  while (tile < n_tiles && ok) {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+      if (tile >= n_tiles || !ok) break;
+      const int64_t ahead = tile + D * stride;
+      __syncwarp();  // every lane has read what the buffer filled next held
+      if (ahead < n_tiles) issue(ahead, (s + D) % STAGES);
+      if (!mbar_wait_bounded(&s_bar[warp][s], (parity >> s) & 1u)) {
+        atomicExch(&g_device_fault, 1);
+        ok = false;
+      }
+      ok = __all_sync(full, ok);
+      parity ^= 1u << s;
+      if (ok) {
+        const unsigned char* buf = wbase + s * stage_bytes;
+        const unsigned vm = vmask[s];
+        const int rows = (int)min((int64_t)R, job.n - tile * R);
+        char* out = job.flat + tile * R * job.row_bytes;
+        const int d = (int)((uintptr_t)out & 15);  // the tile starts at byte d of its first chunk
+        char* chunk0 = out - d;
+        const int n_chunks = (rows * rb + d + 15) >> 4;
+        // ---- chunks inside one row; the lane's starts at byte `off` of row `row`
+        int row = 0, off = (int)lane * 16 - d;
+        if (off < 0) {  // the tile's first chunk is a seam
+          row = -1;
+          off += rb;
+        } else if (off >= rb) {  // off <= 496, and no row is shorter than 256
+          row = 1;
+          off -= rb;
+        }
+        for (int c0 = 0; c0 < n_chunks; c0 += 32) {
+          const int at = __shfl_sync(full, start[s], row & 31) + off;
+          if (off + 16 <= rb && row < rows && row >= 0 && (vm >> row & 1u))
+            st_stream16(chunk0 + (c0 + (int)lane) * 16, shared_unaligned16(buf, row * pitch + at));
+          off += step_off;
+          row += step_row;
+          if (off >= rb) {
+            off -= rb;
+            ++row;
+          }
+        }
+        // ---- seams, one per lane: the chunk that holds the start of row b (b = rows: the tile's end)
+        for (int b0 = 0; b0 <= rows; b0 += 32) {
+          const int b = b0 + (int)lane;
+          const int at0 = __shfl_sync(full, start[s], (b - 1) & 31), at1 = __shfl_sync(full, start[s], b & 31);
+          const int left = (b * rb + d) & 15;  // bytes of the chunk in front of the seam
+          if (b > rows || left == 0) continue;
+          const bool has0 = b > 0 && (vm >> (b - 1) & 1u), has1 = b < rows && (vm >> b & 1u);
+          uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+          if (has0) v0 = shared_unaligned16(buf, (b - 1) * pitch + at0 + rb - left);
+          if (has1) v1 = shared_unaligned16(buf, b * pitch + at1 - left);
+          const uint4 v = join_bytes(v0, v1, left);
+          char* dst = out + b * rb - left;
+          if (has0 && has1)
+            st_stream16(dst, v);
+          else
+            store_bytes(dst, v, has0 ? 0 : left, has1 ? 16 : (has0 ? left : 0));
+        }
+      }
+      tile += stride;
+    }
+  }
+}
+
 // SET == false: table row -> flat (fetch).  SET == true: flat -> table row.
 template <int VEC, bool SET, int U>
 __global__ void __launch_bounds__(kRowThreads) row_copy_kernel(const RowJob job) {
@@ -458,12 +618,55 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   return SHMT_OK;
 }
 
+// Rows that are not 16-byte units.  Buffers of about 5 KB per warp (150,001 rows of 602 bytes: 3.4
+// TB/s read + written with 2 KB, 4.3 with 3 KB, 4.8 with 4 KB, 5.0 with 5 KB; a third buffer gave
+// nothing).  The line at 256 bytes: there the narrow copy of row_copy_kernel still has 2.3 (4-byte
+// rows: 3.4) against 4.2 TB/s and 26 (33) against 35 GB/s from a host table, below it the seams and
+// granules read at both ends of a row outweigh the wider access (132 bytes: 2.9 against 2.3 TB/s, 28
+// against 24 GB/s).  Rows of 8-byte units have a faster narrow copy, which is level at 408 bytes
+// (4.8 against 5.0 TB/s, 41.0 against 40.9 GB/s) and behind at 600 (4.2 against 5.1, 43.1 against 44.2).
+constexpr int kRaggedStages = 2;
+constexpr int64_t kRaggedStageBytes = 5120;
+constexpr int64_t kRaggedMinBytes = 256, kRaggedMinBytes8 = 512;
+
+static size_t ragged_smem_bytes(int64_t row_bytes, int R) {
+  return (size_t)kRowWarps * ((size_t)kRaggedStages * R * ragged_pitch(row_bytes) + 2 * kRaggedPad);
+}
+
+// Rows per ring buffer, 0 if the rows are too small to gain or do not fit.
+static int ragged_rows_per_stage(int64_t row_bytes, int vec, int R_small) {
+  if (vec == 16 || row_bytes < (vec == 8 ? kRaggedMinBytes8 : kRaggedMinBytes)) return 0;
+  int64_t r = kRaggedStageBytes / ragged_pitch(row_bytes);
+  if (r < 1) r = 1;
+  if (r > 32) r = 32;
+  if (r > R_small) r = R_small;
+  return ragged_smem_bytes(row_bytes, (int)r) > kBulkSmemMax ? 0 : (int)r;
+}
+
+static int launch_ragged(RowJob job, int R, cudaStream_t s) {
+  auto kernel = row_gather_ragged_kernel<kRaggedStages>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  SHMT_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && !configured[dev]) {
+    SHMT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBulkSmemMax));
+    configured[dev] = true;
+  }
+  job.rows_per_tile = R;
+  const size_t smem = ragged_smem_bytes(job.row_bytes, R);
+  kernel<<<grid_for_tiles(kernel, job.n, R, smem), kRowThreads, smem, s>>>(job);
+  SHMT_CUDA_TRY(cudaGetLastError());
+  return SHMT_OK;
+}
+
 template <bool SET>
 static int launch_row_copy(const RowJob& job, int vec, cudaStream_t s) {
   {
     static const bool no_bulk = getenv("SHMT_NO_BULK") != nullptr;
     const int R = no_bulk ? 0 : bulk_rows_per_stage(job.row_bytes, vec, job.rows_per_tile);
     if (R >= 1) return launch_bulk<SET>(job, R, s);
+    const int ragged = SET || no_bulk ? 0 : ragged_rows_per_stage(job.row_bytes, vec, job.rows_per_tile);
+    if (ragged >= 1) return launch_ragged(job, ragged, s);
   }
   switch (vec) {
     case 16: return launch_lsu<16, SET>(job, s);

@@ -5,6 +5,7 @@ import torch
 
 from conftest import load_golden
 from oracle import oracle
+from shmtensor_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -312,3 +313,49 @@ def test_cache_replace_keeps_fetch_exact(capi):
         assert torch.equal(gpu_rows[slots.long()].cpu(), torch.from_numpy(table_n[admit]))
     finally:
         capi.unpin_memory(table)
+
+
+@pytest.mark.parametrize("row_bytes", [255, 256, 257, 270, 271, 495, 504, 510, 511, 513, 520, 1031, 2500, 5119, 12_403,
+                                       12_500])
+@pytest.mark.parametrize("n", [1, 31, 4001])
+def test_rows_that_are_no_16_byte_units(capi, row_bytes, n):
+    """Rows that start on any byte: the shortest and the longest that travel as 16-byte granules and
+    their neighbours, tables and outputs off 16-byte boundaries, tiles with a ragged end, hits and
+    host rows side by side; nothing beside the output is written."""
+    rng = np.random.default_rng(row_bytes + n)
+    rows = 700
+    for shift in (0, 1, 6):
+        raw = rng.integers(0, 256, size=rows * row_bytes + 16, dtype=np.uint8)
+        pinned = _pinned(capi, raw)
+        try:
+            host = pinned[shift:shift + rows * row_bytes].view(rows, row_bytes)
+            data = raw[shift:shift + rows * row_bytes].reshape(rows, row_bytes)
+            cached = rng.choice(rows, size=300, replace=False)
+            m = capi.CUCOStaticHashmap(torch.from_numpy(cached).cuda(), torch.arange(300, device="cuda"), 0.5)
+            block = torch.empty(300 * row_bytes + 16, dtype=torch.uint8, device="cuda")
+            gpu = block[shift:shift + 300 * row_bytes].view(300, row_bytes)
+            gpu.copy_(torch.from_numpy(255 - data[cached]))       # so a hit cannot pass for a host row
+            qn = rng.integers(0, rows, size=n)
+            q = torch.from_numpy(qn).cuda()
+            slot = np.full(rows, -1)
+            slot[cached] = np.arange(300)
+            want = np.where((slot[qn] >= 0)[:, None], 255 - data[qn], data[qn])
+            assert _bytes_equal(capi.cache_fetch(host, gpu, q, m), want)
+            assert _bytes_equal(capi.cache_fetch_with_mask(host, gpu, q, m.query(q)), want)
+            around = torch.full((n * row_bytes + 32,), 77, dtype=torch.uint8, device="cuda")
+            capi.uva_fetch(host, q, out=around[8 + shift:8 + shift + n * row_bytes].view(n, row_bytes))
+            got = around.cpu().numpy()
+            assert np.array_equal(got[8 + shift:8 + shift + n * row_bytes].reshape(n, row_bytes), data[qn])
+            assert (got[:8 + shift] == 77).all() and (got[8 + shift + n * row_bytes:] == 77).all()
+            # without a host table a row that is not cached is left as it was
+            around.fill_(77)
+            out = around[8 + shift:8 + shift + n * row_bytes].view(n, row_bytes)
+            _lib.check(_lib.lib.shmt_fetch(m._handle, None, 0, None, gpu.data_ptr(), q.data_ptr(), _lib.I64, n, row_bytes,
+                                           out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+            want = np.where((slot[qn] >= 0)[:, None], 255 - data[qn], np.uint8(77))
+            got = around.cpu().numpy()
+            assert np.array_equal(got[8 + shift:8 + shift + n * row_bytes].reshape(n, row_bytes), want)
+            assert (got[:8 + shift] == 77).all() and (got[8 + shift + n * row_bytes:] == 77).all()
+        finally:
+            capi.unpin_memory(pinned)
+    assert capi.device_fault() == 0
