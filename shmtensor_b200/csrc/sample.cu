@@ -135,6 +135,75 @@ struct HopEdge {
 };
 static_assert(kMaxSeedsPerTile <= 1 << 13, "a seed of the tile takes 13 bits");
 
+// Weighted picks without replacement (Efraimidis-Spirakis 2006): every edge gets the key -log(u) / w
+// (an exponential clock of rate w) and the k smallest keys win, which is sampling without
+// replacement with probabilities proportional to the weights.  The lanes 0..k-1 of a warp hold the k
+// smallest keys seen so far, ascending, equal keys by position; a smaller one is inserted by one
+// shuffle step.
+struct WeightedPicks {
+  float key;
+  int64_t pos;
+
+  // all lanes call with the same candidate
+  __device__ __forceinline__ void insert(float ck, int64_t cp, unsigned lane, int k) {
+    const float left_k = __shfl_up_sync(0xffffffffu, key, 1);
+    const int64_t left_p = __shfl_up_sync(0xffffffffu, pos, 1);
+    if ((int)lane < k && (ck < key || (ck == key && cp < pos))) {
+      const bool here = lane == 0 || left_k < ck || (left_k == ck && left_p < cp);
+      key = here ? ck : left_k;
+      pos = here ? cp : left_p;
+    }
+  }
+
+  // the edges [from, from + 128), then `step` further on, ... of a row of `deg` with weights `w`;
+  // a step's weights are loaded while the one before is looked at
+  __device__ __forceinline__ void scan(const float* w, int64_t from, int64_t step, int64_t deg, unsigned lane, int k,
+                                       const Philox& rng, uint32_t seed_idx, uint32_t off_lo, uint32_t off_hi) {
+    constexpr int U = 4;
+    const unsigned full = 0xffffffffu;
+    const float tiny = 1.17549435e-38f, most = 3.40282347e+38f;  // smallest weight, largest key
+    float next[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) next[u] = from + 32 * u + lane < deg ? __ldg(w + from + 32 * u + lane) : 1.0f;
+    float thr = __shfl_sync(full, key, k - 1);
+    for (int64_t p0 = from; p0 < deg; p0 += step) {
+      float cur[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        cur[u] = next[u];
+        const int64_t ahead = p0 + step + 32 * u + lane;
+        if (ahead < deg) next[u] = __ldg(w + ahead);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t at = p0 + 32 * u + lane;
+        float mine = __int_as_float(0x7f800000);
+        if (at < deg) {
+          const uint4 r = rng(seed_idx, (uint32_t)at, off_lo, off_hi);
+          const float x = ((float)(r.x >> 8) + 1.0f) * (1.0f / 16777216.0f);  // (0, 1]
+          // a weight that is not positive counts as the smallest one; its edge can still be picked
+          mine = fminf(-__logf(x) / fmaxf(cur[u], tiny), most);
+        }
+        unsigned cand = __ballot_sync(full, mine < thr);
+        while (cand) {
+          const int lead = __ffs(cand) - 1;
+          cand &= cand - 1;
+          const float ck = __shfl_sync(full, mine, lead);
+          if (ck < thr) {  // the bound may have dropped since the vote; same on every lane
+            insert(ck, p0 + 32 * u + lead, lane, k);
+            thr = __shfl_sync(full, key, k - 1);
+          }
+        }
+      }
+    }
+  }
+};
+
+// A row longer than this is shared by the warps of the CTA: a hop is as long as its longest row.
+// 1,000 seeds of a power-law graph with rows of up to 10,000 edges: 64 us when one warp took a row
+// with one load in flight, 24 us so.
+constexpr int64_t kWeightedLongRow = 1024;
+
 template <typename IxT, int G>
 __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
   extern __shared__ __align__(16) unsigned char s_dyn[];  // hop_smem_bytes()
@@ -228,7 +297,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const Philox rng(job.rng_seed);
   IxT* out_all = static_cast<IxT*>(job.sub_indices);
   const bool relabel = job.rel_slots != nullptr;
-  const bool listed = G < 32 || (k <= G && !job.weights);  // a smaller group is only launched for such calls
+  const bool listed = G < 32 || (k <= G && !(job.weights && job.replace));  // a smaller group is only launched for such calls
   const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
   const RelRange range{job.rel_slots,
                        relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
@@ -244,7 +313,49 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   // ---- 3. (k <= 32) positions of the picked neighbours, a group of lanes per seed, into a list in
   // output order.  Arithmetic and shuffles only: the memory work is left to step 5, where all
   // threads of the tile share it evenly whatever the rows' lengths.
-  if (listed) {
+  if (G == 32 && listed && job.weights && k > 0) {
+    __shared__ float s_key[G == 32 ? kHopThreads : 1];
+    __shared__ int64_t s_pos[G == 32 ? kHopThreads : 1];
+    const float none = __int_as_float(0x7f800000);
+    auto weights_of = [&](int j) { return (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j]; };
+    auto list = [&](int j, int64_t pos) {
+      s_list[s_off[j] + gl] = HopEdge::pack(s_begin[j] + pos, j, s_hit[j]);
+    };
+    for (int j = group; j < rows; j += kGroups) {
+      const int64_t deg = s_deg[j];
+      if (deg <= k) {
+        if ((int64_t)gl < deg) list(j, gl);
+      } else if (deg <= kWeightedLongRow) {
+        WeightedPicks best{none, -1};
+        best.scan(weights_of(j), 0, 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo, job.off_hi);
+        if ((int64_t)gl < k) list(j, best.pos);
+      }
+    }
+    for (int j = 0; j < rows; ++j) {
+      const int64_t deg = s_deg[j];
+      if (deg <= k || deg <= kWeightedLongRow) continue;  // the same on every thread
+      WeightedPicks best{none, -1};
+      best.scan(weights_of(j), group * 128, kGroups * 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo,
+                job.off_hi);
+      s_key[tid] = best.key;
+      s_pos[tid] = best.pos;
+      __syncthreads();
+      if (group == 0) {
+        for (int w = 1; w < kGroups; ++w)
+          for (int q = 0; q < (int)k; ++q) {
+            const float ck = s_key[w * 32 + q];
+            const int64_t cp = s_pos[w * 32 + q];
+            const float last_k = __shfl_sync(full, best.key, (int)k - 1);
+            const int64_t last_p = __shfl_sync(full, best.pos, (int)k - 1);
+            if (!(ck < last_k || (ck == last_k && cp < last_p))) break;  // nor do the warp's further keys
+            best.insert(ck, cp, gl, (int)k);
+          }
+        if ((int64_t)gl < k) list(j, best.pos);
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+  } else if (listed) {
     for (int j0 = 0; j0 < rows; j0 += kGroups) {
       const int j = j0 + group;
       const bool active = j < rows;
@@ -324,7 +435,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     for (int j = (int)tid; j < rows; j += kHopThreads)
       enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
 
-  // k > 32 (G == 32): one warp per seed
+  // k > 32, or weighted with replacement (G == 32): one warp per seed
   const uint32_t set_slots = job.set_slots;
   uint32_t* set = s_sets + (size_t)(tid >> 5) * set_slots;
   for (int j0 = 0; j0 < rows; j0 += kGroups) {
@@ -345,49 +456,10 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       if (job.out_eids) store_int(job.out_eids, job.indptr64, o, s_begin[j] + pos + s_eshift[j]);
       if (relabel) enter(n + o, val);
     };
-    if (job.weights && deg > 0 && (job.replace || deg > k)) {
+    if (job.weights && deg > 0 && job.replace) {
       const float* w = (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j];
       const float tiny = 1.17549435e-38f;  // a weight that is not positive counts as the smallest one
-      if (!job.replace) {
-        // Efraimidis-Spirakis: every edge gets the key -log(u) / w (an exponential clock of rate
-        // w) and the k smallest keys win, which is sampling without replacement with
-        // probabilities proportional to the weights.  Lanes 0..k-1 hold the k smallest keys seen
-        // so far, ascending; a key below the largest of them is inserted by one shuffle step.
-        float best = __int_as_float(0x7f800000);
-        int64_t bpos = -1;
-        float thr = best;
-        for (int64_t p0 = 0; p0 < deg; p0 += 32) {
-          const int64_t pos = p0 + gl;
-          float key = __int_as_float(0x7f800000);
-          if (pos < deg) {
-            const uint4 r = rng(seed_idx, (uint32_t)pos, job.off_lo, job.off_hi);
-            const float u = ((float)(r.x >> 8) + 1.0f) * (1.0f / 16777216.0f);  // (0, 1]
-            key = -__logf(u) / fmaxf(__ldg(w + pos), tiny);
-          }
-          unsigned cand = __ballot_sync(full, key < thr);
-          while (cand) {
-            const int from = __ffs(cand) - 1;
-            cand &= cand - 1;
-            const float ck = __shfl_sync(full, key, from);
-            const int64_t cp = __shfl_sync(full, pos, from);
-            if (ck < thr) {  // the bound may have dropped since the vote; same on every lane
-              const float left_k = __shfl_up_sync(full, best, 1);
-              const int64_t left_p = __shfl_up_sync(full, bpos, 1);
-              if ((int64_t)gl < k && ck < best) {
-                if (gl == 0 || left_k <= ck) {
-                  best = ck;
-                  bpos = cp;
-                } else {
-                  best = left_k;
-                  bpos = left_p;
-                }
-              }
-              thr = __shfl_sync(full, best, (int)k - 1);
-            }
-          }
-        }
-        if ((int64_t)gl < k) emit(out_at + gl, bpos);
-      } else {
+      {
         // k independent draws proportional to the weights: the row's total, then for 32 draws at
         // a time a second walk that finds where each draw's share of the total falls
         double sum = 0.0;
@@ -581,6 +653,10 @@ int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
                 size_t scratch_off, cudaStream_t stream);
 size_t scan_scratch_bytes(int64_t n);
 
+// The fan-out a hop is laid out for: weighted picks take the lists of fan-outs up to 32, with
+// replacement the warp-per-seed form of larger ones.
+static int64_t hop_layout_k(bool weighted, bool replace, int64_t k) { return !weighted ? k : (replace ? 33 : 32); }
+
 static int pick_seeds_per_tile(int64_t n, int64_t k) {
   int64_t s = (n + (int64_t)sm_count() * 4 - 1) / ((int64_t)sm_count() * 4);
   s = (s + kHopSeedStep - 1) / kHopSeedStep * kHopSeedStep;
@@ -614,7 +690,7 @@ template <typename IxT>
 static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool pdl = false) {
   const unsigned grid = (unsigned)n_tiles;
   job.set_slots = set_slots_for(job.k);
-  const size_t smem = hop_smem_bytes(job.seeds_per_tile, job.weights ? 33 : job.k, job.set_slots);
+  const size_t smem = hop_smem_bytes(job.seeds_per_tile, hop_layout_k(job.weights, job.replace, job.k), job.set_slots);
   if (!job.weights) {
     if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8>, grid, kHopThreads, smem, s, job);
     if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16>, grid, kHopThreads, smem, s, job);
@@ -644,7 +720,7 @@ struct MinibatchPlan {
 };
 
 static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, MinibatchPlan* p,
-                          bool weighted = false) {
+                          bool weighted = false, bool replace = false) {
   SHMT_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops, "mini-batch: 1..%d hops", kMaxHops);
   SHMT_REQUIRE(n_seeds >= 1 && n_seeds < ((int64_t)1 << 31), "mini-batch: seed count out of range");
   SHMT_REQUIRE(fanouts != nullptr, "mini-batch: fanouts is null");
@@ -654,7 +730,7 @@ static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, M
     SHMT_REQUIRE(fanouts[h] >= 1 && fanouts[h] < ((int64_t)1 << 20), "mini-batch: fan-out out of range");
     p->cap[h + 1] = p->cap[h] * (1 + fanouts[h]);
     SHMT_REQUIRE(p->cap[h + 1] < ((int64_t)1 << 30), "mini-batch: worst-case frontier too large");
-    p->spt[h] = pick_seeds_per_tile(p->cap[h], weighted ? 33 : fanouts[h]);  // weighted: warp-per-seed layout
+    p->spt[h] = pick_seeds_per_tile(p->cap[h], hop_layout_k(weighted, replace, fanouts[h]));
     p->hop_tiles[h] = (p->cap[h] + p->spt[h] - 1) / p->spt[h];
     p->rel_tiles[h] = (p->cap[h + 1] + kRelTile - 1) / kRelTile;
     p->off_hop[h] = cursor;
@@ -734,7 +810,7 @@ static int sample_hop_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   job.gpu_edge_base = gpu_edge_base;
   job.weights = weights;
   job.gpu_weights = gpu_weights;
-  job.seeds_per_tile = pick_seeds_per_tile(n, weights ? 33 : k);  // weighted: the warp-per-seed layout
+  job.seeds_per_tile = pick_seeds_per_tile(n, hop_layout_k(weights != nullptr, replace != 0, k));
   const int64_t n_tiles = (n + job.seeds_per_tile - 1) / job.seeds_per_tile;
   if (int rc = ctx_reserve(ctx, tile_state_bytes(n_tiles))) return rc;
   job.st = carve_tile_states(ctx->region(), n_tiles);
@@ -829,7 +905,7 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
 
   // worst-case frontier sizes and the scratch plan: [words][per hop: sample tiles | relabel tiles]
   MinibatchPlan plan;
-  if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &plan, weights != nullptr)) return rc;
+  if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &plan, weights != nullptr, replace != 0)) return rc;
   for (int h = 0; h < n_hops; ++h)
     SHMT_REQUIRE(out_sub_indptr[h] && out_sub_indices[h] && out_relabel[h] && out_frontier[h],
                  "shmt_sample_minibatch: output buffer of hop %d is null", h);

@@ -158,3 +158,33 @@ def test_weighted_minibatch_equals_weighted_hops(capi, cached):
     with pytest.raises(RuntimeError, match="cannot be combined"):
         capi.sample_minibatch(indptr, indices, seeds, [3], False, weights=weights, return_eids=True)
     capi.check_async()
+
+
+@pytest.mark.parametrize("deg", [33, 127, 128, 129, 1023, 1024, 1025, 1153, 2049, 10_000])
+@pytest.mark.parametrize("k", [1, 15, 32])
+def test_rows_around_the_length_that_a_whole_cta_shares(capi, deg, k):
+    """A row with k edges of overwhelming weight yields exactly those, wherever they lie; one whose
+    weights are all zero still yields k different edges; rows of several lengths share a tile."""
+    rng = np.random.default_rng(deg * 40 + k)
+    degs = np.array([deg, 5, deg, 0, 40, deg + 1])
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(degs)])).cuda()
+    indices = torch.arange(int(degs.sum()), dtype=torch.int32, device="cuda")
+    w = rng.random(int(degs.sum())).astype(np.float32) + 0.01
+    heavy = {}
+    for row in (0, 5):
+        heavy[row] = int(indptr[row]) + rng.choice(degs[row], size=k, replace=False)
+        w[heavy[row]] = 1e25
+    w[int(indptr[2]):int(indptr[3])] = 0.0
+    for _ in range(3):
+        p, x = capi.csr_weighted_sampling(indptr, indices, torch.from_numpy(w).cuda(),
+                                          torch.arange(6, dtype=torch.int32, device="cuda"), k, False)
+        p, x = p.cpu().numpy(), x.cpu().numpy()
+        assert np.array_equal(np.diff(p), np.minimum(degs, k))
+        for row in range(6):
+            got = x[p[row]:p[row + 1]]
+            assert np.unique(got).size == got.size
+            assert ((got >= int(indptr[row])) & (got < int(indptr[row + 1]))).all()
+            if row in heavy:
+                assert set(got.tolist()) == set(heavy[row].tolist())
+            if degs[row] <= k:
+                assert np.array_equal(got, np.arange(int(indptr[row]), int(indptr[row + 1])))
