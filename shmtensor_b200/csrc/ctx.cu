@@ -196,6 +196,22 @@ int shmt_ctx_create(int device, shmt_ctx** out) {
     delete ctx;
     return rc;
   }
+  void* scan_state = nullptr;
+  e = cudaMalloc(&scan_state, kScanStateBytes);
+  if (e == cudaSuccess) {
+    ctx->scan_state = static_cast<char*>(scan_state);
+    // zero before any stream's first scan
+    e = cudaMemsetAsync(scan_state, 0, kScanStateBytes, cudaStreamPerThread);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
+  }
+  if (e != cudaSuccess) {
+    set_error("shmt_ctx_create: %s", cudaGetErrorString(e));
+    if (scan_state) cudaFree(scan_state);
+    cudaFree(ctx->scratch);
+    cudaFreeHost(h);
+    delete ctx;
+    return SHMT_ERR_CUDA;
+  }
   ctx->h_words = static_cast<int64_t*>(h);
   memset(ctx->h_words, 0, kCtxWords * sizeof(int64_t));
   *out = ctx;
@@ -207,6 +223,7 @@ int shmt_ctx_destroy(shmt_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->table) cudaFree(ctx->table);
+  if (ctx->scan_state) cudaFree(ctx->scan_state);
   if (ctx->h_words) cudaFreeHost(ctx->h_words);
   if (ctx->tail_event) cudaEventDestroy(ctx->tail_event);
   delete ctx;
@@ -234,7 +251,7 @@ int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, 
 }
 
 int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx) {
-  return ctx ? (int64_t)(ctx->scratch_bytes + ctx->table_bytes) : 0;
+  return ctx ? (int64_t)(ctx->scratch_bytes + ctx->table_bytes + kScanStateBytes) : 0;
 }
 
 }  // extern "C"

@@ -18,6 +18,10 @@ struct shmt_ctx {
   int64_t post_seq = 0;
   cudaEvent_t tail_event = nullptr;
   bool tail_pending = false;
+  // Ticket, count of finished CTAs and tile descriptors of small scans: zero between calls, put back by
+  // the scan kernel itself (see scan.cu).
+  char* scan_state = nullptr;
+  int64_t* scan_words() const { return reinterpret_cast<int64_t*>(scan_state); }
   int64_t* d_words() const { return reinterpret_cast<int64_t*>(scratch); }
   char* region() const { return scratch + 256; }
 };
@@ -25,6 +29,8 @@ struct shmt_ctx {
 namespace shmt {
 
 constexpr int kCtxWords = 128;
+constexpr int kSmallScanTiles = 512;  // tiles whose descriptors live in shmt_ctx::scan_state
+constexpr size_t kScanStateBytes = 16 + (size_t)kSmallScanTiles * 16;
 enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).

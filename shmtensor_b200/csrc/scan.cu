@@ -13,11 +13,11 @@ namespace shmt {
 
 constexpr int kScanThreads = 512;
 constexpr int kScanWarps = kScanThreads / 32;
-constexpr int kScanVecs = 8;                                     // 16-byte vectors per thread
-constexpr int kScanTileBytes = kScanThreads * kScanVecs * 16;    // 64 KB per tile
+constexpr int kScanVecs = 8;                                     // 16-byte vectors per thread, at most
+__host__ __device__ constexpr int scan_tile_bytes(int vecs) { return kScanThreads * vecs * 16; }
+constexpr int kScanTileBytes = scan_tile_bytes(kScanVecs);       // 64 KB per tile
 constexpr int kScanTile = kScanTileBytes / 8;                    // items per tile of the widest type
-constexpr int kScanPartials = kScanVecs * kScanWarps;            // one per (row, warp)
-static_assert(kScanPartials % 32 == 0, "warp 0 scans the per-warp partials, the same number per lane");
+static_assert(kSmallScanTiles <= kScanThreads, "a look-back over a small scan is one step");
 
 template <typename T>
 struct ScanWord;
@@ -26,37 +26,43 @@ struct ScanWord<int> { using type = unsigned; };
 template <>
 struct ScanWord<long long> { using type = unsigned long long; };
 
-// A tile is 8 rows of 512 16-byte vectors (64 KB); thread t owns vector t of every row, so each
+// A tile is VECS rows of 512 16-byte vectors; thread t owns vector t of every row, so each
 // load and store instruction of a warp covers 512 contiguous bytes.  Sums are taken in the unsigned
 // type of the data (wrap-around is defined and the low bits are all the result keeps): inside a
-// vector, across the warp with shuffles, across the 128 (row, warp) partials by warp 0, which
-// also does the look-back; every thread then adds its three offsets and stores.  Large tiles
-// matter: the look-back hands a prefix over at most 32 tiles per round trip through L2, so the
-// bytes per tile bound the rate of the whole scan.
-template <typename T>
+// vector, across the warp with shuffles, across the (row, warp) partials by warp 0; after the
+// look-back every thread adds its three offsets and stores.
+// `clean`: this launch's tile descriptors, ticket and `done` word start at zero and are put back to
+// zero by the CTA whose look-back ends last, so a small scan needs no memset in front of it.
+template <typename T, int VECS>
 __global__ void __launch_bounds__(kScanThreads, 2)
-scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStates st, int64_t* words,
-            const TileDesc* carry) {
+scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStates st, int64_t* ticket, int64_t* status,
+            int64_t* clean, const TileDesc* carry) {
   using U = typename ScanWord<T>::type;
   constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int TILE = kScanTileBytes / (int)sizeof(T);
-  constexpr int PER_LANE = kScanPartials / 32;
-  __shared__ U partial[kScanPartials];  // [row][warp]
+  constexpr int TILE = scan_tile_bytes(VECS) / (int)sizeof(T);
+  constexpr int PARTIALS = VECS * kScanWarps;  // one per (row, warp)
+  constexpr int PER_LANE = PARTIALS / 32;
+  static_assert(PARTIALS % 32 == 0, "warp 0 scans the per-warp partials, the same number per lane");
+  // The sum of a tile of 32-bit numbers is taken and published ahead of the row sums (7.9 M of them:
+  // 14.7 us for 15.6); with 64-bit shuffles that costs more than it gains (1 M: 7.4 for 6.8).
+  constexpr bool kEarly = sizeof(T) == 4;
+  __shared__ U partial[PARTIALS];  // [row][warp]
+  __shared__ U s_warp[kScanWarps];
   __shared__ LookbackShared s_look;
-  __shared__ int64_t s_total;
   __shared__ int s_tile;
   const unsigned full = 0xffffffffu;
   const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tile = take_tile(words + W_TICKET, &s_tile);
+  const int tile = take_tile(ticket, &s_tile);
+  if (clean && tile == 0 && tid == 0) st_relaxed64(status, DEV_OK);  // it reports on this call only
   const int64_t tile_base = (int64_t)tile * TILE;
   union Pack {
     uint4 q;
     U a[VEC];
   };
 
-  U v[kScanVecs][VEC], vsum[kScanVecs], inc[kScanVecs];
+  U v[VECS][VEC], inc[VECS], sum = 0;  // a vector's own sum ends up in its last element
 #pragma unroll
-  for (int k = 0; k < kScanVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const int64_t at = tile_base + ((int64_t)k * kScanThreads + tid) * VEC;
     if (vec_ok && at + VEC <= n) {
       Pack p;
@@ -69,11 +75,25 @@ scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStat
     }
   }
 #pragma unroll
-  for (int k = 0; k < kScanVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
 #pragma unroll
     for (int j = 1; j < VEC; ++j) v[k][j] += v[k][j - 1];
-    vsum[k] = v[k][VEC - 1];
-    inc[k] = vsum[k];
+    sum += v[k][VEC - 1];
+  }
+  // zero-extended aggregate: tile sums add up in 64 bits, of which the low bits are used
+  U total = 0;
+  if (kEarly) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+    if (lane == 0) s_warp[warp] = sum;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) total += s_warp[w];
+    if (tid == 0) lookback_publish(st, tile, (int64_t)(uint64_t)total);
+  }
+#pragma unroll
+  for (int k = 0; k < VECS; ++k) {
+    inc[k] = v[k][VEC - 1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const U up = __shfl_up_sync(full, inc[k], o);
@@ -102,22 +122,29 @@ scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStat
       partial[lane * PER_LANE + q] = run;  // everything ahead of this (row, warp)
       run += a[q];
     }
-    const U total = __shfl_sync(full, linc, 31);
-    // zero-extended aggregate: tile sums add up in 64 bits, of which the low bits are used
-    if (lane == 0) {
-      s_total = (int64_t)(uint64_t)total;
-      lookback_publish(st, tile, s_total);
+    if (!kEarly && lane == 31) {
+      s_warp[0] = run;
+      lookback_publish(st, tile, (int64_t)(uint64_t)run);
     }
   }
-  __syncthreads();
+  if (!kEarly) {
+    __syncthreads();
+    total = s_warp[0];
+  }
   // `carry`: this launch continues a scan whose first part another kernel did (its last
   // descriptor holds the sum of everything before `data`)
-  const U prefix = (U)(uint64_t)(lookback_block(st, tile, s_total, &s_look, words + W_STATUS) +
+  const U prefix = (U)(uint64_t)(lookback_block(st, tile, (int64_t)(uint64_t)total, &s_look, status) +
                                  (carry ? carry->value : 0));
+  __syncthreads();  // nobody in this CTA reads descriptors any more
+  unsigned long long done_before = 0;  // looked at after the stores, so that they do not wait for it
+  if (clean && tid == 0) {
+    __threadfence();
+    done_before = atomicAdd(reinterpret_cast<unsigned long long*>(clean), 1ULL);
+  }
 #pragma unroll
-  for (int k = 0; k < kScanVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const int64_t at = tile_base + ((int64_t)k * kScanThreads + tid) * VEC;
-    const U before = prefix + partial[k * kScanWarps + warp] + (inc[k] - vsum[k]);
+    const U before = prefix + partial[k * kScanWarps + warp] + (inc[k] - v[k][VEC - 1]);
     Pack p;
 #pragma unroll
     for (int j = 0; j < VEC; ++j)
@@ -130,8 +157,14 @@ scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStat
         if (at + j < n) data[at + j] = (T)p.a[j];
     }
   }
+  if (clean && warp == 0 && __shfl_sync(full, done_before, 0) + 1 == gridDim.x) {
+    for (unsigned t = lane; t < gridDim.x; t += 32) st_desc(st.d + t, 0, 0);
+    if (lane == 0) {
+      st_relaxed64(ticket, 0);
+      st_relaxed64(clean, 0);
+    }
+  }
 }
-
 
 // ---- large inputs: persistent clusters ------------------------------------------------------
 // What bounds the kernel above is not bytes but the time a tile sits in registers: ticket,
@@ -436,17 +469,35 @@ static int run_scan_clusters(void* data, int64_t n_super, int exclusive, TileSta
 }
 
 template <typename T>
-static int64_t scan_tiles(int64_t n) {
-  const int64_t tile = kScanTileBytes / (int64_t)sizeof(T);
+static int64_t scan_tiles(int64_t n, int vecs = kScanVecs) {
+  const int64_t tile = scan_tile_bytes(vecs) / (int64_t)sizeof(T);
   return (n + tile - 1) / tile;
 }
 
-template <typename T>
-static void run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_t* words, cudaStream_t s,
-                     const TileDesc* carry = nullptr) {
+template <typename T, int VECS = kScanVecs>
+static void run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_t* ticket, int64_t* status,
+                     cudaStream_t s, int64_t* clean = nullptr, const TileDesc* carry = nullptr) {
   const int vec_ok = ((uintptr_t)data & 15) == 0;
-  scan_kernel<T><<<(unsigned)scan_tiles<T>(n), kScanThreads, 0, s>>>(static_cast<T*>(data), n, exclusive,
-                                                                      vec_ok, st, words, carry);
+  scan_kernel<T, VECS><<<(unsigned)scan_tiles<T>(n, VECS), kScanThreads, 0, s>>>(
+      static_cast<T*>(data), n, exclusive, vec_ok, st, ticket, status, clean, carry);
+}
+
+// Scans of up to kSmallScanTiles 64 KB tiles: look-back state that every launch leaves at zero, and the
+// largest grid of tiles that is resident at once (2 CTAs per SM), so that a small array is loaded and
+// stored by many SMs.  In a row of calls (with a memset and 64 KB tiles -> so): 1,000 int32 6.2 -> 2.5 us, 100,000
+// 8.1 -> 4.1, 1,000,000 8.2 -> 6.1; 2,400,001 int64 11.8 -> 10.6.
+template <typename T>
+static void run_scan_small(shmt_ctx* ctx, void* data, int64_t n, int exclusive, cudaStream_t s) {
+  int64_t* words = ctx->scan_words();
+  const TileStates st = carve_tile_states(reinterpret_cast<char*>(words + 2), kSmallScanTiles);
+  int64_t* status = ctx->d_words() + W_STATUS;
+  const int64_t resident = 2 * (int64_t)sm_count();
+  if (scan_tiles<T>(n, 2) <= resident)
+    run_scan<T, 2>(data, n, exclusive, st, words, status, s, words + 1);
+  else if (scan_tiles<T>(n, 4) <= resident)
+    run_scan<T, 4>(data, n, exclusive, st, words, status, s, words + 1);
+  else
+    run_scan<T, 8>(data, n, exclusive, st, words, status, s, words + 1);
 }
 
 // Large, 16-byte aligned inputs: whole 256 KB super-tiles by the persistent cluster kernel, what
@@ -461,7 +512,8 @@ static int run_scan_large(void* data, int64_t n, int exclusive, char* state_base
   const int64_t rest = n - n_super * per_super;
   if (rest > 0) {
     TileStates tail = carve_tile_states(state_base + tile_state_bytes(n_super), scan_tiles<T>(rest));
-    run_scan<T>(static_cast<T*>(data) + n_super * per_super, rest, exclusive, tail, words, s, st.d + (n_super - 1));
+    run_scan<T>(static_cast<T*>(data) + n_super * per_super, rest, exclusive, tail, words + W_TICKET,
+                words + W_STATUS, s, nullptr, st.d + (n_super - 1));
   }
   return SHMT_OK;
 }
@@ -477,11 +529,22 @@ __global__ void lookback_timeout_probe_kernel(TileStates st, int64_t* words, int
 
 // Launch helper shared with relabel / sub-CSR: scans `n` items in place using
 // ctx scratch at byte offset `scratch_off` for the tile states.
+size_t scan_scratch_bytes(int64_t n);
 int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
                 size_t scratch_off, cudaStream_t stream) {
   if (n <= 0) return SHMT_OK;
   const int64_t n_tiles = (n + kScanTile - 1) / kScanTile;
   SHMT_REQUIRE(n_tiles < (int64_t)1 << 30, "scan: %lld items is too many", (long long)n);
+  static const bool no_clusters = getenv("SHMT_SCAN_NO_CLUSTERS") != nullptr;
+  const bool clusters =
+      !no_clusters && ((uintptr_t)data & 15) == 0 && n * int_itemsize(dtype) >= kScanClusterMinBytes;
+  if (!clusters && (dtype == SHMT_I64 ? scan_tiles<long long>(n) : scan_tiles<int>(n)) <= kSmallScanTiles) {
+    dtype == SHMT_I64 ? run_scan_small<long long>(ctx, data, n, exclusive, stream)
+                      : run_scan_small<int>(ctx, data, n, exclusive, stream);
+    SHMT_CUDA_TRY(cudaGetLastError());
+    return SHMT_OK;
+  }
+  if (int rc = ctx_reserve(ctx, scratch_off + scan_scratch_bytes(n))) return rc;
   TileStates st = carve_tile_states(ctx->region() + scratch_off, n_tiles);
   // status / result / ticket words and the tile descriptors start at zero (one memset when the
   // descriptors sit right behind the words, as they do for a plain scan)
@@ -491,17 +554,16 @@ int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
     SHMT_CUDA_TRY(cudaMemsetAsync(ctx->d_words(), 0, 256, stream));
     SHMT_CUDA_TRY(cudaMemsetAsync(st.d, 0, tile_state_bytes(n_tiles), stream));
   }
-  static const bool no_clusters = getenv("SHMT_SCAN_NO_CLUSTERS") != nullptr;
-  if (!no_clusters && ((uintptr_t)data & 15) == 0 && n * int_itemsize(dtype) >= kScanClusterMinBytes) {
+  if (clusters) {
     // the ticketed kernel's descriptor block is larger than what both kernels need here
     char* base = reinterpret_cast<char*>(st.d);
     if (int rc = dtype == SHMT_I64 ? run_scan_large<long long>(data, n, exclusive, base, ctx->d_words(), stream)
                                    : run_scan_large<int>(data, n, exclusive, base, ctx->d_words(), stream))
       return rc;
   } else if (dtype == SHMT_I64) {
-    run_scan<long long>(data, n, exclusive, st, ctx->d_words(), stream);
+    run_scan<long long>(data, n, exclusive, st, ctx->d_words() + W_TICKET, ctx->d_words() + W_STATUS, stream);
   } else {
-    run_scan<int>(data, n, exclusive, st, ctx->d_words(), stream);
+    run_scan<int>(data, n, exclusive, st, ctx->d_words() + W_TICKET, ctx->d_words() + W_STATUS, stream);
   }
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -561,9 +623,9 @@ extern "C" int shmt_scan_static(void* data, int dtype, int64_t n, int exclusive,
   // words and the descriptors this call will use (they sit right behind the 256-byte header)
   SHMT_CUDA_TRY(cudaMemsetAsync(base, 0, 256 + tile_state_bytes(n_tiles), s));
   if (dtype == SHMT_I64)
-    run_scan<long long>(data, n, exclusive, st, words, s);
+    run_scan<long long>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s);
   else
-    run_scan<int>(data, n, exclusive, st, words, s);
+    run_scan<int>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
 }
@@ -606,6 +668,5 @@ extern "C" int shmt_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int ex
   if (n == 0) return SHMT_OK;
   SHMT_REQUIRE(data != nullptr, "shmt_scan: data is null");
   DeviceGuard guard(ctx->device);
-  if (int rc = ctx_reserve(ctx, scan_scratch_bytes(n))) return rc;
   return launch_scan(ctx, data, dtype, n, exclusive, 0, static_cast<cudaStream_t>(stream));
 }

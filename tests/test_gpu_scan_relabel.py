@@ -76,6 +76,40 @@ def test_scan_large_inputs_through_the_cluster_kernel(capi, dtype):
     assert capi.device_fault() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_small_scans_leave_their_state_clean_and_replay(capi, dtype):
+    """Scans of up to 512 tiles use look-back state that every launch puts back: sizes around the
+    16, 32 and 64 KB tiles and the grid sizes at which the tile grows, twice each; the same calls
+    captured in a graph give the same result on every replay."""
+    item = 4 if dtype == torch.int32 else 8
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sizes = [1, 16384 // item - 1, 16384 // item, 16384 // item + 1, 32768 // item + 3]
+    sizes += [2 * sms * kb * 1024 // item + d for kb in (16, 32) for d in (-1, 0, 1)] + [512 * 65536 // item - 4]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    big = torch.randint(-9, 9, (max(sizes) + 1,), generator=g, device="cuda").to(dtype)
+    for n in sizes:
+        for off in (0, 1):
+            for _ in range(2):
+                work = big.clone()[off:off + n]
+                capi.thrust_scan(work)
+                assert torch.equal(work, torch.cumsum(big[off:off + n], 0, dtype=dtype)), (n, off)
+    n = 2 * sms * 16384 // item + 5
+    work, start = big[:n].clone(), big[:n].clone()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        capi.exclusive_scan_(work)                 # the stream's context exists before the capture
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        work.copy_(start)
+        capi.exclusive_scan_(work)
+    for _ in range(3):
+        work.zero_()
+        graph.replay()
+        assert torch.equal(work, torch.cumsum(start, 0, dtype=dtype) - start)
+    capi.check_async()
+
+
 def test_scan_int32_wraps_like_the_oracle(capi):
     a = torch.full((5000,), 2**30, dtype=torch.int32, device="cuda")
     want = oracle.scan_inclusive(a.cpu().numpy())
