@@ -58,8 +58,14 @@ def _check_contig(t: torch.Tensor, name: str) -> None:
         raise RuntimeError(f"{name} must be contiguous")
 
 
+# torch's current stream of a device as the raw handle, without a Stream object around it (0.1 us
+# against 2.3): every call below asks for it
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    idx = device.index
+    return _raw_stream(torch.cuda.current_device() if idx is None else idx)
 
 
 def _ptr(t) -> int | None:
@@ -77,7 +83,7 @@ def _ctx(device: torch.device) -> int:
     from different torch streams can overlap on the GPU without sharing look-back state, result
     words or the relabel table."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, torch.cuda.current_stream(idx).cuda_stream)
+    key = (idx, _raw_stream(idx))
     h = _contexts.get(key)
     if h is None:
         out = C.c_void_p()
@@ -526,14 +532,15 @@ def tensor_relabel(tensors: List[torch.Tensor]):
         _check_cuda(t, "tensors")
         if t.device != dev:
             raise RuntimeError("tensor_relabel: all tensors must share a device")
-        dt = torch.promote_types(dt, t.dtype)  # what the reference's torch::cat does
+        if t.dtype != dt:
+            dt = torch.promote_types(dt, t.dtype)  # what the reference's torch::cat does
     code = _INT_CODES.get(dt)
     if code is None:
         raise RuntimeError(f"tensor_relabel: ID can only be int32 or int64, got {dt}")
     sizes = [t.numel() for t in tensors]
-    parts = [t.contiguous().reshape(-1).to(dt) for t in tensors]
+    parts = [t.contiguous().to(dt) for t in tensors]
     if len(parts) > 8:
-        parts = [torch.cat(parts, 0)]
+        parts = [torch.cat([p.reshape(-1) for p in parts], 0)]
     total = sum(sizes)
     unique = torch.empty(total, dtype=dt, device=dev)
     relabel = torch.empty(total, dtype=dt, device=dev)
@@ -543,7 +550,7 @@ def tensor_relabel(tensors: List[torch.Tensor]):
     n_unique = C.c_int64(0)
     check(lib.shmt_relabel(_ctx(dev), ptrs, lens, n_parts, code, _ptr(unique), _ptr(relabel),
                            C.byref(n_unique), _stream(dev)))
-    return unique[:n_unique.value], list(relabel.split_with_sizes(sizes, 0))
+    return unique[:n_unique.value], list(relabel.split_with_sizes(sizes))
 
 
 # --------------------------------------------------------------------------- sampling
@@ -770,23 +777,30 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
             _ctx(dev), _ptr(indptr), pdt, _ptr(indices), xdt, _ptr(gpu_indptr), _ptr(gpu_indices),
             map_handle, _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)), _rng["seed"], offset,
             out_ptr, out_idx, out_rel, out_front, sizes, _stream(dev)))
-    # one split per pool gives every exact-size view: per piece (skip, take, rest)
-    cuts_p, cuts_i = [], [0] * (9 * n_hops)
+    # one split per pool gives every exact-size view: per piece the gap in front of it and the piece
+    cuts_p, at_p, cuts_i, at_i = [], 0, [0] * (6 * n_hops), 0
     for h in range(n_hops):
-        n_in, nnz, n_out = sizes[3 * h], sizes[3 * h + 1], sizes[3 * h + 2]
-        room = p_off[h + 1] - p_off[h]
-        cuts_p += [n_in + 1, room - n_in - 1]
-        for piece, skip, take in ((h, 0, nnz), (n_hops + h, n_in, nnz), (2 * n_hops + h, 0, n_out)):
-            room = i_off[piece + 1] - i_off[piece]
-            cuts_i[3 * piece:3 * piece + 3] = [skip, take, room - skip - take]
+        take = sizes[3 * h] + 1
+        cuts_p += (p_off[h] - at_p, take)
+        at_p = p_off[h] + take
     if return_eids:
         for h in range(n_hops):
-            nnz = sizes[3 * h + 1]
-            cuts_p += [nnz, p_off[n_hops + h + 1] - p_off[n_hops + h] - nnz]
+            take = sizes[3 * h + 1]
+            cuts_p += (p_off[n_hops + h] - at_p, take)
+            at_p = p_off[n_hops + h] + take
+    cuts_p.append(p_off[-1] - at_p)
+    for piece in range(3 * n_hops):
+        kind, h = divmod(piece, n_hops)  # neighbours, their new ids (behind the seeds'), the frontier
+        start = i_off[piece] + (sizes[3 * h] if kind == 1 else 0)
+        take = sizes[3 * h + 2] if kind == 2 else sizes[3 * h + 1]
+        cuts_i[2 * piece] = start - at_i
+        cuts_i[2 * piece + 1] = take
+        at_i = start + take
+    cuts_i.append(i_off[-1] - at_i)
     pv = p_pool.split_with_sizes(cuts_p)
     iv = i_pool.split_with_sizes(cuts_i)
-    hops = [(pv[2 * h], iv[3 * h + 1], iv[3 * (n_hops + h) + 1], iv[3 * (2 * n_hops + h) + 1])
-            + ((pv[2 * (n_hops + h)],) if return_eids else ())
+    hops = [(pv[2 * h + 1], iv[2 * h + 1], iv[2 * (n_hops + h) + 1], iv[2 * (2 * n_hops + h) + 1])
+            + ((pv[2 * (n_hops + h) + 1],) if return_eids else ())
             for h in range(n_hops)]
     return hops[-1][3], hops
 

@@ -17,6 +17,8 @@
 // after another with 4-byte accesses and probe the map redundantly on 32 lanes.
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "bulk.cuh"
 #include "ctx.cuh"
 #include "map.cuh"
@@ -556,15 +558,19 @@ static int pick_rows_per_tile(int64_t n) {
 }
 
 // Persistent grid: never more CTAs than are resident at once (tiles are dealt round-robin
-// inside the kernels), so there is no partly filled last wave.
+// inside the kernels), so there is no partly filled last wave.  The occupancy of a kernel with so
+// much shared memory is asked for once (1 us, a fifth of a small call) and kept beside the kernel.
 template <typename Kernel>
-static unsigned grid_for_tiles(Kernel kernel, int64_t n, int R, size_t smem = 0) {
+static unsigned grid_for_tiles(Kernel kernel, std::atomic<uint64_t>* kept, int64_t n, int R, size_t smem = 0) {
   const int64_t tiles = (n + R - 1) / R;
   int64_t blocks = (tiles + kRowWarps - 1) / kRowWarps;
-  int occ = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRowThreads, smem) != cudaSuccess ||
-      occ < 1)
-    occ = 1;
+  const uint64_t have = kept->load(std::memory_order_relaxed);  // smem | CTAs per SM, 0 = not asked yet
+  int occ = (int)(have & 0xFF);
+  if (occ == 0 || (have >> 8) != smem) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRowThreads, smem) != cudaSuccess || occ < 1)
+      occ = 1;
+    kept->store(((uint64_t)smem << 8) | (uint64_t)occ, std::memory_order_relaxed);
+  }
   const int64_t resident = (int64_t)sm_count() * occ;
   if (blocks > resident) blocks = resident;
   return (unsigned)(blocks < 1 ? 1 : blocks);
@@ -572,7 +578,8 @@ static unsigned grid_for_tiles(Kernel kernel, int64_t n, int R, size_t smem = 0)
 
 template <int VEC, bool SET>
 static int launch_lsu(const RowJob& job, cudaStream_t s) {
-  const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, job.n, job.rows_per_tile);
+  static std::atomic<uint64_t> kept{0};
+  const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, job.n, job.rows_per_tile);
   row_copy_kernel<VEC, SET, 8><<<grid, kRowThreads, 0, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -612,7 +619,8 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   }
   job.rows_per_tile = R;
   const size_t smem = (size_t)kRowWarps * kBulkStages * R * job.row_bytes;
-  const unsigned blocks = grid_for_tiles(kernel, job.n, R, smem);
+  static std::atomic<uint64_t> kept{0};
+  const unsigned blocks = grid_for_tiles(kernel, &kept, job.n, R, smem);
   kernel<<<blocks, kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -654,7 +662,8 @@ static int launch_ragged(RowJob job, int R, cudaStream_t s) {
   }
   job.rows_per_tile = R;
   const size_t smem = ragged_smem_bytes(job.row_bytes, R);
-  kernel<<<grid_for_tiles(kernel, job.n, R, smem), kRowThreads, smem, s>>>(job);
+  static std::atomic<uint64_t> kept{0};
+  kernel<<<grid_for_tiles(kernel, &kept, job.n, R, smem), kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
 }
@@ -812,7 +821,8 @@ int shmt_insert_set(shmt_map* map, void* gpu_base, const void* keys, int key_dty
   DeviceGuard guard(map->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int R = pick_rows_per_tile(n);
-  const unsigned grid = grid_for_tiles(insert_set_kernel<16, 8>, n, R);
+  static std::atomic<uint64_t> kept{0};
+  const unsigned grid = grid_for_tiles(insert_set_kernel<16, 8>, &kept, n, R);
   const int vec = pick_vec(row_bytes, {gpu_base, update});
   char* g = static_cast<char*>(gpu_base);
   const char* u = static_cast<const char*>(update);
