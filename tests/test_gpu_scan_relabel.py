@@ -286,3 +286,23 @@ def test_lookback_wait_is_bounded_and_reported(capi):
     assert a[-1].item() == 50_005_000
     u, (r,) = capi.tensor_relabel([torch.tensor([7, 7, 3], device="cuda")])   # table was re-cleaned
     assert u.cpu().tolist() == [7, 3] and r.cpu().tolist() == [0, 0, 1]
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_relabel_in_one_cta_and_just_beyond(capi, n, dtype):
+    """Up to 4,096 ids are relabelled by one CTA with 1, 2 or 4 ids per thread: the edges of each,
+    all ids equal, all distinct and in between, ids that are negative or beyond 32 bits."""
+    rng = np.random.default_rng(n)
+    for hi in (1, max(1, n // 3), 1 << 30):
+        x = rng.integers(0, hi, size=n).astype(np.int64)
+        if hi > 1:
+            x[rng.integers(0, n)] = -7
+        if dtype == torch.int64:
+            x = x * 0x300000001
+        x = x.astype(np.int32 if dtype == torch.int32 else np.int64)
+        cut = n // 3
+        uniq, rel = capi.tensor_relabel([torch.from_numpy(x[:cut]).cuda(), torch.from_numpy(x[cut:]).cuda()])
+        wu, (wr,) = oracle.tensor_relabel([x])
+        assert uniq.dtype == dtype and np.array_equal(uniq.cpu().numpy(), wu)
+        assert np.array_equal(torch.cat(rel).cpu().numpy(), wr)
