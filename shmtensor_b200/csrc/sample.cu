@@ -82,6 +82,9 @@ struct HopJob {
   RelSlot* rel_slots;
   uint32_t rel_cap;
   void* rel_out;
+  // Look-back state that the kernel itself puts back to zero (small single-hop calls): the zeroed word
+  // in which its CTAs count themselves out, or nullptr.
+  int64_t* clean;
   // Single-hop call with a host result: the CTA that finishes its bookkeeping last hands the
   // result words to the host, which returns while the rows are still being written.
   HostPost post;
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     }
     return;
   }
+  if (job.clean && tile == 0 && tid == 0) st_relaxed64(job.status, DEV_OK);  // it reports on this call only
   const int64_t first = (int64_t)tile * S;
   const int rows = (int)min((int64_t)S, n - first);
   const int64_t k = job.k;
@@ -409,7 +413,28 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   }
   if (job.post.host) {  // uniform over the grid; the fused path (which may still flag the relabel table) never posts here
     __syncthreads();
-    if (tid == 0) post_when_last(job.post, n_tiles);
+    if (!job.clean && tid == 0) post_when_last(job.post, n_tiles);
+  }
+  if (job.clean) {  // uniform as well; all look-backs of this CTA are over
+    if (!job.post.host) __syncthreads();
+    if (tid < 32) {
+      bool last = false;
+      if (lane == 0) {
+        __threadfence();
+        last = atomicAdd(reinterpret_cast<unsigned long long*>(job.clean), 1ULL) + 1 == (unsigned long long)n_tiles;
+        if (last) {
+          __threadfence();
+          post_to_host(job.post);
+        }
+      }
+      if (__shfl_sync(full, (int)last, 0)) {
+        for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
+        if (lane == 0) {
+          st_relaxed64(job.ticket, 0);
+          st_relaxed64(job.clean, 0);
+        }
+      }
+    }
   }
 
   // ---- 5. output and relabel slots, one list element per thread and step
@@ -812,19 +837,32 @@ static int sample_hop_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   job.gpu_weights = gpu_weights;
   job.seeds_per_tile = pick_seeds_per_tile(n, hop_layout_k(weights != nullptr, replace != 0, k));
   const int64_t n_tiles = (n + job.seeds_per_tile - 1) / job.seeds_per_tile;
-  if (int rc = ctx_reserve(ctx, tile_state_bytes(n_tiles))) return rc;
-  job.st = carve_tile_states(ctx->region(), n_tiles);
-  job.ticket = ctx->d_words() + W_TICKET;
+  job.n_dev = nullptr;
+  // Up to kSmallScanTiles tiles use look-back state that the kernel leaves at zero: no memset in front
+  // (2 us and a gap on the GPU), and nothing behind the post that the scratch's next user waits for.
+  const bool small = n_tiles <= kSmallScanTiles;
+  int64_t* done = nullptr;
+  if (small) {
+    job.ticket = ctx->scan_words();
+    job.clean = done = ctx->scan_words() + 1;
+    job.st = carve_tile_states(reinterpret_cast<char*>(ctx->scan_words() + 2), kSmallScanTiles);
+  } else {
+    if (int rc = ctx_reserve(ctx, tile_state_bytes(n_tiles))) return rc;
+    done = ctx->d_words() + W_DONE;
+    job.ticket = ctx->d_words() + W_TICKET;
+    job.st = carve_tile_states(ctx->region(), n_tiles);
+    SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + tile_state_bytes(n_tiles), s));
+  }
   job.status = ctx->d_words() + W_STATUS;
   job.result = ctx->d_words() + W_RESULT;
-  job.n_dev = nullptr;
-  if (nnz_host) job.post = ctx_begin_post(ctx, ctx->d_words(), 4, ctx->d_words() + W_DONE);
-  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + tile_state_bytes(n_tiles), s));
+  if (nnz_host) job.post = ctx_begin_post(ctx, ctx->d_words(), 4, done);
   SHMT_CUDA_TRY(indices_dtype == SHMT_I64 ? launch_hop<long long>(job, n_tiles, s)
                                           : launch_hop<int>(job, n_tiles, s));
   SHMT_CUDA_TRY(cudaGetLastError());
   if (nnz_host) {
-    if (int rc = ctx_mark_tail(ctx, s)) return rc;
+    if (!small) {
+      if (int rc = ctx_mark_tail(ctx, s)) return rc;
+    }
     if (int rc = ctx_await_post(ctx, job.post, s)) return rc;
     if (int rc = ctx_status_of_words(ctx, "shmt_sample_hop")) return rc;
     *nnz_host = ctx->h_words[W_RESULT];
