@@ -18,22 +18,37 @@ namespace shmt {
 
 constexpr uint64_t kRelSurveyMinTableBytes = 32ull << 20;
 
-__device__ __forceinline__ void resolve_sizes(Parts& ps, int64_t* numel) {
-  if (ps.dev_n1) {  // |part 0| from the device if given there, else the host's start[1]
-    const int64_t a = ps.dev_n0 ? *ps.dev_n0 : ps.start[1], b = *ps.dev_n1;
-    ps.start[0] = 0;
-#pragma unroll
-    for (int q = 1; q <= kMaxParts; ++q) ps.start[q] = q == 1 ? a : a + b;
-  }
-  *numel = ps.start[kMaxParts];
+// Sizes of the input: the host's, or in the two-part form those an earlier kernel left on the device.
+// Kept beside the parts, which stay the launch's constants: written back into them they would live
+// in local memory, and so would every access by part number (a compact kernel over 300,000 ids spent
+// most of its 32 us queueing for that; see part_elem).
+struct PartSizes {
+  int64_t numel;
+  int64_t split;  // two-part form: elements of part 0; else -1
+};
+__device__ __forceinline__ PartSizes resolve_sizes(const Parts& ps) {
+  if (!ps.dev_n1) return PartSizes{ps.start[kMaxParts], -1};
+  const int64_t a = ps.dev_n0 ? *ps.dev_n0 : ps.start[1];
+  return PartSizes{a + *ps.dev_n1, a};
 }
 
-__device__ __forceinline__ int64_t part_elem(const Parts& ps, int64_t i) {
-  int p = 0;
+__device__ __forceinline__ int64_t part_elem(const Parts& ps, const PartSizes& sz, int64_t i) {
+  const void* p = ps.ptr[0];
+  int64_t from = 0;
+  if (sz.split >= 0) {
+    if (i >= sz.split) {
+      p = ps.ptr[1];
+      from = sz.split;
+    }
+  } else if (ps.n > 1) {
 #pragma unroll
-  for (int q = 1; q < kMaxParts; ++q)
-    if (q < ps.n && i >= ps.start[q]) p = q;
-  return load_int(ps.ptr[p], ps.is64, i - ps.start[p]);
+    for (int q = 1; q < kMaxParts; ++q)
+      if (q < ps.n && i >= ps.start[q]) {
+        p = ps.ptr[q];
+        from = ps.start[q];
+      }
+  }
+  return load_int(p, ps.is64, i - from);
 }
 
 // One id in 2^shift is in the sample, picked by its hash, so that all its occurrences are or none
@@ -51,8 +66,8 @@ __global__ void __launch_bounds__(kRelThreads)
 relabel_survey_kernel(Parts ps, RelSurvey* survey) {
   __shared__ unsigned s_marked[kRelThreads / 32];
   pdl_prologue();
-  int64_t numel;
-  resolve_sizes(ps, &numel);
+  const PartSizes sizes = resolve_sizes(ps);
+  const int64_t numel = sizes.numel;
   const int shift = relabel_sample_shift(numel);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -67,7 +82,9 @@ relabel_survey_kernel(Parts ps, RelSurvey* survey) {
         marked += (atomicOr(survey->bitmap + (at >> 5), bit) & bit) == 0;
     }
   };
-  for (int p = 0; p < ps.n; ++p) {
+#pragma unroll
+  for (int p = 0; p < kMaxParts; ++p) {
+    if (p >= ps.n) break;
     const int64_t n = ps.start[p + 1] - ps.start[p];
     int64_t done = 0;  // elements covered by the 16-byte loads below
     if ((reinterpret_cast<uintptr_t>(ps.ptr[p]) & 15) == 0) {
@@ -118,7 +135,7 @@ relabel_survey_kernel(Parts ps, RelSurvey* survey) {
 // How a call of `numel` ids uses the table.  Without a survey: at least two slots per id, as if all
 // were distinct.  With one: ids that all fit the table are their own slots (a frontier of densely
 // numbered nodes touches a compact part of the table); else kRelSlotsPerId slots per distinct id.
-constexpr double kRelSlotsPerId = 1.5;
+constexpr double kRelSlotsPerId = 2.0;
 __device__ __forceinline__ RelRange relabel_range(const RelTable& t, int64_t numel, const RelSurvey* survey) {
   RelRange r{t.slots, relabel_near((double)numel, relabel_slots_per_id((double)numel, 2.0), t.cap), t.cap, false};
   if (survey) {
@@ -139,17 +156,17 @@ __global__ void __launch_bounds__(kRelThreads, 6)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
                       const RelSurvey* __restrict__ survey) {
   pdl_prologue();
-  int64_t numel;
-  resolve_sizes(ps, &numel);
+  const PartSizes sizes = resolve_sizes(ps);
+  const int64_t numel = sizes.numel;
   const RelRange range = relabel_range(t, numel, survey);
-  // One element per thread and step, its successor's id read ahead: six resident CTAs of 38
-  // registers claim 33.5 M ids in 690 us where two elements per thread (3 CTAs) took 1,150.
+  // One element per thread and step, its successor's id read ahead: eight resident CTAs of 32
+  // registers claim 33.5 M ids in 660 us where two elements per thread (80 registers) took 1,150.
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  long long next = i < numel ? part_elem(ps, i) : 0;
+  long long next = i < numel ? part_elem(ps, sizes, i) : 0;
   for (; i < numel; i += stride) {
     const long long key = next;
-    if (i + stride < numel) next = part_elem(ps, i + stride);
+    if (i + stride < numel) next = part_elem(ps, sizes, i + stride);
     unsigned seen;
     const uint32_t pos = relabel_claim(range, key, status, &seen);
     store_int(out, ps.is64, i, relabel_pack(pos, relabel_settle(range, pos, seen, (unsigned)i), ps.is64));
@@ -171,8 +188,8 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   __shared__ LookbackShared s_look;
   __shared__ int s_tile;
   pdl_prologue();
-  int64_t numel;
-  resolve_sizes(ps, &numel);
+  const PartSizes sizes = resolve_sizes(ps);
+  const int64_t numel = sizes.numel;
   constexpr int kTile = kRelThreads * ITEMS;
   const int64_t n_tiles = (numel + kTile - 1) / kTile;
   const int tile = take_tile(ticket, &s_tile);
@@ -232,7 +249,7 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
     const unsigned row = __ballot_sync(0xffffffffu, is_first >> j & 1u);
     if (is_first >> j & 1u) {
       const int64_t uid = row_uid + __popc(row & ((1u << lane) - 1u));
-      store_int(unique, ps.is64, uid, part_elem(ps, i));
+      store_int(unique, ps.is64, uid, part_elem(ps, sizes, i));
       store_int(slot_of, ps.is64, i, uid);
       *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, ~0u, (unsigned)uid);
     } else if (maybe >> j & 1u) {
@@ -246,8 +263,8 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
 __global__ void __launch_bounds__(kRelThreads)
 relabel_remap_kernel(Parts ps, RelTable t, void* out) {
   pdl_prologue();
-  int64_t numel;
-  resolve_sizes(ps, &numel);
+  const PartSizes sizes = resolve_sizes(ps);
+  const int64_t numel = sizes.numel;
   constexpr int U = 4;  // independent slot reads per thread in flight
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < numel; i0 += U * stride) {
@@ -293,14 +310,15 @@ relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* 
   __shared__ int s_count[ITEMS * kWarps];
   const unsigned full = 0xffffffffu;
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int numel = (int)ps.start[kMaxParts];
+  const PartSizes sizes{ps.start[kMaxParts], -1};
+  const int numel = (int)sizes.numel;
   const uint32_t mask = slots - 1;
   long long id[ITEMS];
   uint32_t pos[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = j * kRelSmallThreads + tid;
-    id[j] = i < numel ? part_elem(ps, i) : 0;
+    id[j] = i < numel ? part_elem(ps, sizes, i) : 0;
   }
   for (uint32_t q = (uint32_t)tid; q < slots; q += kRelSmallThreads) {
     s_key[q] = kEmptyKey;
