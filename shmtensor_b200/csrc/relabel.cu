@@ -194,8 +194,12 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   const int64_t n_tiles = (numel + kTile - 1) / kTile;
   const int tile = take_tile(ticket, &s_tile);
   if (tile >= n_tiles) {  // the grid is sized for the largest input the caller allows
-    if (numel == 0 && tile == 0 && threadIdx.x == 0) {
-      *result = 0;
+    if (numel == 0 && tile == 0 && threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        st_relaxed64(result, 0);
+        __threadfence();
+      }
+      __syncwarp();
       post_to_host(post);
     }
     return;
@@ -240,7 +244,7 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   if (threadIdx.x == 0 && tile == n_tiles - 1) st_relaxed64(result, prefix + total);
   if (post.host) {
     __syncthreads();  // every thread's look-back (which may flag a timeout) is over
-    if (threadIdx.x == 0) post_when_last(post, n_tiles);
+    if (threadIdx.x < 32) post_when_last(post, n_tiles);
   }
   int64_t row_uid = prefix + before;
 #pragma unroll
@@ -382,7 +386,7 @@ relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* 
     }
   }
   __syncthreads();
-  if (tid == 0) post_to_host(post);  // behind the last barrier: nobody waits for its way to the host
+  if (warp == 0) post_to_host(post);  // behind the last barrier: nobody waits for its way to the host
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = j * kRelSmallThreads + tid;

@@ -232,9 +232,13 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const int64_t n_tiles = (n + S - 1) / S;
   const int tile = take_tile(job.ticket, &s_tile);
   if (tile >= n_tiles) {  // the grid is sized for the largest n the caller allows
-    if (n == 0 && tile == 0 && tid == 0) {
-      store_int(job.sub_indptr, job.indptr64, 0, 0);
-      st_relaxed64(job.result, 0);
+    if (n == 0 && tile == 0 && tid < 32) {
+      if (tid == 0) {
+        store_int(job.sub_indptr, job.indptr64, 0, 0);
+        st_relaxed64(job.result, 0);
+        __threadfence();
+      }
+      __syncwarp();
       post_to_host(job.post);
     }
     return;
@@ -413,7 +417,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   }
   if (job.post.host) {  // uniform over the grid; the fused path (which may still flag the relabel table) never posts here
     __syncthreads();
-    if (!job.clean && tid == 0) post_when_last(job.post, n_tiles);
+    if (!job.clean && tid < 32) post_when_last(job.post, n_tiles);
   }
   if (job.clean) {  // uniform as well; all look-backs of this CTA are over
     if (!job.post.host) __syncthreads();
@@ -422,12 +426,10 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       if (lane == 0) {
         __threadfence();
         last = atomicAdd(reinterpret_cast<unsigned long long*>(job.clean), 1ULL) + 1 == (unsigned long long)n_tiles;
-        if (last) {
-          __threadfence();
-          post_to_host(job.post);
-        }
+        __threadfence();
       }
       if (__shfl_sync(full, (int)last, 0)) {
+        post_to_host(job.post);
         for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
         if (lane == 0) {
           st_relaxed64(job.ticket, 0);
