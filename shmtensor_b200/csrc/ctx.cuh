@@ -8,8 +8,8 @@ struct shmt_ctx {
   char* scratch = nullptr;      // device scratch, grown geometrically; the first
   size_t scratch_bytes = 0;     // 256 bytes are the result words (status, result, ticket ...)
   int64_t* h_words = nullptr;   // pinned host mirror of the result words
-  // Relabel table (16-byte slots: key i64, first-index u32, new-id u32).  Keys and first-index words all ones between
-  // calls: the remap kernel restores every slot it leaves, so no per-call memset is needed.
+  // Relabel table (16-byte slots, see relabel.cuh), empty between calls: the kernels that number the
+  // ids empty every slot they leave, so no per-call memset is needed.
   char* table = nullptr;
   size_t table_bytes = 0;
   bool table_dirty = false;     // a failed call may have left entries behind
@@ -36,7 +36,7 @@ enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).
 int ctx_reserve(shmt_ctx* ctx, size_t bytes);
 
-// Make sure ctx->table holds at least `bytes`, all ones.
+// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with).
 int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
 
 // Copy the first `n_words` result words to the host and wait for `stream`.

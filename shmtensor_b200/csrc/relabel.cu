@@ -10,6 +10,8 @@
 // the same kernel, emit unique ids and the slot -> new id table, and put every slot
 // that was used back to "empty", so the table needs no memset between calls;
 // (3) remap the repeats.  Every element probes the table once (the reference four times).
+// Up to 4,096 ids are one CTA's work; more than 2^20 are looked over first and use the smallest
+// form of the table their ids allow, and (2) becomes three kernels without a look-back.
 // The element counts may live on the device (written by an earlier kernel), so a
 // chain of hops can be queued without the host knowing any size.
 #include "relabel.cuh"
@@ -133,24 +135,138 @@ relabel_survey_kernel(Parts ps, RelSurvey* survey) {
 }
 
 // How a call of `numel` ids uses the table.  Without a survey: at least two slots per id, as if all
-// were distinct.  With one: ids that all fit the table are their own slots (a frontier of densely
-// numbered nodes touches a compact part of the table); else kRelSlotsPerId slots per distinct id.
+// were distinct.  With one: kRelSlotsPerId slots per distinct id; or, where fewer bytes per id do:
+// * ids that are all smaller than the table are places themselves (densely numbered nodes): one word
+//   per id, its smallest index, is all there is to keep (RelSmall::stride 1);
+// * ids of few enough bits are kept in half-size slots where full ones would outgrow the L2 cache
+//   (RelSmall::stride 2).
 constexpr double kRelSlotsPerId = 2.0;
-__device__ __forceinline__ RelRange relabel_range(const RelTable& t, int64_t numel, const RelSurvey* survey) {
-  RelRange r{t.slots, relabel_near((double)numel, relabel_slots_per_id((double)numel, 2.0), t.cap), t.cap, false};
-  if (survey) {
-    if (survey->largest < (unsigned long long)t.cap) {
-      r.near = t.cap;
-      r.direct = true;
-    } else {
-      const float bits = (float)(1 << kRelSampleBits), free_bits = bits - (float)survey->marked;
-      const float sampled = free_bits > 0.0f ? -bits * logf(free_bits / bits) : bits * 16.0f;
-      const double ids = (double)sampled * (double)(1ull << relabel_sample_shift(numel));
-      r.near = relabel_near(ids < (double)numel ? ids : (double)numel, kRelSlotsPerId, t.cap);
+
+// Half-size slots.  An id of b bits is mapped one to one onto another number of b bits, whose top bits
+// are the home quad (four slots, 32 bytes) and whose other bits, with the distance from home, are all
+// the slot has to hold to tell the id: {tag 32, first 32} instead of {id 64, first 32, new id 32}.  The
+// new id takes the place of `first`, marked so that no index equals it.  What bounds a large relabel is
+// the sectors its random accesses draw from HBM (2.9 TB/s of them is all there is); half the table
+// means fewer.  An id that finds its 31 quads full goes to an ordinary slot behind them.
+struct RelSmall {
+  unsigned* words;  // the front of the table; nullptr: ordinary slots are used
+  uint32_t n;       // places
+  int stride;       // words per place: 1 = the id is the place, 2 = half-size slot
+  int bits, quad_bits;
+  RelRange rest;    // ordinary slots behind half-size ones; a position is n + index there
+};
+constexpr int kHalfRemainderBits = 26, kHalfQuads = 31;  // the tag is never all ones, which is an empty slot's
+constexpr double kHalfSlotsPerId = 1.6;                  // before rounding up to a power of two
+constexpr double kHalfMinBytes = 40.0 * (1 << 20);       // ordinary slots of this much are in L2 anyway
+
+struct RelUse {
+  RelRange range;
+  RelSmall small;
+};
+__device__ __forceinline__ RelUse relabel_use(const RelTable& t, int64_t numel, const RelSurvey* survey) {
+  RelUse u;
+  u.small = RelSmall{nullptr, 0, 0, 0, 0, {}};
+  u.range = RelRange{t.slots, relabel_near((double)numel, relabel_slots_per_id((double)numel, 2.0), t.cap), t.cap};
+  if (!survey) return u;
+  if (survey->largest < (unsigned long long)t.cap) {
+    u.small = RelSmall{reinterpret_cast<unsigned*>(t.slots), (uint32_t)survey->largest + 1, 1, 0, 0, {}};
+    return u;
+  }
+  const float bits = (float)(1 << kRelSampleBits), free_bits = bits - (float)survey->marked;
+  const float sampled = free_bits > 0.0f ? -bits * logf(free_bits / bits) : bits * 16.0f;
+  double ids = (double)sampled * (double)(1ull << relabel_sample_shift(numel));
+  if (ids > (double)numel) ids = (double)numel;
+  u.range.near = relabel_near(ids, kRelSlotsPerId, t.cap);
+  if (ids * kRelSlotsPerId * sizeof(RelSlot) < kHalfMinBytes || t.cap > (1u << 30)) return u;
+  int quad_bits = 0;
+  while ((double)(4ull << quad_bits) < ids * kHalfSlotsPerId) ++quad_bits;
+  int id_bits = 64 - __clzll((long long)survey->largest);
+  if (id_bits < quad_bits) id_bits = quad_bits;
+  if (id_bits - quad_bits > kHalfRemainderBits) return u;
+  const uint32_t n = 4u << quad_bits, rest = t.cap - n / 2;  // rest: enough for what n places cannot hold
+  u.small = RelSmall{reinterpret_cast<unsigned*>(t.slots), n, 2, id_bits, quad_bits,
+                     RelRange{t.slots + n / 2, rest, rest}};
+  return u;
+}
+
+// One to one on numbers of `bits` bits: every step can be undone (a right shift by half of the bits,
+// a product with an odd number modulo 2^bits).
+__device__ __forceinline__ uint64_t mix_bits(uint64_t x, int bits) {
+  const uint64_t mask = bits >= 64 ? ~0ull : (1ull << bits) - 1;
+  const int half = (bits + 1) / 2;
+  x ^= x >> half;
+  x = (x * 0xff51afd7ed558ccdULL) & mask;
+  x ^= x >> half;
+  x = (x * 0xc4ceb9fe1a85ec53ULL) & mask;
+  x ^= x >> half;
+  return x;
+}
+
+// relabel_claim and relabel_settle for half-size slots: a claim enters the index with the id.
+__device__ __forceinline__ uint32_t relabel_claim_half(const RelSmall& t, long long key, unsigned i, int64_t* status,
+                                                       bool* maybe_first) {
+  const uint64_t x = mix_bits((uint64_t)key, t.bits);
+  const int low = t.bits - t.quad_bits;
+  const uint32_t home = (uint32_t)(x >> low), remainder = (uint32_t)(x & ((1ull << low) - 1));
+  const uint32_t quads = t.n / 4;
+  unsigned long long* slots = reinterpret_cast<unsigned long long*>(t.words);
+  for (uint32_t d = 0; d < kHalfQuads; ++d) {
+    const uint32_t at = ((home + d) & (quads - 1)) * 4, tag = (d << kHalfRemainderBits) | remainder;
+    unsigned long long w[4];
+    asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                 : "l"(slots + at)
+                 : "memory");
+    int found = -1;
+    unsigned seen = 0xFFFFFFFFu;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (found >= 0) continue;
+      if ((uint32_t)(w[q] >> 32) == ~0u) {  // empty, whatever an ordinary slot has left below
+        const unsigned long long empty = w[q];
+        w[q] = atomicCAS(slots + at + q, empty, ((unsigned long long)tag << 32) | i);
+        if (w[q] == empty) {
+          *maybe_first = true;
+          return at + q;
+        }
+      }
+      if ((uint32_t)(w[q] >> 32) == tag) {
+        found = q;
+        seen = (unsigned)w[q];
+      }
+    }
+    if (found >= 0) {
+      *maybe_first = seen > i;
+      if (seen > i) atomicMin(t.words + 2 * (size_t)(at + found), i);
+      return at + found;
     }
   }
-  return r;
+  unsigned seen;
+  const uint32_t pos = relabel_claim(t.rest, key, status, &seen);
+  *maybe_first = relabel_settle(t.rest, pos, seen, i);
+  return t.n + pos;
 }
+
+// Where the later passes of a surveyed call find what they need at position `pos`.
+struct RelView {
+  RelSmall small;
+  RelSlot* slots;  // ordinary slots, by position
+  __device__ __forceinline__ RelView(const RelTable& t, int64_t numel, const RelSurvey* survey) {
+    small = relabel_use(t, numel, survey).small;
+    slots = small.words ? small.rest.slots - small.n : t.slots;  // only indexed from small.n on
+  }
+  __device__ __forceinline__ unsigned* word(uint32_t pos) const { return small.words + (size_t)pos * small.stride; }
+  __device__ __forceinline__ unsigned first(uint32_t pos) const {
+    return __ldcg(pos < small.n ? word(pos) : &slots[pos].first);
+  }
+  __device__ __forceinline__ unsigned newid(uint32_t pos) const { return first(pos) & ~kRelNewId; }
+  __device__ __forceinline__ void number(uint32_t pos, unsigned uid) const {
+    if (pos < small.n)
+      *word(pos) = uid | kRelNewId;
+    else
+      *reinterpret_cast<uint4*>(slots + pos) = make_uint4(~0u, ~0u, uid | kRelNewId, ~0u);
+  }
+};
 
 __global__ void __launch_bounds__(kRelThreads, 6)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
@@ -158,25 +274,48 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
   pdl_prologue();
   const PartSizes sizes = resolve_sizes(ps);
   const int64_t numel = sizes.numel;
-  const RelRange range = relabel_range(t, numel, survey);
-  // One element per thread and step, its successor's id read ahead: eight resident CTAs of 32
-  // registers claim 33.5 M ids in 660 us where two elements per thread (80 registers) took 1,150.
+  const RelUse use = relabel_use(t, numel, survey);
+  // One element per thread and step, its successor's id read ahead: more resident threads are worth
+  // more than more elements on their way per thread (33.5 M ids: 660 us, two elements per thread with
+  // twice the registers 1,150).
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   long long next = i < numel ? part_elem(ps, sizes, i) : 0;
   for (; i < numel; i += stride) {
     const long long key = next;
     if (i + stride < numel) next = part_elem(ps, sizes, i + stride);
-    unsigned seen;
-    const uint32_t pos = relabel_claim(range, key, status, &seen);
-    store_int(out, ps.is64, i, relabel_pack(pos, relabel_settle(range, pos, seen, (unsigned)i), ps.is64));
+    bool maybe_first;
+    uint32_t pos;
+    if (use.small.stride == 1) {
+      pos = (uint32_t)key;
+      maybe_first = __ldcg(use.small.words + pos) > (unsigned)i;
+      if (maybe_first) atomicMin(use.small.words + pos, (unsigned)i);
+    } else if (use.small.stride == 2) {
+      pos = relabel_claim_half(use.small, key, (unsigned)i, status, &maybe_first);
+    } else {
+      unsigned seen;
+      pos = relabel_claim(use.range, key, status, &seen);
+      maybe_first = relabel_settle(use.range, pos, seen, (unsigned)i);
+    }
+    store_int(out, ps.is64, i, relabel_pack(pos, maybe_first, ps.is64));
   }
+}
+
+// Words and half-size slots are not emptied one by one: the front of the table is filled anew.
+__global__ void __launch_bounds__(kRelThreads)
+relabel_clear_kernel(RelTable t, int64_t numel, const RelSurvey* __restrict__ survey) {
+  const RelSmall small = relabel_use(t, numel, survey).small;
+  if (!small.words) return;
+  uint4* dst = reinterpret_cast<uint4*>(small.words);
+  const uint64_t n = ((uint64_t)small.n * small.stride + 3) / 4;  // a little beyond: all ones there already
+  for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (uint64_t)gridDim.x * blockDim.x)
+    dst[q] = make_uint4(~0u, ~0u, ~0u, ~0u);
 }
 
 // Flags first occurrences, numbers them in input order (look-back over the tiles) and finishes
 // everything that can be finished for them: the unique id, the element's own result, and the slot,
-// which gets the new id and is emptied for the next call in the same 16-byte store (a later
-// candidate of the same id still finds an index that is not its own there).  What is left for the
+// which is emptied for the next call and gets the new id in the same 16-byte store (a later
+// candidate of the same id finds no index of its own there).  What is left for the
 // remap kernel are the repeats alone, marked as such.  A warp takes 32 * ITEMS consecutive
 // elements, 32 at a time, so that every access to the streamed arrays is contiguous; all slot
 // reads of a thread are in flight together.
@@ -219,11 +358,17 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
       maybe |= (unsigned)m << j;
     }
   }
-  // only an element the inserting pass did not rule out has to look at its slot
+  // only an element the inserting pass did not rule out has to look at its slot; its id is fetched
+  // along with it (most are first occurrences), so that nothing waits for it behind the look-back
+  int64_t id[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     first[j] = 0xFFFFFFFFu;
-    if (maybe >> j & 1u) first[j] = __ldcg(&t.slots[pos[j]].first);
+    id[j] = 0;
+    if (maybe >> j & 1u) {
+      first[j] = __ldcg(&t.slots[pos[j]].first);
+      id[j] = part_elem(ps, sizes, base + 32 * j);
+    }
   }
   int before = 0, firsts = 0;  // first occurrences of earlier warps and of this one
 #pragma unroll
@@ -253,14 +398,156 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
     const unsigned row = __ballot_sync(0xffffffffu, is_first >> j & 1u);
     if (is_first >> j & 1u) {
       const int64_t uid = row_uid + __popc(row & ((1u << lane) - 1u));
-      store_int(unique, ps.is64, uid, part_elem(ps, sizes, i));
+      store_int(unique, ps.is64, uid, id[j]);
       store_int(slot_of, ps.is64, i, uid);
-      *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, ~0u, (unsigned)uid);
+      *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, (unsigned)uid | kRelNewId, ~0u);
     } else if (maybe >> j & 1u) {
       store_int(slot_of, ps.is64, i, relabel_pack(pos[j], false, ps.is64));
     }
     row_uid += __popc(row);
   }
+}
+
+// The same for a surveyed (large) input, in three kernels without a look-back: flag, number the tiles,
+// number the flagged elements.  Where first occurrences crowd together, as they do at the start of an
+// input with many repeats, a tile is ten times the work of another, and in one kernel every later tile
+// waits for it: 449 us for 33.5 M ids (431 with half-size slots, 339 with one long run per CTA),
+// 310 in three.
+constexpr int kFlagItems = 8;
+constexpr int kFlagTile = kRelThreads * kFlagItems, kFlagWords = kFlagTile / 32;
+inline int64_t flag_tiles(int64_t numel) { return (numel + kFlagTile - 1) / kFlagTile; }
+inline size_t flag_bytes(int64_t numel) {  // a bit per element, then a count per tile
+  return (size_t)flag_tiles(numel) * (kFlagWords * sizeof(uint32_t) + sizeof(int)) + sizeof(int);
+}
+
+__global__ void __launch_bounds__(kRelThreads, 6)
+relabel_flag_kernel(RelTable t, int is64, int64_t numel, void* slot_of, uint32_t* __restrict__ flags,
+                    int* __restrict__ counts, const RelSurvey* __restrict__ survey) {
+  __shared__ int s_count[kRelThreads / 32];
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const RelView view(t, numel, survey);
+  const int64_t word0 = (int64_t)blockIdx.x * kFlagWords + warp * kFlagItems;  // of this warp
+  const int64_t base = word0 * 32 + lane;
+  uint32_t pos[kFlagItems];
+  unsigned first[kFlagItems], maybe = 0;
+#pragma unroll
+  for (int u = 0; u < kFlagItems; ++u) {
+    pos[u] = 0;
+    if (base + 32 * u < numel) {
+      bool m;
+      pos[u] = relabel_unpack(slot_of, is64, base + 32 * u, &m);
+      maybe |= (unsigned)m << u;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kFlagItems; ++u) {
+    first[u] = 0xFFFFFFFFu;
+    if (maybe >> u & 1u) first[u] = view.first(pos[u]);
+  }
+  int firsts = 0;
+#pragma unroll
+  for (int u = 0; u < kFlagItems; ++u) {
+    const bool is_first = first[u] == (unsigned)(base + 32 * u);
+    const unsigned word = __ballot_sync(0xffffffffu, is_first);
+    firsts += __popc(word);
+    if (lane == 0) flags[word0 + u] = word;
+    if (!is_first && (maybe >> u & 1u)) store_int(slot_of, is64, base + 32 * u, relabel_pack(pos[u], false, is64));
+  }
+  if (lane == 0) s_count[warp] = firsts;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int w = 0; w < kRelThreads / 32; ++w) sum += s_count[w];
+    counts[blockIdx.x] = sum;
+  }
+}
+
+// One CTA: counts -> first occurrences ahead of each tile; their number goes to the host.
+constexpr int kTotalThreads = 1024;
+__global__ void __launch_bounds__(kTotalThreads)
+relabel_total_kernel(int* counts, int n_tiles, int64_t* result, HostPost post) {
+  __shared__ int64_t s_sums[32];
+  __shared__ int64_t s_total;
+  // a thread takes consecutive counts, four at a time (the array is 16-byte aligned and, past the
+  // tiles, has room for one more count only)
+  const int per = ((n_tiles + kTotalThreads - 1) / kTotalThreads + 3) & ~3, lo = (int)threadIdx.x * per;
+  const int hi = lo + per < n_tiles ? lo + per : n_tiles;
+  int64_t sum = 0;
+#pragma unroll 4
+  for (int q = lo; q + 4 <= hi; q += 4) {
+    const int4 c = *reinterpret_cast<const int4*>(counts + q);
+    sum += c.x + c.y + c.z + c.w;
+  }
+  for (int q = lo < hi ? lo + ((hi - lo) & ~3) : hi; q < hi; ++q) sum += counts[q];
+  int at = (int)block_exclusive_scan(sum, s_sums, &s_total);
+#pragma unroll 4
+  for (int q = lo; q + 4 <= hi; q += 4) {
+    const int4 c = *reinterpret_cast<const int4*>(counts + q);
+    *reinterpret_cast<int4*>(counts + q) = make_int4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
+    at += c.x + c.y + c.z + c.w;
+  }
+  for (int q = lo < hi ? lo + ((hi - lo) & ~3) : hi; q < hi; ++q) {
+    const int c = counts[q];
+    counts[q] = at;
+    at += c;
+  }
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) {
+      counts[n_tiles] = (int)s_total;
+      st_relaxed64(result, s_total);
+      __threadfence();
+    }
+    __syncwarp();
+    post_to_host(post);
+  }
+}
+
+__global__ void __launch_bounds__(kRelThreads, 5)
+relabel_number_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique,
+                      const uint32_t* __restrict__ flags, const int* __restrict__ before,
+                      const RelSurvey* __restrict__ survey) {
+  const int tile_before = before[blockIdx.x];
+  if (before[blockIdx.x + 1] == tile_before) return;
+  static_assert(kFlagWords == 64, "two words of the tile per lane");
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, full = 0xffffffffu;
+  const PartSizes sizes{ps.start[kMaxParts], -1};
+  const RelView view(t, sizes.numel, survey);
+  const int64_t word0 = (int64_t)blockIdx.x * kFlagWords;
+  // every warp adds up the tile's words, two per lane, and takes kFlagItems of them
+  const uint2 two = reinterpret_cast<const uint2*>(flags + word0)[lane];
+  const int both = __popc(two.x) + __popc(two.y);
+  int inc = both;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(full, inc, o);
+    if (lane >= (unsigned)o) inc += up;
+  }
+  const int ahead = inc - both;  // of this lane's first word
+  const int64_t base = (word0 + warp * kFlagItems) * 32 + lane;
+  uint32_t pos[kFlagItems];
+  int64_t id[kFlagItems];
+  int uid[kFlagItems];
+  unsigned mine = 0;
+#pragma unroll
+  for (int u = 0; u < kFlagItems; ++u) {
+    const int from = (int)(warp * kFlagItems + u) / 2;
+    const uint32_t x = __shfl_sync(full, two.x, from), y = __shfl_sync(full, two.y, from);
+    const uint32_t word = u & 1 ? y : x;
+    uid[u] = tile_before + __shfl_sync(full, ahead, from) + (u & 1 ? __popc(x) : 0) + __popc(word & ((1u << lane) - 1u));
+    if (word >> lane & 1u) {
+      bool m;
+      mine |= 1u << u;
+      pos[u] = relabel_unpack(slot_of, ps.is64, base + 32 * u, &m);
+      id[u] = part_elem(ps, sizes, base + 32 * u);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kFlagItems; ++u)
+    if (mine >> u & 1u) {
+      store_int(unique, ps.is64, uid[u], id[u]);
+      store_int(slot_of, ps.is64, base + 32 * u, uid[u]);
+      view.number(pos[u], (unsigned)uid[u]);
+    }
 }
 
 // The repeats: slot -> new id.  First occurrences hold theirs already.
@@ -287,10 +574,39 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out) {
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (repeat[u]) newid[u] = __ldcg(&t.slots[pos[u]].newid);
+      if (repeat[u]) newid[u] = __ldcg(&t.slots[pos[u]].first) & ~kRelNewId;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (repeat[u]) store_int(out, ps.is64, i0 + u * stride, (int64_t)newid[u]);
+  }
+}
+
+// The same for a surveyed input.
+__global__ void __launch_bounds__(kRelThreads)
+relabel_remap_large_kernel(RelTable t, int is64, int64_t numel, void* out, const RelSurvey* __restrict__ survey) {
+  const RelView view(t, numel, survey);
+  constexpr int U = 4;  // independent slot reads per thread in flight
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < numel; i0 += U * stride) {
+    uint32_t pos[U];
+    unsigned newid[U];
+    bool repeat[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * stride;
+      repeat[u] = false;
+      if (i < numel) {
+        bool done;
+        pos[u] = relabel_unpack(out, is64, i, &done);
+        repeat[u] = !done;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (repeat[u]) newid[u] = view.newid(pos[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (repeat[u]) store_int(out, is64, i0 + u * stride, (int64_t)newid[u]);
   }
 }
 
@@ -414,8 +730,8 @@ static int launch_relabel_small(const Parts& ps, void* out_unique, void* out_rel
 }
 
 // Table for up to `numel_bound` ids at load <= 0.5, in the context's block whose keys and
-// first-index words are all ones between calls (whatever the capacity, so regions of different
-// capacities may overlap freely); the new-id words need no initial value.
+// first-index words are empty between calls (whatever the capacity, so regions of different
+// capacities may overlap freely).
 // Small inputs get four times the room (see kRelRoomy).
 uint64_t relabel_capacity(int64_t numel_bound) {
   uint64_t cap = 64;
@@ -446,7 +762,17 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_insert_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel, status,
                                 (const RelSurvey*)survey));
   }
-  if (numel_bound >= kRelLargeInput) {
+  if (survey) {
+    const int64_t tiles = flag_tiles(numel_bound);  // surveyed inputs are of that size exactly
+    uint32_t* flags = reinterpret_cast<uint32_t*>(survey + 1);
+    int* counts = reinterpret_cast<int*>(flags + tiles * kFlagWords);
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_flag_kernel, (unsigned)tiles, kRelThreads, 0, s, t, ps.is64, numel_bound,
+                                out_relabel, flags, counts, (const RelSurvey*)survey));
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_total_kernel, 1u, kTotalThreads, 0, s, counts, (int)tiles, result,
+                                post ? *post : HostPost{}));
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_number_kernel, (unsigned)tiles, kRelThreads, 0, s, ps, t, out_relabel,
+                                out_unique, (const uint32_t*)flags, (const int*)counts, (const RelSurvey*)survey));
+  } else if (numel_bound >= kRelLargeInput) {
     const int64_t big_tiles = (numel_bound + kRelThreads * kRelItemsLarge - 1) / (kRelThreads * kRelItemsLarge);
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItemsLarge>, (unsigned)big_tiles, kRelThreads, 0, s,
                                 ps, t, out_relabel, out_unique, st, ticket, status, result,
@@ -456,7 +782,14 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
                                 out_relabel, out_unique, st, ticket, status, result,
                                 post ? *post : HostPost{}));
   }
-  SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel));
+  if (!survey) {
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel));
+  } else {
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_large_kernel, grid, kRelThreads, 0, s, t, ps.is64, numel_bound,
+                                out_relabel, (const RelSurvey*)survey));
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_clear_kernel, grid, kRelThreads, 0, s, t, numel_bound,
+                                (const RelSurvey*)survey));
+  }
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
 }
@@ -515,7 +848,7 @@ extern "C" int shmt_relabel(shmt_ctx* ctx, const void* const* parts, const int64
   // a table that fits the L2 cache gains nothing from compact slots; a larger one may
   const bool look = relabel_capacity(numel) * sizeof(RelSlot) > kRelSurveyMinTableBytes;
   const size_t zeroed = look ? states + sizeof(RelSurvey) : tile_state_bytes(n_tiles);
-  if (int rc = ctx_reserve(ctx, zeroed)) return rc;
+  if (int rc = ctx_reserve(ctx, zeroed + (look ? flag_bytes(numel) : 0))) return rc;
   TileStates st = carve_tile_states(ctx->region(), n_tiles);
   RelSurvey* survey = look ? reinterpret_cast<RelSurvey*>(ctx->region() + states) : nullptr;
   // result words, tile descriptors and the survey to zero

@@ -8,12 +8,12 @@
 namespace shmt {
 
 constexpr int kRelThreads = 256;
-// Elements per thread of the compact kernel, and so per tile.  Inputs of kRelLargeInput elements and
-// more use kRelItemsLarge per thread, whose slot reads are all in flight together (33.5 M ids: 505 us
-// with 16, 510 with 8, more with 4); a small input is a few dependent reads long and wants many CTAs.
-// Look-back state is always sized for the small tile.
+// Elements per thread of the compact kernel, and so per tile.  Grids for kRelLargeInput elements and
+// more use kRelItemsLarge per thread (behind a hop of 1.5 M edges: 61 us with 4, 54 with 8, 57 with
+// 16); a small input is a few dependent reads long and wants many CTAs.  Look-back state is always
+// sized for the small tile.
 constexpr int kRelItems = 4;
-constexpr int kRelItemsLarge = 16;
+constexpr int kRelItemsLarge = 8;
 constexpr int64_t kRelLargeInput = 4 << 20;
 constexpr int kRelTile = kRelThreads * kRelItems;
 constexpr int kMaxParts = 8;
@@ -30,12 +30,14 @@ struct Parts {
 };
 
 // One 16-byte slot per distinct id, so that claiming the key and recording the first occurrence
-// touch one sector, as do reading the new id and emptying the slot.
+// touch one sector, as do reading the new id and emptying the slot.  The new id takes the place of
+// `first`, marked so that it is larger than any index: it needs no clearing for the next call.
 struct __align__(16) RelSlot {
-  long long key;   // -1 = empty
-  unsigned first;  // smallest input index holding the key (all ones = none)
-  unsigned newid;  // dense id of the key (written by the compact kernel; needs no initial value)
+  long long key;    // -1 = empty
+  unsigned first;   // smallest input index holding the key; kRelNewId and more: none yet
+  unsigned unused;  // all ones, always
 };
+constexpr unsigned kRelNewId = 0x80000000u;  // indexes and new ids stay below 2^30
 
 struct RelTable {
   RelSlot* slots;  // cap entries
@@ -91,7 +93,6 @@ __device__ __forceinline__ uint32_t relabel_unpack(const void* slot_of, bool is6
 struct RelRange {
   RelSlot* slots;
   uint32_t near, full;  // even
-  bool direct;  // every id of the input lies in [0, near): the id itself is its slot, nothing collides
 };
 constexpr uint32_t kRelNearProbes = 128;
 
@@ -128,7 +129,6 @@ __device__ __forceinline__ long long relabel_cas(RelSlot* slot, long long key) {
 }
 
 __device__ __forceinline__ uint32_t relabel_home(const RelRange& t, long long key) {
-  if (t.direct) return (uint32_t)key;
   return __umulhi((uint32_t)(mix64((uint64_t)key) >> 32), t.near) & ~1u;
 }
 
@@ -180,7 +180,7 @@ __device__ __forceinline__ uint32_t relabel_claim(const RelRange& t, long long k
 // for the atomic's result: an element that lowers the index, or loses to a still smaller one, is
 // simply left among the candidates.
 __device__ __forceinline__ bool relabel_settle(const RelRange& t, uint32_t pos, unsigned seen, unsigned i) {
-  if (seen <= i) return false;
+  if (seen <= i) return false;  // a mark counts as no index
   atomicMin(&t.slots[pos].first, i);
   return true;
 }
@@ -196,7 +196,7 @@ uint64_t relabel_capacity(int64_t numel_bound);
 // of the ids (the fused sampling kernel), so only the compact and remap kernels run.
 // `post`: the compact kernel hands the result words to the host as soon as the unique count is
 // final, i.e. while the remap kernel is still to run (it produces neither sizes nor errors).
-// `survey`: zeroed device memory; when given, a first kernel looks the ids over and the insert
+// `survey`: zeroed device memory, with room for the flags behind it (see relabel_flag_kernel); when given, a first kernel looks the ids over and the insert
 // kernel uses as much of the table as they need (see relabel_survey_kernel).
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
                    int64_t* status, int64_t* result, cudaStream_t s, bool inserted = false,

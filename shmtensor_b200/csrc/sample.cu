@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
   const RelRange range{job.rel_slots,
                        relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
-                       job.rel_cap, false};
+                       job.rel_cap};
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
   auto enter = [&](int64_t i, IxT id) {
     unsigned seen;

@@ -201,6 +201,15 @@ def test_relabel_five_million_ids(capi, spread):
     capi.check_async()
 
 
+def mix64(x):
+    """The 64-bit finaliser of the survey's sample (csrc/common.cuh)."""
+    x = x ^ (x >> np.uint64(33))
+    x = x * np.uint64(0xff51afd7ed558ccd)
+    x = x ^ (x >> np.uint64(33))
+    x = x * np.uint64(0xc4ceb9fe1a85ec53)
+    return x ^ (x >> np.uint64(33))
+
+
 @pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 1, (4 << 20) + 4095])
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 def test_relabel_around_the_survey_and_tile_limits(capi, n, dtype):
@@ -226,12 +235,6 @@ def test_relabel_around_the_survey_and_tile_limits(capi, n, dtype):
 def test_relabel_when_the_survey_sees_far_too_few_ids(capi):
     """Ids picked so that none of them falls into the survey's sample: the part of the table meant
     for them holds almost none, and every id has to find its second home."""
-    def mix64(x):
-        x = x ^ (x >> np.uint64(33))
-        x = x * np.uint64(0xff51afd7ed558ccd)
-        x = x ^ (x >> np.uint64(33))
-        x = x * np.uint64(0xc4ceb9fe1a85ec53)
-        return x ^ (x >> np.uint64(33))
     n = (1 << 20) + 300
     x = np.random.default_rng(3).integers(1 << 30, 1 << 40, size=2 * n).astype(np.int64)
     x = x[mix64(x.astype(np.uint64)) >> np.uint64(62) != 0][:n]   # one id in four is sampled at this size
@@ -244,6 +247,52 @@ def test_relabel_when_the_survey_sees_far_too_few_ids(capi):
     uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(y).cuda()])
     wu, (wr,) = oracle.tensor_relabel([y])
     assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+
+
+@pytest.mark.parametrize("top_bits", [32, 43, 46, 47, 62])
+def test_relabel_in_half_size_slots(capi, top_bits):
+    """Two million distinct ids: up to 46 bits they are kept in half-size slots, beyond in ordinary ones;
+    repeats near and far, every id twice, then ids on which the table must be found clean."""
+    rng = np.random.default_rng(top_bits)
+    ids = np.unique(rng.integers(0, 1 << top_bits, size=2_100_000).astype(np.int64))
+    ids[-1] = (1 << top_bits) - 1
+    rng.shuffle(ids)
+    x = np.concatenate([ids, rng.permutation(ids)[:1_234_567], ids[:3]])
+    for part in (x, x[::-1].copy(), x[:1_500_001]):
+        uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(part).cuda()])
+        wu, (wr,) = oracle.tensor_relabel([part])
+        assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+    capi.check_async()
+
+
+def test_the_three_forms_of_the_table_follow_one_another(capi):
+    """Ordinary slots, a word per id (dense ids) and half-size slots share one table: calls of every
+    form after every other, on the same context, find it empty."""
+    rng = np.random.default_rng(31)
+    n = 2_000_000
+    dense = rng.integers(0, 1_900_000, size=n).astype(np.int64)
+    forms = [dense * 0x10000001 % (1 << 43), dense, dense * 0x3000000000001, rng.integers(0, 60_000, size=50_000) + (1 << 33)]
+    want = [oracle.tensor_relabel([x]) for x in forms]
+    for at in (0, 1, 2, 3, 1, 0, 3, 2, 1, 3, 0, 2, 0):
+        uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(forms[at]).cuda()])
+        assert np.array_equal(uniq.cpu().numpy(), want[at][0]) and np.array_equal(rel.cpu().numpy(), want[at][1][0]), at
+    capi.check_async()
+
+
+def test_relabel_when_half_size_slots_run_over(capi):
+    """The survey sees less than half of the distinct ids (the others evade its sample), so the
+    half-size slots are too few for all of them and some ids go to ordinary slots behind."""
+    rng = np.random.default_rng(12)
+    x = rng.integers(0, 1 << 42, size=16_000_000).astype(np.int64)
+    evading = x[mix64(x.astype(np.uint64)) >> np.uint64(61) != 0][:2_400_000]     # one in 8 is sampled at this size
+    x = np.concatenate([x[-1_400_000:], evading])
+    rng.shuffle(x)
+    x = np.concatenate([x, x[:1000]])
+    for _ in range(2):
+        uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(x).cuda()])
+        wu, (wr,) = oracle.tensor_relabel([x])
+        assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+    capi.check_async()
 
 
 def test_relabel_is_repeatable_and_idempotent(capi):
