@@ -268,7 +268,7 @@ struct RelView {
   }
 };
 
-__global__ void __launch_bounds__(kRelThreads, 6)
+__global__ void __launch_bounds__(kRelThreads, 7)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
                       const RelSurvey* __restrict__ survey) {
   pdl_prologue();
@@ -276,8 +276,8 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
   const int64_t numel = sizes.numel;
   const RelUse use = relabel_use(t, numel, survey);
   // One element per thread and step, its successor's id read ahead: more resident threads are worth
-  // more than more elements on their way per thread (33.5 M ids: 660 us, two elements per thread with
-  // twice the registers 1,150).
+  // more than more elements on their way per thread (33.5 M ids in ordinary slots: 660 us, two elements per thread with
+  // twice the registers 1,150; in half-size slots 480).
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   long long next = i < numel ? part_elem(ps, sizes, i) : 0;
@@ -502,7 +502,7 @@ relabel_total_kernel(int* counts, int n_tiles, int64_t* result, HostPost post) {
   }
 }
 
-__global__ void __launch_bounds__(kRelThreads, 5)
+__global__ void __launch_bounds__(kRelThreads, 4)
 relabel_number_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique,
                       const uint32_t* __restrict__ flags, const int* __restrict__ before,
                       const RelSurvey* __restrict__ survey) {
@@ -556,7 +556,7 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out) {
   pdl_prologue();
   const PartSizes sizes = resolve_sizes(ps);
   const int64_t numel = sizes.numel;
-  constexpr int U = 4;  // independent slot reads per thread in flight
+  constexpr int U = 2;  // independent slot reads per thread in flight
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < numel; i0 += U * stride) {
     uint32_t pos[U];
@@ -582,10 +582,10 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out) {
 }
 
 // The same for a surveyed input.
-__global__ void __launch_bounds__(kRelThreads)
+__global__ void __launch_bounds__(kRelThreads, 8)
 relabel_remap_large_kernel(RelTable t, int is64, int64_t numel, void* out, const RelSurvey* __restrict__ survey) {
   const RelView view(t, numel, survey);
-  constexpr int U = 4;  // independent slot reads per thread in flight
+  constexpr int U = 2;  // 33.5 M ids: 8 reads per thread (5 CTAs) 354 us, 4 (6 CTAs) 232, 2 (8 CTAs) 187, 1 200
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < numel; i0 += U * stride) {
     uint32_t pos[U];
