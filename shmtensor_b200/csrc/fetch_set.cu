@@ -98,6 +98,80 @@ __device__ __forceinline__ char* resolve_row(const RowJob& job, int64_t first, i
   return p;
 }
 
+// The table rows of the tiles a warp goes through, tile0, tile0 + stride, ..., looked up for as many
+// tiles as 32 lanes hold rows of, and while the ones before them are still being copied: a tile of 5
+// rows would leave 27 lanes of the probe idle and wait for its ids, then for its slots, every time.
+// (150,001 rows of 602 bytes: 41 -> 35 us with their lookup.  row_gather_bulk_kernel does without: rows
+// that are in L2 gained there, 134 -> 107 us for 1.2 M of 400 bytes, but its usual batches lost, 158 ->
+// 177: a steadier stream of reads between its writes is slower in HBM.)
+struct RowCursor {
+  int64_t tile0, stride, n_tiles;
+  int tiles;      // looked up together
+  int mine, row;  // the tile of those, and its row, that this lane looks up
+  int64_t at;     // first tile (counted along the warp's way) of those in `here`
+  char* here;
+  char* next;     // of the tiles behind them, once `ready`
+  int64_t next_id;
+  bool ready;
+
+  __device__ __forceinline__ int64_t index_of(const RowJob& job, int64_t from) const {
+    const int64_t tile = tile0 + (from + mine) * stride;
+    const int64_t i = tile * job.rows_per_tile + row;
+    return mine < tiles && tile < n_tiles && i < job.n ? i : -1;
+  }
+  __device__ __forceinline__ void fetch_ids(const RowJob& job, int64_t from) {
+    const int64_t i = index_of(job, from);
+    next_id = i >= 0 ? load_int(job.idx, job.idx64, i) : kEmptyKey;
+    ready = false;
+  }
+  __device__ __forceinline__ void resolve(const RowJob& job, int64_t from, int64_t slot_mask) {
+    next = nullptr;
+    ready = true;
+    if (tile0 + from * stride >= n_tiles) return;  // the same on every lane
+    const int64_t i = index_of(job, from);
+    int64_t v = -1;
+    if (job.mode == MODE_MAP)
+      v = warp_find(job.map, next_id, i >= 0);
+    else if (job.mode == MODE_MASK)
+      v = i >= 0 ? load_int(job.mask, job.mask64, i) : -1;
+    if (i >= 0) {
+      if (v >= 0) {
+        char* base = job.bases[v >> job.owner_shift];
+        if (base) next = base + (v & slot_mask) * job.row_bytes;
+      } else if (job.host) {
+        next = job.host + next_id * job.row_bytes;
+      }
+    }
+  }
+  __device__ __forceinline__ RowCursor(const RowJob& job, int64_t first_tile, int64_t stride_, int64_t slot_mask)
+      : tile0(first_tile), stride(stride_), at(0) {
+    const int lane = (int)(threadIdx.x & 31);
+    n_tiles = (job.n + job.rows_per_tile - 1) / job.rows_per_tile;
+    tiles = 32 / job.rows_per_tile;
+    mine = lane / job.rows_per_tile;
+    row = lane % job.rows_per_tile;
+    fetch_ids(job, 0);
+    resolve(job, 0, slot_mask);
+    here = next;
+    fetch_ids(job, tiles);
+  }
+  // The row of this lane in the k-th tile of the warp (nullptr: none); k goes up by one from call to call.
+  __device__ __forceinline__ char* row_of(const RowJob& job, int64_t k, int64_t slot_mask) {
+    if (k == at + tiles) {
+      if (!ready) resolve(job, k, slot_mask);
+      here = next;
+      at = k;
+      fetch_ids(job, k + tiles);
+    } else if (k == at + 1) {
+      resolve(job, at + tiles, slot_mask);  // its ids have been on their way for a tile
+    }
+    const int lane = (int)(threadIdx.x & 31);
+    const int from = (int)(k - at) * job.rows_per_tile + lane;
+    char* p = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(here), from & 31));
+    return lane < job.rows_per_tile ? p : nullptr;
+  }
+};
+
 // Set by a kernel whose bounded wait ran out; read (and cleared) by shmt_device_fault().
 __device__ int g_device_fault = 0;
 
@@ -332,11 +406,12 @@ row_gather_ragged_kernel(const RowJob job) {
   int start[STAGES];       // byte of this lane's slot at which its row starts
   uint32_t parity = 0;     // bit s: phase of stage s to wait for next
 
-  auto issue = [&](int64_t tile, int s) {
-    const int64_t first = tile * R;
-    const int rows = (int)min((int64_t)R, job.n - first);
-    const int64_t id = load_id(job, first, rows, lane);
-    const char* p = resolve_row(job, first, rows, lane, slot_mask, id);
+  int64_t tile = (int64_t)blockIdx.x * kRowWarps + warp;
+  if (tile >= n_tiles) return;
+  RowCursor cursor(job, tile, stride, slot_mask);
+  int64_t issued = 0;  // tiles of this warp
+  auto issue = [&](int s) {
+    const char* p = cursor.row_of(job, issued++, slot_mask);
     const int sh = (int)((uintptr_t)p & 15);
     const uint32_t bytes = p ? (uint32_t)(sh + rb + 15) & ~15u : 0u;
     const uint32_t total = __reduce_add_sync(full, bytes);
@@ -348,18 +423,17 @@ row_gather_ragged_kernel(const RowJob job) {
   };
 
   constexpr int D = STAGES - 1;
-  int64_t tile = (int64_t)blockIdx.x * kRowWarps + warp;
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < D; ++j)
-    if (tile + j * stride < n_tiles) issue(tile + j * stride, j);
+    if (tile + j * stride < n_tiles) issue(j);
   while (tile < n_tiles && ok) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) {
       if (tile >= n_tiles || !ok) break;
       const int64_t ahead = tile + D * stride;
       __syncwarp();  // every lane has read what the buffer filled next held
-      if (ahead < n_tiles) issue(ahead, (s + D) % STAGES);
+      if (ahead < n_tiles) issue((s + D) % STAGES);
       if (!mbar_wait_bounded(&s_bar[warp][s], (parity >> s) & 1u)) {
         atomicExch(&g_device_fault, 1);
         ok = false;
