@@ -60,7 +60,8 @@ def _check_contig(t: torch.Tensor, name: str) -> None:
 
 # torch's current stream of a device as the raw handle, without a Stream object around it (0.1 us
 # against 2.3): every call below asks for it
-_raw_stream = torch._C._cuda_getCurrentRawStream
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda idx: torch.cuda.current_stream(idx).cuda_stream)
 
 
 def _stream(device: torch.device) -> int:
