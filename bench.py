@@ -2008,7 +2008,7 @@ def run_scan_relabel(args) -> None:
                                   "what": "the same ids numbered 0 .. distinct-1 (ids as slots); the configured "
                                           "workload spreads its ids over 2^43 and is hashed"},
                     "roofline": {"bound": "hbm, rate of random 16-byte slot accesses (2 per id + 2 per distinct id)",
-                                 "kernel": "relabel_insert / relabel_compact / relabel_remap",
+                                 "kernel": "relabel_survey / insert / flag / total / number / remap_large / clear",
                                  "slot_accesses": n_acc,
                                  "achieved": round(n_acc / (t_rel * 1e-3) / 1e9, 3), "peak": round(slot_rate / 1e9, 3),
                                  "unit": "G accesses/s", "frac": round(n_acc / (t_rel * 1e-3) / slot_rate, 4),
@@ -2025,7 +2025,7 @@ def run_scan_relabel(args) -> None:
         "e2e": {"value": round((SR_SCAN_N + SR_IDS) / ((t32 + t_rel) * 1e-3), 1), "unit": "elements/s",
                 "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 8,
                 "note": "device-resident operands, as in their callers; relabel reads its unique count back"},
-        "gpu_launches": steps * 4})
+        "gpu_launches": steps * 8})  # one scan, seven relabel passes
     # the reference's own kernels on the same GPU (thrust inclusive scan, its three-pass relabel)
     try:
         from oracle import build_ref
