@@ -337,9 +337,8 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   const int64_t numel = sizes.numel;
   constexpr int kTile = kRelThreads * ITEMS;
   const int64_t n_tiles = (numel + kTile - 1) / kTile;
-  const int tile = take_tile(ticket, &s_tile);
-  if (tile >= n_tiles) {  // the grid is sized for the largest input the caller allows
-    if (numel == 0 && tile == 0 && threadIdx.x < 32) {
+  if (blockIdx.x >= n_tiles) {  // the grid is sized for the largest input the caller allows
+    if (numel == 0 && blockIdx.x == 0 && threadIdx.x < 32) {
       if (threadIdx.x == 0) {
         st_relaxed64(result, 0);
         __threadfence();
@@ -349,6 +348,7 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
     }
     return;
   }
+  const int tile = take_tile(ticket, &s_tile);  // as many CTAs as tiles are left
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t base = (int64_t)tile * kTile + (int64_t)warp * (32 * ITEMS) + lane;
   uint32_t pos[ITEMS];

@@ -230,9 +230,8 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   uint32_t* s_sets = reinterpret_cast<uint32_t*>(s_hit + S);
   const int64_t n = job.n_dev ? *job.n_dev : job.n;
   const int64_t n_tiles = (n + S - 1) / S;
-  const int tile = take_tile(job.ticket, &s_tile);
-  if (tile >= n_tiles) {  // the grid is sized for the largest n the caller allows
-    if (n == 0 && tile == 0 && tid < 32) {
+  if (blockIdx.x >= n_tiles) {  // the grid is sized for the largest n the caller allows
+    if (n == 0 && blockIdx.x == 0 && tid < 32) {
       if (tid == 0) {
         store_int(job.sub_indptr, job.indptr64, 0, 0);
         st_relaxed64(job.result, 0);
@@ -243,6 +242,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     }
     return;
   }
+  const int tile = take_tile(job.ticket, &s_tile);  // as many CTAs as tiles are left
   if (job.clean && tile == 0 && tid == 0) st_relaxed64(job.status, DEV_OK);  // it reports on this call only
   const int64_t first = (int64_t)tile * S;
   const int rows = (int)min((int64_t)S, n - first);
