@@ -429,12 +429,13 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
         __threadfence();
       }
       if (__shfl_sync(full, (int)last, 0)) {
-        post_to_host(job.post);
         for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
         if (lane == 0) {
           st_relaxed64(job.ticket, 0);
           st_relaxed64(job.clean, 0);
         }
+        // only now: the host may queue the state's next user in another stream as soon as it has the post
+        post_to_host(job.post);
       }
     }
   }
@@ -841,7 +842,8 @@ static int sample_hop_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   const int64_t n_tiles = (n + job.seeds_per_tile - 1) / job.seeds_per_tile;
   job.n_dev = nullptr;
   // Up to kSmallScanTiles tiles use look-back state that the kernel leaves at zero: no memset in front
-  // (2 us and a gap on the GPU), and nothing behind the post that the scratch's next user waits for.
+  // (2 us and a gap on the GPU), and nothing behind the post that the scratch's next user waits for:
+  // the state is zero again before the post, and what follows it writes the caller's outputs only.
   const bool small = n_tiles <= kSmallScanTiles;
   int64_t* done = nullptr;
   if (small) {

@@ -80,3 +80,54 @@ def test_minibatches_on_two_streams_at_once():
             wu, (wr,) = oracle.tensor_relabel([hops[-1][1]])
             assert np.array_equal(uniq, wu) and np.array_equal(rel, wr)
     assert capi.device_fault() == 0
+
+
+@pytest.mark.parametrize("n", [1, 600, 4096])
+def test_one_context_goes_from_stream_to_stream(n):
+    """A hop hands its result to the host before its kernel ends.  What follows on another stream with
+    the same context (up to 512 tiles share look-back state that every kernel leaves at zero) finds
+    that state clean: 300 hops on two streams in turn, scans and relabels in between."""
+    import ctypes as C
+
+    from shmtensor_b200 import _lib
+    lib, check = _lib.lib, _lib.check
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(n)
+    indptr_n, indices_n = _graph(rng, 20_000, 30)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    k, rounds = 10, 300
+    seeds_n = rng.integers(0, 20_000, size=n)
+    seeds = torch.from_numpy(seeds_n).cuda()
+    want = np.concatenate([[0], np.cumsum(np.minimum(indptr_n[seeds_n + 1] - indptr_n[seeds_n], k))])
+    sub_indptr = torch.empty(rounds, n + 1, dtype=torch.int64, device="cuda")
+    sub_indices = torch.empty(rounds, n * k, dtype=torch.int32, device="cuda")
+    unique, relabel = torch.empty(n, dtype=torch.int64, device="cuda"), torch.empty(n, dtype=torch.int64, device="cuda")
+    ones = torch.ones(20_001, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    ctx, got = C.c_void_p(), C.c_int64()
+    check(lib.shmt_ctx_create(0, C.byref(ctx)))
+    try:
+        for i in range(rounds):
+            s = streams[i & 1].cuda_stream
+            check(lib.shmt_sample_hop(ctx, indptr.data_ptr(), _lib.I64, indices.data_ptr(), _lib.I32, None, None, None,
+                                      seeds.data_ptr(), _lib.I64, n, k, 0, 7, i, sub_indptr[i].data_ptr(),
+                                      sub_indices[i].data_ptr(), C.byref(got), s))
+            assert got.value == want[-1], i
+            if i % 3 == 2:
+                other = streams[~i & 1]
+                check(lib.shmt_relabel(ctx, (C.c_void_p * 1)(seeds.data_ptr()), (C.c_int64 * 1)(n), 1, _lib.I64,
+                                       unique.data_ptr(), relabel.data_ptr(), C.byref(got), other.cuda_stream))
+                assert got.value == np.unique(seeds_n).size, i
+                with torch.cuda.stream(other):
+                    ones.fill_(1)
+                check(lib.shmt_scan(ctx, ones.data_ptr(), _lib.I32, ones.numel(), 0, other.cuda_stream))
+                check(lib.shmt_ctx_check(ctx, other.cuda_stream))
+                assert ones[-1].item() == ones.numel(), i
+        torch.cuda.synchronize()
+    finally:
+        lib.shmt_ctx_destroy(ctx)
+    assert np.array_equal(sub_indptr.cpu().numpy(), np.broadcast_to(want, (rounds, n + 1)))
+    for i in (0, 1, rounds - 1):
+        oracle.check_sample_bulk(indptr_n, indices_n, seeds_n, k, False, sub_indptr[i].cpu().numpy(),
+                                 sub_indices[i, :want[-1]].cpu().numpy(), distinct_rows=True)
