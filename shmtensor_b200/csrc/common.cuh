@@ -104,6 +104,10 @@ __device__ __forceinline__ int64_t ld_relaxed64(const int64_t* p) {
 __device__ __forceinline__ void st_relaxed64(int64_t* p, int64_t v) {
   asm volatile("st.relaxed.gpu.global.s64 [%0], %1;" ::"l"(p), "l"((long long)v) : "memory");
 }
+// for the host to see, with everything that happened before it
+__device__ __forceinline__ void st_release_sys64(int64_t* p, int64_t v) {
+  asm volatile("st.release.sys.global.s64 [%0], %1;" ::"l"(p), "l"((long long)v) : "memory");
+}
 
 // 16-byte streaming accesses: rows are touched once per call, so keep them out
 // of L1 and mark them evict-first in L2 on the store side.

@@ -61,15 +61,32 @@ struct HostPost {
 #ifdef __CUDACC__
 // Called by a whole warp: a word per lane.  One thread copying word by word took 0.6 us for each (the
 // next load waits behind the store of the one before), 17 us for the sizes of a three-hop mini-batch,
-// all of it on the way to the host.
+// all of it on the way to the host.  The words are final for every lane (behind a barrier, or a fence
+// and a __syncwarp).  The sequence number is a release at system scope by one lane, behind a
+// __syncwarp: it carries the words of all lanes to the host.
 __device__ __forceinline__ void post_to_host(const HostPost& p) {
   if (!p.host) return;
   const unsigned lane = threadIdx.x & 31;
   for (int i = (int)lane; i < p.n_words; i += 32)
     *reinterpret_cast<volatile int64_t*>(p.host + i) = ld_relaxed64(p.words + i);
-  __threadfence_system();
   __syncwarp();
-  if (lane == 0) *reinterpret_cast<volatile int64_t*>(p.host + p.flag_at) = p.seq;
+  if (lane == 0) st_release_sys64(p.host + p.flag_at, p.seq);
+}
+
+// True on every lane of the calling warp if its CTA is the last of `n_ctas` to count itself out at `done`
+// (zero when the kernel starts).  What the other CTAs did before they counted themselves out, as far
+// as their calling warp had seen it (a CTA-wide barrier before the call), has then happened for every lane:
+// fences around one lane's atomic, and a __syncwarp, for a shuffle orders no memory.
+__device__ __forceinline__ bool last_to_finish(int64_t* done, int64_t n_ctas) {
+  unsigned long long before = 0;
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    before = atomicAdd(reinterpret_cast<unsigned long long*>(done), 1ULL);
+    __threadfence();
+  }
+  before = __shfl_sync(0xffffffffu, before, 0);
+  __syncwarp();
+  return (int64_t)before + 1 == n_ctas;
 }
 
 // Called by one warp of each of the `n_ctas` CTAs that produce results, after a CTA-wide
@@ -77,13 +94,7 @@ __device__ __forceinline__ void post_to_host(const HostPost& p) {
 // sees every CTA's words.
 __device__ __forceinline__ void post_when_last(const HostPost& p, int64_t n_ctas) {
   if (!p.host) return;
-  unsigned long long before = 0;
-  if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    before = atomicAdd(reinterpret_cast<unsigned long long*>(p.done), 1ULL);
-    __threadfence();
-  }
-  if ((int64_t)__shfl_sync(0xffffffffu, before, 0) + 1 == n_ctas) post_to_host(p);
+  if (last_to_finish(p.done, n_ctas)) post_to_host(p);
 }
 #endif
 

@@ -384,3 +384,27 @@ def test_tiles_of_eight_seeds_fused_and_hop_by_hop(capi, n_seeds, k):
     assert torch.equal(fp, p) and torch.equal(fx, x) and torch.equal(fe, e)
     wu, (_, wx) = oracle.tensor_relabel([seeds_n, x.cpu().numpy()])
     assert np.array_equal(frontier.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
+
+
+@pytest.mark.parametrize("n_hops", [1, 4, 8])
+def test_sizes_handed_over_by_a_warp_for_one_to_eight_hops(capi, n_hops):
+    """The sizes of a mini-batch (16 to 72 words, up to three per lane) reach the host ahead of the end
+    of its last kernel: over 100 calls they always describe the outputs."""
+    rng = np.random.default_rng(n_hops)
+    deg = rng.integers(0, 6, size=5000)
+    indptr_n = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    indices_n = rng.integers(0, 5000, size=int(indptr_n[-1])).astype(np.int32)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    batches = []
+    for i in range(100):
+        seeds_n = rng.permutation(5000)[:1 + 3 * i].astype(np.int32)
+        batches.append((seeds_n, capi.sample_minibatch(indptr, indices, torch.from_numpy(seeds_n).cuda(), [1] * n_hops, False)))
+    for seeds_n, (front, hops) in batches:
+        cur = seeds_n
+        for sp, sx, rel, nxt in hops:
+            sp, sx = sp.cpu().numpy(), sx.cpu().numpy()
+            oracle.check_sample_bulk(indptr_n, indices_n, cur, 1, False, sp, sx)
+            wu, (_, wx) = oracle.tensor_relabel([cur, sx])
+            assert np.array_equal(nxt.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
+            cur = wu
+        assert np.array_equal(front.cpu().numpy(), cur)
