@@ -421,22 +421,14 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   }
   if (job.clean) {  // uniform as well; all look-backs of this CTA are over
     if (!job.post.host) __syncthreads();
-    if (tid < 32) {
-      bool last = false;
+    if (tid < 32 && last_to_finish(job.clean, n_tiles)) {
+      for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
       if (lane == 0) {
-        __threadfence();
-        last = atomicAdd(reinterpret_cast<unsigned long long*>(job.clean), 1ULL) + 1 == (unsigned long long)n_tiles;
-        __threadfence();
+        st_relaxed64(job.ticket, 0);
+        st_relaxed64(job.clean, 0);
       }
-      if (__shfl_sync(full, (int)last, 0)) {
-        for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
-        if (lane == 0) {
-          st_relaxed64(job.ticket, 0);
-          st_relaxed64(job.clean, 0);
-        }
-        // only now: the host may queue the state's next user in another stream as soon as it has the post
-        post_to_host(job.post);
-      }
+      // only now: the host may queue the state's next user in another stream as soon as it has the post
+      post_to_host(job.post);
     }
   }
 

@@ -54,6 +54,28 @@ def test_scan_tile_edges_views_and_many_tiles(capi, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_small_scans_leave_their_state_clean_for_the_next(capi, dtype):
+    """Scans of up to 512 tiles use look-back state that the CTA ending last puts back to zero: 400 scans
+    queued in a row, from one tile to 512 and back, a tile more or less at a time, each against cumsum."""
+    item = 4 if dtype == torch.int32 else 8
+    per16k, per64k = 16384 // item, 65536 // item
+    top = 512 * per64k if item == 4 else 511 * per64k
+    g = torch.Generator(device="cuda").manual_seed(item)
+    src = torch.randint(-1000, 1000, (top,), generator=g, device="cuda").to(dtype)
+    want = torch.cumsum(src, 0, dtype=dtype)
+    sizes = [top, 1, 2 * per16k, per16k, 296 * per16k, 296 * per16k + 1, 296 * 2 * per16k, 296 * 2 * per16k + 1]
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(400):
+        n = sizes[i % len(sizes)] if i % 2 else 1 + i * per16k
+        n = min(n, top)
+        work = src[:n].clone()
+        capi.thrust_scan(work)
+        wrong += (work != want[:n]).sum()
+    capi.check_async()
+    assert wrong.item() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 def test_scan_large_inputs_through_the_cluster_kernel(capi, dtype):
     """From 32 MB on, whole 256 KB super-tiles go through the persistent cluster kernel and the
     rest through the ticketed one, which carries on from the last super-tile's sum: lengths at and
