@@ -241,7 +241,8 @@ int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, 
   SHMT_REQUIRE(scratch_bytes >= 0 && relabel_ids >= 0 && relabel_ids < ((int64_t)1 << 30),
                "shmt_ctx_reserve: sizes out of range");
   DeviceGuard guard(ctx->device);
-  if (int rc = ctx_reserve(ctx, (size_t)scratch_bytes)) return rc;
+  const size_t relabel = relabel_scratch_bytes(relabel_ids);
+  if (int rc = ctx_reserve(ctx, (size_t)scratch_bytes > relabel ? (size_t)scratch_bytes : relabel)) return rc;
   if (relabel_ids > 0) {
     if (int rc = ctx_reserve_table(ctx, relabel_capacity(relabel_ids) * sizeof(RelSlot),
                                    static_cast<cudaStream_t>(stream)))

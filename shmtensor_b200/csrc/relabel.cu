@@ -746,6 +746,25 @@ uint64_t relabel_capacity(int64_t numel_bound) {
   return cap;
 }
 
+// Where a call of `numel` ids keeps what: look-back descriptors, or, when it is surveyed, the survey and
+// the flags behind it.
+struct RelScratch {
+  bool look;           // a table that fits the L2 cache gains nothing from compact slots; a larger one may
+  size_t zeroed;       // bytes that start at zero; the survey lies behind `states` of them
+  size_t states, all;
+};
+static RelScratch relabel_scratch(int64_t numel) {
+  RelScratch r{};
+  if (numel <= kRelSmallMax) return r;  // one CTA, all in shared memory
+  const int64_t n_tiles = (numel + kRelTile - 1) / kRelTile;
+  r.look = relabel_capacity(numel) * sizeof(RelSlot) > kRelSurveyMinTableBytes;
+  r.states = (tile_state_bytes(n_tiles) + 255) & ~(size_t)255;
+  r.zeroed = r.look ? r.states + sizeof(RelSurvey) : tile_state_bytes(n_tiles);
+  r.all = r.zeroed + (r.look ? flag_bytes(numel) : 0);
+  return r;
+}
+size_t relabel_scratch_bytes(int64_t numel) { return relabel_scratch(numel).all; }
+
 int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s) {
   const uint64_t cap = relabel_capacity(numel_bound);
   if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s)) return rc;
@@ -849,16 +868,12 @@ extern "C" int shmt_relabel(shmt_ctx* ctx, const void* const* parts, const int64
     *n_unique_host = ctx->h_words[W_RESULT];
     return SHMT_OK;
   }
-  const int64_t n_tiles = (numel + kRelTile - 1) / kRelTile;
-  const size_t states = (tile_state_bytes(n_tiles) + 255) & ~(size_t)255;
-  // a table that fits the L2 cache gains nothing from compact slots; a larger one may
-  const bool look = relabel_capacity(numel) * sizeof(RelSlot) > kRelSurveyMinTableBytes;
-  const size_t zeroed = look ? states + sizeof(RelSurvey) : tile_state_bytes(n_tiles);
-  if (int rc = ctx_reserve(ctx, zeroed + (look ? flag_bytes(numel) : 0))) return rc;
-  TileStates st = carve_tile_states(ctx->region(), n_tiles);
-  RelSurvey* survey = look ? reinterpret_cast<RelSurvey*>(ctx->region() + states) : nullptr;
+  const RelScratch at = relabel_scratch(numel);
+  if (int rc = ctx_reserve(ctx, at.all)) return rc;
+  TileStates st = carve_tile_states(ctx->region(), (numel + kRelTile - 1) / kRelTile);
+  RelSurvey* survey = at.look ? reinterpret_cast<RelSurvey*>(ctx->region() + at.states) : nullptr;
   // result words, tile descriptors and the survey to zero
-  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + zeroed, s));
+  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + at.zeroed, s));
   int64_t* w = ctx->d_words();
   // with a count to return, the compact kernel posts it and the call returns while the remap
   // kernel runs; the next user of the context waits for that kernel first

@@ -189,6 +189,9 @@ __device__ __forceinline__ bool relabel_settle(const RelRange& t, uint32_t pos, 
 // Slots of the table that serves up to `numel_bound` ids.
 uint64_t relabel_capacity(int64_t numel_bound);
 
+// Context scratch that shmt_relabel takes for up to `numel` ids.
+size_t relabel_scratch_bytes(int64_t numel);
+
 // Queue the three relabel kernels.  `numel_bound` >= the real element count sizes the
 // table and the grids; ticket/status/result are zeroed device words.
 // `pdl`: launch with programmatic stream serialization (see pdl_prologue in common.cuh).

@@ -377,3 +377,30 @@ def test_relabel_in_one_cta_and_just_beyond(capi, n, dtype):
         wu, (wr,) = oracle.tensor_relabel([x])
         assert uniq.dtype == dtype and np.array_equal(uniq.cpu().numpy(), wu)
         assert np.array_equal(torch.cat(rel).cpu().numpy(), wr)
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 1 << 20, (1 << 20) + 1, 8_000_001])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_a_reserved_context_relabels_without_allocating(capi, n, sparse):
+    """shmt_ctx_reserve(relabel_ids) covers all that a relabel of so many ids takes (table, look-back
+    state and, above 2^20 ids, the survey and a flag bit per id), and of fewer."""
+    import ctypes as C
+
+    from shmtensor_b200 import _lib
+    lib, check = _lib.lib, _lib.check
+    stream = torch.cuda.current_stream().cuda_stream
+    x = torch.randint(0, n // 2 + 1, (n,), device="cuda") * (0x10000001 if sparse else 1)
+    unique, relabel = torch.empty_like(x), torch.empty_like(x)
+    ctx, got = C.c_void_p(), C.c_int64()
+    check(lib.shmt_ctx_create(0, C.byref(ctx)))
+    try:
+        check(lib.shmt_ctx_reserve(ctx, 0, n, stream))
+        reserved = lib.shmt_ctx_scratch_bytes(ctx)
+        for m in (n, n // 2 + 1, 1000, n):
+            check(lib.shmt_relabel(ctx, (C.c_void_p * 1)(x.data_ptr()), (C.c_int64 * 1)(m), 1, _lib.I64,
+                                   unique.data_ptr(), relabel.data_ptr(), C.byref(got), stream))
+            assert lib.shmt_ctx_scratch_bytes(ctx) == reserved, m
+            assert torch.equal(unique[:got.value][relabel[:m]], x[:m])
+            assert got.value == torch.unique(x[:m]).numel()
+    finally:
+        lib.shmt_ctx_destroy(ctx)
