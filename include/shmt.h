@@ -51,8 +51,9 @@ int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx);
  * allocate device memory (which stalls the device): at least scratch_bytes of look-back state
  * (16 bytes per tile; a scan of n items of 8 bytes needs n / 512 bytes), and what relabel calls of up
  * to relabel_ids ids take, their scratch and their table.  shmt_ctx_reserve_minibatch sizes both
- * for shmt_sample_minibatch calls of up to n_seeds seeds with these fan-outs.  No counterpart in
- * the reference, which allocates temporaries on every call (src/cache_graph_sampling.cu:50-56).   */
+ * for shmt_sample_minibatch calls, weighted or not, of up to n_seeds seeds with these fan-outs.
+ * No counterpart in the reference, which allocates temporaries on every call
+ * (src/cache_graph_sampling.cu:50-56).                                                     */
 int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, void* stream);
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                int n_hops, void* stream);

@@ -771,10 +771,13 @@ extern "C" {
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts, int n_hops,
                                void* stream) {
   SHMT_REQUIRE(ctx != nullptr, "shmt_ctx_reserve_minibatch: ctx is null");
-  MinibatchPlan plan;
+  // weighted hops without replacement have the smaller tiles, and so the more descriptors, of the two
+  MinibatchPlan plan, weighted;
   if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &plan)) return rc;
+  if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &weighted, /*weighted=*/true)) return rc;
   DeviceGuard guard(ctx->device);
-  if (int rc = ctx_reserve(ctx, plan.scratch_bytes)) return rc;
+  if (int rc = ctx_reserve(ctx, weighted.scratch_bytes > plan.scratch_bytes ? weighted.scratch_bytes : plan.scratch_bytes))
+    return rc;
   RelTable t;
   return relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream));
 }

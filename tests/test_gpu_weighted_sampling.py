@@ -188,3 +188,25 @@ def test_rows_around_the_length_that_a_whole_cta_shares(capi, deg, k):
                 assert set(got.tolist()) == set(heavy[row].tolist())
             if degs[row] <= k:
                 assert np.array_equal(got, np.arange(int(indptr[row]), int(indptr[row + 1])))
+
+
+@pytest.mark.parametrize("replace", [False, True])
+def test_a_reserved_context_samples_weighted_batches_without_allocating(replace):
+    """capi.reserve_minibatch covers weighted hops too, whose tiles hold at most 64 seeds where others
+    hold up to 256: look-back state of 62,500 tiles for 4,000,000 seeds."""
+    from shmtensor_b200 import capi
+    n = 4_000_000
+    indptr = torch.arange(1001, device="cuda") * 4
+    indices = torch.arange(4000, device="cuda", dtype=torch.int32) % 1000
+    weights = torch.rand(4000, device="cuda") + 0.1
+    seeds = torch.arange(n, device="cuda", dtype=torch.int32) % 1000
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+        capi.reserve_minibatch(n, [2])
+        reserved = capi.context_scratch_bytes()
+        front, [(sp, sx, rel, _)] = capi.sample_minibatch(indptr, indices, seeds, [2], replace, weights=weights)
+        assert capi.context_scratch_bytes() == reserved
+        capi.sample_minibatch(indptr, indices, seeds, [2], replace)
+        assert capi.context_scratch_bytes() == reserved
+    torch.cuda.synchronize()
+    assert sx.numel() == 2 * n and torch.equal(front[rel.long()], sx)
