@@ -17,10 +17,9 @@
 // after another with 4-byte accesses and probe the map redundantly on 32 lanes.
 #include <stdlib.h>
 
-#include <atomic>
-
 #include "bulk.cuh"
 #include "ctx.cuh"
+#include "kept.h"
 #include "map.cuh"
 
 namespace shmt {
@@ -633,18 +632,16 @@ static int pick_rows_per_tile(int64_t n) {
 
 // Persistent grid: never more CTAs than are resident at once (tiles are dealt round-robin
 // inside the kernels), so there is no partly filled last wave.  The occupancy of a kernel with so
-// much shared memory is asked for once (1 us, a fifth of a small call) and kept beside the kernel.
+// much shared memory is asked for once per device (1 us, a fifth of a small call) and kept beside the kernel.
 template <typename Kernel>
-static unsigned grid_for_tiles(Kernel kernel, std::atomic<uint64_t>* kept, int64_t n, int R, size_t smem = 0) {
+static unsigned grid_for_tiles(Kernel kernel, KeptOccupancy* kept, int64_t n, int R, size_t smem = 0) {
   const int64_t tiles = (n + R - 1) / R;
   int64_t blocks = (tiles + kRowWarps - 1) / kRowWarps;
-  const uint64_t have = kept->load(std::memory_order_relaxed);  // smem | CTAs per SM, 0 = not asked yet
-  int occ = (int)(have & 0xFF);
-  if (occ == 0 || (have >> 8) != smem) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRowThreads, smem) != cudaSuccess || occ < 1)
-      occ = 1;
-    kept->store(((uint64_t)smem << 8) | (uint64_t)occ, std::memory_order_relaxed);
-  }
+  int dev = -1;
+  cudaGetDevice(&dev);
+  const int occ = kept->get(dev, smem, [&](int* ctas) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, kRowThreads, smem) == cudaSuccess;
+  });
   const int64_t resident = (int64_t)sm_count() * occ;
   if (blocks > resident) blocks = resident;
   return (unsigned)(blocks < 1 ? 1 : blocks);
@@ -652,7 +649,7 @@ static unsigned grid_for_tiles(Kernel kernel, std::atomic<uint64_t>* kept, int64
 
 template <int VEC, bool SET>
 static int launch_lsu(const RowJob& job, cudaStream_t s) {
-  static std::atomic<uint64_t> kept{0};
+  static KeptOccupancy kept;
   const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, job.n, job.rows_per_tile);
   row_copy_kernel<VEC, SET, 8><<<grid, kRowThreads, 0, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
@@ -693,7 +690,7 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   }
   job.rows_per_tile = R;
   const size_t smem = (size_t)kRowWarps * kBulkStages * R * job.row_bytes;
-  static std::atomic<uint64_t> kept{0};
+  static KeptOccupancy kept;
   const unsigned blocks = grid_for_tiles(kernel, &kept, job.n, R, smem);
   kernel<<<blocks, kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
@@ -736,7 +733,7 @@ static int launch_ragged(RowJob job, int R, cudaStream_t s) {
   }
   job.rows_per_tile = R;
   const size_t smem = ragged_smem_bytes(job.row_bytes, R);
-  static std::atomic<uint64_t> kept{0};
+  static KeptOccupancy kept;
   kernel<<<grid_for_tiles(kernel, &kept, job.n, R, smem), kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -895,7 +892,7 @@ int shmt_insert_set(shmt_map* map, void* gpu_base, const void* keys, int key_dty
   DeviceGuard guard(map->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int R = pick_rows_per_tile(n);
-  static std::atomic<uint64_t> kept{0};
+  static KeptOccupancy kept;
   const unsigned grid = grid_for_tiles(insert_set_kernel<16, 8>, &kept, n, R);
   const int vec = pick_vec(row_bytes, {gpu_base, update});
   char* g = static_cast<char*>(gpu_base);
