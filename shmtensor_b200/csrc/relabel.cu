@@ -189,7 +189,10 @@ __device__ __forceinline__ RelUse relabel_use(const RelTable& t, int64_t numel, 
   int id_bits = 64 - __clzll((long long)survey->largest);
   if (id_bits < quad_bits) id_bits = quad_bits;
   if (id_bits - quad_bits > kHalfRemainderBits) return u;
-  const uint32_t n = 4u << quad_bits, rest = t.cap - n / 2;  // rest: enough for what n places cannot hold
+  // The ordinary slots behind the n places would hold every id of the call, whatever the survey saw and wherever
+  // the homes lie: cap / 2 is a power of two P >= numel, and n / 2, a power of two below 1.6 * numel, is
+  // at most P, so that cap - n / 2 >= numel.
+  const uint32_t n = 4u << quad_bits, rest = t.cap - n / 2;
   u.small = RelSmall{reinterpret_cast<unsigned*>(t.slots), n, 2, id_bits, quad_bits,
                      RelRange{t.slots + n / 2, rest, rest}};
   return u;

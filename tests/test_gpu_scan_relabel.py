@@ -317,6 +317,31 @@ def test_relabel_when_half_size_slots_run_over(capi):
     capi.check_async()
 
 
+def unmix_bits(x, bits):
+    """The inverse of the mix that gives half-size slots their homes (csrc/relabel.cu, mix_bits)."""
+    mask, half = np.uint64((1 << bits) - 1), np.uint64((bits + 1) // 2)
+    x = x ^ (x >> half)
+    for factor in (0xc4ceb9fe1a85ec53, 0xff51afd7ed558ccd):
+        x = (x * np.uint64(pow(factor, -1, 1 << bits))) & mask
+        x = x ^ (x >> half)
+    return x
+
+
+def test_relabel_of_ids_made_against_the_half_size_slots(capi):
+    """1.5 million distinct ids of 46 bits that all have the same home: 124 fill the places near it, every
+    other one goes on to the ordinary slots behind, which hold as many ids as the call has."""
+    rng = np.random.default_rng(5)
+    low = np.unique(rng.integers(0, 1 << 26, size=1_600_000).astype(np.uint64))[:1_500_000]
+    ids = unmix_bits((np.uint64(12_345) << np.uint64(26)) | low, 46).astype(np.int64)   # 2^20 homes
+    assert ids.size == 1_500_000 and int(ids.max()).bit_length() == 46
+    rng.shuffle(ids)
+    x = np.concatenate([ids, ids[:30_000]])
+    for part in (x, x[:1_400_000]):
+        uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(part).cuda()])
+        wu, (wr,) = oracle.tensor_relabel([part])
+        assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+
+
 def test_relabel_is_repeatable_and_idempotent(capi):
     g = torch.Generator(device="cuda").manual_seed(1)
     x = torch.randint(0, 100_000, (500_000,), generator=g, device="cuda")
