@@ -192,8 +192,9 @@ int shmt_scan_static_check(void* stream);
 
 /* Test hook for the failure path of every look-back scan: runs one warp whose predecessor
  * tile never publishes, with a short spin limit, and returns what the host sees --
- * SHMT_ERR_TIMEOUT -- leaving the context usable.  Nothing faults, traps or hangs.
- * No counterpart in the reference.                                                    */
+ * SHMT_ERR_TIMEOUT -- leaving the context usable.  The relabel table, if the context has one,
+ * is left with an index in every slot, as a call that failed halfway may leave it.  Nothing
+ * faults, traps or hangs.  No counterpart in the reference.                            */
 int shmt_debug_lookback_timeout(shmt_ctx* ctx, void* stream);
 
 /* ---- relabel ---------------------------------------------------------------

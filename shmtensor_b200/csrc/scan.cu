@@ -3,11 +3,13 @@
 // Semantics follow cub_exclusiveSum (reference src/cache_graph_sampling.cu:30-45)
 // and the intended meaning of thrust_scan (reference src/thrust_scan.cu:9-18,
 // whose own lambda races); integer arithmetic wraps.
+#include <stddef.h>
 #include <stdlib.h>
 
 #include "bulk.cuh"
 #include "ctx.cuh"
 #include "lookback.cuh"
+#include "relabel.cuh"
 
 namespace shmt {
 
@@ -661,6 +663,9 @@ extern "C" int shmt_debug_lookback_timeout(shmt_ctx* ctx, void* stream) {
   SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + tile_state_bytes(2), s));
   lookback_timeout_probe_kernel<<<1, 32, 0, s>>>(st, ctx->d_words(), 1 << 10);
   SHMT_CUDA_TRY(cudaGetLastError());
+  if (ctx->table)  // index 0 in every slot of the relabel table
+    SHMT_CUDA_TRY(cudaMemset2DAsync(ctx->table + offsetof(RelSlot, first), sizeof(RelSlot), 0, sizeof(RelSlot::first),
+                                    ctx->table_bytes / sizeof(RelSlot), s));
   return ctx_fetch_words(ctx, s, "shmt_debug_lookback_timeout");
 }
 

@@ -368,10 +368,17 @@ def test_relabel_errors(capi):
     assert u.numel() == 0 and r.numel() == 0
 
 
-def test_lookback_wait_is_bounded_and_reported(capi):
-    """A look-back whose predecessor never publishes gives up after its spin limit: the host
-    gets SHMT_ERR_TIMEOUT, and the same context keeps working afterwards."""
+@pytest.mark.parametrize("n, step", [(5000, 1), (1_200_000, 1), (1_200_000, 0x10000001)])
+def test_lookback_wait_is_bounded_and_reported(capi, n, step):
+    """A look-back whose predecessor never publishes gives up after its spin limit: the host gets
+    SHMT_ERR_TIMEOUT, and the same context keeps working afterwards.  The relabel table, which the failed
+    call leaves with an index in every slot, is empty again for the next call, whichever form of it that
+    uses (ordinary slots, a word per id, slots of ids spread wide)."""
     from shmtensor_b200 import _lib
+    x = np.random.default_rng(n).integers(0, n // 3, size=n).astype(np.int64) * step
+    wu, (wr,) = oracle.tensor_relabel([x])
+    ids = torch.from_numpy(x).cuda()
+    capi.tensor_relabel([ids])                                                # the context has its table
     dev = torch.device("cuda", torch.cuda.current_device())
     ctx = capi._ctx(dev)
     rc = _lib.lib.shmt_debug_lookback_timeout(ctx, torch.cuda.current_stream().cuda_stream)
@@ -380,8 +387,10 @@ def test_lookback_wait_is_bounded_and_reported(capi):
     capi.thrust_scan(a)
     capi.check_async()
     assert a[-1].item() == 50_005_000
-    u, (r,) = capi.tensor_relabel([torch.tensor([7, 7, 3], device="cuda")])   # table was re-cleaned
+    u, (r,) = capi.tensor_relabel([torch.tensor([7, 7, 3], device="cuda")])   # in one CTA, without the table
     assert u.cpu().tolist() == [7, 3] and r.cpu().tolist() == [0, 0, 1]
+    u, (r,) = capi.tensor_relabel([ids])                                      # table was re-cleaned
+    assert np.array_equal(u.cpu().numpy(), wu) and np.array_equal(r.cpu().numpy(), wr)
 
 
 @pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097])
