@@ -196,14 +196,15 @@ int shmt_ctx_create(int device, shmt_ctx** out) {
     delete ctx;
     return rc;
   }
+  // zero before any stream's first scan; in a stream of its own, which waits for nobody's work (the
+  // per-thread stream would wait for all that is queued in the default stream)
   void* scan_state = nullptr;
+  cudaStream_t own = nullptr;
   e = cudaMalloc(&scan_state, kScanStateBytes);
-  if (e == cudaSuccess) {
-    ctx->scan_state = static_cast<char*>(scan_state);
-    // zero before any stream's first scan
-    e = cudaMemsetAsync(scan_state, 0, kScanStateBytes, cudaStreamPerThread);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamPerThread);
-  }
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(scan_state, 0, kScanStateBytes, own);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+  if (own) cudaStreamDestroy(own);
   if (e != cudaSuccess) {
     set_error("shmt_ctx_create: %s", cudaGetErrorString(e));
     if (scan_state) cudaFree(scan_state);
@@ -212,6 +213,7 @@ int shmt_ctx_create(int device, shmt_ctx** out) {
     delete ctx;
     return SHMT_ERR_CUDA;
   }
+  ctx->scan_state = static_cast<char*>(scan_state);
   ctx->h_words = static_cast<int64_t*>(h);
   memset(ctx->h_words, 0, kCtxWords * sizeof(int64_t));
   *out = ctx;

@@ -131,3 +131,23 @@ def test_one_context_goes_from_stream_to_stream(n):
     for i in (0, 1, rounds - 1):
         oracle.check_sample_bulk(indptr_n, indices_n, seeds_n, k, False, sub_indptr[i].cpu().numpy(),
                                  sub_indices[i, :want[-1]].cpu().numpy(), distinct_rows=True)
+
+
+def test_a_new_context_waits_for_no_stream():
+    """The first call on a stream creates its context; that must not wait for what other streams, the
+    default stream among them, still have queued."""
+    import ctypes as C
+
+    from shmtensor_b200 import _lib
+    torch.cuda.set_device(0)
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    torch.cuda._sleep(400_000_000)       # about 200 ms
+    done.record()
+    ctx = C.c_void_p()
+    _lib.check(_lib.lib.shmt_ctx_create(0, C.byref(ctx)))
+    busy = not done.query()
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib.shmt_ctx_destroy(ctx))
+    assert busy
