@@ -1975,21 +1975,25 @@ def run_scan_relabel(args) -> None:
                                     for _ in range(steps))
     del ids_dense
     b32, b64 = SR_SCAN_N * 8, SR_SCAN_N // 2 * 16
-    # relabel: ids read by insert and compact (8 each), slot written + read + new id written (8 each x 3),
-    # unique ids written; the table (12 bytes per slot at load <= 0.5) is written, read and cleaned
-    cap = 1
-    while cap < 2 * SR_IDS:
-        cap <<= 1
-    b_rel = SR_IDS * (8 + 8 + 8 * 3) + uniq.numel() * 8
-    # what bounds relabel is the rate of random 16-byte slot accesses in a table beyond L2: per id one to
-    # claim the slot / lower its first index and one to read the new id; per distinct id (at least) one to
-    # confirm the first occurrence and write the new id, and one to empty the slot
-    n_acc = 2 * SR_IDS + 2 * uniq.numel()
+    # The table of the configured ids: half-size slots of 8 bytes, the smallest power of two of at least 1.6
+    # per distinct id (csrc/relabel.cu).  Streamed per id: read by the survey and the insert pass, its slot
+    # written, read by the flag and the remap pass (8 bytes each), its flag bit written and read; per
+    # repeat its new id written; per distinct id its slot and id read, unique id and new id written; the table
+    # emptied once.
+    n_uniq = uniq.numel()
+    slots = 4
+    while slots < 1.6 * n_uniq:
+        slots *= 2
+    b_rel = SR_IDS * (5 * 8) + SR_IDS // 4 + (SR_IDS - n_uniq) * 8 + n_uniq * (4 * 8) + slots * 8
+    # What bounds relabel is the rate of random accesses to that table: per id one read to claim or find
+    # its slot, per distinct id a claim, a look at its first index and its new id's store, per repeat
+    # one read of the new id
+    n_acc = SR_IDS + 3 * n_uniq + (SR_IDS - n_uniq)
     from shmtensor_b200._lib import check, lib as shm_lib
     sink = torch.zeros(1, dtype=torch.int64, device=dev)
-    tbl = torch.empty(cap * 16, dtype=torch.uint8, device=dev)
+    tbl = torch.empty(slots * 8, dtype=torch.uint8, device=dev)
     n_probe = 1 << 26
-    probe = lambda c=[0]: (check(shm_lib.shmt_random_read(tbl.data_ptr(), tbl.numel(), n_probe, 16, c[0], sink.data_ptr(),
+    probe = lambda c=[0]: (check(shm_lib.shmt_random_read(tbl.data_ptr(), tbl.numel(), n_probe, 32, c[0], sink.data_ptr(),
                                                           stream.cuda_stream)), c.__setitem__(0, c[0] + 1))
     probe()
     slot_rate = n_probe / (min(time_launches(probe, 1, stream) for _ in range(5)) * 1e-3)
@@ -2003,17 +2007,19 @@ def run_scan_relabel(args) -> None:
                        "roofline": {"bound": "hbm", "achieved": round(b64 / (t64 * 1e6), 1), "peak": peak, "unit": "GB/s",
                                     "frac": round(b64 / (t64 * 1e6) / peak, 4)}},
         "relabel": {"ms": round(t_rel, 4), "ids_per_s": round(SR_IDS / (t_rel * 1e-3), 1), "unique": uniq.numel(),
-                    "table_slots": cap,
+                    "table_slots": slots,
                     "dense_ids": {"ms": round(t_rel_dense, 4), "ids_per_s": round(SR_IDS / (t_rel_dense * 1e-3), 1),
                                   "what": "the same ids numbered 0 .. distinct-1 (ids as slots); the configured "
                                           "workload spreads its ids over 2^43 and is hashed"},
-                    "roofline": {"bound": "hbm, rate of random 16-byte slot accesses (2 per id + 2 per distinct id)",
+                    "roofline": {"bound": "rate of random accesses to the table (L2 and HBM): 2 per id + 2 per distinct id",
                                  "kernel": "relabel_survey / insert / flag / total / number / remap_large / clear",
                                  "slot_accesses": n_acc,
                                  "achieved": round(n_acc / (t_rel * 1e-3) / 1e9, 3), "peak": round(slot_rate / 1e9, 3),
                                  "unit": "G accesses/s", "frac": round(n_acc / (t_rel * 1e-3) / slot_rate, 4),
-                                 "peak_source": "shmt_random_read, 16-byte reads over a buffer of the table's size "
-                                                "(1 GiB), measured in this run",
+                                 "peak_source": "shmt_random_read, independent 32-byte reads over a buffer of the "
+                                                f"{slots * 8 >> 20} MB the table takes and nothing else, measured in this run; "
+                                                "the call also streams its ids and slots through the same L2",
+                                 "streamed_bytes": b_rel,
                                  "streamed_bytes_frac_of_hbm": round(b_rel / (t_rel * 1e6) / peak, 4)}},
         "cub_scan": {"int32_ms": round(cub32, 4), "int64_ms": round(cub64, 4),
                      "int32_gbs": round(b32 / (cub32 * 1e6), 1), "int64_gbs": round(b64 / (cub64 * 1e6), 1),
