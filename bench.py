@@ -1153,11 +1153,14 @@ def sampling_object(steps: int, local_rank: int, full: bool = True) -> dict:
     link_reads = int(cold.size + touched[d_cold > 0].sum())
     sink = torch.zeros(1, dtype=torch.int64, device=dev)
     n_probe = 1 << 21
-    probe = lambda c=[0]: (check(shm_lib.shmt_random_read(indices.data_ptr(), indices.numel() * 4, n_probe, 16, c[0],
-                                                          sink.data_ptr(), stream.cuda_stream)), c.__setitem__(0, c[0] + 1))
-    probe()
-    probe_ms = min(time_launches(probe, 1, stream) for _ in range(5))
-    ceiling = n_probe / (probe_ms * 1e-3)
+
+    def small_read_rate(t):
+        probe = lambda c=[0]: (check(shm_lib.shmt_random_read(t.data_ptr(), t.numel() * t.element_size(), n_probe, 16, c[0],
+                                                              sink.data_ptr(), stream.cuda_stream)), c.__setitem__(0, c[0] + 1))
+        probe()
+        return n_probe / (min(time_launches(probe, 1, stream) for _ in range(5)) * 1e-3)
+    # the rate falls with the span of the addresses (translation): the row offsets are 19 MB, the neighbours 248
+    ceiling, ceiling_indices = small_read_rate(indptr), small_read_rate(indices)
     peak, peak_src = measured_peaks()
     sizes = [(N_SEEDS, 0)]
     alg = 0
@@ -1174,14 +1177,16 @@ def sampling_object(steps: int, local_rank: int, full: bool = True) -> dict:
         "kernel_ms": round(hop_ms, 5), "kernel_share_of_step": round(hop_ms / ms, 3),
         "link_reads_per_launch": link_reads, "achieved": round(link_reads / (hop_ms * 1e-3) / 1e9, 4),
         "peak": round(ceiling / 1e9, 4), "unit": "G reads/s", "frac": round(link_reads / (hop_ms * 1e-3) / ceiling, 4),
-        "peak_source": "shmt_random_read: independent 16-byte reads (one request each) of the same pinned indices "
-                       "array, 4 per thread in flight, measured in this run",
+        "peak_source": "shmt_random_read: independent 16-byte reads (one request each) of the same pinned indptr array, "
+                       "4 per thread in flight, measured in this run",
+        "peak_over_the_indices_array": round(ceiling_indices / 1e9, 4),
         "cold_rows_per_launch": int(cold.size), "frontier_rows_per_launch": int(fr.size),
         "algorithmic_bytes": int(alg), "hbm_achieved_gbs": round(alg / (ms * 1e6), 1), "hbm_peak": peak,
         "hbm_frac": round(alg / (ms * 1e6) / peak, 5), "hbm_peak_source": peak_src, "traffic": None,
         "note": "a cold row of the frontier costs one request for its row-offset pair and then one per 128-byte line of "
-                "its adjacency list that a pick falls in, the second depending on the first; the link serves about 0.3 G "
-                "such requests per second whatever their size, so bytes do not matter here"}
+                "its adjacency list that a pick falls in, the second depending on the first; the link serves 0.3 G "
+                "such requests per second over a gigabyte, 0.35 G over 248 MB and 0.45 G over 19 MB, so bytes do not "
+                "matter here"}
 
     if full:
         # uncached (every row over UVA) and fully GPU-resident graph, for the cache's effect
