@@ -992,14 +992,11 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
     job.ticket = w + 0;
     job.status = status;
     job.result = w + 1;
-    const bool fuse_insert = true;  // every sampler claims the relabel slots of what it emits
-    if (fuse_insert) {
-      RelTable t;
-      if (int rc = relabel_table(ctx, cap[h + 1], &t, s)) return rc;
-      job.rel_slots = t.slots;
-      job.rel_cap = t.cap;
-      job.rel_out = out_relabel[h];
-    }
+    RelTable t;  // every sampler claims the relabel slots of what it emits
+    if (int rc = relabel_table(ctx, cap[h + 1], &t, s)) return rc;
+    job.rel_slots = t.slots;
+    job.rel_cap = t.cap;
+    job.rel_out = out_relabel[h];
     SHMT_CUDA_TRY(indices_dtype == SHMT_I64 ? launch_hop<long long>(job, hop_tiles[h], s, /*pdl=*/h > 0)
                                             : launch_hop<int>(job, hop_tiles[h], s, /*pdl=*/h > 0));
     SHMT_CUDA_TRY(cudaGetLastError());
@@ -1017,7 +1014,7 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
     if (h == n_hops - 1) post = ctx_begin_post(ctx, words, n_hops * 8 + 8, w + 4);
     if (int rc = launch_relabel(ctx, ps, cap[h + 1], out_frontier[h], out_relabel[h],
                                 carve_tile_states(base + off_rel[h], rel_tiles[h]), w + 2, status,
-                                w + 3, s, fuse_insert, /*pdl=*/true, h == n_hops - 1 ? &post : nullptr))
+                                w + 3, s, /*inserted=*/true, /*pdl=*/true, h == n_hops - 1 ? &post : nullptr))
       return rc;
     cur_seeds = out_frontier[h];
   }
