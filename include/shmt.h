@@ -202,9 +202,9 @@ int shmt_debug_lookback_timeout(shmt_ctx* ctx, void* stream);
  * order (out_unique, capacity = total) and, for every input element, the index
  * of its id in out_unique (out_relabel, total elements, same dtype).  Ids must
  * not be -1.  If n_unique_host != NULL the call waits for the number of distinct
- * ids and stores it there; it returns as soon as that number is known, while the
- * last kernel may still be writing out_relabel (consume the outputs in `stream`
- * order, or synchronise).  TensorRelabel (src/tensor_relabel.cu:125-209).        */
+ * ids and stores it there; it returns as soon as that number is known, while up to
+ * four kernels may still be writing out_unique and out_relabel (consume the outputs in
+ * `stream` order, or synchronise).  TensorRelabel (src/tensor_relabel.cu:125-209).    */
 int shmt_relabel(shmt_ctx* ctx, const void* const* parts,
                  const int64_t* part_sizes, int n_parts, int dtype,
                  void* out_unique, void* out_relabel, int64_t* n_unique_host,

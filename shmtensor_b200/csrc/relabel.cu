@@ -11,7 +11,8 @@
 // that was used back to "empty", so the table needs no memset between calls;
 // (3) remap the repeats.  Every element probes the table once (the reference four times).
 // Up to 4,096 ids are one CTA's work; more than 2^20 are looked over first and use the smallest
-// form of the table their ids allow, and (2) becomes three kernels without a look-back.
+// form of the table their ids allow, (2) becomes three kernels without a look-back, and a last one
+// empties what (3) leaves of the small forms.
 // The element counts may live on the device (written by an earlier kernel), so a
 // chain of hops can be queued without the host knowing any size.
 #include "relabel.cuh"
@@ -285,8 +286,9 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
   const int64_t numel = sizes.numel;
   const RelUse use = relabel_use(t, numel, survey);
   // One element per thread and step, its successor's id read ahead: more resident threads are worth
-  // more than more elements on their way per thread (33.5 M ids in ordinary slots: 660 us, two elements per thread with
-  // twice the registers 1,150; in half-size slots 480).
+  // more than more elements on their way per thread (33.5 M ids in ordinary slots: 660 us, two elements per
+  // thread with twice the registers 1,150; in half-size slots 480).  The 7 CTAs per SM leave 32 registers, and
+  // 24 bytes a thread are spilled; it took 492 us before 7 were asked for.
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   long long next = i < numel ? part_elem(ps, sizes, i) : 0;

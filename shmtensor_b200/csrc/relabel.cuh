@@ -24,7 +24,8 @@ struct Parts {
   int n;
   int is64;
   // Two-part form whose sizes were produced on the device (dev_n1 set): |part 1| = *dev_n1,
-  // |part 0| = *dev_n0, or the host's start[1] if dev_n0 is null; the kernels fill start[].
+  // |part 0| = *dev_n0, or the host's start[1] if dev_n0 is null.  start[] stays as the host left it: the
+  // kernels keep the sizes they read beside the parts (PartSizes in relabel.cu).
   const int64_t* dev_n0;
   const int64_t* dev_n1;
 };
@@ -46,7 +47,8 @@ struct RelTable {
 
 // Slots per id.  A small input waits for its longest walk (at half load a few of 5,000 ids walk six
 // pairs, 1 us each), so it spreads out over up to kRelRoomy slots; a large one is bound by the
-// sectors it draws from HBM and stays compact.
+// sectors it draws from HBM and stays compact.  The price is memory: a context that serves 300,000 ids
+// holds 48 MB of table where two slots per id would be 24.
 constexpr double kRelRoomy = (double)(1 << 21);  // 32 MB
 
 // What a first look at a large input says about it.
@@ -166,7 +168,7 @@ __device__ __forceinline__ uint32_t relabel_claim(const RelRange& t, long long k
       const long long old = relabel_cas(t.slots + pos, key);
       if (old == kEmptyKey || old == key) return pos;
     }
-    if (round > t.full) {  // the table holds twice the ids: cannot happen
+    if (round > t.full) {  // there are never fewer slots than ids: cannot happen
       atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
       return pos;
     }
@@ -192,18 +194,21 @@ uint64_t relabel_capacity(int64_t numel_bound);
 // Context scratch that shmt_relabel takes for up to `numel` ids.
 size_t relabel_scratch_bytes(int64_t numel);
 
-// Queue the three relabel kernels.  `numel_bound` >= the real element count sizes the
-// table and the grids; ticket/status/result are zeroed device words.
+// Queue the relabel kernels: insert, compact and remap, or, of a surveyed input, survey, insert, flag,
+// total, number, remap and clear.  `numel_bound` >= the real element count sizes the table and the
+// grids; ticket/status/result are zeroed device words.
 // `pdl`: launch with programmatic stream serialization (see pdl_prologue in common.cuh).
 // `inserted`: the slots were already claimed and recorded in out_relabel by the producer
 // of the ids (the fused sampling kernel), so only the compact and remap kernels run.
-// `post`: the compact kernel hands the result words to the host as soon as the unique count is
-// final, i.e. while the remap kernel is still to run (it produces neither sizes nor errors).
-// `survey`: zeroed device memory, with room for the flags behind it (see relabel_flag_kernel); when given, a first kernel looks the ids over and the insert
-// kernel uses as much of the table as they need (see relabel_survey_kernel).
-int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
-                   int64_t* status, int64_t* result, cudaStream_t s, bool inserted = false,
-                   bool pdl = false, const HostPost* post = nullptr, RelSurvey* survey = nullptr);
+// `post`: the compact (or total) kernel hands the result words to the host as soon as the unique count
+// is final; the kernels still to run then produce neither sizes nor errors.
+// `survey`: zeroed device memory, with room for the flags behind it (relabel_scratch_bytes in all); when
+// given, a first kernel looks the ids over and the others use the form of the table that suits them
+// (see relabel_survey_kernel, relabel_use).
+int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel,
+                   TileStates st, int64_t* ticket, int64_t* status, int64_t* result, cudaStream_t s,
+                   bool inserted = false, bool pdl = false, const HostPost* post = nullptr,
+                   RelSurvey* survey = nullptr);
 
 // The context's table for `numel_bound` ids (reserving it).
 int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s);

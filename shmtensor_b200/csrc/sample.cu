@@ -33,7 +33,8 @@ constexpr int kHopThreads = 256;
 // A hop is a chain of dependent reads per edge (row bounds, neighbour, relabel slot), so resident
 // threads count for more than reads in flight per thread: the third hop of 8,192 seeds x 5/10/15
 // took 118 us with four edges per thread (64 registers, 4 CTAs per SM), 99 with two (5 CTAs) and 94
-// with one (6 CTAs).
+// with one (6 CTAs).  At 6 the 40 registers do not hold everything: 20 to 28 bytes a thread are spilled,
+// and are part of the 94.
 constexpr int kHopCtasPerSm = 6;
 // Seeds of a tile come in steps of 8: a small hop is as long as its slowest CTA, and 1,024 seeds over
 // a host graph took 20 us in 32 CTAs of 32 seeds and 16 us in 128 CTAs of 8.

@@ -1,5 +1,5 @@
-// In-place prefix sum in one pass with decoupled look-back: a ticketed kernel over 64 KB tiles
-// for small inputs, a persistent thread-block-cluster kernel with early sums for large ones.
+// In-place prefix sum in one pass with decoupled look-back: a ticketed kernel over tiles of 16, 32 or
+// 64 KB for small inputs, a persistent thread-block-cluster kernel with early sums for large ones.
 // Semantics follow cub_exclusiveSum (reference src/cache_graph_sampling.cu:30-45)
 // and the intended meaning of thrust_scan (reference src/thrust_scan.cu:9-18,
 // whose own lambda races); integer arithmetic wraps.
@@ -33,6 +33,7 @@ struct ScanWord<long long> { using type = unsigned long long; };
 // type of the data (wrap-around is defined and the low bits are all the result keeps): inside a
 // vector, across the warp with shuffles, across the (row, warp) partials by warp 0; after the
 // look-back every thread adds its three offsets and stores.
+// Two CTAs per SM leave 64 registers; 64-bit numbers in 64 KB tiles spill 24 bytes a thread there.
 // `clean`: this launch's tile descriptors, ticket and `done` word start at zero and are put back to
 // zero by the CTA whose look-back ends last, so a small scan needs no memset in front of it.
 template <typename T, int VECS>
