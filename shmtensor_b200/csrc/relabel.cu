@@ -64,12 +64,18 @@ __device__ __forceinline__ int relabel_sample_shift(int64_t numel) {
 }
 
 // A look at a large input before any slot is claimed: its largest id (a negative id counts as
-// huge), and how many distinct ids it holds, from a sample.
+// huge), and how many distinct ids it holds, from a sample.  A sampled id that many elements share would be
+// looked up in the bitmap, one sector of L2, by every warp (3,000,000 ids, a tenth of them the same: 38 us
+// for 24 without such ids); a CTA therefore remembers what it has looked up.
+constexpr int kRelKnown = 1024;
 __global__ void __launch_bounds__(kRelThreads, 8)
 relabel_survey_kernel(Parts ps, RelSurvey* survey) {
   __shared__ unsigned s_marked[kRelThreads / 32];
   __shared__ unsigned long long s_largest[kRelThreads / 32];
+  __shared__ uint32_t s_known[kRelKnown];  // bits this CTA has looked up or set, the last at each place
   pdl_prologue();
+  for (int q = (int)threadIdx.x; q < kRelKnown; q += kRelThreads) s_known[q] = ~0u;
+  __syncthreads();
   const PartSizes sizes = resolve_sizes(ps);
   const int64_t numel = sizes.numel;
   const int shift = relabel_sample_shift(numel);
@@ -82,7 +88,10 @@ relabel_survey_kernel(Parts ps, RelSurvey* survey) {
     const uint64_t h = mix64((uint64_t)id);
     if (shift == 0 || (h >> (64 - shift)) == 0) {
       const uint32_t at = (uint32_t)h & ((1u << kRelSampleBits) - 1u), bit = 1u << (at & 31);
-      if (!(__ldcg(survey->bitmap + (at >> 5)) & bit))
+      volatile uint32_t* known = s_known + at % kRelKnown;
+      if (*known == at) return;
+      *known = at;
+      if (!(__ldcg(survey->bitmap + (at >> 5)) & bit) && relabel_lowest(at))
         marked += (atomicOr(survey->bitmap + (at >> 5), bit) & bit) == 0;
     }
   };
@@ -212,7 +221,7 @@ __device__ __forceinline__ uint64_t mix_bits(uint64_t x, int bits) {
   return x;
 }
 
-// relabel_claim and relabel_settle for half-size slots: a claim enters the index with the id.
+// relabel_enter for half-size slots: a claim enters the index with the id.
 __device__ __forceinline__ uint32_t relabel_claim_half(const RelSmall& t, long long key, unsigned i, int64_t* status,
                                                        bool* maybe_first) {
   const uint64_t x = mix_bits((uint64_t)key, t.bits);
@@ -251,10 +260,7 @@ __device__ __forceinline__ uint32_t relabel_claim_half(const RelSmall& t, long l
       return at + found;
     }
   }
-  unsigned seen;
-  const uint32_t pos = relabel_claim(t.rest, key, status, &seen);
-  *maybe_first = relabel_settle(t.rest, pos, seen, i);
-  return t.n + pos;
+  return t.n + relabel_enter<true>(t.rest, key, i, status, maybe_first);
 }
 
 // Where the later passes of a surveyed call find what they need at position `pos`.
@@ -278,7 +284,9 @@ struct RelView {
   }
 };
 
-__global__ void __launch_bounds__(kRelThreads, 7)
+constexpr unsigned kRelSms = 148, kRelInsertCtas = 7;  // CTAs per SM
+
+__global__ void __launch_bounds__(kRelThreads, kRelInsertCtas)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
                       const RelSurvey* __restrict__ survey) {
   pdl_prologue();
@@ -288,10 +296,15 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
   // One element per thread and step, its successor's id read ahead: more resident threads are worth
   // more than more elements on their way per thread (33.5 M ids in ordinary slots: 660 us, two elements per
   // thread with twice the registers 1,150; in half-size slots 480).  The 7 CTAs per SM leave 32 registers, and
-  // 24 bytes a thread are spilled; it took 492 us before 7 were asked for.
+  // 16 bytes a thread are spilled; it took 492 us before 7 were asked for.
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   long long next = i < numel ? part_elem(ps, sizes, i) : 0;
+  // The CTAs of the first wave start a little apart: an id that many elements share is claimed by the first of
+  // them and found by the others, instead of being met unclaimed by all (see relabel_enter).  1,048,576 ids, a
+  // tenth of them the same: 121 us a call with all at once, 108 with 1 us between the CTAs of an SM, 103 with 2;
+  // 300,000 distinct ids take 54 us with 0 and 1, 57 with 2.
+  if (blockIdx.x >= kRelSms && blockIdx.x < kRelSms * kRelInsertCtas) __nanosleep(blockIdx.x / kRelSms * 1000);
   for (; i < numel; i += stride) {
     const long long key = next;
     if (i + stride < numel) next = part_elem(ps, sizes, i + stride);
@@ -300,13 +313,14 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
     if (use.small.stride == 1) {
       pos = (uint32_t)key;
       maybe_first = __ldcg(use.small.words + pos) > (unsigned)i;
-      if (maybe_first) atomicMin(use.small.words + pos, (unsigned)i);
+      if (maybe_first) {
+        maybe_first = relabel_lowest(pos);
+        if (maybe_first) atomicMin(use.small.words + pos, (unsigned)i);
+      }
     } else if (use.small.stride == 2) {
       pos = relabel_claim_half(use.small, key, (unsigned)i, status, &maybe_first);
     } else {
-      unsigned seen;
-      pos = relabel_claim(use.range, key, status, &seen);
-      maybe_first = relabel_settle(use.range, pos, seen, (unsigned)i);
+      pos = relabel_enter<true>(use.range, key, (unsigned)i, status, &maybe_first);
     }
     store_int(out, ps.is64, i, relabel_pack(pos, maybe_first, ps.is64));
   }

@@ -148,43 +148,55 @@ __device__ __forceinline__ uint32_t relabel_next(const RelRange& t, long long ke
   return at == t.full ? t.near : at;
 }
 
-// Claim (or find) the slot of `key`.  What bounds a claim is latency: a read of the home, then a CAS
-// if it had room, 0.7 - 1 us each and more under load.  *seen is the first index the slot held (all
-// ones if it was claimed just now, by this element or by another one of the same id).
-__device__ __forceinline__ uint32_t relabel_claim(const RelRange& t, long long key, int64_t* status,
-                                                  unsigned* seen) {
+// Whether the calling lane is the lowest, of those that call together, with its `at`.
+__device__ __forceinline__ bool relabel_lowest(uint32_t at) {
+  return __ffs(__match_any_sync(__activemask(), at)) - 1 == (int)(threadIdx.x & 31);
+}
+
+// Claim (or find) the slot of `key` and enter index `i` for it as a candidate first occurrence;
+// *maybe_first is false if it certainly is not one.
+// What bounds this is latency: a read of the home, then a CAS if it had room, 0.7 - 1 us each and more under
+// load.  `first` only ever goes down: when the index seen there is already smaller than this one the
+// atomic would change nothing, and most elements of a frontier are such repeats.  Nothing waits for
+// the atomic's result: an element that lowers the index, or loses to a still smaller one, is simply left
+// among the candidates.
+// CROWDED: an id that many elements share is met unclaimed by every warp on its way when the call starts, and
+// atomics on one address are served one after the other (1,048,576 ids, a tenth of them the same: 146 us a
+// call, 108 so).  The lanes of a warp that are about to change the same slot leave it to the lowest of them
+// (indexes go up with the lanes), and one that lost its claim to another warp looks at the index once more
+// first.  A sampling hop, whose warps arrive spread out by their reads of the graph, is better without (8,192 seeds
+// 5/10/15 on a graph whose neighbours crowd: 161 us for 164).
+template <bool CROWDED>
+__device__ __forceinline__ uint32_t relabel_enter(const RelRange& t, long long key, unsigned i, int64_t* status,
+                                                  bool* maybe_first) {
   uint32_t pos = relabel_home(t, key);
-  *seen = 0xFFFFFFFFu;
   for (uint32_t round = 0;; ++round) {
+    if (round > t.full + 32) {  // there are never fewer slots than ids: cannot happen
+      atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
+      *maybe_first = false;
+      return pos;
+    }
     const RelPair p = relabel_load_pair(t.slots, pos & ~1u);
     const bool second = (pos & 1u) || (p.key0 != key && p.key0 != kEmptyKey);
     const long long cur = second ? p.key1 : p.key0;
     pos |= (uint32_t)second;
     if (cur == key) {
-      *seen = second ? p.first1 : p.first0;
+      *maybe_first = (second ? p.first1 : p.first0) > i;  // a mark counts as no index
+      if (CROWDED && *maybe_first) *maybe_first = relabel_lowest(pos);
+      if (*maybe_first) atomicMin(&t.slots[pos].first, i);
       return pos;
     }
     if (cur == kEmptyKey) {
+      if (CROWDED && !relabel_lowest(pos)) continue;  // reads next what the lowest lane did
       const long long old = relabel_cas(t.slots + pos, key);
-      if (old == kEmptyKey || old == key) return pos;
-    }
-    if (round > t.full) {  // there are never fewer slots than ids: cannot happen
-      atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
-      return pos;
+      if (old == kEmptyKey || old == key) {
+        *maybe_first = !CROWDED || old == kEmptyKey || *reinterpret_cast<volatile unsigned*>(&t.slots[pos].first) > i;
+        if (*maybe_first) atomicMin(&t.slots[pos].first, i);
+        return pos;
+      }
     }
     pos = relabel_next(t, key, pos);
   }
-}
-
-// Enter index `i` for the slot as a candidate first occurrence; false if it certainly is not one.
-// `first` only ever goes down: when the index seen there is already smaller than this one the
-// atomic would change nothing, and most elements of a frontier are such repeats.  Nothing waits
-// for the atomic's result: an element that lowers the index, or loses to a still smaller one, is
-// simply left among the candidates.
-__device__ __forceinline__ bool relabel_settle(const RelRange& t, uint32_t pos, unsigned seen, unsigned i) {
-  if (seen <= i) return false;  // a mark counts as no index
-  atomicMin(&t.slots[pos].first, i);
-  return true;
 }
 #endif
 

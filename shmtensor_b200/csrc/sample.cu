@@ -313,9 +313,8 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
                        job.rel_cap};
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
   auto enter = [&](int64_t i, IxT id) {
-    unsigned seen;
-    const uint32_t at = relabel_claim(range, (long long)id, job.status, &seen);
-    const bool maybe_first = relabel_settle(range, at, seen, (unsigned)i);
+    bool maybe_first;
+    const uint32_t at = relabel_enter<false>(range, (long long)id, (unsigned)i, job.status, &maybe_first);
     store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
   };
 

@@ -317,6 +317,23 @@ def test_relabel_when_half_size_slots_run_over(capi):
     capi.check_async()
 
 
+@pytest.mark.parametrize("n", [4097, 300_001, (1 << 20) + 1, 3_000_000])
+@pytest.mark.parametrize("share", [0.1, 0.5, 1.0])
+def test_relabel_of_ids_that_many_elements_share(capi, n, share):
+    """Lanes of a warp that are about to change the same slot, word or survey bit leave it to one of them:
+    a few ids take a share of the elements, anywhere among them, in every form of the table (a word per
+    id, ordinary slots, half-size slots) and width, the first elements among the shared ones or not."""
+    rng = np.random.default_rng(n + int(10 * share))
+    few = rng.integers(0, n, size=5)
+    x = np.where(rng.random(n) < share, few[rng.integers(0, 5, size=n) // rng.integers(1, 6, size=n)], rng.permutation(n))
+    for make in (lambda y: y.astype(np.int32), lambda y: y, lambda y: y * 0x100001, lambda y: y * 0x1000000000 - 7):
+        for y in (make(x), make(x)[::-1].copy()):
+            uniq, (rel,) = capi.tensor_relabel([torch.from_numpy(y).cuda()])
+            wu, (wr,) = oracle.tensor_relabel([y])
+            assert np.array_equal(uniq.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wr)
+    capi.check_async()
+
+
 def unmix_bits(x, bits):
     """The inverse of the mix that gives half-size slots their homes (csrc/relabel.cu, mix_bits)."""
     mask, half = np.uint64((1 << bits) - 1), np.uint64((bits + 1) // 2)
