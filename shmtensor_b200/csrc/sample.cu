@@ -203,12 +203,22 @@ struct WeightedPicks {
   }
 };
 
-// A row longer than this is shared by the warps of the CTA: a hop is as long as its longest row.
-// 1,000 seeds of a power-law graph with rows of up to 10,000 edges: 64 us when one warp took a row
-// with one load in flight, 24 us so.
-constexpr int64_t kWeightedLongRow = 1024;
+// Which rows of a tile the warps of the CTA share (a row's edges dealt out 128 at a time, the warps' picks
+// then ranked against one another), and which ones a warp takes alone: a hop is as long as its slowest
+// tile.  Alone rows run beside one another, shared rows one after the other, and a shared row is less
+// than an eighth as long: each warp still inserts its own k best.  So the longest rows are shared, as
+// many of them as make the tile's estimate smallest.  1,000 seeds of a power-law graph with rows of up to
+// 10,000 edges: 64 us with none shared and one load in flight, 24 with the longest shared; 8 rows of 2,000 edges, 15
+// picks each, in a tile: 138 us with all shared and merged one pick after the other, 39 with none.
+constexpr int64_t kWeightedLongRow = 1024;  // shorter rows are never shared
+// Times in edges looked at (6.6 ns): an insertion is worth 17, and a warp that looks at d edges inserts
+// about k * (1 + ln(d / k)) of them.
+__device__ __forceinline__ float weighted_cost(float edges, float k) {
+  return edges <= k ? k : edges + 17.0f * k * (1.0f + __logf(edges / k));
+}
+constexpr float kWeightedShareCost = 200.0f;  // barriers, and the ranking
 
-template <typename IxT, int G>
+template <typename IxT, int G, bool EARLY = false>
 __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
   extern __shared__ __align__(16) unsigned char s_dyn[];  // hop_smem_bytes()
   __shared__ int64_t warp_sums[32];
@@ -318,49 +328,122 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
   };
 
+  // the tile's place in the output, and what the host waits for
+  auto place = [&]() -> int64_t {
+    const int64_t prefix = lookback_block(job.st, tile, s_total, &s_look, job.status);
+    for (int j = (int)tid; j < rows; j += kHopThreads)
+      store_int(job.sub_indptr, job.indptr64, first + j, prefix + s_off[j]);
+    if (tile == n_tiles - 1 && tid == 0) {
+      store_int(job.sub_indptr, job.indptr64, n, prefix + s_total);
+      st_relaxed64(job.result, prefix + s_total);
+    }
+    if (job.post.host) {  // uniform over the grid; the fused path (which may still flag the relabel table) never posts here
+      __syncthreads();
+      if (!job.clean && tid < 32) post_when_last(job.post, n_tiles);
+    }
+    if (job.clean) {  // uniform as well; all look-backs of this CTA are over
+      if (!job.post.host) __syncthreads();
+      if (tid < 32 && last_to_finish(job.clean, n_tiles)) {
+        for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
+        if (lane == 0) {
+          st_relaxed64(job.ticket, 0);
+          st_relaxed64(job.clean, 0);
+        }
+        // only now: the host may queue the state's next user in another stream as soon as it has the post
+        post_to_host(job.post);
+      }
+    }
+    return prefix;
+  };
+
+  // EARLY: picking by weight takes long, and a host that waits for the count need not wait for it, so the
+  // tile takes its place first (8 rows of 1,000 edges, 15 picks each: 46.6 us a call, 31.2 so).  Both orders in one
+  // kernel cost the other one: a weighted mini-batch of 1,000 seeds 130 us for 125.
+  const int64_t placed = EARLY ? place() : 0;
+
   // ---- 3. (k <= 32) positions of the picked neighbours, a group of lanes per seed, into a list in
   // output order.  Arithmetic and shuffles only: the memory work is left to step 5, where all
   // threads of the tile share it evenly whatever the rows' lengths.
   if (G == 32 && listed && job.weights && k > 0) {
     __shared__ float s_key[G == 32 ? kHopThreads : 1];
     __shared__ int64_t s_pos[G == 32 ? kHopThreads : 1];
+    __shared__ unsigned long long s_cut;
     const float none = __int_as_float(0x7f800000);
     auto weights_of = [&](int j) { return (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j]; };
-    auto list = [&](int j, int64_t pos) {
-      s_list[s_off[j] + gl] = HopEdge::pack(s_begin[j] + pos, j, s_hit[j]);
+    auto list = [&](int j, int at, int64_t pos) {
+      s_list[s_off[j] + at] = HopEdge::pack(s_begin[j] + pos, j, s_hit[j]);
+    };
+    // rows in falling order of length (then by place): those ahead of row `cut` are shared.  A single long
+    // row always is.
+    int cut = -1;
+    int64_t cut_deg = kWeightedLongRow;
+    const int64_t my_deg = (int)tid < rows ? s_deg[tid] : -1;  // thread `rows` stands behind the last row
+    const int n_long = __syncthreads_count(my_deg > kWeightedLongRow);
+    if (n_long == 1) cut = 0;
+    if (n_long > 1) {
+      const float fk = (float)k;
+      if (tid == 0) s_cut = ~0ull;
+      if ((int)tid < rows) {
+        s_key[tid] = weighted_cost((float)my_deg, fk);
+        reinterpret_cast<float*>(s_pos)[tid] = weighted_cost((float)my_deg / kGroups, fk) + kWeightedShareCost;
+      }
+      __syncthreads();
+      if ((int)tid <= rows) {
+        float shared = 0.0f, alone = 0.0f;
+        bool allowed = true;
+        for (int j = 0; j < rows; ++j) {
+          if (s_deg[j] > my_deg || (s_deg[j] == my_deg && j < (int)tid)) {
+            shared += reinterpret_cast<const float*>(s_pos)[j];
+            allowed = allowed && s_deg[j] > kWeightedLongRow;
+          } else {
+            alone += s_key[j];
+          }
+        }
+        const float mine = (int)tid < rows ? s_key[tid] : 0.0f;
+        const float estimate = shared + fmaxf(mine, alone / kGroups);
+        if (allowed) atomicMin(&s_cut, ((unsigned long long)__float_as_uint(estimate) << 32) | tid);
+      }
+      __syncthreads();
+      cut = (int)(s_cut & 0xFFFFFFFFull);
+      cut_deg = cut < rows ? s_deg[cut] : -1;
+    }
+    auto is_shared = [&](int j) {  // the same on every thread
+      return cut >= 0 && (s_deg[j] > cut_deg || (s_deg[j] == cut_deg && j < cut));
     };
     for (int j = group; j < rows; j += kGroups) {
       const int64_t deg = s_deg[j];
       if (deg <= k) {
-        if ((int64_t)gl < deg) list(j, gl);
-      } else if (deg <= kWeightedLongRow) {
+        if ((int64_t)gl < deg) list(j, (int)gl, gl);
+      } else if (!is_shared(j)) {
         WeightedPicks best{none, -1};
         best.scan(weights_of(j), 0, 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo, job.off_hi);
-        if ((int64_t)gl < k) list(j, best.pos);
+        if ((int64_t)gl < k) list(j, (int)gl, best.pos);
       }
     }
-    for (int j = 0; j < rows; ++j) {
-      const int64_t deg = s_deg[j];
-      if (deg <= k || deg <= kWeightedLongRow) continue;  // the same on every thread
+    for (int j = 0; cut >= 0 && j < rows; ++j) {
+      if (!is_shared(j)) continue;
       WeightedPicks best{none, -1};
-      best.scan(weights_of(j), group * 128, kGroups * 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo,
+      best.scan(weights_of(j), group * 128, kGroups * 128, s_deg[j], gl, (int)k, rng, (uint32_t)(first + j), job.off_lo,
                 job.off_hi);
+      __syncthreads();  // the row before has been ranked (and the estimates read)
       s_key[tid] = best.key;
       s_pos[tid] = best.pos;
       __syncthreads();
-      if (group == 0) {
-        for (int w = 1; w < kGroups; ++w)
-          for (int q = 0; q < (int)k; ++q) {
-            const float ck = s_key[w * 32 + q];
-            const int64_t cp = s_pos[w * 32 + q];
-            const float last_k = __shfl_sync(full, best.key, (int)k - 1);
-            const int64_t last_p = __shfl_sync(full, best.pos, (int)k - 1);
-            if (!(ck < last_k || (ck == last_k && cp < last_p))) break;  // nor do the warp's further keys
-            best.insert(ck, cp, gl, (int)k);
-          }
-        if ((int64_t)gl < k) list(j, best.pos);
+      // a pick's place is the number of picks ahead of it, found in each warp's ascending list; one that
+      // its warp has not filled has k ahead of it
+      int ahead[kGroups] = {0}, rank = 0;
+      for (int step = 1 << (31 - __clz((int)k)); step > 0; step >>= 1) {
+#pragma unroll
+        for (int w = 0; w < kGroups; ++w) {
+          const int at = w * 32 + min(ahead[w] + step, (int)k) - 1;
+          const float ck = s_key[at];
+          const bool less = ck < best.key || (ck == best.key && s_pos[at] < best.pos);
+          if (less && ahead[w] + step <= (int)k) ahead[w] += step;
+        }
       }
-      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kGroups; ++w) rank += ahead[w];
+      if ((int64_t)gl < k && rank < (int)k) list(j, rank, best.pos);
     }
     __syncthreads();
   } else if (listed) {
@@ -408,29 +491,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     return __ldg(static_cast<const IxT*>(x.hit() ? job.gpu_indices : job.indices) + x.at());
   };
   IxT next = fetch((int)tid);
-  const int64_t prefix = lookback_block(job.st, tile, s_total, &s_look, job.status);
-  for (int j = (int)tid; j < rows; j += kHopThreads)
-    store_int(job.sub_indptr, job.indptr64, first + j, prefix + s_off[j]);
-  if (tile == n_tiles - 1 && tid == 0) {
-    store_int(job.sub_indptr, job.indptr64, n, prefix + s_total);
-    st_relaxed64(job.result, prefix + s_total);
-  }
-  if (job.post.host) {  // uniform over the grid; the fused path (which may still flag the relabel table) never posts here
-    __syncthreads();
-    if (!job.clean && tid < 32) post_when_last(job.post, n_tiles);
-  }
-  if (job.clean) {  // uniform as well; all look-backs of this CTA are over
-    if (!job.post.host) __syncthreads();
-    if (tid < 32 && last_to_finish(job.clean, n_tiles)) {
-      for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
-      if (lane == 0) {
-        st_relaxed64(job.ticket, 0);
-        st_relaxed64(job.clean, 0);
-      }
-      // only now: the host may queue the state's next user in another stream as soon as it has the post
-      post_to_host(job.post);
-    }
-  }
+  const int64_t prefix = EARLY ? placed : place();
 
   // ---- 5. output and relabel slots, one list element per thread and step
   if (listed) {
@@ -715,6 +776,8 @@ static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool 
     if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8>, grid, kHopThreads, smem, s, job);
     if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16>, grid, kHopThreads, smem, s, job);
   }
+  if (job.weights && !job.replace && job.post.host)  // the lists of fan-outs up to 32: within 48 KB
+    return launch_kernel(pdl, sample_hop_kernel<IxT, 32, true>, grid, kHopThreads, smem, s, job);
   if (smem > (48 << 10)) {
     static bool configured[64] = {false};
     int dev = 0;

@@ -210,3 +210,31 @@ def test_a_reserved_context_samples_weighted_batches_without_allocating(replace)
         assert capi.context_scratch_bytes() == reserved
     torch.cuda.synchronize()
     assert sx.numel() == 2 * n and torch.equal(front[rel.long()], sx)
+
+
+@pytest.mark.parametrize("deg", [1025, 1500, 5000, 10_000])
+@pytest.mark.parametrize("k", [1, 7, 32])
+def test_a_row_yields_the_same_picks_alone_and_shared(capi, deg, k):
+    """Whether the warps of a CTA share a long row depends on the rows it shares a tile with; what is
+    drawn for it does not: its place among the seeds decides.  Weights of which many are equal, or zero."""
+    rng = np.random.default_rng(deg + k)
+    degs = np.concatenate([np.full(8, deg), rng.integers(40, 200, size=8), [deg + 700, 3 * deg]])
+    indptr_n = np.concatenate([[0], np.cumsum(degs)])
+    indptr = torch.from_numpy(indptr_n).cuda()
+    indices = torch.arange(int(indptr_n[-1]), dtype=torch.int32, device="cuda")
+    w = torch.from_numpy((rng.integers(0, 4, size=int(indptr_n[-1])) ** 2).astype(np.float32)).cuda()
+
+    def picks(seeds):
+        capi.set_sampling_seed(77)
+        p, x = capi.csr_weighted_sampling(indptr, indices, w, torch.tensor(seeds, dtype=torch.int32, device="cuda"), k, False)
+        return [r.tolist() for r in torch.tensor_split(x.cpu(), p.cpu()[1:-1])]
+
+    crowded = picks(list(range(8)))                              # eight rows of one length: none is shared
+    for at in range(8):
+        seeds = [8 + j for j in range(8)]
+        seeds[at] = at
+        assert picks(seeds)[at] == crowded[at]                   # one long row among short ones: shared
+        seeds[(at + 3) % 8], seeds[(at + 6) % 8] = 16, 17
+        assert picks(seeds)[at] == crowded[at]                   # among the longer ones of three
+    assert picks([0])[0] == crowded[0]                           # and on its own
+    assert len({tuple(r) for r in crowded}) == 8 and all(len(set(r)) == k for r in crowded)
