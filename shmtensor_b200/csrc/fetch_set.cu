@@ -704,21 +704,37 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
 // granules read at both ends of a row outweigh the wider access (132 bytes: 2.9 against 2.3 TB/s, 28
 // against 24 GB/s).  Rows of 8-byte units have a faster narrow copy, which is level at 408 bytes
 // (4.8 against 5.0 TB/s, 41.0 against 40.9 GB/s) and behind at 600 (4.2 against 5.1, 43.1 against 44.2).
+// A small batch read from the host alone is a wait for its few rows, to which granules add a trip through
+// shared memory: rows of 4- and 8-byte units take the narrow copy up to 512 KB a batch, and up to 4 MB where
+// they are shorter than 512 and 600 bytes (300 rows of 808 bytes 9.3 us against 9.9, 3,000 of 260 bytes 24.0
+// against 26.7, of 520 38.5 against 40.0; but 20,000 of 260 bytes 158 against 146, of 520 245 against 237).
+// 2-byte units are faster in granules from 1,000 rows of 258 bytes on (12.6 against 11.7).
+// A batch that may hit the cache takes granules whatever its size: how many of its rows miss is not known here.
+// Where all hit, the narrow copy is 0.5 to 3 us faster up to about 40 MB of 8-byte units or 5 MB of 4-byte units
+// (30,000 rows of 1,000 bytes 11.3 against 12.4); where a fifth of those rows miss, granules are by 5 (135
+// against 130).
 constexpr int kRaggedStages = 2;
 constexpr int64_t kRaggedStageBytes = 5120;
 constexpr int64_t kRaggedMinBytes = 256, kRaggedMinBytes8 = 512;
+constexpr int64_t kRaggedHostBytes = 512 << 10, kRaggedHostBytesShort = 4 << 20;  // of a batch from the host alone
+constexpr int64_t kRaggedHostRow4 = 512, kRaggedHostRow8 = 600;                     // rows below are short
 
 static size_t ragged_smem_bytes(int64_t row_bytes, int R) {
   return (size_t)kRowWarps * ((size_t)kRaggedStages * R * ragged_pitch(row_bytes) + 2 * kRaggedPad);
 }
 
-// Rows per ring buffer, 0 if the rows are too small to gain or do not fit.
-static int ragged_rows_per_stage(int64_t row_bytes, int vec, int R_small) {
+// Rows per ring buffer, 0 if the batch is not to gain or its rows do not fit.
+static int ragged_rows_per_stage(const RowJob& job, int vec) {
+  const int64_t row_bytes = job.row_bytes;
   if (vec == 16 || row_bytes < (vec == 8 ? kRaggedMinBytes8 : kRaggedMinBytes)) return 0;
+  if (job.mode == MODE_HOST && vec >= 4) {
+    const bool is_short = row_bytes < (vec == 8 ? kRaggedHostRow8 : kRaggedHostRow4);
+    if (job.n * row_bytes < (is_short ? kRaggedHostBytesShort : kRaggedHostBytes)) return 0;
+  }
   int64_t r = kRaggedStageBytes / ragged_pitch(row_bytes);
   if (r < 1) r = 1;
   if (r > 32) r = 32;
-  if (r > R_small) r = R_small;
+  if (r > job.rows_per_tile) r = job.rows_per_tile;
   return ragged_smem_bytes(row_bytes, (int)r) > kBulkSmemMax ? 0 : (int)r;
 }
 
@@ -745,7 +761,7 @@ static int launch_row_copy(const RowJob& job, int vec, cudaStream_t s) {
     static const bool no_bulk = getenv("SHMT_NO_BULK") != nullptr;
     const int R = no_bulk ? 0 : bulk_rows_per_stage(job.row_bytes, vec, job.rows_per_tile);
     if (R >= 1) return launch_bulk<SET>(job, R, s);
-    const int ragged = SET || no_bulk ? 0 : ragged_rows_per_stage(job.row_bytes, vec, job.rows_per_tile);
+    const int ragged = SET || no_bulk ? 0 : ragged_rows_per_stage(job, vec);
     if (ragged >= 1) return launch_ragged(job, ragged, s);
   }
   switch (vec) {

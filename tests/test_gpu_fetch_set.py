@@ -359,3 +359,19 @@ def test_rows_that_are_no_16_byte_units(capi, row_bytes, n):
         finally:
             capi.unpin_memory(pinned)
     assert capi.device_fault() == 0
+
+
+@pytest.mark.parametrize("row_bytes, n", [(260, 16_131), (260, 16_133), (508, 8256), (516, 1016), (516, 1017), (520, 8065),
+                                          (520, 8067), (600, 873), (600, 874)])
+def test_host_rows_around_the_line_between_narrow_copies_and_granules(capi, row_bytes, n):
+    """Batches from the host table alone: rows of 4- and 8-byte units on both sides of 4 MB a batch, and from
+    516 and 600 bytes on of 512 KB."""
+    rng = np.random.default_rng(row_bytes + n)
+    data = rng.integers(0, 256, size=(3000, row_bytes), dtype=np.uint8)
+    host = _pinned(capi, data.reshape(-1)).view(3000, row_bytes)
+    try:
+        q = rng.integers(0, 3000, size=n)
+        assert _bytes_equal(capi.uva_fetch(host, torch.from_numpy(q).cuda()), data[q])
+    finally:
+        capi.unpin_memory(host)
+    assert capi.device_fault() == 0
