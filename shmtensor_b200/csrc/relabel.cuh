@@ -171,11 +171,6 @@ __device__ __forceinline__ uint32_t relabel_enter(const RelRange& t, long long k
                                                   bool* maybe_first) {
   uint32_t pos = relabel_home(t, key);
   for (uint32_t round = 0;; ++round) {
-    if (round > t.full + 32) {  // there are never fewer slots than ids: cannot happen
-      atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
-      *maybe_first = false;
-      return pos;
-    }
     const RelPair p = relabel_load_pair(t.slots, pos & ~1u);
     const bool second = (pos & 1u) || (p.key0 != key && p.key0 != kEmptyKey);
     const long long cur = second ? p.key1 : p.key0;
@@ -187,13 +182,19 @@ __device__ __forceinline__ uint32_t relabel_enter(const RelRange& t, long long k
       return pos;
     }
     if (cur == kEmptyKey) {
-      if (CROWDED && !relabel_lowest(pos)) continue;  // reads next what the lowest lane did
+      // reads next what the lowest lane did: once per lane below this one at most, for the slot is taken then
+      if (CROWDED && !relabel_lowest(pos)) continue;
       const long long old = relabel_cas(t.slots + pos, key);
       if (old == kEmptyKey || old == key) {
         *maybe_first = !CROWDED || old == kEmptyKey || *reinterpret_cast<volatile unsigned*>(&t.slots[pos].first) > i;
         if (*maybe_first) atomicMin(&t.slots[pos].first, i);
         return pos;
       }
+    }
+    if (round > t.full) {  // there are never fewer slots than ids: cannot happen
+      atomicMax(reinterpret_cast<unsigned long long*>(status), (unsigned long long)DEV_OVERFLOW);
+      *maybe_first = false;
+      return pos;
     }
     pos = relabel_next(t, key, pos);
   }
