@@ -634,11 +634,9 @@ static int pick_rows_per_tile(int64_t n) {
 // inside the kernels), so there is no partly filled last wave.  The occupancy of a kernel with so
 // much shared memory is asked for once per device (1 us, a fifth of a small call) and kept beside the kernel.
 template <typename Kernel>
-static unsigned grid_for_tiles(Kernel kernel, KeptOccupancy* kept, int64_t n, int R, size_t smem = 0) {
+static unsigned grid_for_tiles(Kernel kernel, KeptOccupancy* kept, int dev, int64_t n, int R, size_t smem = 0) {
   const int64_t tiles = (n + R - 1) / R;
   int64_t blocks = (tiles + kRowWarps - 1) / kRowWarps;
-  int dev = -1;
-  cudaGetDevice(&dev);
   const int occ = kept->get(dev, smem, [&](int* ctas) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, kernel, kRowThreads, smem) == cudaSuccess;
   });
@@ -650,7 +648,9 @@ static unsigned grid_for_tiles(Kernel kernel, KeptOccupancy* kept, int64_t n, in
 template <int VEC, bool SET>
 static int launch_lsu(const RowJob& job, cudaStream_t s) {
   static KeptOccupancy kept;
-  const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, job.n, job.rows_per_tile);
+  int dev = 0;
+  SHMT_CUDA_TRY(cudaGetDevice(&dev));
+  const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, dev, job.n, job.rows_per_tile);
   row_copy_kernel<VEC, SET, 8><<<grid, kRowThreads, 0, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -691,7 +691,7 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   job.rows_per_tile = R;
   const size_t smem = (size_t)kRowWarps * kBulkStages * R * job.row_bytes;
   static KeptOccupancy kept;
-  const unsigned blocks = grid_for_tiles(kernel, &kept, job.n, R, smem);
+  const unsigned blocks = grid_for_tiles(kernel, &kept, dev, job.n, R, smem);
   kernel<<<blocks, kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
@@ -750,7 +750,7 @@ static int launch_ragged(RowJob job, int R, cudaStream_t s) {
   job.rows_per_tile = R;
   const size_t smem = ragged_smem_bytes(job.row_bytes, R);
   static KeptOccupancy kept;
-  kernel<<<grid_for_tiles(kernel, &kept, job.n, R, smem), kRowThreads, smem, s>>>(job);
+  kernel<<<grid_for_tiles(kernel, &kept, dev, job.n, R, smem), kRowThreads, smem, s>>>(job);
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
 }
@@ -909,7 +909,7 @@ int shmt_insert_set(shmt_map* map, void* gpu_base, const void* keys, int key_dty
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int R = pick_rows_per_tile(n);
   static KeptOccupancy kept;
-  const unsigned grid = grid_for_tiles(insert_set_kernel<16, 8>, &kept, n, R);
+  const unsigned grid = grid_for_tiles(insert_set_kernel<16, 8>, &kept, map->device, n, R);
   const int vec = pick_vec(row_bytes, {gpu_base, update});
   char* g = static_cast<char*>(gpu_base);
   const char* u = static_cast<const char*>(update);
