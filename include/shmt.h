@@ -57,6 +57,9 @@ int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx);
 int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, void* stream);
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                int n_hops, void* stream);
+/* The same, with room for a word per node of a graph of n_nodes (see shmt_sample_minibatch_pooled). */
+int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
+                                     int n_hops, int64_t n_nodes, void* stream);
 /* Wait for `stream` and report what the last asynchronous op on this context (a scan,
  * or a hop / relabel called without a host result pointer) left in its status word:
  * SHMT_OK, SHMT_ERR_TIMEOUT or SHMT_ERR_CAPACITY.  No counterpart in the reference.  */
@@ -318,6 +321,24 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
                                void* const* out_sub_indptr, void* const* out_sub_indices,
                                void* const* out_edge_ids, void* const* out_relabel,
                                void* const* out_frontier, int64_t* sizes_host, void* stream);
+
+/* The three mini-batches above as one call (weights, gpu_edge_base and what belongs to them may be null) that
+ * is also told how many rows indptr has: on graphs of up to 2^25 nodes ids are then relabelled through a
+ * word per node, behind the relabel table of the context, instead of hashed slots (n_nodes = 0: not known; ids of
+ * n_nodes and more are accepted and hashed).  The outputs lie in two pools, one per dtype: hop h's sub_indptr at
+ * element layout[h] of indptr_pool, its edge ids (if with_edge_ids) at layout[n_hops + h], and in
+ * indices_pool its sub_indices at layout[2 * n_hops + h], relabelled ids at layout[3 * n_hops + h] and frontier
+ * at layout[4 * n_hops + h].  Same results.  A context whose table was sized by shmt_ctx_reserve_minibatch
+ * does not grow for the words.                                                             */
+int shmt_sample_minibatch_pooled(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
+                                 const void* indices, int indices_dtype, const float* weights,
+                                 const void* gpu_indptr, const void* gpu_indices,
+                                 const float* gpu_weights, const void* gpu_edge_base,
+                                 const shmt_map* map, const void* seeds, int64_t n_seeds,
+                                 const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
+                                 uint64_t rng_offset, void* indptr_pool, void* indices_pool,
+                                 const int64_t* layout, int with_edge_ids, int64_t* sizes_host,
+                                 void* stream);
 
 /* Compact CSR of the selected rows, in the given order: CreateCacheCSR
  * (src/cache_graph_sampling.cu:455-492).  _count writes the n+1 offsets and

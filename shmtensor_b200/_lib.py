@@ -51,6 +51,7 @@ SIGNATURES = {
     "shmt_ctx_check": (_i, [_vp, _vp]),
     "shmt_ctx_reserve": (_i, [_vp, _i64, _i64, _vp]),
     "shmt_ctx_reserve_minibatch": (_i, [_vp, _i64, _pi64, _i, _vp]),
+    "shmt_ctx_reserve_minibatch_nodes": (_i, [_vp, _i64, _pi64, _i, _i64, _vp]),
     "shmt_map_table_bytes": (_i64, [_i64, _i64]),
     "shmt_map_create": (_i, [_i, _i64, _i64, _i, _i, _vp, _vp, _pvp]),
     "shmt_map_insert": (_i, [_vp, _vp, _vp, _i64, _vp]),
@@ -85,6 +86,8 @@ SIGNATURES = {
                                             _u64, _u64, _pvp, _pvp, _pvp, _pvp, _pi64, _vp]),
     "shmt_sample_minibatch_eids": (_i, [_vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i64, _pi64, _i, _i, _u64,
                                         _u64, _pvp, _pvp, _pvp, _pvp, _pvp, _pi64, _vp]),
+    "shmt_sample_minibatch_pooled": (_i, [_vp, _vp, _i, _i64, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _pi64,
+                                          _i, _i, _u64, _u64, _vp, _vp, _pi64, _i, _pi64, _vp]),
     "shmt_subcsr_count": (_i, [_vp, _vp, _i, _vp, _i, _i64, _vp, _pi64, _vp]),
     "shmt_subcsr_fill": (_i, [_vp, _i, _vp, _i, _vp, _i, _i64, _vp, _vp, _vp]),
     "shmt_shm_create": (_i, [_s, _i64, _i, _pi64, _pi64]),

@@ -93,14 +93,16 @@ def _ctx(device: torch.device) -> int:
     return h
 
 
-def reserve_minibatch(n_seeds: int, fanouts: Sequence[int], device="cuda") -> None:
+def reserve_minibatch(n_seeds: int, fanouts: Sequence[int], device="cuda", n_nodes: int = 0) -> None:
     """Extension: size the current stream's context for ``sample_minibatch`` calls of up to
-    ``n_seeds`` seeds with these fan-outs, so the first mini-batch does not stop to allocate."""
+    ``n_seeds`` seeds with these fan-outs, so the first mini-batch does not stop to allocate.
+    ``n_nodes``: rows of the graph, so that there is room for a word per node as well."""
     device = torch.device(device)
     if device.index is None:
         device = torch.device("cuda", torch.cuda.current_device())
     fan = (C.c_int64 * len(fanouts))(*[int(k) for k in fanouts])
-    check(lib.shmt_ctx_reserve_minibatch(_ctx(device), int(n_seeds), fan, len(fanouts), _stream(device)))
+    check(lib.shmt_ctx_reserve_minibatch_nodes(_ctx(device), int(n_seeds), fan, len(fanouts), int(n_nodes),
+                                               _stream(device)))
 
 
 def context_scratch_bytes(device="cuda") -> int:
@@ -691,7 +693,7 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
                      fanouts: Sequence[int], replace: bool = False, gpu_indptr=None,
                      gpu_indices=None, hashmap: "CUCOStaticHashmap | None" = None,
                      gpu_edge_base=None, return_eids: bool = False, weights=None, gpu_weights=None):
-    """Extension: all hops of a mini-batch in one native call (``shmt_sample_minibatch``).
+    """Extension: all hops of a mini-batch in one native call (``shmt_sample_minibatch_pooled``).
 
     Equivalent to, for each ``k`` in ``fanouts`` in the given order::
 
@@ -736,48 +738,31 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
     layout = _minibatch_layouts.get(key)
     if layout is None:
         def plan(dtype, counts):
-            item = _ITEMSIZE[dtype]
-            step = 16 // item
+            step = 16 // _ITEMSIZE[dtype]
             offs, lo = [], 0
             for c in counts:
                 offs.append(lo)
                 lo += -(-c // step) * step
-            return offs + [lo], item
-        p_off, p_item = plan(indptr.dtype, [caps[h] + 1 for h in range(n_hops)]
-                             + ([caps[h] * int(fanouts[h]) for h in range(n_hops)] if return_eids else []))
-        i_off, i_item = plan(indices.dtype, [caps[h] * int(fanouts[h]) for h in range(n_hops)]
-                             + [caps[h + 1] for h in range(n_hops)] * 2)
+            return offs + [lo]
+        p_off = plan(indptr.dtype, [caps[h] + 1 for h in range(n_hops)]
+                     + ([caps[h] * int(fanouts[h]) for h in range(n_hops)] if return_eids else []))
+        i_off = plan(indices.dtype, [caps[h] * int(fanouts[h]) for h in range(n_hops)]
+                     + [caps[h + 1] for h in range(n_hops)] * 2)
         fan = (C.c_int64 * n_hops)(*[int(k) for k in fanouts])
-        layout = _minibatch_layouts[key] = (p_off, p_item, i_off, i_item, fan)
-    p_off, p_item, i_off, i_item, fan = layout
+        eid_off = p_off[n_hops:2 * n_hops] if return_eids else [0] * n_hops
+        where = (C.c_int64 * (5 * n_hops))(*p_off[:n_hops], *eid_off, *i_off[:3 * n_hops])
+        layout = _minibatch_layouts[key] = (p_off, i_off, fan, where)
+    p_off, i_off, fan, where = layout
     p_pool = torch.empty(p_off[-1], dtype=indptr.dtype, device=dev)
     i_pool = torch.empty(i_off[-1], dtype=indices.dtype, device=dev)
-    p_base, i_base = p_pool.data_ptr(), i_pool.data_ptr()
-    VP = C.c_void_p * n_hops
     sizes = (C.c_int64 * (3 * n_hops))()
     offset = _rng["calls"] + 1
     _rng["calls"] += n_hops
-    out_ptr = VP(*[p_base + p_off[h] * p_item for h in range(n_hops)])
-    out_idx = VP(*[i_base + i_off[h] * i_item for h in range(n_hops)])
-    out_rel = VP(*[i_base + i_off[n_hops + h] * i_item for h in range(n_hops)])
-    out_front = VP(*[i_base + i_off[2 * n_hops + h] * i_item for h in range(n_hops)])
-    map_handle = hashmap._handle if hashmap is not None else None
-    if return_eids:
-        out_eid = VP(*[p_base + p_off[n_hops + h] * p_item for h in range(n_hops)])
-        check(lib.shmt_sample_minibatch_eids(
-            _ctx(dev), _ptr(indptr), pdt, _ptr(indices), xdt, _ptr(gpu_indptr), _ptr(gpu_indices),
-            _ptr(gpu_edge_base), map_handle, _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)),
-            _rng["seed"], offset, out_ptr, out_idx, out_eid, out_rel, out_front, sizes, _stream(dev)))
-    elif weights is not None:
-        check(lib.shmt_sample_minibatch_weighted(
-            _ctx(dev), _ptr(indptr), pdt, _ptr(indices), xdt, _ptr(weights), _ptr(gpu_indptr), _ptr(gpu_indices),
-            _ptr(gpu_weights), map_handle, _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)),
-            _rng["seed"], offset, out_ptr, out_idx, out_rel, out_front, sizes, _stream(dev)))
-    else:
-        check(lib.shmt_sample_minibatch(
-            _ctx(dev), _ptr(indptr), pdt, _ptr(indices), xdt, _ptr(gpu_indptr), _ptr(gpu_indices),
-            map_handle, _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)), _rng["seed"], offset,
-            out_ptr, out_idx, out_rel, out_front, sizes, _stream(dev)))
+    check(lib.shmt_sample_minibatch_pooled(
+        _ctx(dev), _ptr(indptr), pdt, max(indptr.numel() - 1, 0), _ptr(indices), xdt, _ptr(weights), _ptr(gpu_indptr),
+        _ptr(gpu_indices), _ptr(gpu_weights), _ptr(gpu_edge_base), hashmap._handle if hashmap is not None else None,
+        _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)), _rng["seed"], offset, p_pool.data_ptr(),
+        i_pool.data_ptr(), where, int(bool(return_eids)), sizes, _stream(dev)))
     # one split per pool gives every exact-size view: per piece the gap in front of it and the piece
     cuts_p, at_p, cuts_i, at_i = [], 0, [0] * (6 * n_hops), 0
     for h in range(n_hops):

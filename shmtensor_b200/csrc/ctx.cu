@@ -121,13 +121,15 @@ int ctx_reserve(shmt_ctx* ctx, size_t bytes) {
   return SHMT_OK;
 }
 
-int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
+int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words) {
   if (int rc = ctx_join_tail(ctx)) return rc;
-  if (bytes > ctx->table_bytes) {
+  if (bytes + words > ctx->table_bytes) {
     if (ctx->table) SHMT_CUDA_TRY(cudaFree(ctx->table));
     ctx->table = nullptr;
     ctx->table_bytes = 0;
+    ctx->table_words_bytes = 0;
     size_t want = bytes + bytes / 2;
+    if (want < bytes + words) want = bytes + words;
     if (want < ((size_t)4 << 20)) want = (size_t)4 << 20;
     want = (want + 255) & ~(size_t)255;
     void* p = nullptr;
@@ -139,7 +141,14 @@ int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
   if (ctx->table_dirty) {
     SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table, 0xFF, ctx->table_bytes, stream));
     ctx->table_dirty = false;
+    ctx->table_words_bytes = 0;
   }
+  if (bytes > ctx->table_bytes - ctx->table_words_bytes) {  // slots in the place of words
+    SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table + ctx->table_bytes - ctx->table_words_bytes, 0xFF, ctx->table_words_bytes,
+                                  stream));
+    ctx->table_words_bytes = 0;
+  }
+  if (words > ctx->table_words_bytes) ctx->table_words_bytes = words;  // empty slots are words at rest
   return SHMT_OK;
 }
 

@@ -13,6 +13,11 @@ struct shmt_ctx {
   char* table = nullptr;
   size_t table_bytes = 0;
   bool table_dirty = false;     // a failed call may have left entries behind
+  // Words of mini-batches (RelTable in relabel.cuh): the last table_words_bytes of the block.  At rest they
+  // hold marked numbers, not the all ones of empty slots, so slots that reach into them need them cleared.
+  size_t table_words_bytes = 0;
+  bool table_reserved = false;  // the caller sized the table for mini-batches: none of them grows it for words
+  unsigned* table_words(int64_t n) const { return reinterpret_cast<unsigned*>(table + table_bytes) - n; }
   // Early hand-over of result words (see HostPost): sequence number of the last post, and an
   // event behind the kernels that were still running when the call returned.
   int64_t post_seq = 0;
@@ -36,8 +41,9 @@ enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).
 int ctx_reserve(shmt_ctx* ctx, size_t bytes);
 
-// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with).
-int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
+// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with), and behind them `words`
+// bytes of words.
+int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words = 0);
 
 // Copy the first `n_words` result words to the host and wait for `stream`.
 // Returns SHMT_ERR_TIMEOUT / SHMT_ERR_CAPACITY if the kernel flagged either.

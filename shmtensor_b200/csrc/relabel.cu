@@ -391,8 +391,8 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
     first[j] = 0xFFFFFFFFu;
     id[j] = 0;
     if (maybe >> j & 1u) {
-      first[j] = __ldcg(&t.slots[pos[j]].first);
-      id[j] = part_elem(ps, sizes, base + 32 * j);
+      first[j] = __ldcg(relabel_first(t, pos[j]));
+      id[j] = pos[j] < t.n_words ? (int64_t)pos[j] : part_elem(ps, sizes, base + 32 * j);
     }
   }
   int before = 0, firsts = 0;  // first occurrences of earlier warps and of this one
@@ -425,7 +425,10 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
       const int64_t uid = row_uid + __popc(row & ((1u << lane) - 1u));
       store_int(unique, ps.is64, uid, id[j]);
       store_int(slot_of, ps.is64, i, uid);
-      *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, (unsigned)uid | kRelNewId, ~0u);
+      if (pos[j] < t.n_words)
+        t.words[pos[j]] = (unsigned)uid | kRelNewId;
+      else
+        *reinterpret_cast<uint4*>(t.slots + (pos[j] - t.n_words)) = make_uint4(~0u, ~0u, (unsigned)uid | kRelNewId, ~0u);
     } else if (maybe >> j & 1u) {
       store_int(slot_of, ps.is64, i, relabel_pack(pos[j], false, ps.is64));
     }
@@ -599,7 +602,7 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out) {
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (repeat[u]) newid[u] = __ldcg(&t.slots[pos[u]].first) & ~kRelNewId;
+      if (repeat[u]) newid[u] = __ldcg(relabel_first(t, pos[u])) & ~kRelNewId;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (repeat[u]) store_int(out, ps.is64, i0 + u * stride, (int64_t)newid[u]);
@@ -784,19 +787,21 @@ static RelScratch relabel_scratch(int64_t numel) {
 }
 size_t relabel_scratch_bytes(int64_t numel) { return relabel_scratch(numel).all; }
 
-int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s) {
+int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, int64_t n_words) {
   const uint64_t cap = relabel_capacity(numel_bound);
-  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s)) return rc;
+  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s, (size_t)n_words * sizeof(unsigned))) return rc;
   t->slots = reinterpret_cast<RelSlot*>(ctx->table);
   t->cap = (uint32_t)cap;
+  t->words = n_words ? ctx->table_words(n_words) : nullptr;
+  t->n_words = (uint32_t)n_words;
   return SHMT_OK;
 }
 
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
                    int64_t* status, int64_t* result, cudaStream_t s, bool inserted, bool pdl,
-                   const HostPost* post, RelSurvey* survey) {
+                   const HostPost* post, RelSurvey* survey, int64_t n_words) {
   RelTable t;
-  if (int rc = relabel_table(ctx, numel_bound, &t, s)) return rc;
+  if (int rc = relabel_table(ctx, numel_bound, &t, s, n_words)) return rc;
   const int64_t n_tiles = (numel_bound + kRelTile - 1) / kRelTile;
   int64_t blocks = (numel_bound + kRelThreads - 1) / kRelThreads;
   const int64_t cap_blocks = (int64_t)sm_count() * 16;

@@ -82,6 +82,8 @@ struct HopJob {
   // kernel would otherwise wait on memory.  rel_slots == nullptr: off.
   RelSlot* rel_slots;
   uint32_t rel_cap;
+  unsigned* rel_words;  // ids below rel_n_words take no slot (see RelTable)
+  uint32_t rel_n_words;
   void* rel_out;
   // Look-back state that the kernel itself puts back to zero (small single-hop calls): the zeroed word
   // in which its CTAs count themselves out, or nullptr.
@@ -324,7 +326,14 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
   auto enter = [&](int64_t i, IxT id) {
     bool maybe_first;
-    const uint32_t at = relabel_enter<false>(range, (long long)id, (unsigned)i, job.status, &maybe_first);
+    uint32_t at;
+    if ((uint64_t)(long long)id < job.rel_n_words) {
+      at = (uint32_t)id;
+      maybe_first = __ldcg(job.rel_words + at) > (unsigned)i;  // a mark counts as no index
+      if (maybe_first) atomicMin(job.rel_words + at, (unsigned)i);
+    } else {
+      at = job.rel_n_words + relabel_enter<false>(range, (long long)id, (unsigned)i, job.status, &maybe_first);
+    }
     store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
   };
 
@@ -834,6 +843,17 @@ static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, M
   return SHMT_OK;
 }
 
+// Words for the ids of a mini-batch of up to `numel_bound` of them on a graph of `n_nodes` (0: not known): all
+// or none.  None where positions would not fit 31 bits, or where a table that the caller has sized
+// would have to grow.
+static int64_t minibatch_words(const shmt_ctx* ctx, int64_t numel_bound, int64_t n_nodes) {
+  if (n_nodes > kRelMaxWords) return 0;
+  const uint64_t cap = relabel_capacity(numel_bound);
+  if (cap + (uint64_t)n_nodes >= kRelNotFirst32) return 0;
+  const bool fits = cap * sizeof(RelSlot) + (size_t)n_nodes * sizeof(unsigned) <= ctx->table_bytes;
+  return fits || !ctx->table_reserved ? n_nodes : 0;
+}
+
 }  // namespace shmt
 
 using namespace shmt;
@@ -842,7 +862,13 @@ extern "C" {
 
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts, int n_hops,
                                void* stream) {
+  return shmt_ctx_reserve_minibatch_nodes(ctx, n_seeds, fanouts, n_hops, 0, stream);
+}
+
+int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts, int n_hops,
+                                     int64_t n_nodes, void* stream) {
   SHMT_REQUIRE(ctx != nullptr, "shmt_ctx_reserve_minibatch: ctx is null");
+  SHMT_REQUIRE(n_nodes >= 0, "shmt_ctx_reserve_minibatch: negative node count");
   // weighted hops without replacement have the smaller tiles, and so the more descriptors, of the two
   MinibatchPlan plan, weighted;
   if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &plan)) return rc;
@@ -851,7 +877,11 @@ int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fa
   if (int rc = ctx_reserve(ctx, weighted.scratch_bytes > plan.scratch_bytes ? weighted.scratch_bytes : plan.scratch_bytes))
     return rc;
   RelTable t;
-  return relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream));
+  ctx->table_reserved = false;
+  const int64_t n_words = minibatch_words(ctx, plan.cap[n_hops], n_nodes);
+  if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream), n_words)) return rc;
+  ctx->table_reserved = true;
+  return SHMT_OK;
 }
 
 static int sample_hop_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
@@ -998,7 +1028,8 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
                                  void* const* out_sub_indices, void* const* out_relabel,
                                  void* const* out_frontier, int64_t* sizes_host, void* stream,
                                  const void* gpu_edge_base, void* const* out_edge_ids,
-                                 const float* weights = nullptr, const float* gpu_weights = nullptr) {
+                                 const float* weights = nullptr, const float* gpu_weights = nullptr,
+                                 int64_t n_nodes = 0) {
   SHMT_REQUIRE(ctx != nullptr, "shmt_sample_minibatch: ctx is null");
   SHMT_REQUIRE(valid_int_dtype(indptr_dtype) && valid_int_dtype(indices_dtype),
                "shmt_sample_minibatch: ID can only be int32 or int64");
@@ -1029,9 +1060,11 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
   SHMT_CUDA_TRY(cudaMemsetAsync(base, 0, cursor, s));  // words, tickets and every tile descriptor
   int64_t* status = words + n_hops * 8;
 
-  {  // the relabel table for the largest hop, reserved before anything is queued
+  // the relabel table for the largest hop, reserved before anything is queued
+  const int64_t n_words = minibatch_words(ctx, cap[n_hops], n_nodes);
+  {
     RelTable biggest;
-    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s)) return rc;
+    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s, n_words)) return rc;
   }
   const void* cur_seeds = seeds;
   HostPost post{};
@@ -1065,9 +1098,11 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
     job.status = status;
     job.result = w + 1;
     RelTable t;  // every sampler claims the relabel slots of what it emits
-    if (int rc = relabel_table(ctx, cap[h + 1], &t, s)) return rc;
+    if (int rc = relabel_table(ctx, cap[h + 1], &t, s, n_words)) return rc;
     job.rel_slots = t.slots;
     job.rel_cap = t.cap;
+    job.rel_words = t.words;
+    job.rel_n_words = t.n_words;
     job.rel_out = out_relabel[h];
     SHMT_CUDA_TRY(indices_dtype == SHMT_I64 ? launch_hop<long long>(job, hop_tiles[h], s, /*pdl=*/h > 0)
                                             : launch_hop<int>(job, hop_tiles[h], s, /*pdl=*/h > 0));
@@ -1086,7 +1121,8 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
     if (h == n_hops - 1) post = ctx_begin_post(ctx, words, n_hops * 8 + 8, w + 4);
     if (int rc = launch_relabel(ctx, ps, cap[h + 1], out_frontier[h], out_relabel[h],
                                 carve_tile_states(base + off_rel[h], rel_tiles[h]), w + 2, status,
-                                w + 3, s, /*inserted=*/true, /*pdl=*/true, h == n_hops - 1 ? &post : nullptr))
+                                w + 3, s, /*inserted=*/true, /*pdl=*/true, h == n_hops - 1 ? &post : nullptr,
+                                /*survey=*/nullptr, n_words))
       return rc;
     cur_seeds = out_frontier[h];
   }
@@ -1159,6 +1195,43 @@ int shmt_sample_minibatch_weighted(shmt_ctx* ctx, const void* indptr, int indptr
                                seeds, n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
                                out_sub_indices, out_relabel, out_frontier, sizes_host, stream, nullptr, nullptr,
                                weights, gpu_weights);
+}
+
+int shmt_sample_minibatch_pooled(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
+                                 const void* indices, int indices_dtype, const float* weights,
+                                 const void* gpu_indptr, const void* gpu_indices, const float* gpu_weights,
+                                 const void* gpu_edge_base, const shmt_map* map, const void* seeds, int64_t n_seeds,
+                                 const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
+                                 uint64_t rng_offset, void* indptr_pool, void* indices_pool, const int64_t* layout,
+                                 int with_edge_ids, int64_t* sizes_host, void* stream) {
+  SHMT_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops, "shmt_sample_minibatch_pooled: 1..%d hops", kMaxHops);
+  SHMT_REQUIRE(valid_int_dtype(indptr_dtype) && valid_int_dtype(indices_dtype),
+               "shmt_sample_minibatch_pooled: ID can only be int32 or int64");
+  SHMT_REQUIRE(indptr_pool && indices_pool && layout, "shmt_sample_minibatch_pooled: null argument");
+  SHMT_REQUIRE(n_nodes >= 0, "shmt_sample_minibatch_pooled: negative node count");
+  SHMT_REQUIRE(!weights || !with_edge_ids, "shmt_sample_minibatch_pooled: weights and edge ids cannot be combined");
+  SHMT_REQUIRE(!with_edge_ids || map == nullptr || gpu_edge_base != nullptr,
+               "shmt_sample_minibatch_pooled: edge ids of a cached graph need gpu_edge_base (shmt_subcsr_edge_base)");
+  SHMT_REQUIRE(!weights || map == nullptr || gpu_weights != nullptr,
+               "shmt_sample_minibatch_pooled: a cached graph needs gpu_weights");
+  for (int h = 0; weights && fanouts && h < n_hops; ++h)
+    SHMT_REQUIRE(replace || fanouts[h] <= 32,
+                 "shmt_sample_minibatch_pooled: without replacement the fan-out is at most 32 (hop %d has %lld)", h,
+                 (long long)fanouts[h]);
+  void *sub_indptr[kMaxHops], *sub_indices[kMaxHops], *relabel[kMaxHops], *frontier[kMaxHops], *edge_ids[kMaxHops];
+  char *p = static_cast<char*>(indptr_pool), *x = static_cast<char*>(indices_pool);
+  const int p_item = int_itemsize(indptr_dtype), x_item = int_itemsize(indices_dtype);
+  for (int h = 0; h < n_hops; ++h) {
+    sub_indptr[h] = p + layout[h] * p_item;
+    edge_ids[h] = with_edge_ids ? p + layout[n_hops + h] * p_item : nullptr;
+    sub_indices[h] = x + layout[2 * n_hops + h] * x_item;
+    relabel[h] = x + layout[3 * n_hops + h] * x_item;
+    frontier[h] = x + layout[4 * n_hops + h] * x_item;
+  }
+  return sample_minibatch_impl(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds,
+                               n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, sub_indptr, sub_indices,
+                               relabel, frontier, sizes_host, stream, gpu_edge_base, with_edge_ids ? edge_ids : nullptr,
+                               weights, gpu_weights, n_nodes);
 }
 
 int shmt_subcsr_count(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* seeds,

@@ -94,7 +94,8 @@ class GPUSamplingDataloader:
             # scratch belongs to the stream the sampling runs on)
             with torch.cuda.stream(self._side) if self._side is not None else contextlib.nullcontext():
                 capi.reserve_minibatch(max(1, min(self.batchsize, max(1, self.seeds.numel()))),
-                                       list(reversed(self.num_picks)), self.seeds.device)
+                                       list(reversed(self.num_picks)), self.seeds.device,
+                                       n_nodes=self.indptr.numel() - 1)
 
     # ------------------------------------------------------------------ seed bookkeeping
     def _local_share(self, seeds):

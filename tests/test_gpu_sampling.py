@@ -408,3 +408,52 @@ def test_sizes_handed_over_by_a_warp_for_one_to_eight_hops(capi, n_hops):
             assert np.array_equal(nxt.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
             cur = wu
         assert np.array_equal(front.cpu().numpy(), cur)
+
+
+@pytest.mark.parametrize("dt", [torch.int32, torch.int64])
+@pytest.mark.parametrize("k", [5, 16, 32, 40])
+def test_minibatch_relabel_by_words_and_slots(capi, dt, k):
+    """Ids below the row count are relabelled through a word per node, others (here half of the last hop's,
+    which have no row and are never sampled from) through slots.  Relabels of other sizes in between use the whole
+    table as slots, the words' place included; a table sized by reserve_minibatch does without words."""
+    rng = np.random.default_rng(k)
+    n = 3001
+    deg = rng.integers(0, 2 * k, size=n)
+    indptr_n = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    near = rng.integers(0, n, size=int(indptr_n[-1])).astype(DT[dt])
+    far = np.where(rng.random(near.size) < 0.5, near, near.astype(np.int64) + 2**30).astype(DT[dt])
+    indptr = torch.from_numpy(indptr_n).cuda()
+
+    def check(indices_n, fanouts, seeds_n):
+        front, hops = capi.sample_minibatch(indptr, torch.from_numpy(indices_n).cuda(), torch.from_numpy(seeds_n).cuda(),
+                                            fanouts, False)
+        cur = seeds_n
+        for (sp, sx, rel, nxt), fan in zip(hops, fanouts):
+            sp, sx = sp.cpu().numpy(), sx.cpu().numpy()
+            oracle.check_sample_bulk(indptr_n, indices_n, cur, fan, False, sp, sx)
+            wu, (_, wx) = oracle.tensor_relabel([cur, sx])
+            assert np.array_equal(nxt.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
+            cur = wu
+
+    def relabel(m):
+        ids = rng.integers(0, m, size=m).astype(DT[dt]) * 7
+        wu, (wx,) = oracle.tensor_relabel([ids])
+        unique, (local,) = capi.tensor_relabel([torch.from_numpy(ids).cuda()])
+        assert np.array_equal(unique.cpu().numpy(), wu) and np.array_equal(local.cpu().numpy(), wx)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):  # a context of its own, whose table starts small
+        for round_ in range(3):
+            check(far, [k], rng.permutation(n)[:200].astype(DT[dt]))
+            relabel((5_000, 30_000, 200_000)[round_])
+            check(near, [k, 3], rng.permutation(n)[:50 + 400 * round_].astype(DT[dt]))
+            check(far, [k], np.arange(n, dtype=DT[dt]))
+    other = torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(other):
+        capi.reserve_minibatch(n, [k])
+        held = capi.context_scratch_bytes()
+        check(far, [k], np.arange(n, dtype=DT[dt]))
+        assert capi.context_scratch_bytes() == held
+    torch.cuda.synchronize()
