@@ -41,6 +41,8 @@ enum : int { DEV_OK = 0, DEV_OVERFLOW = 1, DEV_TIMEOUT = 2 };
 
 // Launch `kernel` allowing it to overlap its scheduling with the tail of the previous kernel
 // in `stream` (see pdl_prologue); plain launch when `pdl` is false.
+// A launch takes 0.4 us longer where its parameters end in the last 16 bytes of a 64-byte line or at the line's end
+// (240, 256, 304, 320, 512 bytes: 6.9 us there and back; 208, 224, 272, 288, 352, 400: 6.5).
 #ifdef __CUDACC__
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block,

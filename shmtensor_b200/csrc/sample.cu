@@ -45,20 +45,22 @@ constexpr int kHopSeedStep = 8;
 constexpr double kHopSlotsPerEdge = 1.25;
 constexpr int kMaxSeedsPerTile = 1024;
 
-struct HopJob {
+struct HopJob {  // 288 bytes: see launch_kernel
   const void* indptr;
-  int indptr64;
   const void* indices;      // host / full graph
   const void* gpu_indptr;   // compact cached CSR (nullable)
   const void* gpu_indices;
   MapView map;
   const void* seeds;
-  int seeds64;
   int64_t n;
   int64_t k;
+  int indptr64, seeds64;
   int replace;
-  uint64_t rng_seed;
+  uint32_t rel_cap, rel_n_words;  // see rel_slots
   uint32_t off_lo, off_hi;
+  int seeds_per_tile;
+  uint32_t set_slots;     // fan-out > 32: words of the per-warp set of chosen positions (0: none)
+  uint64_t rng_seed;
   void* sub_indptr;
   void* sub_indices;
   TileStates st;
@@ -66,8 +68,6 @@ struct HopJob {
   int64_t* status;        // device status word
   int64_t* result;        // receives nnz
   const int64_t* n_dev;   // if set, the seed count is read here (it was produced on the device)
-  int seeds_per_tile;
-  uint32_t set_slots;     // fan-out > 32: words of the per-warp set of chosen positions (0: none)
   // Edge ids (optional): for every sampled neighbour its position in the full `indices` array,
   // in the dtype of indptr.  A cached row's position there is gpu_edge_base[slot] + offset in row.
   void* out_eids;
@@ -79,11 +79,9 @@ struct HopJob {
   // Fused relabel insert (multi-hop path): the kernel also claims a relabel-table slot for
   // every seed and every sampled neighbour, at its index in [seeds | neighbours], and
   // records the slot in rel_out -- the work of relabel's first kernel, done while this
-  // kernel would otherwise wait on memory.  rel_slots == nullptr: off.
+  // kernel would otherwise wait on memory.  rel_slots == nullptr: off (HOP_FUSED otherwise).
   RelSlot* rel_slots;
-  uint32_t rel_cap;
   unsigned* rel_words;  // ids below rel_n_words take no slot (see RelTable)
-  uint32_t rel_n_words;
   void* rel_out;
   // Look-back state that the kernel itself puts back to zero (small single-hop calls): the zeroed word
   // in which its CTAs count themselves out, or nullptr.
@@ -143,9 +141,42 @@ static_assert(kMaxSeedsPerTile <= 1 << 13, "a seed of the tile takes 13 bits");
 
 // Weighted picks without replacement (Efraimidis-Spirakis 2006): every edge gets the key -log(u) / w
 // (an exponential clock of rate w) and the k smallest keys win, which is sampling without
-// replacement with probabilities proportional to the weights.  The lanes 0..k-1 of a warp hold the k
-// smallest keys seen so far, ascending, equal keys by position; a smaller one is inserted by one
-// shuffle step.
+// replacement with probabilities proportional to the weights.  While a warp looks at a row, a candidate is one
+// number, its key above its position, so that numbers compare as keys, equal ones by position; the warp
+// holds the 32 smallest, ascending across its lanes.
+using Mark = unsigned long long;
+constexpr int kMarkPosBits = 32;
+constexpr Mark kNoMark = ~0ull;
+constexpr int kFewPicks = 4;      // taken as minima: 5,000 rows of 1,000 edges, one pick, 54 us sorted, 44 so
+constexpr int kMarkBuffer = 160;  // candidates a warp collects before it sorts them: up to 31 left and 128 new
+
+template <int N>
+__device__ __forceinline__ void sort_step(Mark (&v)[N], unsigned stride, bool ascending, unsigned lane) {
+  const bool low = ((lane & stride) == 0) == ascending;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const Mark other = __shfl_xor_sync(0xffffffffu, v[i], stride);
+    v[i] = (v[i] < other) == low ? v[i] : other;
+  }
+}
+// every v[i] ascending across the warp (bitonic)
+template <int N>
+__device__ __forceinline__ void sort_marks(Mark (&v)[N], unsigned lane) {
+#pragma unroll
+  for (unsigned size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (unsigned stride = size >> 1; stride > 0; stride >>= 1) sort_step<N>(v, stride, (lane & size) == 0, lane);
+}
+// the 32 smallest of v[i] and with[i], both ascending, into v[i]
+template <int N>
+__device__ __forceinline__ void merge_marks(Mark (&v)[N], const Mark* with, unsigned lane) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = min(v[i], __shfl_sync(0xffffffffu, with[i], 31 - lane));
+#pragma unroll
+  for (unsigned stride = 16; stride > 0; stride >>= 1) sort_step<N>(v, stride, true, lane);
+}
+
+// The k picks of a row, one per lane (0..k-1), ascending.
 struct WeightedPicks {
   float key;
   int64_t pos;
@@ -161,45 +192,121 @@ struct WeightedPicks {
     }
   }
 
-  // the edges [from, from + 128), then `step` further on, ... of a row of `deg` with weights `w`;
-  // a step's weights are loaded while the one before is looked at
-  __device__ __forceinline__ void scan(const float* w, int64_t from, int64_t step, int64_t deg, unsigned lane, int k,
-                                       const Philox& rng, uint32_t seed_idx, uint32_t off_lo, uint32_t off_hi) {
+  // The smallest marks of the edges [from, from + 128), then `step` further on, ... of `deg` with weights `w`; a
+  // step's weights are loaded while the one before is looked at.  Candidates, those below the k-th smallest key
+  // so far, go to `buf` and are sorted 32 to 128 at a time, the first 128 edges at once.  What bounds it is the
+  // warp's chain of instructions: put in one after the other, each by a shuffle step that waits for the one
+  // before, candidates cost 110 ns apiece; and with a vote and a division for every 32 edges the draws of a step
+  // waited for one another, 6.6 ns an edge and warp, 4.1 now.  Calls of 5,000 rows of 200 edges: 15 picks 43 -> 30 us,
+  // 32 picks 58 -> 31, of 1,000 edges 77 -> 59 and 102 -> 65; one row of 10,000: 38 -> 28, 100 of 100,000: 760 -> 540.
+  static __device__ __forceinline__ Mark scan_marks(const float* w, unsigned from, unsigned step, unsigned deg,
+                                                    unsigned lane, int k, const Philox& rng, uint32_t seed_idx,
+                                                    uint32_t counter0, uint32_t off_lo, uint32_t off_hi, Mark* buf) {
     constexpr int U = 4;
     const unsigned full = 0xffffffffu;
     const float tiny = 1.17549435e-38f, most = 3.40282347e+38f;  // smallest weight, largest key
     float next[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) next[u] = from + 32 * u + lane < deg ? __ldg(w + from + 32 * u + lane) : 1.0f;
-    float thr = __shfl_sync(full, key, k - 1);
-    for (int64_t p0 = from; p0 < deg; p0 += step) {
+    Mark best[1] = {kNoMark};
+    float thr = __int_as_float(0x7f800000), above = thr;  // the bound, and one that roundings do not reach
+    int held = 0;
+    for (unsigned p0 = from; p0 < deg; p0 += step) {
       float cur[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         cur[u] = next[u];
-        const int64_t ahead = p0 + step + 32 * u + lane;
+        const unsigned ahead = p0 + step + 32 * u + lane;
         if (ahead < deg) next[u] = __ldg(w + ahead);
       }
+      // the key is clock / weight; whether any may lie below the bound is seen without dividing, and at once
+      float clock[U];
+      bool maybe = false;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int64_t at = p0 + 32 * u + lane;
-        float mine = __int_as_float(0x7f800000);
-        if (at < deg) {
-          const uint4 r = rng(seed_idx, (uint32_t)at, off_lo, off_hi);
-          const float x = ((float)(r.x >> 8) + 1.0f) * (1.0f / 16777216.0f);  // (0, 1]
-          // a weight that is not positive counts as the smallest one; its edge can still be picked
-          mine = fminf(-__logf(x) / fmaxf(cur[u], tiny), most);
+        const unsigned at = p0 + 32 * u + lane;
+        const uint4 r = rng(seed_idx, counter0 + at, off_lo, off_hi);
+        const float x = ((float)(r.x >> 8) + 1.0f) * (1.0f / 16777216.0f);  // (0, 1]
+        clock[u] = -__logf(x);
+        cur[u] = fmaxf(cur[u], tiny);  // a weight that is not positive counts as the smallest; its edge can still be picked
+        maybe = maybe || (at < deg && clock[u] <= above * cur[u]);
+      }
+      if (__any_sync(full, maybe)) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const unsigned at = p0 + 32 * u + lane;
+          const float mine = fabsf(fminf(clock[u] / cur[u], most));  // no negative zero
+          const bool cand = at < deg && mine < thr;
+          const unsigned votes = __ballot_sync(full, cand);
+          if (cand) buf[held + __popc(votes & ((1u << lane) - 1u))] = ((Mark)__float_as_uint(mine) << kMarkPosBits) | at;
+          held += __popc(votes);
         }
-        unsigned cand = __ballot_sync(full, mine < thr);
-        while (cand) {
-          const int lead = __ffs(cand) - 1;
-          cand &= cand - 1;
-          const float ck = __shfl_sync(full, mine, lead);
-          if (ck < thr) {  // the bound may have dropped since the vote; same on every lane
-            insert(ck, p0 + 32 * u + lead, lane, k);
-            thr = __shfl_sync(full, key, k - 1);
+      }
+      const bool last = p0 + step >= deg;
+      while (held >= 32 || (last && held > 0)) {
+        __syncwarp();
+        const int n = min(held, 128);
+        held -= n;
+        if (k <= kFewPicks) {  // the k smallest one after the other
+          Mark v[5] = {best[0]}, kept = kNoMark;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u + 1] = 32 * u + (int)lane < n ? buf[held + 32 * u + lane] : kNoMark;
+          for (int t = 0; t < k; ++t) {
+            Mark least = v[0];
+#pragma unroll
+            for (int u = 1; u < 5; ++u) least = min(least, v[u]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) least = min(least, __shfl_xor_sync(full, least, o));
+            if ((int)lane == t) kept = least;
+#pragma unroll
+            for (int u = 0; u < 5; ++u)
+              if (v[u] == least) v[u] = kNoMark;
           }
+          best[0] = kept;
+        } else if (n <= 32) {
+          Mark v[1] = {(int)lane < n ? buf[held + lane] : kNoMark};
+          sort_marks<1>(v, lane);
+          merge_marks<1>(best, v, lane);
+        } else {
+          Mark v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u] = 32 * u + (int)lane < n ? buf[held + 32 * u + lane] : kNoMark;
+          sort_marks<4>(v, lane);
+          Mark two[2] = {v[0], v[1]};
+          merge_marks<2>(two, v + 2, lane);
+          Mark one[1] = {two[0]};
+          merge_marks<1>(one, two + 1, lane);
+          merge_marks<1>(best, one, lane);
         }
+        const unsigned bits = (unsigned)(__shfl_sync(full, best[0], k - 1) >> kMarkPosBits);
+        thr = __uint_as_float(min(bits, 0x7f800000u));
+        above = thr * 1.0001f;
+        __syncwarp();
+      }
+    }
+    return best[0];
+  }
+
+  // The same of a whole row (or this warp's share of it).  `key` and `pos` are those of no pick where there are
+  // fewer than k.  Rows of more than 2^31 edges are looked at piece by piece.
+  __device__ __forceinline__ void scan(const float* w, unsigned from, unsigned step, int64_t deg, unsigned lane, int k,
+                                       const Philox& rng, uint32_t seed_idx, uint32_t off_lo, uint32_t off_hi,
+                                       Mark* buf) {
+    constexpr int64_t kPiece = (int64_t)1 << 31;
+    for (int64_t p0 = 0; p0 < deg; p0 += kPiece) {
+      const Mark m = scan_marks(w + p0, from, step, (unsigned)min(deg - p0, kPiece), lane, k, rng, seed_idx, (uint32_t)p0, off_lo,
+                                off_hi, buf);
+      const float mk = m == kNoMark ? __int_as_float(0x7f800000) : __uint_as_float((unsigned)(m >> kMarkPosBits));
+      const int64_t mp = m == kNoMark ? -1 : p0 + (int64_t)(unsigned)m;
+      if (p0 == 0) {
+        key = mk;
+        pos = mp;
+        continue;
+      }
+      for (int t = 0; t < k; ++t) {
+        const float ck = __shfl_sync(0xffffffffu, mk, t);
+        const int64_t cp = __shfl_sync(0xffffffffu, mp, t);
+        if (cp >= 0) insert(ck, cp, lane, k);
       }
     }
   }
@@ -208,19 +315,24 @@ struct WeightedPicks {
 // Which rows of a tile the warps of the CTA share (a row's edges dealt out 128 at a time, the warps' picks
 // then ranked against one another), and which ones a warp takes alone: a hop is as long as its slowest
 // tile.  Alone rows run beside one another, shared rows one after the other, and a shared row is less
-// than an eighth as long: each warp still inserts its own k best.  So the longest rows are shared, as
-// many of them as make the tile's estimate smallest.  1,000 seeds of a power-law graph with rows of up to
-// 10,000 edges: 64 us with none shared and one load in flight, 24 with the longest shared; 8 rows of 2,000 edges, 15
-// picks each, in a tile: 138 us with all shared and merged one pick after the other, 39 with none.
-constexpr int64_t kWeightedLongRow = 1024;  // shorter rows are never shared
-// Times in edges looked at (6.6 ns): an insertion is worth 17, and a warp that looks at d edges inserts
-// about k * (1 + ln(d / k)) of them.
+// than an eighth as long: each warp still sorts its own candidates.  So the longest rows are shared, as
+// many of them as make the tile's estimate smallest.
+// Shorter rows are never shared (lines at 256 and 512: the same within 1 %, and 2 % behind on hops of 4,000 seeds).
+constexpr int64_t kWeightedLongRow = 1024;
+// Times in edges looked at (4 ns): the first sort is worth 170; behind the first 128 edges about k * ln(edges / 128)
+// candidates are collected, and sorted 32 at a time for 100.
 __device__ __forceinline__ float weighted_cost(float edges, float k) {
-  return edges <= k ? k : edges + 17.0f * k * (1.0f + __logf(edges / k));
+  if (edges <= k) return k;
+  return edges + 170.0f + (edges > 128.0f ? 100.0f + 3.0f * k * __logf(edges / 128.0f) : 0.0f);
 }
 constexpr float kWeightedShareCost = 200.0f;  // barriers, and the ranking
 
-template <typename IxT, int G, bool EARLY = false>
+// HOP_FUSED: a hop of a mini-batch, which also claims relabel slots.  HOP_SINGLE: a call of its own.  Kernels
+// apart, because the claims' code and registers cost a small call 0.7 of 24 us though it never runs it.  HOP_EARLY: a
+// weighted call whose count the host waits for (see step 3).
+enum : int { HOP_FUSED = 0, HOP_SINGLE = 1, HOP_EARLY = 2 };
+
+template <typename IxT, int G, int MODE>
 __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
   extern __shared__ __align__(16) unsigned char s_dyn[];  // hop_smem_bytes()
   __shared__ int64_t warp_sums[32];
@@ -256,7 +368,8 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     return;
   }
   const int tile = take_tile(job.ticket, &s_tile);  // as many CTAs as tiles are left
-  if (job.clean && tile == 0 && tid == 0) st_relaxed64(job.status, DEV_OK);  // it reports on this call only
+  constexpr bool kFused = MODE == HOP_FUSED, kEarly = MODE == HOP_EARLY;
+  if (!kFused && job.clean && tile == 0 && tid == 0) st_relaxed64(job.status, DEV_OK);  // it reports on this call only
   const int64_t first = (int64_t)tile * S;
   const int rows = (int)min((int64_t)S, n - first);
   const int64_t k = job.k;
@@ -317,11 +430,10 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const int group = (int)(tid / G);
   const Philox rng(job.rng_seed);
   IxT* out_all = static_cast<IxT*>(job.sub_indices);
-  const bool relabel = job.rel_slots != nullptr;
   const bool listed = G < 32 || (k <= G && !(job.weights && job.replace));  // a smaller group is only launched for such calls
   const double most = (double)n * (double)(1 + k);  // ids of this hop, were every row that long
   const RelRange range{job.rel_slots,
-                       relabel ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
+                       kFused ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
                        job.rel_cap};
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
   auto enter = [&](int64_t i, IxT id) {
@@ -346,11 +458,11 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       store_int(job.sub_indptr, job.indptr64, n, prefix + s_total);
       st_relaxed64(job.result, prefix + s_total);
     }
-    if (job.post.host) {  // uniform over the grid; the fused path (which may still flag the relabel table) never posts here
+    if (!kFused && job.post.host) {  // uniform over the grid
       __syncthreads();
       if (!job.clean && tid < 32) post_when_last(job.post, n_tiles);
     }
-    if (job.clean) {  // uniform as well; all look-backs of this CTA are over
+    if (!kFused && job.clean) {  // uniform as well; all look-backs of this CTA are over
       if (!job.post.host) __syncthreads();
       if (tid < 32 && last_to_finish(job.clean, n_tiles)) {
         for (int64_t t = lane; t < n_tiles; t += 32) st_desc(job.st.d + t, 0, 0);
@@ -365,10 +477,10 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     return prefix;
   };
 
-  // EARLY: picking by weight takes long, and a host that waits for the count need not wait for it, so the
+  // Picking by weight takes long, and a host that waits for the count need not wait for it, so the
   // tile takes its place first (8 rows of 1,000 edges, 15 picks each: 46.6 us a call, 31.2 so).  Both orders in one
   // kernel cost the other one: a weighted mini-batch of 1,000 seeds 130 us for 125.
-  const int64_t placed = EARLY ? place() : 0;
+  const int64_t placed = kEarly ? place() : 0;
 
   // ---- 3. (k <= 32) positions of the picked neighbours, a group of lanes per seed, into a list in
   // output order.  Arithmetic and shuffles only: the memory work is left to step 5, where all
@@ -378,6 +490,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     __shared__ int64_t s_pos[G == 32 ? kHopThreads : 1];
     __shared__ unsigned long long s_cut;
     const float none = __int_as_float(0x7f800000);
+    Mark* marks = reinterpret_cast<Mark*>(s_list + S * 32) + group * kMarkBuffer;  // behind the list
     auto weights_of = [&](int j) { return (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j]; };
     auto list = [&](int j, int at, int64_t pos) {
       s_list[s_off[j] + at] = HopEdge::pack(s_begin[j] + pos, j, s_hit[j]);
@@ -425,7 +538,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
         if ((int64_t)gl < deg) list(j, (int)gl, gl);
       } else if (!is_shared(j)) {
         WeightedPicks best{none, -1};
-        best.scan(weights_of(j), 0, 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo, job.off_hi);
+        best.scan(weights_of(j), 0, 128, deg, gl, (int)k, rng, (uint32_t)(first + j), job.off_lo, job.off_hi, marks);
         if ((int64_t)gl < k) list(j, (int)gl, best.pos);
       }
     }
@@ -433,7 +546,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       if (!is_shared(j)) continue;
       WeightedPicks best{none, -1};
       best.scan(weights_of(j), group * 128, kGroups * 128, s_deg[j], gl, (int)k, rng, (uint32_t)(first + j), job.off_lo,
-                job.off_hi);
+                job.off_hi, marks);
       __syncthreads();  // the row before has been ranked (and the estimates read)
       s_key[tid] = best.key;
       s_pos[tid] = best.pos;
@@ -491,7 +604,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
 
   // ---- 4. the tile's place in the output.  The first neighbours are fetched ahead of the look-back,
   // so that the two waits overlap.
-  const int lead = relabel ? rows : 0;  // the seeds come first: they are relabelled too
+  const int lead = kFused ? rows : 0;  // the seeds come first: they are relabelled too
   const int n_items = listed ? lead + (int)s_total : 0;
   auto fetch = [&](int e) -> IxT {
     if (e >= n_items) return IxT(0);
@@ -500,7 +613,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     return __ldg(static_cast<const IxT*>(x.hit() ? job.gpu_indices : job.indices) + x.at());
   };
   IxT next = fetch((int)tid);
-  const int64_t prefix = EARLY ? placed : place();
+  const int64_t prefix = kEarly ? placed : place();
 
   // ---- 5. output and relabel slots, one list element per thread and step
   if (listed) {
@@ -517,11 +630,11 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
           store_int(job.out_eids, job.indptr64, o, x.at() + s_eshift[x.seed()]);
         }
       }
-      if (relabel) enter(i, v);
+      if (kFused) enter(i, v);
     }
     return;
   }
-  if (relabel)
+  if (kFused)
     for (int j = (int)tid; j < rows; j += kHopThreads)
       enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
 
@@ -544,7 +657,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       const IxT val = __ldg(in + pos);
       out_all[o] = val;
       if (job.out_eids) store_int(job.out_eids, job.indptr64, o, s_begin[j] + pos + s_eshift[j]);
-      if (relabel) enter(n + o, val);
+      if (kFused) enter(n + o, val);
     };
     if (job.weights && deg > 0 && job.replace) {
       const float* w = (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j];
@@ -590,9 +703,9 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       auto drawn = [&](int64_t p) {
         return (int64_t)draw_below(rng, seed_idx, (uint32_t)p, job.off_lo, job.off_hi, (uint64_t)deg);
       };
-      // The plain hop has a short loop of its own, not unrolled: with the slot claims inlined into it 200,000
-      // seeds with 200 draws took 247 us, so 185 (two draws a step 184, but 33 to 40 draws 107 for 84).
-      if (!relabel && !job.out_eids) {
+      // The plain hop has a short loop of its own, not unrolled: 200,000 seeds with 200 draws take 185 us (two draws a
+      // step 184, but 33 to 40 draws 107 for 84).
+      if (!kFused && !job.out_eids) {
 #pragma unroll 1
         for (int64_t p = gl; p < k; p += 32) out_all[out_at + p] = __ldg(in + drawn(p));
       } else {
@@ -779,35 +892,43 @@ static uint32_t set_slots_for(int64_t k) {
 }
 
 // The per-seed arrays of a tile and what lies behind them (see the kernel).
-static size_t hop_smem_bytes(int seeds_per_tile, int64_t k, uint32_t set_slots) {
+static size_t hop_smem_bytes(int seeds_per_tile, int64_t k, uint32_t set_slots, bool marks = false) {
   const size_t list = k <= 32 ? (size_t)seeds_per_tile * (size_t)k * sizeof(uint64_t) : 0;
   const size_t sets = (size_t)set_slots * sizeof(uint32_t) * (kHopThreads / 32);
-  return (size_t)seeds_per_tile * (4 * sizeof(int64_t) + 1) + (list > sets ? list : sets);
+  return (size_t)seeds_per_tile * (4 * sizeof(int64_t) + 1) + (list > sets ? list : sets) +
+         (marks ? kMarkBuffer * sizeof(Mark) * (kHopThreads / 32) : 0);
+}
+
+template <typename IxT, int MODE>
+static cudaError_t launch_hop_as(const HopJob& job, unsigned grid, size_t smem, cudaStream_t s, bool pdl) {
+  if (!job.weights) {
+    if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8, MODE>, grid, kHopThreads, smem, s, job);
+    if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16, MODE>, grid, kHopThreads, smem, s, job);
+  }
+  if (smem > (48 << 10)) {
+    static bool configured[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev]) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(sample_hop_kernel<IxT, 32, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)hop_smem_bytes(kMaxSeedsPerTile, 33, 2 * kMaxSetPicks));
+      if (e != cudaSuccess) return e;
+      configured[dev] = true;
+    }
+  }
+  return launch_kernel(pdl, sample_hop_kernel<IxT, 32, MODE>, grid, kHopThreads, smem, s, job);
 }
 
 template <typename IxT>
 static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool pdl = false) {
   const unsigned grid = (unsigned)n_tiles;
   job.set_slots = set_slots_for(job.k);
-  const size_t smem = hop_smem_bytes(job.seeds_per_tile, hop_layout_k(job.weights, job.replace, job.k), job.set_slots);
-  if (!job.weights) {
-    if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8>, grid, kHopThreads, smem, s, job);
-    if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16>, grid, kHopThreads, smem, s, job);
-  }
+  const size_t smem = hop_smem_bytes(job.seeds_per_tile, hop_layout_k(job.weights, job.replace, job.k), job.set_slots,
+                                     job.weights && !job.replace);
+  if (job.rel_slots) return launch_hop_as<IxT, HOP_FUSED>(job, grid, smem, s, pdl);
   if (job.weights && !job.replace && job.post.host)  // the lists of fan-outs up to 32: within 48 KB
-    return launch_kernel(pdl, sample_hop_kernel<IxT, 32, true>, grid, kHopThreads, smem, s, job);
-  if (smem > (48 << 10)) {
-    static bool configured[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev]) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(sample_hop_kernel<IxT, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)hop_smem_bytes(kMaxSeedsPerTile, 33, 2 * kMaxSetPicks));
-      if (e != cudaSuccess) return e;
-      configured[dev] = true;
-    }
-  }
-  return launch_kernel(pdl, sample_hop_kernel<IxT, 32>, grid, kHopThreads, smem, s, job);
+    return launch_kernel(pdl, sample_hop_kernel<IxT, 32, HOP_EARLY>, grid, kHopThreads, smem, s, job);
+  return launch_hop_as<IxT, HOP_SINGLE>(job, grid, smem, s, pdl);
 }
 
 // Scratch layout of a multi-hop mini-batch, from its worst-case sizes (c_0 = n_seeds,

@@ -238,3 +238,31 @@ def test_a_row_yields_the_same_picks_alone_and_shared(capi, deg, k):
         assert picks(seeds)[at] == crowded[at]                   # among the longer ones of three
     assert picks([0])[0] == crowded[0]                           # and on its own
     assert len({tuple(r) for r in crowded}) == 8 and all(len(set(r)) == k for r in crowded)
+
+
+@pytest.mark.parametrize("k", [1, 4, 5, 15, 31, 32])
+def test_the_k_heavy_edges_win_wherever_they_lie(capi, k):
+    """k edges outweigh the others by more than any two clocks differ (2^-24 to 17, against 10^30), so they
+    are the picks exactly: candidates sorted 32 or 128 at a time, several sorts a row where the light edges
+    grow heavier along it, rows shared by a CTA and not, and fan-outs small enough to be picked one by one."""
+    rng = np.random.default_rng(k)
+    deg = np.array([k + 1, 32, 33, 64, 127, 128, 129, 159, 161, 500, 1000, 1024, 1025, 3000, 9000])
+    deg = np.maximum(deg, k + 1)
+    indptr_n = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    w = np.empty(indptr_n[-1], np.float32)
+    heavy = []
+    for b, d in zip(indptr_n, deg):
+        w[b:b + d] = 1e-20 * (1 + np.arange(d)) ** 2
+        at = rng.choice(d, size=k, replace=False)
+        if d > 40:
+            at = np.concatenate([[d - 1], at[at != d - 1]])[:k] if d % 2 else at
+        w[b + at] = np.float32(1e20) * (1 + rng.random(k)).astype(np.float32)
+        heavy.append(np.sort(at))
+    indptr, weights = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(w).cuda()
+    indices = torch.from_numpy(np.concatenate([np.arange(d) for d in deg]).astype(np.int32)).cuda()
+    for n in (1, 15, 600):
+        seeds_n = rng.integers(0, deg.size, size=n) if n != 15 else np.arange(deg.size)
+        p, x = capi.csr_weighted_sampling(indptr, indices, weights, torch.from_numpy(seeds_n).cuda(), k, False)
+        got = np.sort(x.cpu().numpy().reshape(n, k), 1)
+        assert np.array_equal(got, np.stack([heavy[s] for s in seeds_n]))
+        assert np.array_equal(p.cpu().numpy(), np.arange(n + 1) * k)
