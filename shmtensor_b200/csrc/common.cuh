@@ -41,12 +41,25 @@ enum : int { DEV_OK = 0, DEV_OVERFLOW = 1, DEV_TIMEOUT = 2 };
 
 // Launch `kernel` allowing it to overlap its scheduling with the tail of the previous kernel
 // in `stream` (see pdl_prologue); plain launch when `pdl` is false.
-// A launch takes 0.4 us longer where its parameters end in the last 16 bytes of a 64-byte line or at the line's end
-// (240, 256, 304, 320, 512 bytes: 6.9 us there and back; 208, 224, 272, 288, 352, 400: 6.5).
+//
+// The parameters of every kernel that a small call launches take 32 bytes modulo 64, with a LaunchPad at their end:
+// a launch takes least host time so (there and back 6.2 us; 24 or 40 modulo 64: 6.6; the others, 0 and 48 among
+// them: 6.9; sizes from 40 to 320 bytes).
+template <int BYTES>
+struct LaunchPad {
+  unsigned char unused[BYTES];
+};
+template <typename... P>
+constexpr size_t param_bytes() {
+  size_t at = 0;
+  ((at = (at + alignof(P) - 1) / alignof(P) * alignof(P) + sizeof(P)), ...);
+  return at;
+}
 #ifdef __CUDACC__
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block,
                                  size_t smem, cudaStream_t stream, Args... args) {
+  static_assert(param_bytes<KArgs...>() % 64 == 32, "see LaunchPad");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);

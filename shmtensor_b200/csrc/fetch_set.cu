@@ -44,6 +44,7 @@ struct RowJob {
   int64_t row_bytes;
   char* flat;             // fetch: output; set: update rows (request order)
   int rows_per_tile;      // R, 1..32
+  LaunchPad<60> pad;
 };
 
 template <int VEC> struct VecT;
@@ -651,8 +652,7 @@ static int launch_lsu(const RowJob& job, cudaStream_t s) {
   int dev = 0;
   SHMT_CUDA_TRY(cudaGetDevice(&dev));
   const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, dev, job.n, job.rows_per_tile);
-  row_copy_kernel<VEC, SET, 8><<<grid, kRowThreads, 0, s>>>(job);
-  SHMT_CUDA_TRY(cudaGetLastError());
+  SHMT_CUDA_TRY(launch_kernel(false, row_copy_kernel<VEC, SET, 8>, grid, kRowThreads, 0, s, job));
   return SHMT_OK;
 }
 
@@ -692,8 +692,7 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   const size_t smem = (size_t)kRowWarps * kBulkStages * R * job.row_bytes;
   static KeptOccupancy kept;
   const unsigned blocks = grid_for_tiles(kernel, &kept, dev, job.n, R, smem);
-  kernel<<<blocks, kRowThreads, smem, s>>>(job);
-  SHMT_CUDA_TRY(cudaGetLastError());
+  SHMT_CUDA_TRY(launch_kernel(false, kernel, blocks, kRowThreads, smem, s, job));
   return SHMT_OK;
 }
 
@@ -750,8 +749,7 @@ static int launch_ragged(RowJob job, int R, cudaStream_t s) {
   job.rows_per_tile = R;
   const size_t smem = ragged_smem_bytes(job.row_bytes, R);
   static KeptOccupancy kept;
-  kernel<<<grid_for_tiles(kernel, &kept, dev, job.n, R, smem), kRowThreads, smem, s>>>(job);
-  SHMT_CUDA_TRY(cudaGetLastError());
+  SHMT_CUDA_TRY(launch_kernel(false, kernel, grid_for_tiles(kernel, &kept, dev, job.n, R, smem), kRowThreads, smem, s, job));
   return SHMT_OK;
 }
 

@@ -69,7 +69,7 @@ __device__ __forceinline__ int relabel_sample_shift(int64_t numel) {
 // for 24 without such ids); a CTA therefore remembers what it has looked up.
 constexpr int kRelKnown = 1024;
 __global__ void __launch_bounds__(kRelThreads, 8)
-relabel_survey_kernel(Parts ps, RelSurvey* survey) {
+relabel_survey_kernel(Parts ps, RelSurvey* survey, LaunchPad<56>) {
   __shared__ unsigned s_marked[kRelThreads / 32];
   __shared__ unsigned long long s_largest[kRelThreads / 32];
   __shared__ uint32_t s_known[kRelKnown];  // bits this CTA has looked up or set, the last at each place
@@ -288,7 +288,7 @@ constexpr unsigned kRelSms = 148, kRelInsertCtas = 7;  // CTAs per SM
 
 __global__ void __launch_bounds__(kRelThreads, kRelInsertCtas)
 relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* status,
-                      const RelSurvey* __restrict__ survey) {
+                      const RelSurvey* __restrict__ survey, LaunchPad<8>) {
   pdl_prologue();
   const PartSizes sizes = resolve_sizes(ps);
   const int64_t numel = sizes.numel;
@@ -328,7 +328,7 @@ relabel_insert_kernel(Parts ps, RelTable t, void* __restrict__ out, int64_t* sta
 
 // Words and half-size slots are not emptied one by one: the front of the table is filled anew.
 __global__ void __launch_bounds__(kRelThreads)
-relabel_clear_kernel(RelTable t, int64_t numel, const RelSurvey* __restrict__ survey) {
+relabel_clear_kernel(RelTable t, int64_t numel, const RelSurvey* __restrict__ survey, LaunchPad<48>) {
   const RelSmall small = relabel_use(t, numel, survey).small;
   if (!small.words) return;
   uint4* dst = reinterpret_cast<uint4*>(small.words);
@@ -347,7 +347,7 @@ relabel_clear_kernel(RelTable t, int64_t numel, const RelSurvey* __restrict__ su
 template <int ITEMS>
 __global__ void __launch_bounds__(kRelThreads, 4)
 relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique, TileStates st,
-                       int64_t* ticket, int64_t* status, int64_t* result, HostPost post) {
+                       int64_t* ticket, int64_t* status, int64_t* result, HostPost post, LaunchPad<8>) {
   __shared__ int s_warp_firsts[kRelThreads / 32];
   __shared__ LookbackShared s_look;
   __shared__ int s_tile;
@@ -450,7 +450,7 @@ inline size_t flag_bytes(int64_t numel) {  // a bit per element, then a count pe
 
 __global__ void __launch_bounds__(kRelThreads, 6)
 relabel_flag_kernel(RelTable t, int is64, int64_t numel, void* slot_of, uint32_t* __restrict__ flags,
-                    int* __restrict__ counts, const RelSurvey* __restrict__ survey) {
+                    int* __restrict__ counts, const RelSurvey* __restrict__ survey, LaunchPad<16>) {
   __shared__ int s_count[kRelThreads / 32];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const RelView view(t, numel, survey);
@@ -493,7 +493,7 @@ relabel_flag_kernel(RelTable t, int is64, int64_t numel, void* slot_of, uint32_t
 // One CTA: counts -> first occurrences ahead of each tile; their number goes to the host.
 constexpr int kTotalThreads = 1024;
 __global__ void __launch_bounds__(kTotalThreads)
-relabel_total_kernel(int* counts, int n_tiles, int64_t* result, HostPost post) {
+relabel_total_kernel(int* counts, int n_tiles, int64_t* result, HostPost post, LaunchPad<32>) {
   __shared__ int64_t s_sums[32];
   __shared__ int64_t s_total;
   // a thread takes consecutive counts, four at a time (the array is 16-byte aligned and, past the
@@ -533,7 +533,7 @@ relabel_total_kernel(int* counts, int n_tiles, int64_t* result, HostPost post) {
 __global__ void __launch_bounds__(kRelThreads, 4)
 relabel_number_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique,
                       const uint32_t* __restrict__ flags, const int* __restrict__ before,
-                      const RelSurvey* __restrict__ survey) {
+                      const RelSurvey* __restrict__ survey, LaunchPad<56>) {
   const int tile_before = before[blockIdx.x];
   if (before[blockIdx.x + 1] == tile_before) return;
   static_assert(kFlagWords == 64, "two words of the tile per lane");
@@ -580,7 +580,7 @@ relabel_number_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ un
 
 // The repeats: slot -> new id.  First occurrences hold theirs already.
 __global__ void __launch_bounds__(kRelThreads)
-relabel_remap_kernel(Parts ps, RelTable t, void* out) {
+relabel_remap_kernel(Parts ps, RelTable t, void* out, LaunchPad<24>) {
   pdl_prologue();
   const PartSizes sizes = resolve_sizes(ps);
   const int64_t numel = sizes.numel;
@@ -611,7 +611,8 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out) {
 
 // The same for a surveyed input.
 __global__ void __launch_bounds__(kRelThreads, 8)
-relabel_remap_large_kernel(RelTable t, int is64, int64_t numel, void* out, const RelSurvey* __restrict__ survey) {
+relabel_remap_large_kernel(RelTable t, int is64, int64_t numel, void* out, const RelSurvey* __restrict__ survey,
+                           LaunchPad<32>) {
   const RelView view(t, numel, survey);
   constexpr int U = 2;  // 33.5 M ids: 8 reads per thread (5 CTAs) 354 us, 4 (6 CTAs) 232, 2 (8 CTAs) 187, 1 200
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -650,7 +651,7 @@ static size_t rel_small_smem(uint32_t slots) { return (size_t)slots * (sizeof(lo
 template <int ITEMS>
 __global__ void __launch_bounds__(kRelSmallThreads)
 relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* __restrict__ out, int64_t* status,
-                     int64_t* result, HostPost post) {
+                     int64_t* result, HostPost post, LaunchPad<48>) {
   constexpr int kWarps = kRelSmallThreads / 32;
   extern __shared__ __align__(16) unsigned char s_table[];
   long long* s_key = reinterpret_cast<long long*>(s_table);
@@ -751,9 +752,9 @@ static int launch_relabel_small(const Parts& ps, void* out_unique, void* out_rel
                                        (int)rel_small_smem(2 * ITEMS * kRelSmallThreads)));
     configured[dev] = true;
   }
-  relabel_small_kernel<ITEMS><<<1, kRelSmallThreads, rel_small_smem(slots), s>>>(
-      ps, slots, out_unique, out_relabel, words + W_STATUS, words + W_RESULT, post);
-  SHMT_CUDA_TRY(cudaGetLastError());
+  SHMT_CUDA_TRY(launch_kernel(false, relabel_small_kernel<ITEMS>, 1u, kRelSmallThreads, rel_small_smem(slots), s, ps,
+                              slots, out_unique, out_relabel, words + W_STATUS, words + W_RESULT, post,
+                              LaunchPad<48>{}));
   return SHMT_OK;
 }
 
@@ -807,37 +808,37 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
   const int64_t cap_blocks = (int64_t)sm_count() * 16;
   const unsigned grid = (unsigned)(blocks < cap_blocks ? blocks : cap_blocks);
   if (!inserted) {
-    if (survey) SHMT_CUDA_TRY(launch_kernel(pdl, relabel_survey_kernel, grid, kRelThreads, 0, s, ps, survey));
+    if (survey) SHMT_CUDA_TRY(launch_kernel(pdl, relabel_survey_kernel, grid, kRelThreads, 0, s, ps, survey, LaunchPad<56>{}));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_insert_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel, status,
-                                (const RelSurvey*)survey));
+                                (const RelSurvey*)survey, LaunchPad<8>{}));
   }
   if (survey) {
     const int64_t tiles = flag_tiles(numel_bound);  // surveyed inputs are of that size exactly
     uint32_t* flags = reinterpret_cast<uint32_t*>(survey + 1);
     int* counts = reinterpret_cast<int*>(flags + tiles * kFlagWords);
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_flag_kernel, (unsigned)tiles, kRelThreads, 0, s, t, ps.is64, numel_bound,
-                                out_relabel, flags, counts, (const RelSurvey*)survey));
+                                out_relabel, flags, counts, (const RelSurvey*)survey, LaunchPad<16>{}));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_total_kernel, 1u, kTotalThreads, 0, s, counts, (int)tiles, result,
-                                post ? *post : HostPost{}));
+                                post ? *post : HostPost{}, LaunchPad<32>{}));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_number_kernel, (unsigned)tiles, kRelThreads, 0, s, ps, t, out_relabel,
-                                out_unique, (const uint32_t*)flags, (const int*)counts, (const RelSurvey*)survey));
+                                out_unique, (const uint32_t*)flags, (const int*)counts, (const RelSurvey*)survey, LaunchPad<56>{}));
   } else if (numel_bound >= kRelLargeInput) {
     const int64_t big_tiles = (numel_bound + kRelThreads * kRelItemsLarge - 1) / (kRelThreads * kRelItemsLarge);
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItemsLarge>, (unsigned)big_tiles, kRelThreads, 0, s,
                                 ps, t, out_relabel, out_unique, st, ticket, status, result,
-                                post ? *post : HostPost{}));
+                                post ? *post : HostPost{}, LaunchPad<8>{}));
   } else {
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItems>, (unsigned)n_tiles, kRelThreads, 0, s, ps, t,
                                 out_relabel, out_unique, st, ticket, status, result,
-                                post ? *post : HostPost{}));
+                                post ? *post : HostPost{}, LaunchPad<8>{}));
   }
   if (!survey) {
-    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel));
+    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel, LaunchPad<24>{}));
   } else {
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_large_kernel, grid, kRelThreads, 0, s, t, ps.is64, numel_bound,
-                                out_relabel, (const RelSurvey*)survey));
+                                out_relabel, (const RelSurvey*)survey, LaunchPad<32>{}));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_clear_kernel, grid, kRelThreads, 0, s, t, numel_bound,
-                                (const RelSurvey*)survey));
+                                (const RelSurvey*)survey, LaunchPad<48>{}));
   }
   SHMT_CUDA_TRY(cudaGetLastError());
   return SHMT_OK;
