@@ -57,7 +57,7 @@ int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx);
 int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, void* stream);
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                int n_hops, void* stream);
-/* The same, with room for a word per node of a graph of n_nodes (see shmt_sample_minibatch_pooled). */
+/* The same, with room for a word per node of a graph of n_nodes (see shmt_minibatch_start). */
 int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                      int n_hops, int64_t n_nodes, void* stream);
 /* Wait for `stream` and report what the last asynchronous op on this context (a scan,
@@ -329,16 +329,20 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
  * element layout[h] of indptr_pool, its edge ids (if with_edge_ids) at layout[n_hops + h], and in
  * indices_pool its sub_indices at layout[2 * n_hops + h], relabelled ids at layout[3 * n_hops + h] and frontier
  * at layout[4 * n_hops + h].  Same results.  A context whose table was sized by shmt_ctx_reserve_minibatch
- * does not grow for the words.                                                             */
-int shmt_sample_minibatch_pooled(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
-                                 const void* indices, int indices_dtype, const float* weights,
-                                 const void* gpu_indptr, const void* gpu_indices,
-                                 const float* gpu_weights, const void* gpu_edge_base,
-                                 const shmt_map* map, const void* seeds, int64_t n_seeds,
-                                 const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
-                                 uint64_t rng_offset, void* indptr_pool, void* indices_pool,
-                                 const int64_t* layout, int with_edge_ids, int64_t* sizes_host,
-                                 void* stream);
+ * does not grow for the words.
+ *
+ * shmt_minibatch_start returns when everything is queued.  shmt_minibatch_hop waits until the sizes of a hop are
+ * known (seeds in, edges sampled, distinct ids out), while the hops behind it may still run; asked for the last
+ * hop it also reports an error of any of them, and the mini-batch is over.  No other call uses the context
+ * in between.                                                                                */
+int shmt_minibatch_start(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
+                         const void* indices, int indices_dtype, const float* weights,
+                         const void* gpu_indptr, const void* gpu_indices, const float* gpu_weights,
+                         const void* gpu_edge_base, const shmt_map* map, const void* seeds,
+                         int64_t n_seeds, const int64_t* fanouts, int n_hops, int replace,
+                         uint64_t rng_seed, uint64_t rng_offset, void* indptr_pool,
+                         void* indices_pool, const int64_t* layout, int with_edge_ids, void* stream);
+int shmt_minibatch_hop(shmt_ctx* ctx, int hop, int64_t* sizes_host);
 
 /* Compact CSR of the selected rows, in the given order: CreateCacheCSR
  * (src/cache_graph_sampling.cu:455-492).  _count writes the n+1 offsets and

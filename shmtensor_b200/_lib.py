@@ -86,8 +86,9 @@ SIGNATURES = {
                                             _u64, _u64, _pvp, _pvp, _pvp, _pvp, _pi64, _vp]),
     "shmt_sample_minibatch_eids": (_i, [_vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i64, _pi64, _i, _i, _u64,
                                         _u64, _pvp, _pvp, _pvp, _pvp, _pvp, _pi64, _vp]),
-    "shmt_sample_minibatch_pooled": (_i, [_vp, _vp, _i, _i64, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _pi64,
-                                          _i, _i, _u64, _u64, _vp, _vp, _pi64, _i, _pi64, _vp]),
+    "shmt_minibatch_start": (_i, [_vp, _vp, _i, _i64, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _pi64, _i, _i,
+                                  _u64, _u64, _vp, _vp, _pi64, _i, _vp]),
+    "shmt_minibatch_hop": (_i, [_vp, _i, _pi64]),
     "shmt_subcsr_count": (_i, [_vp, _vp, _i, _vp, _i, _i64, _vp, _pi64, _vp]),
     "shmt_subcsr_fill": (_i, [_vp, _i, _vp, _i, _vp, _i, _i64, _vp, _vp, _vp]),
     "shmt_shm_create": (_i, [_s, _i64, _i, _pi64, _pi64]),

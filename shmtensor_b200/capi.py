@@ -123,6 +123,7 @@ def _row_bytes(data: torch.Tensor) -> int:
 _rng = {"seed": 7777, "calls": 0}
 _ITEMSIZE = {torch.int32: 4, torch.int64: 8}
 _minibatch_layouts: dict = {}
+_ONE = (1,)
 
 
 def set_sampling_seed(seed: int) -> None:
@@ -531,29 +532,44 @@ def tensor_relabel(tensors: List[torch.Tensor]):
         raise RuntimeError("tensor_relabel: expected a non-empty list of tensors")
     dev = tensors[0].device
     dt = tensors[0].dtype
+    plain = True
     for t in tensors:
         _check_cuda(t, "tensors")
         if t.device != dev:
             raise RuntimeError("tensor_relabel: all tensors must share a device")
         if t.dtype != dt:
             dt = torch.promote_types(dt, t.dtype)  # what the reference's torch::cat does
+            plain = False
+        plain = plain and t.is_contiguous()
     code = _INT_CODES.get(dt)
     if code is None:
         raise RuntimeError(f"tensor_relabel: ID can only be int32 or int64, got {dt}")
-    sizes = [t.numel() for t in tensors]
-    parts = [t.contiguous().to(dt) for t in tensors]
-    if len(parts) > 8:
-        parts = [torch.cat([p.reshape(-1) for p in parts], 0)]
+    parts = tensors if plain else [t.contiguous().to(dt) for t in tensors]
+    sizes = [t.numel() for t in parts]
     total = sum(sizes)
-    unique = torch.empty(total, dtype=dt, device=dev)
-    relabel = torch.empty(total, dtype=dt, device=dev)
     n_parts = len(parts)
-    ptrs = (C.c_void_p * n_parts)(*[_ptr(p) for p in parts])
-    lens = (C.c_int64 * n_parts)(*[p.numel() for p in parts])
+    if n_parts > 8:
+        parts, n_parts = [torch.cat([p.reshape(-1) for p in parts], 0)], 1
     n_unique = C.c_int64(0)
-    check(lib.shmt_relabel(_ctx(dev), ptrs, lens, n_parts, code, _ptr(unique), _ptr(relabel),
-                           C.byref(n_unique), _stream(dev)))
-    return unique[:n_unique.value], list(relabel.split_with_sizes(sizes))
+    # small results share an allocation and are cut from it at once
+    pooled = total <= _SMALL_RELABEL
+    unique = torch.empty(2 * total if pooled else total, dtype=dt, device=dev)
+    relabel = None if pooled else torch.empty(total, dtype=dt, device=dev)
+    u_ptr = unique.data_ptr()
+    ptrs, lens = _PTRS[n_parts](*[_ptr(p) for p in parts]), _LENS[n_parts](*(sizes if len(sizes) == n_parts else [total]))
+    check(lib.shmt_relabel(_ctx(dev), ptrs, lens, n_parts, code, u_ptr or None,
+                           (u_ptr + total * _ITEMSIZE[dt] if pooled else relabel.data_ptr()) or None, C.byref(n_unique),
+                           _stream(dev)))
+    found = n_unique.value
+    if pooled:
+        cut = unique.split_with_sizes([found, total - found, *sizes])
+        return cut[0], list(cut[2:])
+    return unique[:found], list(relabel.split_with_sizes(sizes))
+
+
+_SMALL_RELABEL = 1 << 16
+_PTRS = [C.c_void_p * n for n in range(9)]
+_LENS = [C.c_int64 * n for n in range(9)]
 
 
 # --------------------------------------------------------------------------- sampling
@@ -561,8 +577,8 @@ def _sample(indptr, indices, gpu_indptr, gpu_indices, hashmap, seeds, num_picks,
     _check_cuda(seeds, "seeds")
     seeds = seeds.contiguous()
     dev = seeds.device
-    for t, nm in ((indptr, "indptr"), (indices, "indices")):
-        _check_contig(t, nm)
+    _check_contig(indptr, "indptr")
+    _check_contig(indices, "indices")
     pdt, xdt, sdt = _int_code(indptr, who), _int_code(indices, who), _int_code(seeds, who)
     if hashmap is not None:
         _check_cuda(gpu_indptr, "gpu_indptr")
@@ -576,10 +592,10 @@ def _sample(indptr, indices, gpu_indptr, gpu_indices, hashmap, seeds, num_picks,
     _rng["calls"] += 1
     check(lib.shmt_sample_hop(_ctx(dev), _ptr(indptr), pdt, _ptr(indices), xdt, _ptr(gpu_indptr),
                               _ptr(gpu_indices), hashmap._handle if hashmap is not None else None,
-                              _ptr(seeds), sdt, n, k, int(bool(replace)), _rng["seed"],
+                              _ptr(seeds), sdt, n, k, bool(replace), _rng["seed"],
                               _rng["calls"], sub_indptr.data_ptr(), _ptr(sub_indices),
                               C.byref(nnz), _stream(dev)))
-    return sub_indptr, sub_indices[:nnz.value]
+    return sub_indptr, sub_indices.as_strided((nnz.value,), _ONE)
 
 
 def csr_sampling(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.Tensor,
@@ -693,7 +709,7 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
                      fanouts: Sequence[int], replace: bool = False, gpu_indptr=None,
                      gpu_indices=None, hashmap: "CUCOStaticHashmap | None" = None,
                      gpu_edge_base=None, return_eids: bool = False, weights=None, gpu_weights=None):
-    """Extension: all hops of a mini-batch in one native call (``shmt_sample_minibatch_pooled``).
+    """Extension: all hops of a mini-batch queued by one native call (``shmt_minibatch_start``).
 
     Equivalent to, for each ``k`` in ``fanouts`` in the given order::
 
@@ -710,16 +726,12 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
     """
     _check_cuda(seeds, "seeds")
     dev = seeds.device
-    for t, nm in ((indptr, "indptr"), (indices, "indices")):
-        _check_contig(t, nm)
+    _check_contig(indptr, "indptr")
+    _check_contig(indices, "indices")
     pdt, xdt = _int_code(indptr, "sample_minibatch"), _int_code(indices, "sample_minibatch")
-    seeds = seeds.contiguous().to(indices.dtype)
-    n_hops = len(fanouts)
-    caps = [seeds.numel()]
-    for k in fanouts:
-        caps.append(caps[-1] * (1 + int(k)))
-    # two allocations (one per dtype); the per-hop outputs are 16-byte aligned pieces of them,
-    # handed to the library as raw addresses and turned into views only once sizes are known
+    if seeds.dtype is not indices.dtype or not seeds.is_contiguous():
+        seeds = seeds.contiguous().to(indices.dtype)
+    n_seeds = seeds.numel()
     if return_eids and hashmap is not None and gpu_edge_base is None:
         raise RuntimeError("sample_minibatch: edge ids of a cached graph need gpu_edge_base")
     if weights is not None:
@@ -734,61 +746,66 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
             _check_cuda(gpu_weights, "gpu_weights")
             if gpu_weights.dtype != torch.float32 or gpu_weights.numel() != gpu_indices.numel():
                 raise RuntimeError("sample_minibatch: gpu_weights must be float32, one per cached edge")
-    key = (seeds.numel(), tuple(int(k) for k in fanouts), indptr.dtype, indices.dtype, bool(return_eids))
-    layout = _minibatch_layouts.get(key)
-    if layout is None:
-        def plan(dtype, counts):
-            step = 16 // _ITEMSIZE[dtype]
-            offs, lo = [], 0
-            for c in counts:
-                offs.append(lo)
-                lo += -(-c // step) * step
-            return offs + [lo]
-        p_off = plan(indptr.dtype, [caps[h] + 1 for h in range(n_hops)]
-                     + ([caps[h] * int(fanouts[h]) for h in range(n_hops)] if return_eids else []))
-        i_off = plan(indices.dtype, [caps[h] * int(fanouts[h]) for h in range(n_hops)]
-                     + [caps[h + 1] for h in range(n_hops)] * 2)
-        fan = (C.c_int64 * n_hops)(*[int(k) for k in fanouts])
-        eid_off = p_off[n_hops:2 * n_hops] if return_eids else [0] * n_hops
-        where = (C.c_int64 * (5 * n_hops))(*p_off[:n_hops], *eid_off, *i_off[:3 * n_hops])
-        layout = _minibatch_layouts[key] = (p_off, i_off, fan, where)
-    p_off, i_off, fan, where = layout
-    p_pool = torch.empty(p_off[-1], dtype=indptr.dtype, device=dev)
-    i_pool = torch.empty(i_off[-1], dtype=indices.dtype, device=dev)
-    sizes = (C.c_int64 * (3 * n_hops))()
+    # two allocations (one per dtype); the per-hop outputs are 16-byte aligned pieces of them, which become
+    # views as their sizes arrive
+    fan = tuple(fanouts)
+    if not all(type(k) is int for k in fan):
+        fan = tuple(int(k) for k in fan)
+    key = (n_seeds, fan, pdt, xdt, bool(return_eids))
+    layout = _minibatch_layouts.get(key) or _minibatch_layout(key)
+    p_size, i_size, fan_c, where_c, where = layout
+    n_hops = len(fan)
+    p_pool = torch.empty(p_size, dtype=indptr.dtype, device=dev)
+    i_pool = torch.empty(i_size, dtype=indices.dtype, device=dev)
     offset = _rng["calls"] + 1
     _rng["calls"] += n_hops
-    check(lib.shmt_sample_minibatch_pooled(
-        _ctx(dev), _ptr(indptr), pdt, max(indptr.numel() - 1, 0), _ptr(indices), xdt, _ptr(weights), _ptr(gpu_indptr),
+    ctx = _ctx(dev)
+    check(lib.shmt_minibatch_start(
+        ctx, _ptr(indptr), pdt, max(indptr.numel() - 1, 0), _ptr(indices), xdt, _ptr(weights), _ptr(gpu_indptr),
         _ptr(gpu_indices), _ptr(gpu_weights), _ptr(gpu_edge_base), hashmap._handle if hashmap is not None else None,
-        _ptr(seeds), seeds.numel(), fan, n_hops, int(bool(replace)), _rng["seed"], offset, p_pool.data_ptr(),
-        i_pool.data_ptr(), where, int(bool(return_eids)), sizes, _stream(dev)))
-    # one split per pool gives every exact-size view: per piece the gap in front of it and the piece
-    cuts_p, at_p, cuts_i, at_i = [], 0, [0] * (6 * n_hops), 0
-    for h in range(n_hops):
-        take = sizes[3 * h] + 1
-        cuts_p += (p_off[h] - at_p, take)
-        at_p = p_off[h] + take
-    if return_eids:
-        for h in range(n_hops):
-            take = sizes[3 * h + 1]
-            cuts_p += (p_off[n_hops + h] - at_p, take)
-            at_p = p_off[n_hops + h] + take
-    cuts_p.append(p_off[-1] - at_p)
-    for piece in range(3 * n_hops):
-        kind, h = divmod(piece, n_hops)  # neighbours, their new ids (behind the seeds'), the frontier
-        start = i_off[piece] + (sizes[3 * h] if kind == 1 else 0)
-        take = sizes[3 * h + 2] if kind == 2 else sizes[3 * h + 1]
-        cuts_i[2 * piece] = start - at_i
-        cuts_i[2 * piece + 1] = take
-        at_i = start + take
-    cuts_i.append(i_off[-1] - at_i)
-    pv = p_pool.split_with_sizes(cuts_p)
-    iv = i_pool.split_with_sizes(cuts_i)
-    hops = [(pv[2 * h + 1], iv[2 * h + 1], iv[2 * (n_hops + h) + 1], iv[2 * (2 * n_hops + h) + 1])
-            + ((pv[2 * (n_hops + h) + 1],) if return_eids else ())
-            for h in range(n_hops)]
+        _ptr(seeds), n_seeds, fan_c, n_hops, bool(replace), _rng["seed"], offset, p_pool.data_ptr(),
+        i_pool.data_ptr(), where_c, bool(return_eids), _stream(dev)))
+    # the sizes of a hop arrive while those behind it run, and its views are made meanwhile
+    sizes = (C.c_int64 * 3)()
+    hops = []
+    for h, (p_at, e_at, x_at, r_at, f_at) in enumerate(where):
+        check(lib.shmt_minibatch_hop(ctx, h, sizes))
+        n_in, nnz, n_out = sizes
+        hop = (p_pool.as_strided((n_in + 1,), _ONE, p_at), i_pool.as_strided((nnz,), _ONE, x_at),
+               i_pool.as_strided((nnz,), _ONE, r_at + n_in),  # behind the seeds' new ids
+               i_pool.as_strided((n_out,), _ONE, f_at))
+        hops.append(hop + (p_pool.as_strided((nnz,), _ONE, e_at),) if return_eids else hop)
     return hops[-1][3], hops
+
+
+def _minibatch_layout(key):
+    """Sizes of the two pools of ``sample_minibatch``, and where in them the outputs of every hop lie:
+    ``(sub_indptr, edge ids)`` and ``(sub_indices, relabelled ids, frontier)``."""
+    n_seeds, fan, pdt, xdt, return_eids = key
+    caps = [n_seeds]
+    for k in fan:
+        caps.append(caps[-1] * (1 + k))
+    n_hops = len(fan)
+
+    def plan(code, counts):
+        step = 16 // _ITEMSIZE[_CODE_DTYPES[code]]
+        offs, lo = [], 0
+        for c in counts:
+            offs.append(lo)
+            lo += -(-c // step) * step
+        return offs, lo
+
+    edges = [caps[h] * fan[h] for h in range(n_hops)]
+    p_off, p_size = plan(pdt, [c + 1 for c in caps[:-1]] + (edges if return_eids else []))
+    i_off, i_size = plan(xdt, edges + caps[1:] * 2)
+    p_off += [0] * (2 * n_hops - len(p_off))
+    flat = p_off + i_off
+    where = [tuple(flat[piece * n_hops + h] for piece in range(5)) for h in range(n_hops)]
+    if len(_minibatch_layouts) >= 1024:  # as many different batches as a program has; not without end
+        _minibatch_layouts.clear()
+    layout = _minibatch_layouts[key] = (p_size, i_size, (C.c_int64 * n_hops)(*fan), (C.c_int64 * (5 * n_hops))(*flat),
+                                        where)
+    return layout
 
 
 def create_subcsr(uva_indptr: torch.Tensor, uva_indices: torch.Tensor, seeds: torch.Tensor):

@@ -88,6 +88,32 @@ int ctx_await_post(shmt_ctx* ctx, const HostPost& post, cudaStream_t stream) {
   return SHMT_OK;
 }
 
+HostPost ctx_begin_note(shmt_ctx* ctx, int at) {
+  HostPost p = ctx_begin_post(ctx, nullptr, 0, nullptr);
+  p.flag_at = at;
+  ctx->h_words[at] = ctx->h_words[at + 1] = -1;
+  return p;
+}
+
+int ctx_await_note(shmt_ctx* ctx, int at, cudaStream_t stream) {
+  const int64_t* note = ctx->h_words + at;
+  auto here = [&] {
+    return __atomic_load_n(note, __ATOMIC_ACQUIRE) >= 0 && __atomic_load_n(note + 1, __ATOMIC_ACQUIRE) >= 0;
+  };
+  for (uint64_t it = 1;; ++it) {
+    if (here()) return SHMT_OK;
+    if ((it & 0xFFF) == 0) {
+      const cudaError_t q = cudaStreamQuery(stream);
+      if (q == cudaSuccess) return here() ? SHMT_OK : -1;
+      if (q != cudaErrorNotReady) {
+        set_error("waiting for the sizes of a hop: %s", cudaGetErrorString(q));
+        return SHMT_ERR_CUDA;
+      }
+    }
+    cpu_relax();
+  }
+}
+
 int ctx_mark_tail(shmt_ctx* ctx, cudaStream_t stream) {
   if (!ctx->tail_event)
     SHMT_CUDA_TRY(cudaEventCreateWithFlags(&ctx->tail_event, cudaEventDisableTiming));

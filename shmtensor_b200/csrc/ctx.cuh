@@ -3,6 +3,26 @@
 
 #include "common.cuh"
 
+namespace shmt {
+
+// Result words handed to the host without a copy and before the stream drains: the thread that
+// completes them stores them into the context's pinned host words and then a sequence number,
+// which the host polls for.  Whatever the stream still runs behind that point must not produce
+// results or errors the host needs.
+//
+// A note (n_words = 0) is two numbers, stored to host[flag_at] and the word behind it by the thread that has
+// them, as soon as it has them and in no order with anything; the host has set both words to -1.
+struct HostPost {
+  int64_t* host;         // pinned host words as the device sees them; nullptr = no post
+  const int64_t* words;  // device words to mirror
+  int n_words;
+  int flag_at;           // index of the sequence word (the last pinned word)
+  int64_t seq;           // stored to host[flag_at] after the words
+  int64_t* done;         // zeroed device word counting the CTAs that have finished
+};
+
+}  // namespace shmt
+
 struct shmt_ctx {
   int device = 0;
   char* scratch = nullptr;      // device scratch, grown geometrically; the first
@@ -23,6 +43,14 @@ struct shmt_ctx {
   int64_t post_seq = 0;
   cudaEvent_t tail_event = nullptr;
   bool tail_pending = false;
+  // The mini-batch that has been queued and not yet been waited for (shmt_minibatch_start).
+  struct {
+    shmt::HostPost post{};
+    void* stream = nullptr;
+    int n_hops = 0;  // 0: none
+    int64_t n_seeds = 0;
+    bool noted = false;  // sizes of all hops but the last come as notes
+  } batch;
   // Ticket, count of finished CTAs and tile descriptors of small scans: zero between calls, put back by
   // the scan kernel itself (see scan.cu).
   char* scan_state = nullptr;
@@ -34,6 +62,7 @@ struct shmt_ctx {
 namespace shmt {
 
 constexpr int kCtxWords = 128;
+constexpr int kNoteWord = 96;  // notes of a mini-batch's hops in shmt_ctx::h_words, two words each
 constexpr int kSmallScanTiles = 512;  // tiles whose descriptors live in shmt_ctx::scan_state
 constexpr size_t kScanStateBytes = 16 + (size_t)kSmallScanTiles * 16;
 enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
@@ -51,19 +80,6 @@ int ctx_fetch_words(shmt_ctx* ctx, cudaStream_t stream, const char* what);
 // The same check on words that are already in ctx->h_words.
 int ctx_status_of_words(shmt_ctx* ctx, const char* what);
 
-// Result words handed to the host without a copy and before the stream drains: the thread that
-// completes them stores them into the context's pinned host words and then a sequence number,
-// which the host polls for.  Whatever the stream still runs behind that point must not produce
-// results or errors the host needs.
-struct HostPost {
-  int64_t* host;         // pinned host words as the device sees them; nullptr = no post
-  const int64_t* words;  // device words to mirror
-  int n_words;
-  int flag_at;           // index of the sequence word (the last pinned word)
-  int64_t seq;           // stored to host[flag_at] after the words
-  int64_t* done;         // zeroed device word counting the CTAs that have finished
-};
-
 #ifdef __CUDACC__
 // Called by a whole warp: a word per lane.  One thread copying word by word took 0.6 us for each (the
 // next load waits behind the store of the one before), 17 us for the sizes of a three-hop mini-batch,
@@ -77,6 +93,11 @@ __device__ __forceinline__ void post_to_host(const HostPost& p) {
     *reinterpret_cast<volatile int64_t*>(p.host + i) = ld_relaxed64(p.words + i);
   __syncwarp();
   if (lane == 0) st_release_sys64(p.host + p.flag_at, p.seq);
+}
+
+__device__ __forceinline__ void post_note(const HostPost& p, int64_t a, int64_t b) {
+  *reinterpret_cast<volatile int64_t*>(p.host + p.flag_at) = a;
+  *reinterpret_cast<volatile int64_t*>(p.host + p.flag_at + 1) = b;
 }
 
 // True on every lane of the calling warp if its CTA is the last of `n_ctas` to count itself out at `done`
@@ -111,6 +132,9 @@ __device__ __forceinline__ void post_when_last(const HostPost& p, int64_t n_ctas
 // still be running; the next user of the context's scratch waits for them first.
 HostPost ctx_begin_post(shmt_ctx* ctx, const int64_t* dev_words, int n_words, int64_t* done_word);
 int ctx_await_post(shmt_ctx* ctx, const HostPost& post, cudaStream_t stream);
+// A note for the next call, and the wait for it (SHMT_OK, an error, or -1: the stream has drained without it).
+HostPost ctx_begin_note(shmt_ctx* ctx, int at);
+int ctx_await_note(shmt_ctx* ctx, int at, cudaStream_t stream);
 int ctx_mark_tail(shmt_ctx* ctx, cudaStream_t stream);
 int ctx_join_tail(shmt_ctx* ctx);
 

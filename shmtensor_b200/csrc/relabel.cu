@@ -363,7 +363,10 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
         __threadfence();
       }
       __syncwarp();
-      post_to_host(post);
+      if (post.n_words)
+        post_to_host(post);
+      else if (post.host && threadIdx.x == 0)
+        post_note(post, 0, 0);
     }
     return;
   }
@@ -411,8 +414,11 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   }
   if (threadIdx.x == 0) lookback_publish(st, tile, total);
   const int64_t prefix = lookback_block(st, tile, total, &s_look, status);
-  if (threadIdx.x == 0 && tile == n_tiles - 1) st_relaxed64(result, prefix + total);
-  if (post.host) {
+  if (threadIdx.x == 0 && tile == n_tiles - 1) {
+    st_relaxed64(result, prefix + total);
+    if (post.host && !post.n_words) post_note(post, numel - sizes.split, prefix + total);
+  }
+  if (post.n_words) {
     __syncthreads();  // every thread's look-back (which may flag a timeout) is over
     if (threadIdx.x < 32) post_when_last(post, n_tiles);
   }

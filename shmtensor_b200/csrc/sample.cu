@@ -1141,23 +1141,23 @@ int shmt_sample_hop_eids(shmt_ctx* ctx, const void* indptr, int indptr_dtype, co
 // to back; each reads the size of its input from the device word the previous stage
 // wrote, with grids sized for the largest frontier the fan-outs allow.  The host waits
 // once, at the end, for all the sizes.
-static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
+static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
                                  int indices_dtype, const void* gpu_indptr, const void* gpu_indices,
                                  const shmt_map* map, const void* seeds, int64_t n_seeds,
                                  const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
                                  uint64_t rng_offset, void* const* out_sub_indptr,
                                  void* const* out_sub_indices, void* const* out_relabel,
-                                 void* const* out_frontier, int64_t* sizes_host, void* stream,
+                                 void* const* out_frontier, void* stream,
                                  const void* gpu_edge_base, void* const* out_edge_ids,
                                  const float* weights = nullptr, const float* gpu_weights = nullptr,
-                                 int64_t n_nodes = 0) {
+                                 int64_t n_nodes = 0, bool notes = false) {
   SHMT_REQUIRE(ctx != nullptr, "shmt_sample_minibatch: ctx is null");
   SHMT_REQUIRE(valid_int_dtype(indptr_dtype) && valid_int_dtype(indices_dtype),
                "shmt_sample_minibatch: ID can only be int32 or int64");
   SHMT_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops, "shmt_sample_minibatch: 1..%d hops", kMaxHops);
   SHMT_REQUIRE(n_seeds >= 1 && n_seeds < ((int64_t)1 << 31), "shmt_sample_minibatch: seed count out of range");
   SHMT_REQUIRE(indptr && indices && seeds && fanouts && out_sub_indptr && out_sub_indices &&
-                   out_relabel && out_frontier && sizes_host,
+                   out_relabel && out_frontier,
                "shmt_sample_minibatch: null argument");
   SHMT_REQUIRE(map == nullptr || (gpu_indptr != nullptr && gpu_indices != nullptr),
                "shmt_sample_minibatch: a map needs gpu_indptr and gpu_indices");
@@ -1189,6 +1189,8 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
   }
   const void* cur_seeds = seeds;
   HostPost post{};
+  ctx->batch.n_hops = 0;
+  ctx->batch.noted = notes;
   for (int h = 0; h < n_hops; ++h) {
     int64_t* w = words + h * 8;  // [0] hop ticket, [1] nnz, [2] relabel ticket, [3] n_unique, [4] CTAs done
     HopJob job{};
@@ -1239,16 +1241,31 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
     ps.dev_n1 = w + 1;
     // every size and the status word are final once the last hop's ids are counted: that kernel
     // hands them to the host, which returns while the last remap kernel is still running
-    if (h == n_hops - 1) post = ctx_begin_post(ctx, words, n_hops * 8 + 8, w + 4);
+    if (h == n_hops - 1)
+      post = ctx_begin_post(ctx, words, n_hops * 8 + 8, w + 4);
+    else
+      post = notes ? ctx_begin_note(ctx, kNoteWord + 2 * h) : HostPost{};
+    if (h < n_hops - 1 && !post.host) ctx->batch.noted = false;
     if (int rc = launch_relabel(ctx, ps, cap[h + 1], out_frontier[h], out_relabel[h],
                                 carve_tile_states(base + off_rel[h], rel_tiles[h]), w + 2, status,
-                                w + 3, s, /*inserted=*/true, /*pdl=*/true, h == n_hops - 1 ? &post : nullptr,
-                                /*survey=*/nullptr, n_words))
+                                w + 3, s, /*inserted=*/true, /*pdl=*/true, &post, /*survey=*/nullptr, n_words))
       return rc;
     cur_seeds = out_frontier[h];
   }
   if (int rc = ctx_mark_tail(ctx, s)) return rc;
-  if (int rc = ctx_await_post(ctx, post, s)) return rc;
+  ctx->batch.post = post;
+  ctx->batch.stream = stream;
+  ctx->batch.n_hops = n_hops;
+  ctx->batch.n_seeds = n_seeds;
+  return SHMT_OK;
+}
+
+// Waits for the end of the queued mini-batch: all sizes are in ctx->h_words then.
+static int await_minibatch(shmt_ctx* ctx) {
+  const int n_hops = ctx->batch.n_hops;
+  SHMT_REQUIRE(n_hops > 0, "mini-batch: none has been started");
+  ctx->batch.n_hops = 0;
+  if (int rc = ctx_await_post(ctx, ctx->batch.post, static_cast<cudaStream_t>(ctx->batch.stream))) return rc;
   const int64_t st = ctx->h_words[n_hops * 8];
   if (st != DEV_OK) {
     ctx->table_dirty = true;
@@ -1256,13 +1273,20 @@ static int sample_minibatch_impl(shmt_ctx* ctx, const void* indptr, int indptr_d
               st == DEV_TIMEOUT ? "a bounded look-back wait ran out" : "relabel table overflow");
     return st == DEV_TIMEOUT ? SHMT_ERR_TIMEOUT : SHMT_ERR_CAPACITY;
   }
-  int64_t n_in = n_seeds;
-  for (int h = 0; h < n_hops; ++h) {
-    sizes_host[3 * h + 0] = n_in;
-    sizes_host[3 * h + 1] = ctx->h_words[h * 8 + 1];
-    sizes_host[3 * h + 2] = ctx->h_words[h * 8 + 3];
-    n_in = sizes_host[3 * h + 2];
-  }
+  return SHMT_OK;
+}
+
+// {seeds in, edges sampled, distinct ids out} of hop `h`, from the words of a mini-batch that is over.
+static void hop_sizes(const shmt_ctx* ctx, int h, int64_t* sizes) {
+  sizes[0] = h == 0 ? ctx->batch.n_seeds : ctx->h_words[(h - 1) * 8 + 3];
+  sizes[1] = ctx->h_words[h * 8 + 1];
+  sizes[2] = ctx->h_words[h * 8 + 3];
+}
+
+static int finish_minibatch(shmt_ctx* ctx, int64_t* sizes_host) {
+  const int n_hops = ctx->batch.n_hops;
+  if (int rc = await_minibatch(ctx)) return rc;
+  for (int h = 0; h < n_hops; ++h) hop_sizes(ctx, h, sizes_host + 3 * h);
   return SHMT_OK;
 }
 
@@ -1273,9 +1297,12 @@ int shmt_sample_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, c
                           uint64_t rng_offset, void* const* out_sub_indptr,
                           void* const* out_sub_indices, void* const* out_relabel,
                           void* const* out_frontier, int64_t* sizes_host, void* stream) {
-  return sample_minibatch_impl(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map,
-                               seeds, n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
-                               out_sub_indices, out_relabel, out_frontier, sizes_host, stream, nullptr, nullptr);
+  SHMT_REQUIRE(sizes_host != nullptr, "shmt_sample_minibatch: null argument");
+  if (int rc = queue_minibatch(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds,
+                               n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
+                               out_sub_indices, out_relabel, out_frontier, stream, nullptr, nullptr))
+    return rc;
+  return finish_minibatch(ctx, sizes_host);
 }
 
 int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
@@ -1291,10 +1318,12 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
                "shmt_sample_minibatch_eids: a cached graph needs gpu_edge_base (shmt_subcsr_edge_base)");
   for (int h = 0; h < n_hops && h < 8; ++h)
     SHMT_REQUIRE(out_edge_ids[h] != nullptr, "shmt_sample_minibatch_eids: edge-id buffer of hop %d is null", h);
-  return sample_minibatch_impl(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map,
-                               seeds, n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
-                               out_sub_indices, out_relabel, out_frontier, sizes_host, stream, gpu_edge_base,
-                               out_edge_ids);
+  SHMT_REQUIRE(sizes_host != nullptr, "shmt_sample_minibatch_eids: null argument");
+  if (int rc = queue_minibatch(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds,
+                               n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
+                               out_sub_indices, out_relabel, out_frontier, stream, gpu_edge_base, out_edge_ids))
+    return rc;
+  return finish_minibatch(ctx, sizes_host);
 }
 
 int shmt_sample_minibatch_weighted(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
@@ -1312,32 +1341,34 @@ int shmt_sample_minibatch_weighted(shmt_ctx* ctx, const void* indptr, int indptr
     SHMT_REQUIRE(replace || fanouts[h] <= 32,
                  "shmt_sample_minibatch_weighted: without replacement the fan-out is at most 32 (hop %d has %lld)", h,
                  (long long)fanouts[h]);
-  return sample_minibatch_impl(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map,
-                               seeds, n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
-                               out_sub_indices, out_relabel, out_frontier, sizes_host, stream, nullptr, nullptr,
-                               weights, gpu_weights);
+  SHMT_REQUIRE(sizes_host != nullptr, "shmt_sample_minibatch_weighted: null argument");
+  if (int rc = queue_minibatch(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds,
+                               n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, out_sub_indptr,
+                               out_sub_indices, out_relabel, out_frontier, stream, nullptr, nullptr, weights,
+                               gpu_weights))
+    return rc;
+  return finish_minibatch(ctx, sizes_host);
 }
 
-int shmt_sample_minibatch_pooled(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
-                                 const void* indices, int indices_dtype, const float* weights,
-                                 const void* gpu_indptr, const void* gpu_indices, const float* gpu_weights,
-                                 const void* gpu_edge_base, const shmt_map* map, const void* seeds, int64_t n_seeds,
-                                 const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
-                                 uint64_t rng_offset, void* indptr_pool, void* indices_pool, const int64_t* layout,
-                                 int with_edge_ids, int64_t* sizes_host, void* stream) {
-  SHMT_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops, "shmt_sample_minibatch_pooled: 1..%d hops", kMaxHops);
+int shmt_minibatch_start(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes, const void* indices,
+                         int indices_dtype, const float* weights, const void* gpu_indptr, const void* gpu_indices,
+                         const float* gpu_weights, const void* gpu_edge_base, const shmt_map* map, const void* seeds,
+                         int64_t n_seeds, const int64_t* fanouts, int n_hops, int replace, uint64_t rng_seed,
+                         uint64_t rng_offset, void* indptr_pool, void* indices_pool, const int64_t* layout,
+                         int with_edge_ids, void* stream) {
+  SHMT_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops, "shmt_minibatch_start: 1..%d hops", kMaxHops);
   SHMT_REQUIRE(valid_int_dtype(indptr_dtype) && valid_int_dtype(indices_dtype),
-               "shmt_sample_minibatch_pooled: ID can only be int32 or int64");
-  SHMT_REQUIRE(indptr_pool && indices_pool && layout, "shmt_sample_minibatch_pooled: null argument");
-  SHMT_REQUIRE(n_nodes >= 0, "shmt_sample_minibatch_pooled: negative node count");
-  SHMT_REQUIRE(!weights || !with_edge_ids, "shmt_sample_minibatch_pooled: weights and edge ids cannot be combined");
+               "shmt_minibatch_start: ID can only be int32 or int64");
+  SHMT_REQUIRE(indptr_pool && indices_pool && layout, "shmt_minibatch_start: null argument");
+  SHMT_REQUIRE(n_nodes >= 0, "shmt_minibatch_start: negative node count");
+  SHMT_REQUIRE(!weights || !with_edge_ids, "shmt_minibatch_start: weights and edge ids cannot be combined");
   SHMT_REQUIRE(!with_edge_ids || map == nullptr || gpu_edge_base != nullptr,
-               "shmt_sample_minibatch_pooled: edge ids of a cached graph need gpu_edge_base (shmt_subcsr_edge_base)");
+               "shmt_minibatch_start: edge ids of a cached graph need gpu_edge_base (shmt_subcsr_edge_base)");
   SHMT_REQUIRE(!weights || map == nullptr || gpu_weights != nullptr,
-               "shmt_sample_minibatch_pooled: a cached graph needs gpu_weights");
+               "shmt_minibatch_start: a cached graph needs gpu_weights");
   for (int h = 0; weights && fanouts && h < n_hops; ++h)
     SHMT_REQUIRE(replace || fanouts[h] <= 32,
-                 "shmt_sample_minibatch_pooled: without replacement the fan-out is at most 32 (hop %d has %lld)", h,
+                 "shmt_minibatch_start: without replacement the fan-out is at most 32 (hop %d has %lld)", h,
                  (long long)fanouts[h]);
   void *sub_indptr[kMaxHops], *sub_indices[kMaxHops], *relabel[kMaxHops], *frontier[kMaxHops], *edge_ids[kMaxHops];
   char *p = static_cast<char*>(indptr_pool), *x = static_cast<char*>(indices_pool);
@@ -1349,10 +1380,33 @@ int shmt_sample_minibatch_pooled(shmt_ctx* ctx, const void* indptr, int indptr_d
     relabel[h] = x + layout[3 * n_hops + h] * x_item;
     frontier[h] = x + layout[4 * n_hops + h] * x_item;
   }
-  return sample_minibatch_impl(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds,
-                               n_seeds, fanouts, n_hops, replace, rng_seed, rng_offset, sub_indptr, sub_indices,
-                               relabel, frontier, sizes_host, stream, gpu_edge_base, with_edge_ids ? edge_ids : nullptr,
-                               weights, gpu_weights, n_nodes);
+  return queue_minibatch(ctx, indptr, indptr_dtype, indices, indices_dtype, gpu_indptr, gpu_indices, map, seeds, n_seeds,
+                         fanouts, n_hops, replace, rng_seed, rng_offset, sub_indptr, sub_indices, relabel, frontier,
+                         stream, gpu_edge_base, with_edge_ids ? edge_ids : nullptr, weights, gpu_weights, n_nodes,
+                         /*notes=*/true);
+}
+
+int shmt_minibatch_hop(shmt_ctx* ctx, int hop, int64_t* sizes_host) {
+  SHMT_REQUIRE(ctx != nullptr && sizes_host != nullptr, "shmt_minibatch_hop: null argument");
+  const int n_hops = ctx->batch.n_hops;
+  SHMT_REQUIRE(n_hops > 0 && hop >= 0 && hop < n_hops, "shmt_minibatch_hop: no such hop has been started");
+  DeviceGuard guard(ctx->device);
+  if (hop < n_hops - 1 && ctx->batch.noted) {
+    int rc = SHMT_OK;
+    for (int h = hop > 0 ? hop - 1 : 0; h <= hop && rc == SHMT_OK; ++h)
+      rc = ctx_await_note(ctx, kNoteWord + 2 * h, static_cast<cudaStream_t>(ctx->batch.stream));
+    if (rc > 0) return rc;
+    if (rc == SHMT_OK) {
+      sizes_host[0] = hop == 0 ? ctx->batch.n_seeds : ctx->h_words[kNoteWord + 2 * hop - 1];
+      sizes_host[1] = ctx->h_words[kNoteWord + 2 * hop];
+      sizes_host[2] = ctx->h_words[kNoteWord + 2 * hop + 1];
+      return SHMT_OK;
+    }
+  }
+  if (int rc = await_minibatch(ctx)) return rc;
+  if (hop < n_hops - 1) ctx->batch.n_hops = n_hops;  // the others may be asked for
+  hop_sizes(ctx, hop, sizes_host);
+  return SHMT_OK;
 }
 
 int shmt_subcsr_count(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* seeds,

@@ -457,3 +457,33 @@ def test_minibatch_relabel_by_words_and_slots(capi, dt, k):
         check(far, [k], np.arange(n, dtype=DT[dt]))
         assert capi.context_scratch_bytes() == held
     torch.cuda.synchronize()
+
+
+def test_hop_sizes_of_a_started_minibatch_in_any_order(capi):
+    """shmt_minibatch_hop: sizes of a hop while later ones may still run, asked for out of order and twice; the last
+    hop ends the mini-batch, and there is none to ask about before or after."""
+    import ctypes as C
+    from shmtensor_b200 import _lib
+    lib = _lib.lib
+    rng = np.random.default_rng(5)
+    deg = rng.integers(0, 9, size=4000)
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)).cuda()
+    indices = torch.from_numpy(rng.integers(0, 4000, size=int(deg.sum())).astype(np.int32)).cuda()
+    seeds = torch.arange(300, dtype=torch.int32, device="cuda")
+    capi.set_sampling_seed(31)
+    _, hops = capi.sample_minibatch(indptr, indices, seeds, [3, 2, 2], False)
+    want = [[sp.numel() - 1, sx.numel(), f.numel()] for sp, sx, _, f in hops]
+    ctx, stream, sizes = capi._ctx(seeds.device), capi._stream(seeds.device), (C.c_int64 * 3)()
+    assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.ERR_INVALID
+    p_size, i_size, fan, where, _ = capi._minibatch_layout((300, (3, 2, 2), 1, 0, False))
+    p_pool = torch.empty(p_size, dtype=torch.int64, device="cuda")
+    i_pool = torch.empty(i_size, dtype=torch.int32, device="cuda")
+    for order in ((0, 1, 2), (1, 0, 1, 2), (2,)):
+        _lib.check(lib.shmt_minibatch_start(ctx, indptr.data_ptr(), 1, 4000, indices.data_ptr(), 0, None, None, None, None,
+                                            None, None, seeds.data_ptr(), 300, fan, 3, 0, 31, 1, p_pool.data_ptr(),
+                                            i_pool.data_ptr(), where, 0, stream))
+        assert lib.shmt_minibatch_hop(ctx, 3, sizes) == _lib.ERR_INVALID
+        for h in order:
+            _lib.check(lib.shmt_minibatch_hop(ctx, h, sizes))
+            assert list(sizes) == want[h]
+        assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.ERR_INVALID
