@@ -174,7 +174,21 @@ int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t w
                                   stream));
     ctx->table_words_bytes = 0;
   }
-  if (words > ctx->table_words_bytes) ctx->table_words_bytes = words;  // empty slots are words at rest
+  if (words > ctx->table_words_bytes) {
+    // every word of an empty slot has its top bit set
+    if (ctx->table_words_bytes == 0 || ctx->words_tag > 0x80000000u) ctx->words_tag = 0x80000000u;
+    ctx->table_words_bytes = words;
+  }
+  return SHMT_OK;
+}
+
+int ctx_take_tags(shmt_ctx* ctx, unsigned count, unsigned* first, cudaStream_t stream) {
+  if (ctx->words_tag < count) {
+    SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table + ctx->table_bytes - ctx->table_words_bytes, 0xFF, ctx->table_words_bytes,
+                                  stream));
+    ctx->words_tag = 0xFFFFFFFFu;
+  }
+  *first = ctx->words_tag -= count;
   return SHMT_OK;
 }
 

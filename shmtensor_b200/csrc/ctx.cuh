@@ -33,9 +33,10 @@ struct shmt_ctx {
   char* table = nullptr;
   size_t table_bytes = 0;
   bool table_dirty = false;     // a failed call may have left entries behind
-  // Words of mini-batches (RelTable in relabel.cuh): the last table_words_bytes of the block.  At rest they
-  // hold marked numbers, not the all ones of empty slots, so slots that reach into them need them cleared.
+  // Words of mini-batches (RelTable in relabel.cuh): the last table_words_bytes of the block.  They hold
+  // numbers from words_tag on, not the all ones of empty slots, so slots that reach into them need them cleared.
   size_t table_words_bytes = 0;
+  unsigned words_tag = 0;
   bool table_reserved = false;  // the caller sized the table for mini-batches: none of them grows it for words
   unsigned* table_words(int64_t n) const { return reinterpret_cast<unsigned*>(table + table_bytes) - n; }
   // Early hand-over of result words (see HostPost): sequence number of the last post, and an
@@ -73,6 +74,9 @@ int ctx_reserve(shmt_ctx* ctx, size_t bytes);
 // Make sure ctx->table holds at least `bytes`, empty (all ones to begin with), and behind them `words`
 // bytes of words.
 int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words = 0);
+
+// `count` numbers below all that the words hold: *first and those behind it.
+int ctx_take_tags(shmt_ctx* ctx, unsigned count, unsigned* first, cudaStream_t stream);
 
 // Copy the first `n_words` result words to the host and wait for `stream`.
 // Returns SHMT_ERR_TIMEOUT / SHMT_ERR_CAPACITY if the kernel flagged either.

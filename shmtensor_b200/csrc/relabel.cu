@@ -284,6 +284,7 @@ struct RelView {
   }
 };
 
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 constexpr unsigned kRelSms = 148, kRelInsertCtas = 7;  // CTAs per SM
 
 __global__ void __launch_bounds__(kRelThreads, kRelInsertCtas)
@@ -344,7 +345,13 @@ relabel_clear_kernel(RelTable t, int64_t numel, const RelSurvey* __restrict__ su
 // remap kernel are the repeats alone, marked as such.  A warp takes 32 * ITEMS consecutive
 // elements, 32 at a time, so that every access to the streamed arrays is contiguous; all slot
 // reads of a thread are in flight together.
-template <int ITEMS>
+// WORDS: ids below t.n_words have a word instead of a slot, and nothing in slot_of yet; a word is final, and
+// stays as it is.  A repeat takes down its first occurrence's index.  The seeds of all hops but the first
+// are distinct (they are the hop before's unique ids), so theirs need not be looked at.  What bounds it is random
+// reads of the words, from L2.  8,192 seeds 5/10/15 on 10 M nodes, behind the last hop (2.8 M ids, 2.4 M of them
+// distinct): 45 us with the new ids written to the words, 35 so; the hop, which reads no word any more before it
+// lowers it, 62 -> 55.  (The look-back is 3 of the 45; 5 or 6 CTAs per SM, half the tile, a loop over 592 CTAs: the same.)
+template <int ITEMS, bool WORDS>
 __global__ void __launch_bounds__(kRelThreads, 4)
 relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ unique, TileStates st,
                        int64_t* ticket, int64_t* status, int64_t* result, HostPost post, LaunchPad<8>) {
@@ -376,26 +383,52 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
   uint32_t pos[ITEMS];
   unsigned first[ITEMS];
   unsigned maybe = 0, is_first = 0;  // one bit per element of this thread
-#pragma unroll
-  for (int j = 0; j < ITEMS; ++j) {
-    const int64_t i = base + 32 * j;
-    pos[j] = 0;
-    if (i < numel) {
-      bool m;
-      pos[j] = relabel_unpack(slot_of, ps.is64, i, &m);
-      maybe |= (unsigned)m << j;
-    }
-  }
-  // only an element the inserting pass did not rule out has to look at its slot; its id is fetched
-  // along with it (most are first occurrences), so that nothing waits for it behind the look-back
   int64_t id[ITEMS];
+  if (WORDS) {
+    const int64_t distinct = ps.dev_n0 ? sizes.split : 0;
 #pragma unroll
-  for (int j = 0; j < ITEMS; ++j) {
-    first[j] = 0xFFFFFFFFu;
-    id[j] = 0;
-    if (maybe >> j & 1u) {
-      first[j] = __ldcg(relabel_first(t, pos[j]));
-      id[j] = pos[j] < t.n_words ? (int64_t)pos[j] : part_elem(ps, sizes, base + 32 * j);
+    for (int j = 0; j < ITEMS; ++j) {
+      const int64_t i = base + 32 * j;
+      id[j] = i < numel ? part_elem(ps, sizes, i) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {  // all reads on their way before anything is done with one
+      const int64_t i = base + 32 * j;
+      first[j] = t.tag + (unsigned)i;
+      if (i >= distinct && i < numel && (uint64_t)id[j] < t.n_words) first[j] = __ldcg(t.words + id[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int64_t i = base + 32 * j;
+      pos[j] = kNoSlot;
+      first[j] = i < numel ? first[j] - t.tag : 0xFFFFFFFFu;
+      if (i < numel && (uint64_t)id[j] >= t.n_words) {
+        bool m;
+        pos[j] = relabel_unpack(slot_of, ps.is64, i, &m);
+        first[j] = m ? __ldcg(&t.slots[pos[j]].first) : 0xFFFFFFFFu;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int64_t i = base + 32 * j;
+      pos[j] = 0;
+      if (i < numel) {
+        bool m;
+        pos[j] = relabel_unpack(slot_of, ps.is64, i, &m);
+        maybe |= (unsigned)m << j;
+      }
+    }
+    // only an element the inserting pass did not rule out has to look at its slot; its id is fetched
+    // along with it (most are first occurrences), so that nothing waits for it behind the look-back
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      first[j] = 0xFFFFFFFFu;
+      id[j] = 0;
+      if (maybe >> j & 1u) {
+        first[j] = __ldcg(&t.slots[pos[j]].first);
+        id[j] = part_elem(ps, sizes, base + 32 * j);
+      }
     }
   }
   int before = 0, firsts = 0;  // first occurrences of earlier warps and of this one
@@ -431,10 +464,12 @@ relabel_compact_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ u
       const int64_t uid = row_uid + __popc(row & ((1u << lane) - 1u));
       store_int(unique, ps.is64, uid, id[j]);
       store_int(slot_of, ps.is64, i, uid);
-      if (pos[j] < t.n_words)
-        t.words[pos[j]] = (unsigned)uid | kRelNewId;
-      else
-        *reinterpret_cast<uint4*>(t.slots + (pos[j] - t.n_words)) = make_uint4(~0u, ~0u, (unsigned)uid | kRelNewId, ~0u);
+      if (!WORDS || pos[j] != kNoSlot)
+        *reinterpret_cast<uint4*>(t.slots + pos[j]) = make_uint4(~0u, ~0u, (unsigned)uid | kRelNewId, ~0u);
+    } else if (WORDS) {
+      if (i < numel)
+        store_int(slot_of, ps.is64, i,
+                  relabel_pack(pos[j] == kNoSlot ? first[j] : pos[j] | kRelRepeatSlot, false, ps.is64));
     } else if (maybe >> j & 1u) {
       store_int(slot_of, ps.is64, i, relabel_pack(pos[j], false, ps.is64));
     }
@@ -584,7 +619,8 @@ relabel_number_kernel(Parts ps, RelTable t, void* slot_of, void* __restrict__ un
     }
 }
 
-// The repeats: slot -> new id.  First occurrences hold theirs already.
+// The repeats: slot, or with WORDS first occurrence, -> new id.  First occurrences hold theirs already.
+template <bool WORDS>
 __global__ void __launch_bounds__(kRelThreads)
 relabel_remap_kernel(Parts ps, RelTable t, void* out, LaunchPad<24>) {
   pdl_prologue();
@@ -600,6 +636,7 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out, LaunchPad<24>) {
     for (int u = 0; u < U; ++u) {
       const int64_t i = i0 + u * stride;
       repeat[u] = false;
+      pos[u] = 0;
       if (i < numel) {
         bool done;
         pos[u] = relabel_unpack(out, ps.is64, i, &done);
@@ -607,11 +644,14 @@ relabel_remap_kernel(Parts ps, RelTable t, void* out, LaunchPad<24>) {
       }
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (repeat[u]) newid[u] = __ldcg(relabel_first(t, pos[u])) & ~kRelNewId;
+    for (int u = 0; u < U; ++u) {  // reads only under a condition: they all are on their way before one is waited for
+      const unsigned* at = &t.slots[WORDS ? pos[u] & ~kRelRepeatSlot : pos[u]].first;
+      if (WORDS && !(pos[u] & kRelRepeatSlot)) at = static_cast<const unsigned*>(out) + ((size_t)pos[u] << ps.is64);
+      if (repeat[u]) newid[u] = __ldcg(at);
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (repeat[u]) store_int(out, ps.is64, i0 + u * stride, (int64_t)newid[u]);
+      if (repeat[u]) store_int(out, ps.is64, i0 + u * stride, (int64_t)(newid[u] & ~kRelNewId));
   }
 }
 
@@ -794,21 +834,22 @@ static RelScratch relabel_scratch(int64_t numel) {
 }
 size_t relabel_scratch_bytes(int64_t numel) { return relabel_scratch(numel).all; }
 
-int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, int64_t n_words) {
+int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, const RelWords& words) {
   const uint64_t cap = relabel_capacity(numel_bound);
-  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s, (size_t)n_words * sizeof(unsigned))) return rc;
+  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s, (size_t)words.n * sizeof(unsigned))) return rc;
   t->slots = reinterpret_cast<RelSlot*>(ctx->table);
   t->cap = (uint32_t)cap;
-  t->words = n_words ? ctx->table_words(n_words) : nullptr;
-  t->n_words = (uint32_t)n_words;
+  t->words = words.n ? ctx->table_words(words.n) : nullptr;
+  t->n_words = (uint32_t)words.n;
+  t->tag = words.tag;
   return SHMT_OK;
 }
 
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel, TileStates st, int64_t* ticket,
                    int64_t* status, int64_t* result, cudaStream_t s, bool inserted, bool pdl,
-                   const HostPost* post, RelSurvey* survey, int64_t n_words) {
+                   const HostPost* post, RelSurvey* survey, const RelWords& words) {
   RelTable t;
-  if (int rc = relabel_table(ctx, numel_bound, &t, s, n_words)) return rc;
+  if (int rc = relabel_table(ctx, numel_bound, &t, s, words)) return rc;
   const int64_t n_tiles = (numel_bound + kRelTile - 1) / kRelTile;
   int64_t blocks = (numel_bound + kRelThreads - 1) / kRelThreads;
   const int64_t cap_blocks = (int64_t)sm_count() * 16;
@@ -828,18 +869,16 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
                                 post ? *post : HostPost{}, LaunchPad<32>{}));
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_number_kernel, (unsigned)tiles, kRelThreads, 0, s, ps, t, out_relabel,
                                 out_unique, (const uint32_t*)flags, (const int*)counts, (const RelSurvey*)survey, LaunchPad<56>{}));
-  } else if (numel_bound >= kRelLargeInput) {
-    const int64_t big_tiles = (numel_bound + kRelThreads * kRelItemsLarge - 1) / (kRelThreads * kRelItemsLarge);
-    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItemsLarge>, (unsigned)big_tiles, kRelThreads, 0, s,
-                                ps, t, out_relabel, out_unique, st, ticket, status, result,
-                                post ? *post : HostPost{}, LaunchPad<8>{}));
   } else {
-    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_compact_kernel<kRelItems>, (unsigned)n_tiles, kRelThreads, 0, s, ps, t,
-                                out_relabel, out_unique, st, ticket, status, result,
-                                post ? *post : HostPost{}, LaunchPad<8>{}));
+    const bool big = numel_bound >= kRelLargeInput;
+    const int64_t big_tiles = (numel_bound + kRelThreads * kRelItemsLarge - 1) / (kRelThreads * kRelItemsLarge);
+    auto kernel = big ? (words.n ? relabel_compact_kernel<kRelItemsLarge, true> : relabel_compact_kernel<kRelItemsLarge, false>)
+                      : (words.n ? relabel_compact_kernel<kRelItems, true> : relabel_compact_kernel<kRelItems, false>);
+    SHMT_CUDA_TRY(launch_kernel(pdl, kernel, (unsigned)(big ? big_tiles : n_tiles), kRelThreads, 0, s, ps, t, out_relabel,
+                                out_unique, st, ticket, status, result, post ? *post : HostPost{}, LaunchPad<8>{}));
   }
   if (!survey) {
-    SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_kernel, grid, kRelThreads, 0, s, ps, t, out_relabel, LaunchPad<24>{}));
+    SHMT_CUDA_TRY(launch_kernel(pdl, words.n ? relabel_remap_kernel<true> : relabel_remap_kernel<false>, grid, kRelThreads, 0, s, ps, t, out_relabel, LaunchPad<24>{}));
   } else {
     SHMT_CUDA_TRY(launch_kernel(pdl, relabel_remap_large_kernel, grid, kRelThreads, 0, s, t, ps.is64, numel_bound,
                                 out_relabel, (const RelSurvey*)survey, LaunchPad<32>{}));

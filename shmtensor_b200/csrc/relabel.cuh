@@ -40,22 +40,27 @@ struct __align__(16) RelSlot {
 };
 constexpr unsigned kRelNewId = 0x80000000u;  // indexes and new ids stay below 2^30
 
-// Mini-batches on a graph of up to kRelMaxWords nodes: a word per node, the smallest index of that id or,
-// marked as in a slot, its new id.  An id below `n_words` is its own position and nothing has to be claimed:
-// one 4-byte read and one minimum, without waiting for either, where a slot takes a 32-byte read, a
-// compare-and-swap and a minimum; and the words of a graph fit the L2 cache where the slots of a large
-// frontier do not.  Other ids (a last hop may reach nodes that have no row) take slots, at positions from
-// n_words on.  Like slots, words need nothing between calls: a new id counts as no index.
+// Mini-batches on a graph of up to kRelMaxWords nodes: a word per node, the smallest index of that id in the hop,
+// plus the hop's `tag`.  An id below `n_words` is its own position and nothing has to be claimed: a minimum, which
+// nobody waits for, where a slot takes a 32-byte read, a compare-and-swap and a minimum; and the words
+// of a graph fit the L2 cache where the slots of a large frontier do not.  Tags go down from hop to hop by
+// as many numbers as it can have indices, so that whatever earlier hops have left is larger than all of this
+// one's, and no word is ever put back (but all of them when the tags have come down, every 200 batches of
+// 10 M ids).  An element that finds another's index in its word is a repeat of that element, whose result it takes.
+// Other ids (a last hop may reach nodes that have no row) take slots.
 // Slots against words, 8,192 seeds 5/10/15, int64 ids: 2.4 M nodes 416 us and 292, 10 M 536 and 354, 24 M 579
 // and 438, 50 M 597 and 580, 110 M 606 and 712; 1,024 seeds 161 and 138, 165 and 142, 163 and 149, 164 and 156, 164
-// and 178; 50 seeds 93 and 86 at every size.  The line is where the words are the size of the L2 cache.
+// and 178; 50 seeds 93 and 86 at every size (words that held the new ids too).  The line is where the words
+// are the size of the L2 cache.
 struct RelTable {
   RelSlot* slots;  // cap entries
   uint32_t cap;
-  unsigned* words;   // n_words entries; nullptr: none
   uint32_t n_words;
+  unsigned* words;  // n_words entries; nullptr: none
+  unsigned tag;
 };
 constexpr int64_t kRelMaxWords = 1 << 25;
+constexpr int64_t kRelMaxWordIds = 1 << 29;  // with words, ids per hop: an index or a slot and two marks fit 32 bits
 
 // Slots per id.  A small input waits for its longest walk (at half load a few of 5,000 ids walk six
 // pairs, 1 us each), so it spreads out over up to kRelRoomy slots; a large one is bound by the
@@ -80,6 +85,8 @@ struct RelSurvey {
 // table never has more than 2^31 slots (inputs stay below 2^30 ids).
 constexpr unsigned long long kRelNotFirst64 = 1ull << 40;
 constexpr uint32_t kRelNotFirst32 = 0x80000000u;
+// With words, a repeat is marked and holds its first occurrence's index, or, so marked too, a slot.
+constexpr uint32_t kRelRepeatSlot = 1u << 30;
 
 __device__ __forceinline__ int64_t relabel_pack(uint32_t pos, bool unmarked, bool is64) {
   if (is64) return (int64_t)((unsigned long long)pos | (unmarked ? 0ull : kRelNotFirst64));
@@ -160,11 +167,6 @@ __device__ __forceinline__ uint32_t relabel_next(const RelRange& t, long long ke
   return at == t.full ? t.near : at;
 }
 
-// Where position `pos` of a call keeps the smallest index of its id, later its new id.
-__device__ __forceinline__ unsigned* relabel_first(const RelTable& t, uint32_t pos) {
-  return pos < t.n_words ? t.words + pos : &t.slots[pos - t.n_words].first;
-}
-
 // Whether the calling lane is the lowest, of those that call together, with its `at`.
 __device__ __forceinline__ bool relabel_lowest(uint32_t at) {
   return __ffs(__match_any_sync(__activemask(), at)) - 1 == (int)(threadIdx.x & 31);
@@ -224,6 +226,12 @@ uint64_t relabel_capacity(int64_t numel_bound);
 // Context scratch that shmt_relabel takes for up to `numel` ids.
 size_t relabel_scratch_bytes(int64_t numel);
 
+// Words of a hop (n = 0: none).
+struct RelWords {
+  int64_t n = 0;
+  unsigned tag = 0;
+};
+
 // Queue the relabel kernels: insert, compact and remap, or, of a surveyed input, survey, insert, flag,
 // total, number, remap and clear.  `numel_bound` >= the real element count sizes the table and the
 // grids; ticket/status/result are zeroed device words.
@@ -232,16 +240,16 @@ size_t relabel_scratch_bytes(int64_t numel);
 // of the ids (the fused sampling kernel), so only the compact and remap kernels run.
 // `post`: the compact (or total) kernel hands the result words to the host as soon as the unique count
 // is final; the kernels still to run then produce neither sizes nor errors.
-// `n_words`: what the producer that `inserted` was given (relabel_table).
+// `words`: what the producer that `inserted` was given.
 // `survey`: zeroed device memory, with room for the flags behind it (relabel_scratch_bytes in all); when
 // given, a first kernel looks the ids over and the others use the form of the table that suits them
 // (see relabel_survey_kernel, relabel_use).
 int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* out_unique, void* out_relabel,
                    TileStates st, int64_t* ticket, int64_t* status, int64_t* result, cudaStream_t s,
                    bool inserted = false, bool pdl = false, const HostPost* post = nullptr,
-                   RelSurvey* survey = nullptr, int64_t n_words = 0);
+                   RelSurvey* survey = nullptr, const RelWords& words = {});
 
-// The context's table for `numel_bound` ids (reserving it), with words for ids below `n_words` if given.
-int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, int64_t n_words = 0);
+// The context's table for `numel_bound` ids (reserving it).
+int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, const RelWords& words = {});
 
 }  // namespace shmt

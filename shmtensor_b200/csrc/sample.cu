@@ -45,7 +45,7 @@ constexpr int kHopSeedStep = 8;
 constexpr double kHopSlotsPerEdge = 1.25;
 constexpr int kMaxSeedsPerTile = 1024;
 
-struct HopJob {  // 288 bytes: see launch_kernel
+struct HopJob {
   const void* indptr;
   const void* indices;      // host / full graph
   const void* gpu_indptr;   // compact cached CSR (nullable)
@@ -54,9 +54,9 @@ struct HopJob {  // 288 bytes: see launch_kernel
   const void* seeds;
   int64_t n;
   int64_t k;
-  int indptr64, seeds64;
-  int replace;
-  uint32_t rel_cap, rel_n_words;  // see rel_slots
+  bool indptr64, seeds64;
+  bool replace;
+  uint32_t rel_cap, rel_n_words, rel_tag;  // see rel_slots
   uint32_t off_lo, off_hi;
   int seeds_per_tile;
   uint32_t set_slots;     // fan-out > 32: words of the per-warp set of chosen positions (0: none)
@@ -81,7 +81,7 @@ struct HopJob {  // 288 bytes: see launch_kernel
   // records the slot in rel_out -- the work of relabel's first kernel, done while this
   // kernel would otherwise wait on memory.  rel_slots == nullptr: off (HOP_FUSED otherwise).
   RelSlot* rel_slots;
-  unsigned* rel_words;  // ids below rel_n_words take no slot (see RelTable)
+  unsigned* rel_words;  // ids below rel_n_words take no slot, and are not recorded (see RelTable)
   void* rel_out;
   // Look-back state that the kernel itself puts back to zero (small single-hop calls): the zeroed word
   // in which its CTAs count themselves out, or nullptr.
@@ -89,6 +89,7 @@ struct HopJob {  // 288 bytes: see launch_kernel
   // Single-hop call with a host result: the CTA that finishes its bookkeeping last hands the
   // result words to the host, which returns while the rows are still being written.
   HostPost post;
+  LaunchPad<8> pad;
 };
 
 // indptr[i] and indptr[i+1] with one load when the pair is naturally aligned (one request on
@@ -437,15 +438,12 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
                        job.rel_cap};
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
   auto enter = [&](int64_t i, IxT id) {
-    bool maybe_first;
-    uint32_t at;
     if ((uint64_t)(long long)id < job.rel_n_words) {
-      at = (uint32_t)id;
-      maybe_first = __ldcg(job.rel_words + at) > (unsigned)i;  // a mark counts as no index
-      if (maybe_first) atomicMin(job.rel_words + at, (unsigned)i);
-    } else {
-      at = job.rel_n_words + relabel_enter<false>(range, (long long)id, (unsigned)i, job.status, &maybe_first);
+      atomicMin(job.rel_words + id, job.rel_tag + (unsigned)i);
+      return;
     }
+    bool maybe_first;
+    const uint32_t at = relabel_enter<false>(range, (long long)id, (unsigned)i, job.status, &maybe_first);
     store_int(job.rel_out, sizeof(IxT) == 8, i, relabel_pack(at, maybe_first, sizeof(IxT) == 8));
   };
 
@@ -965,12 +963,10 @@ static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, M
 }
 
 // Words for the ids of a mini-batch of up to `numel_bound` of them on a graph of `n_nodes` (0: not known): all
-// or none.  None where positions would not fit 31 bits, or where a table that the caller has sized
-// would have to grow.
+// or none.  None where a table that the caller has sized would have to grow.
 static int64_t minibatch_words(const shmt_ctx* ctx, int64_t numel_bound, int64_t n_nodes) {
-  if (n_nodes > kRelMaxWords) return 0;
+  if (n_nodes > kRelMaxWords || numel_bound > kRelMaxWordIds) return 0;
   const uint64_t cap = relabel_capacity(numel_bound);
-  if (cap + (uint64_t)n_nodes >= kRelNotFirst32) return 0;
   const bool fits = cap * sizeof(RelSlot) + (size_t)n_nodes * sizeof(unsigned) <= ctx->table_bytes;
   return fits || !ctx->table_reserved ? n_nodes : 0;
 }
@@ -999,8 +995,9 @@ int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64
     return rc;
   RelTable t;
   ctx->table_reserved = false;
-  const int64_t n_words = minibatch_words(ctx, plan.cap[n_hops], n_nodes);
-  if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream), n_words)) return rc;
+  RelWords words;
+  words.n = minibatch_words(ctx, plan.cap[n_hops], n_nodes);
+  if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream), words)) return rc;
   ctx->table_reserved = true;
   return SHMT_OK;
 }
@@ -1182,10 +1179,17 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   int64_t* status = words + n_hops * 8;
 
   // the relabel table for the largest hop, reserved before anything is queued
-  const int64_t n_words = minibatch_words(ctx, cap[n_hops], n_nodes);
+  RelWords rel_words;
+  rel_words.n = minibatch_words(ctx, cap[n_hops], n_nodes);
   {
     RelTable biggest;
-    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s, n_words)) return rc;
+    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s, rel_words)) return rc;
+  }
+  if (rel_words.n) {
+    unsigned ids = 0;
+    for (int h = 0; h < n_hops; ++h) ids += (unsigned)cap[h + 1];
+    if (int rc = ctx_take_tags(ctx, ids, &rel_words.tag, s)) return rc;
+    rel_words.tag += ids;  // goes down hop by hop
   }
   const void* cur_seeds = seeds;
   HostPost post{};
@@ -1221,11 +1225,13 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
     job.status = status;
     job.result = w + 1;
     RelTable t;  // every sampler claims the relabel slots of what it emits
-    if (int rc = relabel_table(ctx, cap[h + 1], &t, s, n_words)) return rc;
+    if (rel_words.n) rel_words.tag -= (unsigned)cap[h + 1];
+    if (int rc = relabel_table(ctx, cap[h + 1], &t, s, rel_words)) return rc;
     job.rel_slots = t.slots;
     job.rel_cap = t.cap;
     job.rel_words = t.words;
     job.rel_n_words = t.n_words;
+    job.rel_tag = t.tag;
     job.rel_out = out_relabel[h];
     SHMT_CUDA_TRY(indices_dtype == SHMT_I64 ? launch_hop<long long>(job, hop_tiles[h], s, /*pdl=*/h > 0)
                                             : launch_hop<int>(job, hop_tiles[h], s, /*pdl=*/h > 0));
@@ -1248,7 +1254,7 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
     if (h < n_hops - 1 && !post.host) ctx->batch.noted = false;
     if (int rc = launch_relabel(ctx, ps, cap[h + 1], out_frontier[h], out_relabel[h],
                                 carve_tile_states(base + off_rel[h], rel_tiles[h]), w + 2, status,
-                                w + 3, s, /*inserted=*/true, /*pdl=*/true, &post, /*survey=*/nullptr, n_words))
+                                w + 3, s, /*inserted=*/true, /*pdl=*/true, &post, /*survey=*/nullptr, rel_words))
       return rc;
     cur_seeds = out_frontier[h];
   }

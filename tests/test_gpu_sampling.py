@@ -487,3 +487,26 @@ def test_hop_sizes_of_a_started_minibatch_in_any_order(capi):
             _lib.check(lib.shmt_minibatch_hop(ctx, h, sizes))
             assert list(sizes) == want[h]
         assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.ERR_INVALID
+
+
+def test_minibatch_words_when_their_tags_run_out(capi):
+    """Every hop takes as many tags as it can have ids (here 20,020,000 of 2^32); when there are none left
+    the words start over.  240 batches, through the start of the tags, their end and past it, are all alike."""
+    rng = np.random.default_rng(12)
+    n = 60_000
+    deg = rng.integers(0, 8, size=n)
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)).cuda()
+    indices = torch.from_numpy(rng.integers(0, n, size=int(deg.sum())).astype(np.int32)).cuda()
+    seeds = torch.from_numpy(rng.permutation(n)[:20_000].astype(np.int32)).cuda()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = None
+        for i in range(240):
+            front, [(sp, sx, rel, _)] = capi.sample_minibatch(indptr, indices, seeds, [1000], False)
+            if want is None:
+                want = [t.clone() for t in (front, sp, sx, rel)]
+                wu, (_, wx) = oracle.tensor_relabel([seeds.cpu().numpy(), sx.cpu().numpy()])
+                assert np.array_equal(front.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
+            assert all(torch.equal(a, b) for a, b in zip(want, (front, sp, sx, rel))), i
+    torch.cuda.synchronize()
