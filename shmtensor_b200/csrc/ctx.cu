@@ -118,19 +118,25 @@ int ctx_mark_tail(shmt_ctx* ctx, cudaStream_t stream) {
   if (!ctx->tail_event)
     SHMT_CUDA_TRY(cudaEventCreateWithFlags(&ctx->tail_event, cudaEventDisableTiming));
   SHMT_CUDA_TRY(cudaEventRecord(ctx->tail_event, stream));
+  SHMT_CUDA_TRY(cudaStreamGetId(stream, &ctx->tail_stream));
   ctx->tail_pending = true;
   return SHMT_OK;
 }
 
-int ctx_join_tail(shmt_ctx* ctx) {
+int ctx_join_tail(shmt_ctx* ctx, cudaStream_t stream) {
   if (!ctx->tail_pending) return SHMT_OK;
+  // In the tail's own stream everything is queued behind it.  A mini-batch that nobody has waited for could
+  // still write to the host words, though.
+  unsigned long long id = 0;
+  SHMT_CUDA_TRY(cudaStreamGetId(stream, &id));
+  if (id == ctx->tail_stream && ctx->batch.n_hops == 0) return SHMT_OK;
   ctx->tail_pending = false;
   SHMT_CUDA_TRY(cudaEventSynchronize(ctx->tail_event));
   return SHMT_OK;
 }
 
-int ctx_reserve(shmt_ctx* ctx, size_t bytes) {
-  if (int rc = ctx_join_tail(ctx)) return rc;
+int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
+  if (int rc = ctx_join_tail(ctx, stream)) return rc;
   bytes += 256;  // result words live in front of the region
   if (bytes <= ctx->scratch_bytes) return SHMT_OK;
   // cudaFree waits for work that may still read the old block.
@@ -148,7 +154,7 @@ int ctx_reserve(shmt_ctx* ctx, size_t bytes) {
 }
 
 int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words) {
-  if (int rc = ctx_join_tail(ctx)) return rc;
+  if (int rc = ctx_join_tail(ctx, stream)) return rc;
   if (bytes + words > ctx->table_bytes) {
     if (ctx->table) SHMT_CUDA_TRY(cudaFree(ctx->table));
     ctx->table = nullptr;
@@ -240,7 +246,7 @@ int shmt_ctx_create(int device, shmt_ctx** out) {
     delete ctx;
     return SHMT_ERR_CUDA;
   }
-  if (int rc = ctx_reserve(ctx, 0)) {
+  if (int rc = ctx_reserve(ctx, 0, nullptr)) {
     cudaFreeHost(h);
     delete ctx;
     return rc;
@@ -293,7 +299,9 @@ int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, 
                "shmt_ctx_reserve: sizes out of range");
   DeviceGuard guard(ctx->device);
   const size_t relabel = relabel_scratch_bytes(relabel_ids);
-  if (int rc = ctx_reserve(ctx, (size_t)scratch_bytes > relabel ? (size_t)scratch_bytes : relabel)) return rc;
+  if (int rc = ctx_reserve(ctx, (size_t)scratch_bytes > relabel ? (size_t)scratch_bytes : relabel,
+                           static_cast<cudaStream_t>(stream)))
+    return rc;
   if (relabel_ids > 0) {
     if (int rc = ctx_reserve_table(ctx, relabel_capacity(relabel_ids) * sizeof(RelSlot),
                                    static_cast<cudaStream_t>(stream)))

@@ -43,6 +43,7 @@ struct shmt_ctx {
   // event behind the kernels that were still running when the call returned.
   int64_t post_seq = 0;
   cudaEvent_t tail_event = nullptr;
+  unsigned long long tail_stream = 0;  // its id: a handle may be another stream's by now
   bool tail_pending = false;
   // The mini-batch that has been queued and not yet been waited for (shmt_minibatch_start).
   struct {
@@ -69,7 +70,7 @@ constexpr size_t kScanStateBytes = 16 + (size_t)kSmallScanTiles * 16;
 enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).
-int ctx_reserve(shmt_ctx* ctx, size_t bytes);
+int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
 
 // Make sure ctx->table holds at least `bytes`, empty (all ones to begin with), and behind them `words`
 // bytes of words.
@@ -140,7 +141,7 @@ int ctx_await_post(shmt_ctx* ctx, const HostPost& post, cudaStream_t stream);
 HostPost ctx_begin_note(shmt_ctx* ctx, int at);
 int ctx_await_note(shmt_ctx* ctx, int at, cudaStream_t stream);
 int ctx_mark_tail(shmt_ctx* ctx, cudaStream_t stream);
-int ctx_join_tail(shmt_ctx* ctx);
+int ctx_join_tail(shmt_ctx* ctx, cudaStream_t stream);
 
 // Device that owns a device pointer (the current device if the runtime cannot tell).
 int device_of_pointer(const void* p);

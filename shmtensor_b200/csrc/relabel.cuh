@@ -60,7 +60,6 @@ struct RelTable {
   unsigned tag;
 };
 constexpr int64_t kRelMaxWords = 1 << 25;
-constexpr int64_t kRelMaxWordIds = 1 << 29;  // with words, ids per hop: an index or a slot and two marks fit 32 bits
 
 // Slots per id.  A small input waits for its longest walk (at half load a few of 5,000 ids walk six
 // pairs, 1 us each), so it spreads out over up to kRelRoomy slots; a large one is bound by the
@@ -85,8 +84,7 @@ struct RelSurvey {
 // table never has more than 2^31 slots (inputs stay below 2^30 ids).
 constexpr unsigned long long kRelNotFirst64 = 1ull << 40;
 constexpr uint32_t kRelNotFirst32 = 0x80000000u;
-// With words, a repeat is marked and holds its first occurrence's index, or, so marked too, a slot.
-constexpr uint32_t kRelRepeatSlot = 1u << 30;
+// With words, a repeat is marked and holds its first occurrence's index.
 
 __device__ __forceinline__ int64_t relabel_pack(uint32_t pos, bool unmarked, bool is64) {
   if (is64) return (int64_t)((unsigned long long)pos | (unmarked ? 0ull : kRelNotFirst64));
@@ -248,6 +246,18 @@ int launch_relabel(shmt_ctx* ctx, const Parts& ps, int64_t numel_bound, void* ou
                    TileStates st, int64_t* ticket, int64_t* status, int64_t* result, cudaStream_t s,
                    bool inserted = false, bool pdl = false, const HostPost* post = nullptr,
                    RelSurvey* survey = nullptr, const RelWords& words = {});
+
+// The repeats of the hops of a mini-batch that was relabelled with words: `out` as the compact kernels left it,
+// `words` the sizes ([8 h + 1] edges and [8 h + 3] distinct ids of hop h).  launch_relabel leaves them out.
+struct RelRepeats {
+  void* out[8];
+  const int64_t* words;
+  int64_t n_seeds;
+  int n_hops;
+  unsigned first_cta[8];  // of each hop; set by launch_relabel_repeats
+};
+// `numel_bounds`: most elements of every hop.
+int launch_relabel_repeats(RelRepeats r, const int64_t* numel_bounds, bool is64, cudaStream_t s);
 
 // The context's table for `numel_bound` ids (reserving it).
 int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, const RelWords& words = {});

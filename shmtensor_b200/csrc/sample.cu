@@ -965,7 +965,7 @@ static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, M
 // Words for the ids of a mini-batch of up to `numel_bound` of them on a graph of `n_nodes` (0: not known): all
 // or none.  None where a table that the caller has sized would have to grow.
 static int64_t minibatch_words(const shmt_ctx* ctx, int64_t numel_bound, int64_t n_nodes) {
-  if (n_nodes > kRelMaxWords || numel_bound > kRelMaxWordIds) return 0;
+  if (n_nodes > kRelMaxWords) return 0;
   const uint64_t cap = relabel_capacity(numel_bound);
   const bool fits = cap * sizeof(RelSlot) + (size_t)n_nodes * sizeof(unsigned) <= ctx->table_bytes;
   return fits || !ctx->table_reserved ? n_nodes : 0;
@@ -991,7 +991,8 @@ int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64
   if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &plan)) return rc;
   if (int rc = plan_minibatch(n_seeds, fanouts, n_hops, &weighted, /*weighted=*/true)) return rc;
   DeviceGuard guard(ctx->device);
-  if (int rc = ctx_reserve(ctx, weighted.scratch_bytes > plan.scratch_bytes ? weighted.scratch_bytes : plan.scratch_bytes))
+  if (int rc = ctx_reserve(ctx, weighted.scratch_bytes > plan.scratch_bytes ? weighted.scratch_bytes : plan.scratch_bytes,
+                           static_cast<cudaStream_t>(stream)))
     return rc;
   RelTable t;
   ctx->table_reserved = false;
@@ -1066,7 +1067,7 @@ static int sample_hop_impl(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
     job.clean = done = ctx->scan_words() + 1;
     job.st = carve_tile_states(reinterpret_cast<char*>(ctx->scan_words() + 2), kSmallScanTiles);
   } else {
-    if (int rc = ctx_reserve(ctx, tile_state_bytes(n_tiles))) return rc;
+    if (int rc = ctx_reserve(ctx, tile_state_bytes(n_tiles), s)) return rc;
     done = ctx->d_words() + W_DONE;
     job.ticket = ctx->d_words() + W_TICKET;
     job.st = carve_tile_states(ctx->region(), n_tiles);
@@ -1172,7 +1173,7 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   const int* spt = plan.spt;
   const size_t *off_hop = plan.off_hop, *off_rel = plan.off_rel;
   const size_t cursor = plan.scratch_bytes;
-  if (int rc = ctx_reserve(ctx, cursor)) return rc;
+  if (int rc = ctx_reserve(ctx, cursor, s)) return rc;
   char* base = ctx->region();
   int64_t* words = reinterpret_cast<int64_t*>(base);
   SHMT_CUDA_TRY(cudaMemsetAsync(base, 0, cursor, s));  // words, tickets and every tile descriptor
@@ -1193,6 +1194,9 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   }
   const void* cur_seeds = seeds;
   HostPost post{};
+  RelRepeats repeats{};
+  repeats.words = words;
+  repeats.n_seeds = n_seeds;
   ctx->batch.n_hops = 0;
   ctx->batch.noted = notes;
   for (int h = 0; h < n_hops; ++h) {
@@ -1256,7 +1260,12 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
                                 carve_tile_states(base + off_rel[h], rel_tiles[h]), w + 2, status,
                                 w + 3, s, /*inserted=*/true, /*pdl=*/true, &post, /*survey=*/nullptr, rel_words))
       return rc;
+    repeats.out[h] = out_relabel[h];
     cur_seeds = out_frontier[h];
+  }
+  if (rel_words.n) {
+    repeats.n_hops = n_hops;
+    if (int rc = launch_relabel_repeats(repeats, cap + 1, indices_dtype == SHMT_I64, s)) return rc;
   }
   if (int rc = ctx_mark_tail(ctx, s)) return rc;
   ctx->batch.post = post;
@@ -1425,7 +1434,7 @@ int shmt_subcsr_count(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const
   SHMT_REQUIRE(indptr && out_gpu_indptr && (n == 0 || seeds), "shmt_subcsr_count: null argument");
   DeviceGuard guard(ctx->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int rc = ctx_reserve(ctx, scan_scratch_bytes(n + 1))) return rc;
+  if (int rc = ctx_reserve(ctx, scan_scratch_bytes(n + 1), s)) return rc;
   int64_t blocks = (n + 1 + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   subcsr_degree_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(

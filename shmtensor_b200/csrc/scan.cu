@@ -551,7 +551,7 @@ int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
     SHMT_CUDA_TRY(cudaGetLastError());
     return SHMT_OK;
   }
-  if (int rc = ctx_reserve(ctx, scratch_off + scan_scratch_bytes(n))) return rc;
+  if (int rc = ctx_reserve(ctx, scratch_off + scan_scratch_bytes(n), stream)) return rc;
   TileStates st = carve_tile_states(ctx->region() + scratch_off, n_tiles);
   // status / result / ticket words and the tile descriptors start at zero (one memset when the
   // descriptors sit right behind the words, as they do for a plain scan)
@@ -659,7 +659,7 @@ extern "C" int shmt_debug_lookback_timeout(shmt_ctx* ctx, void* stream) {
   SHMT_REQUIRE(ctx != nullptr, "shmt_debug_lookback_timeout: ctx is null");
   DeviceGuard guard(ctx->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int rc = ctx_reserve(ctx, tile_state_bytes(2))) return rc;
+  if (int rc = ctx_reserve(ctx, tile_state_bytes(2), s)) return rc;
   TileStates st = carve_tile_states(ctx->region(), 2);
   SHMT_CUDA_TRY(cudaMemsetAsync(ctx->scratch, 0, 256 + tile_state_bytes(2), s));
   lookback_timeout_probe_kernel<<<1, 32, 0, s>>>(st, ctx->d_words(), 1 << 10);

@@ -487,6 +487,26 @@ def test_hop_sizes_of_a_started_minibatch_in_any_order(capi):
             _lib.check(lib.shmt_minibatch_hop(ctx, h, sizes))
             assert list(sizes) == want[h]
         assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.ERR_INVALID
+    # the context in one stream, then in another, while kernels of the call before may still run; a mini-batch that
+    # is never asked about
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    pools = []
+    torch.cuda.synchronize()
+    for i in range(24):
+        pools.append((torch.empty(p_size, dtype=torch.int64, device="cuda"), torch.empty(i_size, dtype=torch.int32, device="cuda")))
+        _lib.check(lib.shmt_minibatch_start(ctx, indptr.data_ptr(), 1, 4000, indices.data_ptr(), 0, None, None, None, None,
+                                            None, None, seeds.data_ptr(), 300, fan, 3, 0, 31, 1, pools[-1][0].data_ptr(),
+                                            pools[-1][1].data_ptr(), where, 0, streams[i // 2 % 2].cuda_stream))
+        for h in range(3) if i % 5 else ():
+            _lib.check(lib.shmt_minibatch_hop(ctx, h, sizes))
+            assert list(sizes) == want[h]
+    torch.cuda.synchronize()
+    for p_pool, i_pool in pools:
+        for h, (sp, sx, rel, f) in enumerate(hops):
+            p_at, _, x_at, r_at, f_at = capi._minibatch_layouts[(300, (3, 2, 2), 1, 0, False)][4][h]
+            n_in, nnz, n_out = want[h]
+            assert torch.equal(p_pool[p_at:p_at + n_in + 1], sp) and torch.equal(i_pool[x_at:x_at + nnz], sx)
+            assert torch.equal(i_pool[r_at + n_in:r_at + n_in + nnz], rel) and torch.equal(i_pool[f_at:f_at + n_out], f)
 
 
 def test_minibatch_words_when_their_tags_run_out(capi):
