@@ -186,6 +186,7 @@ __device__ int g_device_fault = 0;
 template <int STAGES>
 __global__ void __launch_bounds__(kRowThreads)
 row_gather_bulk_kernel(const RowJob job) {
+  pdl_launch_next();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar[kRowWarps][STAGES];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -201,6 +202,7 @@ row_gather_bulk_kernel(const RowJob job) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[warp][s], 1);
   mbar_init_fence();
   __syncwarp();
+  pdl_wait();
 
   unsigned vmask[STAGES];  // lanes whose row is being loaded into the stage
   int nrows[STAGES];
@@ -267,6 +269,7 @@ row_gather_bulk_kernel(const RowJob job) {
 template <int STAGES>
 __global__ void __launch_bounds__(kRowThreads)
 row_scatter_bulk_kernel(const RowJob job) {
+  pdl_launch_next();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar[kRowWarps][STAGES];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -282,6 +285,7 @@ row_scatter_bulk_kernel(const RowJob job) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[warp][s], 1);
   mbar_init_fence();
   __syncwarp();
+  pdl_wait();
 
   char* dst_row[STAGES];  // where this lane's row of the stage goes (nullptr: nowhere)
   uint32_t parity = 0;
@@ -384,6 +388,7 @@ constexpr int kRaggedPad = 32;  // in front of and behind a warp's buffers: what
 template <int STAGES>
 __global__ void __launch_bounds__(kRowThreads)
 row_gather_ragged_kernel(const RowJob job) {
+  pdl_launch_next();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar[kRowWarps][STAGES];
   const unsigned full = 0xffffffffu;
@@ -401,6 +406,7 @@ row_gather_ragged_kernel(const RowJob job) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&s_bar[warp][s], 1);
   mbar_init_fence();
   __syncwarp();
+  pdl_wait();
 
   unsigned vmask[STAGES];  // lanes whose row is being loaded into the stage
   int start[STAGES];       // byte of this lane's slot at which its row starts
@@ -494,6 +500,7 @@ row_gather_ragged_kernel(const RowJob job) {
 // SET == false: table row -> flat (fetch).  SET == true: flat -> table row.
 template <int VEC, bool SET, int U>
 __global__ void __launch_bounds__(kRowThreads) row_copy_kernel(const RowJob job) {
+  pdl_prologue();
   using V = typename VecT<VEC>::type;
   __shared__ char* s_row[kRowWarps][32];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -652,7 +659,7 @@ static int launch_lsu(const RowJob& job, cudaStream_t s) {
   int dev = 0;
   SHMT_CUDA_TRY(cudaGetDevice(&dev));
   const unsigned grid = grid_for_tiles(row_copy_kernel<VEC, SET, 8>, &kept, dev, job.n, job.rows_per_tile);
-  SHMT_CUDA_TRY(launch_kernel(false, row_copy_kernel<VEC, SET, 8>, grid, kRowThreads, 0, s, job));
+  SHMT_CUDA_TRY(launch_kernel(true, row_copy_kernel<VEC, SET, 8>, grid, kRowThreads, 0, s, job));
   return SHMT_OK;
 }
 
@@ -692,7 +699,7 @@ static int launch_bulk(RowJob job, int R, cudaStream_t s) {
   const size_t smem = (size_t)kRowWarps * kBulkStages * R * job.row_bytes;
   static KeptOccupancy kept;
   const unsigned blocks = grid_for_tiles(kernel, &kept, dev, job.n, R, smem);
-  SHMT_CUDA_TRY(launch_kernel(false, kernel, blocks, kRowThreads, smem, s, job));
+  SHMT_CUDA_TRY(launch_kernel(true, kernel, blocks, kRowThreads, smem, s, job));
   return SHMT_OK;
 }
 
@@ -749,7 +756,7 @@ static int launch_ragged(RowJob job, int R, cudaStream_t s) {
   job.rows_per_tile = R;
   const size_t smem = ragged_smem_bytes(job.row_bytes, R);
   static KeptOccupancy kept;
-  SHMT_CUDA_TRY(launch_kernel(false, kernel, grid_for_tiles(kernel, &kept, dev, job.n, R, smem), kRowThreads, smem, s, job));
+  SHMT_CUDA_TRY(launch_kernel(true, kernel, grid_for_tiles(kernel, &kept, dev, job.n, R, smem), kRowThreads, smem, s, job));
   return SHMT_OK;
 }
 

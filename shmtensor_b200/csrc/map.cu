@@ -51,6 +51,7 @@ map_erase_kernel(MapView m, const void* __restrict__ keys, int keys64, int64_t n
 __global__ void __launch_bounds__(kMapThreads, SHMT_QUERY_CTAS)
 map_query_kernel(MapView m, const void* __restrict__ req, int req64, int64_t n,
                  void* __restrict__ out, int out64, LaunchPad<36>) {
+  pdl_prologue();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = threadIdx.x & 31;
@@ -194,7 +195,7 @@ int shmt_map_query(const shmt_map* map, const void* requests, int req_dtype, int
   if (n == 0) return SHMT_OK;
   SHMT_REQUIRE(requests != nullptr && out != nullptr, "shmt_map_query: requests/out are null");
   DeviceGuard guard(map->device);
-  SHMT_CUDA_TRY(launch_kernel(false, map_query_kernel, grid_for_warps(n), kMapThreads, 0, static_cast<cudaStream_t>(stream),
+  SHMT_CUDA_TRY(launch_kernel(true, map_query_kernel, grid_for_warps(n), kMapThreads, 0, static_cast<cudaStream_t>(stream),
                               map->view, requests, req_dtype == SHMT_I64, n, out, map->val_dtype == SHMT_I64,
                               LaunchPad<36>{}));
   return SHMT_OK;

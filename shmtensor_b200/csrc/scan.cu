@@ -40,6 +40,7 @@ template <typename T, int VECS>
 __global__ void __launch_bounds__(kScanThreads, 2)
 scan_kernel(T* __restrict__ data, int64_t n, int exclusive, int vec_ok, TileStates st, int64_t* ticket, int64_t* status,
             int64_t* clean, const TileDesc* carry, LaunchPad<32>) {
+  pdl_prologue();
   using U = typename ScanWord<T>::type;
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr int TILE = scan_tile_bytes(VECS) / (int)sizeof(T);
@@ -485,7 +486,7 @@ template <typename T, int VECS = kScanVecs>
 static void run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_t* ticket, int64_t* status,
                      cudaStream_t s, int64_t* clean = nullptr, const TileDesc* carry = nullptr) {
   const int vec_ok = ((uintptr_t)data & 15) == 0;
-  launch_kernel(false, scan_kernel<T, VECS>, (unsigned)scan_tiles<T>(n, VECS), kScanThreads, 0, s,
+  launch_kernel(true, scan_kernel<T, VECS>, (unsigned)scan_tiles<T>(n, VECS), kScanThreads, 0, s,
                 static_cast<T*>(data), n, exclusive, vec_ok, st, ticket, status, clean, carry, LaunchPad<32>{});
 }
 

@@ -151,3 +151,47 @@ def test_a_new_context_waits_for_no_stream():
     torch.cuda.synchronize()
     _lib.check(_lib.lib.shmt_ctx_destroy(ctx))
     assert busy
+
+
+@pytest.mark.parametrize("dim,dt", [(100, torch.float32), (301, torch.bfloat16), (33, torch.bfloat16)])
+def test_lookups_fetches_and_scans_in_a_row_and_captured(dim, dt):
+    """These kernels are scheduled while the one before them still runs: each reads what the one before it writes,
+    called one after the other and replayed from a graph."""
+    from shmtensor_b200 import capi
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    rows, n = 50_000, 30_011
+    hmap = capi.CUCOStaticHashmap(torch.arange(rows, device="cuda"), torch.arange(rows, dtype=torch.int32, device="cuda"), 0.5)
+    table = torch.randn(rows, dim, generator=g, device="cuda").to(dt)
+    ids = torch.randint(0, rows, (n,), generator=g, device="cuda")
+    x = torch.ones(300_001, dtype=torch.int64, device="cuda")
+
+    def step():
+        at = (ids * 7 + 3) % rows
+        mask = hmap.query(at)
+        one = capi.cache_fetch_with_mask(None, table, at, mask)
+        two = capi.cache_fetch(None, table, mask.long(), hmap)
+        capi.thrust_scan(x)
+        capi.thrust_scan(x)
+        return at, one, two
+
+    def check(got):
+        at, one, two = got
+        assert torch.equal(one, table[at]) and torch.equal(two, table[at])
+        i = torch.arange(1, x.numel() + 1, device="cuda")
+        assert torch.equal(x, i * (i + 1) // 2)
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for _ in range(20):
+            x.fill_(1)
+            check(step())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        got = step()
+    for _ in range(10):
+        ids.random_(0, rows, generator=g)
+        x.fill_(1)
+        graph.replay()
+        check(got)
