@@ -664,19 +664,32 @@ static int launch_lsu(const RowJob& job, cudaStream_t s) {
 }
 
 // Ring geometry of the bulk path: two buffers per warp of about 2 KB each (5 rows of
-// 400 bytes, 4 of 512): measured best on B200 among 0.5 .. 12 KB buffers and 2 .. 4 stages.
+// 400 bytes): measured best on B200 among 0.5 .. 12 KB buffers and 2 .. 4 stages.
 constexpr int kBulkStages = 2;
 constexpr int64_t kBulkStageBytes = 2048;
+// A fetch looks a tile's rows up in one go and waits for it, so few rows a tile means few lookups on their way.
+// Rows of 512 bytes and more therefore come 6 a
+// buffer, as long as these fit.  Popular ids, 0.6 GB fetched: 512 bytes 179 -> 155 us, 640 180 -> 150, 800 196 -> 163, 1,024
+// 159 -> 147, 1,200 238 -> 165, 1,600 184 -> 160, 2,048 150 -> 143, 2,800 166 -> 146; 60,000 rows of 800 bytes 18.3 -> 14.7.
+// Ids drawn evenly from 1.6 GB of rows: 1,024 bytes 225 -> 219 us, 1,200 253 -> 224, 2,048 223 -> 213, but 512 229 -> 238
+// and 576 to 900 bytes 7 to 9 % behind (more scattered reads between the writes than HBM likes), which no cache is
+// filled for.  Sets have their own line: 512 bytes 124 us with 4 rows and 129 with 6, 800 bytes 189 with 2 and 208.
+constexpr int64_t kWideRowBytes = 512, kWideStageBytes = 12800;
+constexpr int kWideRows = 6;
 constexpr size_t kBulkSmemMax = 200 * 1024;
 
 // Rows per ring buffer, 0 if the rows are not 16-byte units or do not fit.
-static int bulk_rows_per_stage(int64_t row_bytes, int vec, int R_small) {
+static int bulk_rows_per_stage(int64_t row_bytes, int vec, int R_small, bool set) {
   if (vec != 16) return 0;
   static const int forced = [] {
     const char* e = getenv("SHMT_BULK_ROWS");
     return e ? atoi(e) : 0;
   }();
   int64_t r = forced > 0 ? forced : kBulkStageBytes / row_bytes;
+  if (forced <= 0 && !set && row_bytes >= kWideRowBytes) {
+    r = kWideStageBytes / row_bytes;
+    if (r > kWideRows) r = kWideRows;
+  }
   if (r < 1) r = 1;
   if (r > 32) r = 32;
   if (r > R_small) r = R_small;
@@ -764,7 +777,7 @@ template <bool SET>
 static int launch_row_copy(const RowJob& job, int vec, cudaStream_t s) {
   {
     static const bool no_bulk = getenv("SHMT_NO_BULK") != nullptr;
-    const int R = no_bulk ? 0 : bulk_rows_per_stage(job.row_bytes, vec, job.rows_per_tile);
+    const int R = no_bulk ? 0 : bulk_rows_per_stage(job.row_bytes, vec, job.rows_per_tile, SET);
     if (R >= 1) return launch_bulk<SET>(job, R, s);
     const int ragged = SET || no_bulk ? 0 : ragged_rows_per_stage(job, vec);
     if (ragged >= 1) return launch_ragged(job, ragged, s);

@@ -375,3 +375,29 @@ def test_host_rows_around_the_line_between_narrow_copies_and_granules(capi, row_
     finally:
         capi.unpin_memory(host)
     assert capi.device_fault() == 0
+
+
+@pytest.mark.parametrize("row_bytes", [496, 512, 528, 1024, 2048, 2128, 2144, 6400, 6416, 12_800, 12_816])
+def test_rows_of_512_bytes_and_more_several_a_buffer(capi, row_bytes):
+    """Six rows a ring buffer from 512 bytes on, fewer where six do not fit (2,133 bytes), one (6,416), none
+    (12,816: the copy without a ring); batches of less than a tile and of many, the last tile partly filled, rows
+    cached, in host memory, and in neither."""
+    g = torch.Generator(device="cuda").manual_seed(row_bytes)
+    rows = 3000
+    host = torch.randint(0, 256, (rows, row_bytes), generator=g, device="cuda", dtype=torch.uint8).cpu().pin_memory()
+    cached = torch.randperm(rows, generator=g, device="cuda")[:2000]
+    gpu = host.cuda()[cached] ^ 85                       # a hit that reads the host row is seen
+    m = capi.CUCOStaticHashmap(cached, torch.arange(2000, dtype=torch.int32, device="cuda"), 0.5)
+    truth = host.cuda()
+    truth[cached] = gpu
+    for n in (1, 7, 5000, min(28_423, 200_000_000 // row_bytes)):
+        ids = torch.randint(0, rows, (n,), generator=g, device="cuda")
+        out = torch.full((n + 2, row_bytes), 7, dtype=torch.uint8, device="cuda")
+        got = capi.cache_fetch(host, gpu, ids, m)
+        assert torch.equal(got, truth[ids])
+        assert torch.equal(capi.cache_fetch_with_mask(host, gpu, ids, m.query(ids)), got)
+        capi._fetch(None, gpu, ids, m, None, "rows in neither", out=out[1:n + 1])
+        hit = m.query(ids) >= 0
+        assert torch.equal(out[1:n + 1], torch.where(hit[:, None], got, torch.full_like(got, 7)))
+        assert (out[0] == 7).all() and (out[n + 1] == 7).all()
+    assert capi.device_fault() == 0
