@@ -100,6 +100,15 @@ __device__ __forceinline__ void post_to_host(const HostPost& p) {
   if (lane == 0) st_release_sys64(p.host + p.flag_at, p.seq);
 }
 
+// The same with the first four words, as far as they are not W_RESULT, zero, and by a warp that has the result.
+__device__ __forceinline__ void post_result(const HostPost& p, int64_t result) {
+  if (!p.host) return;
+  const int lane = (int)(threadIdx.x & 31);
+  if (lane < p.n_words) *reinterpret_cast<volatile int64_t*>(p.host + lane) = lane == W_RESULT ? result : 0;
+  __syncwarp();
+  if (lane == 0) st_release_sys64(p.host + p.flag_at, p.seq);
+}
+
 __device__ __forceinline__ void post_note(const HostPost& p, int64_t a, int64_t b) {
   *reinterpret_cast<volatile int64_t*>(p.host + p.flag_at) = a;
   *reinterpret_cast<volatile int64_t*>(p.host + p.flag_at + 1) = b;

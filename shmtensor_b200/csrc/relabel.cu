@@ -757,6 +757,7 @@ relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* 
   long long* s_key = reinterpret_cast<long long*>(s_table);
   unsigned* s_first = reinterpret_cast<unsigned*>(s_key + slots);  // smallest index of the id; later its new id
   __shared__ int s_count[ITEMS * kWarps];
+  __shared__ int s_found;
   const unsigned full = 0xffffffffu;
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const PartSizes sizes{ps.start[kMaxParts], -1};
@@ -816,6 +817,7 @@ relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* 
       run += __shfl_sync(full, inc, 31);
     }
     if (lane == 0) {
+      s_found = run;
       st_relaxed64(status, DEV_OK);
       st_relaxed64(result, run);
     }
@@ -831,7 +833,7 @@ relabel_small_kernel(Parts ps, uint32_t slots, void* __restrict__ unique, void* 
     }
   }
   __syncthreads();
-  if (warp == 0) post_to_host(post);  // behind the last barrier: nobody waits for its way to the host
+  if (warp == 0) post_result(post, s_found);  // behind the last barrier: nobody waits for its way to the host
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = j * kRelSmallThreads + tid;

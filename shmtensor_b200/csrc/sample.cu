@@ -22,6 +22,8 @@
 //      ones (or, for rows shorter than 2k, the deg-k to leave out) are held: O(k) draws, no
 //      global atomics.  Only beyond 1024 picks per seed does it fall back to the reference's
 //      reservoir on the output row.
+#include <type_traits>
+
 #include "ctx.cuh"
 #include "lookback.cuh"
 #include "map.cuh"
@@ -331,7 +333,14 @@ constexpr float kWeightedShareCost = 200.0f;  // barriers, and the ranking
 // HOP_FUSED: a hop of a mini-batch, which also claims relabel slots.  HOP_SINGLE: a call of its own.  Kernels
 // apart, because the claims' code and registers cost a small call 0.7 of 24 us though it never runs it.  HOP_EARLY: a
 // weighted call whose count the host waits for (see step 3).
-enum : int { HOP_FUSED = 0, HOP_SINGLE = 1, HOP_EARLY = 2 };
+// HOP_TINY: a call of its own for few seeds.  Every CTA looks all seeds up and adds up all picks itself: no ticket, no
+// look-back, nobody counts anybody out, and the count is on its way to the host before a position is picked.  100
+// seeds on the GPU 23.6 us a call, 19.5 so; 1,024 24.0 and 22.4.
+enum : int { HOP_FUSED = 0, HOP_SINGLE = 1, HOP_EARLY = 2, HOP_TINY = 3 };
+// Beyond a few seeds a thread the CTAs' repeated lookups cost what the look-back does.  Over a host graph each CTA reads
+// all row bounds across the link: 50 seeds 25.0 us the other way and 22.7 so, 100 seeds 26.0 and 26.6, 256 seeds 26.9
+// and 51.7.
+constexpr int64_t kTinySeeds = 4 * kHopThreads, kTinyHostSeeds = 64;
 
 template <typename IxT, int G, int MODE>
 __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
@@ -340,6 +349,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   __shared__ int64_t s_total;
   __shared__ LookbackShared s_look;
   __shared__ int s_tile;
+  __shared__ int64_t s_prefix, s_end;  // HOP_TINY
 
   pdl_prologue();
   const unsigned full = 0xffffffffu;
@@ -368,15 +378,84 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     }
     return;
   }
-  const int tile = take_tile(job.ticket, &s_tile);  // as many CTAs as tiles are left
-  constexpr bool kFused = MODE == HOP_FUSED, kEarly = MODE == HOP_EARLY;
+  constexpr bool kFused = MODE == HOP_FUSED, kEarly = MODE == HOP_EARLY, kTiny = MODE == HOP_TINY;
+  const int tile = kTiny ? (int)blockIdx.x : take_tile(job.ticket, &s_tile);  // as many CTAs as tiles are left
   if (!kFused && job.clean && tile == 0 && tid == 0) st_relaxed64(job.status, DEV_OK);  // it reports on this call only
   const int64_t first = (int64_t)tile * S;
   const int rows = (int)min((int64_t)S, n - first);
   const int64_t k = job.k;
 
   // ---- 1. row bounds and pick counts, one seed per thread
-  for (int j0 = (int)(tid & ~31u); j0 < S; j0 += kHopThreads) {
+  if (kTiny) {  // of all seeds, a few in a row per thread; this CTA's are kept
+    auto add_up = [&](auto most) -> int64_t {
+      constexpr int kMost = decltype(most)::value;
+      const int per = kMost == 1 ? 1 : (int)((n + kHopThreads - 1) / kHopThreads);
+      int64_t row[kMost], slot[kMost], b[kMost], e[kMost];
+#pragma unroll
+      for (int q = 0; q < kMost; ++q) {
+        const int i = (int)tid * per + q;
+        row[q] = q < per && i < n ? load_int(job.seeds, job.seeds64, i) : kEmptyKey;
+      }
+#pragma unroll
+      for (int q = 0; q < kMost; ++q) {
+        if (q >= per) break;
+        const bool valid = (int64_t)tid * per + q < n;
+        slot[q] = -1;
+        if (job.map.slots) slot[q] = warp_find(job.map, row[q], valid);
+        b[q] = e[q] = 0;
+        if (valid) {
+          if (slot[q] >= 0)
+            load_bounds(job.gpu_indptr, job.indptr64, slot[q], &b[q], &e[q]);
+          else
+            load_bounds(job.indptr, job.indptr64, row[q], &b[q], &e[q]);
+        }
+      }
+      auto picks = [&](int q) -> int64_t {
+        if (q >= per || (int64_t)tid * per + q >= n) return 0;
+        const int64_t deg = e[q] - b[q];
+        return job.replace ? (deg > 0 ? k : 0) : (deg < k ? deg : k);
+      };
+      int64_t sum = 0;
+#pragma unroll
+      for (int q = 0; q < kMost; ++q) sum += picks(q);
+      int64_t run = block_exclusive_scan(sum, warp_sums, &s_total);
+#pragma unroll
+      for (int q = 0; q < kMost; ++q) {
+        const int i = (int)tid * per + q, j = i - (int)first;
+        if (q < per && j >= 0 && j < rows) {
+          s_begin[j] = b[q];
+          s_deg[j] = e[q] - b[q];
+          s_hit[j] = slot[q] >= 0;
+          s_off[j] = run;
+          if (job.out_eids) s_eshift[j] = slot[q] >= 0 ? load_int(job.gpu_edge_base, job.indptr64, slot[q]) - b[q] : 0;
+          store_int(job.sub_indptr, job.indptr64, i, run);
+          if (j == rows - 1) s_end = run + picks(q);
+        }
+        run += picks(q);
+      }
+      return s_total;
+    };
+    const int64_t total = n <= kHopThreads ? add_up(std::integral_constant<int, 1>{})
+                                           : add_up(std::integral_constant<int, (int)(kTinySeeds / kHopThreads)>{});
+    if (tile == 0 && tid < 32) {
+      if (tid == 0) {
+        store_int(job.sub_indptr, job.indptr64, n, total);
+        st_relaxed64(job.status, DEV_OK);
+        st_relaxed64(job.result, total);
+      }
+      post_result(job.post, total);
+    }
+    __syncthreads();
+    const int64_t prefix = s_off[0];
+    __syncthreads();
+    for (int j = (int)tid; j < rows; j += kHopThreads) s_off[j] -= prefix;
+    if (tid == 0) {
+      s_prefix = prefix;
+      s_total = s_end - prefix;
+    }
+    __syncthreads();
+  }
+  for (int j0 = (int)(tid & ~31u); !kTiny && j0 < S; j0 += kHopThreads) {
     const int j = j0 + (int)lane;
     const bool valid = j < rows;
     const int64_t row = valid ? load_int(job.seeds, job.seeds64, first + j) : kEmptyKey;
@@ -403,7 +482,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
 
   // ---- 2. offsets inside the tile.  The tile's sum goes out now: the tiles behind it then never
   // wait for the neighbour loads and slot claims below.
-  {
+  if (!kTiny) {
     const int ch = (S + kHopThreads - 1) / kHopThreads;  // seeds per thread, 1..4
     int64_t c[kMaxSeedsPerTile / kHopThreads];
     int64_t sum = 0;
@@ -478,7 +557,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   // Picking by weight takes long, and a host that waits for the count need not wait for it, so the
   // tile takes its place first (8 rows of 1,000 edges, 15 picks each: 46.6 us a call, 31.2 so).  Both orders in one
   // kernel cost the other one: a weighted mini-batch of 1,000 seeds 130 us for 125.
-  const int64_t placed = kEarly ? place() : 0;
+  const int64_t placed = kEarly ? place() : (kTiny ? s_prefix : 0);
 
   // ---- 3. (k <= 32) positions of the picked neighbours, a group of lanes per seed, into a list in
   // output order.  Arithmetic and shuffles only: the memory work is left to step 5, where all
@@ -611,7 +690,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
     return __ldg(static_cast<const IxT*>(x.hit() ? job.gpu_indices : job.indices) + x.at());
   };
   IxT next = fetch((int)tid);
-  const int64_t prefix = kEarly ? placed : place();
+  const int64_t prefix = kEarly || kTiny ? placed : place();
 
   // ---- 5. output and relabel slots, one list element per thread and step
   if (listed) {
@@ -917,6 +996,13 @@ static cudaError_t launch_hop_as(const HopJob& job, unsigned grid, size_t smem, 
   return launch_kernel(pdl, sample_hop_kernel<IxT, 32, MODE>, grid, kHopThreads, smem, s, job);
 }
 
+static bool on_device(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeDevice;
+  cudaGetLastError();  // a failed query must not poison the next launch check
+  return false;
+}
+
 template <typename IxT>
 static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool pdl = false) {
   const unsigned grid = (unsigned)n_tiles;
@@ -924,6 +1010,8 @@ static cudaError_t launch_hop(HopJob job, int64_t n_tiles, cudaStream_t s, bool 
   const size_t smem = hop_smem_bytes(job.seeds_per_tile, hop_layout_k(job.weights, job.replace, job.k), job.set_slots,
                                      job.weights && !job.replace);
   if (job.rel_slots) return launch_hop_as<IxT, HOP_FUSED>(job, grid, smem, s, pdl);
+  if (!job.weights && (job.n <= kTinyHostSeeds || (job.n <= kTinySeeds && on_device(job.indptr))))
+    return launch_hop_as<IxT, HOP_TINY>(job, grid, smem, s, pdl);
   if (job.weights && !job.replace && job.post.host)  // the lists of fan-outs up to 32: within 48 KB
     return launch_kernel(pdl, sample_hop_kernel<IxT, 32, HOP_EARLY>, grid, kHopThreads, smem, s, job);
   return launch_hop_as<IxT, HOP_SINGLE>(job, grid, smem, s, pdl);

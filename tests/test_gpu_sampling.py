@@ -530,3 +530,35 @@ def test_minibatch_words_when_their_tags_run_out(capi):
                 assert np.array_equal(front.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
             assert all(torch.equal(a, b) for a, b in zip(want, (front, sp, sx, rel))), i
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 64, 65, 256, 257, 1023, 1024, 1025])
+@pytest.mark.parametrize("k", [1, 8, 9, 32, 40])
+def test_hops_in_which_every_cta_adds_up_all_picks(capi, n, k):
+    """Up to 1,024 seeds on the GPU and 64 over a host graph every CTA adds up all picks itself; more take their
+    places from one another.  Offsets, rows, edge ids, a cached graph's rows and repeated seeds; the same draws from
+    the graph on the GPU, in host memory, and cached."""
+    rng = np.random.default_rng(n * 100 + k)
+    deg = rng.integers(0, 3 * k + 2, size=700)
+    indptr_n = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    indices_n = np.concatenate([rng.permutation(5000)[:d] for d in deg]).astype(np.int32)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    hot = torch.from_numpy(rng.permutation(700)[:300]).cuda()
+    gp, gi = capi.create_subcsr(indptr, indices, hot)
+    hmap = capi.CUCOStaticHashmap(hot, torch.arange(300, device="cuda"), 0.5)
+    base = capi.subcsr_edge_base(indptr, hot)
+    seeds_n = rng.integers(0, 700, size=n)
+    seeds = torch.from_numpy(seeds_n).cuda()
+    for replace in (False, True):
+        capi.set_sampling_seed(6)
+        p, x = capi.csr_sampling(indptr, indices, seeds, k, replace)
+        oracle.check_sample_bulk(indptr_n, indices_n, seeds_n, k, replace, p.cpu().numpy(), x.cpu().numpy(), distinct_rows=True)
+        capi.set_sampling_seed(6)
+        p2, x2 = capi.csr_cache_sampling(indptr, indices, gp, gi, hmap, seeds, k, replace)
+        assert torch.equal(p, p2) and torch.equal(x, x2)
+        capi.set_sampling_seed(6)
+        p3, x3, e3 = capi.csr_sampling_with_eids(indptr, indices, seeds, k, replace, gp, gi, base, hmap)
+        assert torch.equal(p, p3) and torch.equal(x, x3) and torch.equal(indices[e3], x)
+        capi.set_sampling_seed(6)
+        p4, x4 = capi.csr_cache_sampling(indptr.cpu().pin_memory(), indices.cpu().pin_memory(), gp, gi, hmap, seeds, k, replace)
+        assert torch.equal(p, p4) and torch.equal(x, x4)
