@@ -324,7 +324,7 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
 
 /* The three mini-batches above as one call (weights, gpu_edge_base and what belongs to them may be null) that
  * is also told how many rows indptr has: on graphs of up to 2^25 nodes ids are then relabelled through a
- * word per node, behind the relabel table of the context, instead of hashed slots (n_nodes = 0: not known; ids of
+ * word per node, kept by the context, instead of hashed slots (n_nodes = 0: not known; ids of
  * n_nodes and more are accepted and hashed).  The outputs lie in two pools, one per dtype: hop h's sub_indptr at
  * element layout[h] of indptr_pool, its edge ids (if with_edge_ids) at layout[n_hops + h], and in
  * indices_pool its sub_indices at layout[2 * n_hops + h], relabelled ids at layout[3 * n_hops + h] and frontier

@@ -153,15 +153,13 @@ int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
   return SHMT_OK;
 }
 
-int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words) {
+int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
   if (int rc = ctx_join_tail(ctx, stream)) return rc;
-  if (bytes + words > ctx->table_bytes) {
+  if (bytes > ctx->table_bytes) {
     if (ctx->table) SHMT_CUDA_TRY(cudaFree(ctx->table));
     ctx->table = nullptr;
     ctx->table_bytes = 0;
-    ctx->table_words_bytes = 0;
     size_t want = bytes + bytes / 2;
-    if (want < bytes + words) want = bytes + words;
     if (want < ((size_t)4 << 20)) want = (size_t)4 << 20;
     want = (want + 255) & ~(size_t)255;
     void* p = nullptr;
@@ -173,27 +171,36 @@ int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t w
   if (ctx->table_dirty) {
     SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table, 0xFF, ctx->table_bytes, stream));
     ctx->table_dirty = false;
-    ctx->table_words_bytes = 0;
-  }
-  if (bytes > ctx->table_bytes - ctx->table_words_bytes) {  // slots in the place of words
-    SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table + ctx->table_bytes - ctx->table_words_bytes, 0xFF, ctx->table_words_bytes,
-                                  stream));
-    ctx->table_words_bytes = 0;
-  }
-  if (words > ctx->table_words_bytes) {
-    // every word of an empty slot has its top bit set
-    if (ctx->table_words_bytes == 0 || ctx->words_tag > 0x80000000u) ctx->words_tag = 0x80000000u;
-    ctx->table_words_bytes = words;
   }
   return SHMT_OK;
 }
 
-int ctx_take_tags(shmt_ctx* ctx, unsigned count, unsigned* first, cudaStream_t stream) {
-  if (ctx->words_tag < count) {
-    SHMT_CUDA_TRY(cudaMemsetAsync(ctx->table + ctx->table_bytes - ctx->table_words_bytes, 0xFF, ctx->table_words_bytes,
-                                  stream));
-    ctx->words_tag = 0xFFFFFFFFu;
+static int empty_words(shmt_ctx* ctx, cudaStream_t stream) {
+  SHMT_CUDA_TRY(cudaMemsetAsync(ctx->words, 0xFF, ctx->words_bytes, stream));
+  ctx->words_tag = 0xFFFFFFFFu;
+  ctx->words_dirty = false;
+  return SHMT_OK;
+}
+
+int ctx_reserve_words(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
+  if (int rc = ctx_join_tail(ctx, stream)) return rc;
+  if (bytes > ctx->words_bytes) {
+    if (ctx->words) SHMT_CUDA_TRY(cudaFree(ctx->words));
+    ctx->words = nullptr;
+    ctx->words_bytes = 0;
+    const size_t want = (bytes + 255) & ~(size_t)255;
+    void* p = nullptr;
+    SHMT_CUDA_TRY(cudaMalloc(&p, want));
+    ctx->words = static_cast<unsigned*>(p);
+    ctx->words_bytes = want;
+    ctx->words_dirty = true;
   }
+  return ctx->words_dirty && ctx->words ? empty_words(ctx, stream) : SHMT_OK;
+}
+
+int ctx_take_tags(shmt_ctx* ctx, unsigned count, unsigned* first, cudaStream_t stream) {
+  if (ctx->words_tag < count)
+    if (int rc = empty_words(ctx, stream)) return rc;
   *first = ctx->words_tag -= count;
   return SHMT_OK;
 }
@@ -207,7 +214,7 @@ int ctx_fetch_words(shmt_ctx* ctx, cudaStream_t stream, const char* what) {
 
 int ctx_status_of_words(shmt_ctx* ctx, const char* what) {
   const int64_t st = ctx->h_words[W_STATUS];
-  if (st != DEV_OK) ctx->table_dirty = true;
+  if (st != DEV_OK) ctx_table_failed(ctx);
   if (st == DEV_TIMEOUT) {
     set_error("%s: a bounded look-back wait ran out (device status %lld)", what, (long long)st);
     return SHMT_ERR_TIMEOUT;
@@ -280,6 +287,7 @@ int shmt_ctx_destroy(shmt_ctx* ctx) {
   DeviceGuard guard(ctx->device);
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->table) cudaFree(ctx->table);
+  if (ctx->words) cudaFree(ctx->words);
   if (ctx->scan_state) cudaFree(ctx->scan_state);
   if (ctx->h_words) cudaFreeHost(ctx->h_words);
   if (ctx->tail_event) cudaEventDestroy(ctx->tail_event);
@@ -311,7 +319,7 @@ int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, 
 }
 
 int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx) {
-  return ctx ? (int64_t)(ctx->scratch_bytes + ctx->table_bytes + kScanStateBytes) : 0;
+  return ctx ? (int64_t)(ctx->scratch_bytes + ctx->table_bytes + ctx->words_bytes + kScanStateBytes) : 0;
 }
 
 }  // extern "C"

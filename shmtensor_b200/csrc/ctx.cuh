@@ -33,12 +33,13 @@ struct shmt_ctx {
   char* table = nullptr;
   size_t table_bytes = 0;
   bool table_dirty = false;     // a failed call may have left entries behind
-  // Words of mini-batches (RelTable in relabel.cuh): the last table_words_bytes of the block.  They hold
-  // numbers from words_tag on, not the all ones of empty slots, so slots that reach into them need them cleared.
-  size_t table_words_bytes = 0;
+  // Words of mini-batches (RelTable in relabel.cuh), in a block of their own: they hold numbers from words_tag on,
+  // which would be taken for slots, and a table that grew for them would leave captured relabels without theirs.
+  unsigned* words = nullptr;
+  size_t words_bytes = 0;
   unsigned words_tag = 0;
-  bool table_reserved = false;  // the caller sized the table for mini-batches: none of them grows it for words
-  unsigned* table_words(int64_t n) const { return reinterpret_cast<unsigned*>(table + table_bytes) - n; }
+  bool words_dirty = false;     // a failed call may have left numbers below words_tag behind
+  bool words_reserved = false;  // the caller sized the context for mini-batches: none of them grows it for words
   // Early hand-over of result words (see HostPost): sequence number of the last post, and an
   // event behind the kernels that were still running when the call returned.
   int64_t post_seq = 0;
@@ -72,9 +73,14 @@ enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).
 int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
 
-// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with), and behind them `words`
-// bytes of words.
-int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream, size_t words = 0);
+// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with).
+int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
+
+// Make sure ctx->words holds at least `bytes`, every word of them above words_tag - 1.
+int ctx_reserve_words(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
+
+// A failed call may have left entries in the table and the words.
+inline void ctx_table_failed(shmt_ctx* ctx) { ctx->table_dirty = ctx->words_dirty = true; }
 
 // `count` numbers below all that the words hold: *first and those behind it.
 int ctx_take_tags(shmt_ctx* ctx, unsigned count, unsigned* first, cudaStream_t stream);

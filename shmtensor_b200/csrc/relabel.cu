@@ -892,10 +892,10 @@ size_t relabel_scratch_bytes(int64_t numel) { return relabel_scratch(numel).all;
 
 int relabel_table(shmt_ctx* ctx, int64_t numel_bound, RelTable* t, cudaStream_t s, const RelWords& words) {
   const uint64_t cap = relabel_capacity(numel_bound);
-  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s, (size_t)words.n * sizeof(unsigned))) return rc;
+  if (int rc = ctx_reserve_table(ctx, cap * sizeof(RelSlot), s)) return rc;
   t->slots = reinterpret_cast<RelSlot*>(ctx->table);
   t->cap = (uint32_t)cap;
-  t->words = words.n ? ctx->table_words(words.n) : nullptr;
+  t->words = words.n ? ctx->words : nullptr;
   t->n_words = (uint32_t)words.n;
   t->tag = words.tag;
   return SHMT_OK;

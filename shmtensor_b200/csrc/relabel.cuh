@@ -45,7 +45,7 @@ constexpr unsigned kRelNewId = 0x80000000u;  // indexes and new ids stay below 2
 // nobody waits for, where a slot takes a 32-byte read, a compare-and-swap and a minimum; and the words
 // of a graph fit the L2 cache where the slots of a large frontier do not.  Tags go down from hop to hop by
 // as many numbers as it can have indices, so that whatever earlier hops have left is larger than all of this
-// one's, and no word is ever put back (but all of them when the tags have come down, every 200 batches of
+// one's, and no word is ever put back (but all of them when the tags have come down, every 429 batches of
 // 10 M ids).  An element that finds another's index in its word is a repeat of that element, whose result it takes.
 // Other ids (a last hop may reach nodes that have no row) take slots.
 // Slots against words, 8,192 seeds 5/10/15, int64 ids: 2.4 M nodes 416 us and 292, 10 M 536 and 354, 24 M 579
@@ -224,7 +224,7 @@ uint64_t relabel_capacity(int64_t numel_bound);
 // Context scratch that shmt_relabel takes for up to `numel` ids.
 size_t relabel_scratch_bytes(int64_t numel);
 
-// Words of a hop (n = 0: none).
+// Words of a hop (n = 0: none), which ctx_reserve_words has made room for.
 struct RelWords {
   int64_t n = 0;
   unsigned tag = 0;

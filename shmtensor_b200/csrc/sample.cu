@@ -1050,13 +1050,12 @@ static int plan_minibatch(int64_t n_seeds, const int64_t* fanouts, int n_hops, M
   return SHMT_OK;
 }
 
-// Words for the ids of a mini-batch of up to `numel_bound` of them on a graph of `n_nodes` (0: not known): all
-// or none.  None where a table that the caller has sized would have to grow.
-static int64_t minibatch_words(const shmt_ctx* ctx, int64_t numel_bound, int64_t n_nodes) {
+// Words for the ids of a mini-batch on a graph of `n_nodes` (0: not known): all or none.  None where a context
+// that the caller has sized would have to grow.
+static int64_t minibatch_words(const shmt_ctx* ctx, int64_t n_nodes) {
   if (n_nodes > kRelMaxWords) return 0;
-  const uint64_t cap = relabel_capacity(numel_bound);
-  const bool fits = cap * sizeof(RelSlot) + (size_t)n_nodes * sizeof(unsigned) <= ctx->table_bytes;
-  return fits || !ctx->table_reserved ? n_nodes : 0;
+  const bool fits = (size_t)n_nodes * sizeof(unsigned) <= ctx->words_bytes;
+  return fits || !ctx->words_reserved ? n_nodes : 0;
 }
 
 }  // namespace shmt
@@ -1083,11 +1082,14 @@ int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64
                            static_cast<cudaStream_t>(stream)))
     return rc;
   RelTable t;
-  ctx->table_reserved = false;
-  RelWords words;
-  words.n = minibatch_words(ctx, plan.cap[n_hops], n_nodes);
-  if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream), words)) return rc;
-  ctx->table_reserved = true;
+  if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream))) return rc;
+  // where the node count is not known: room for the words of a small graph, as much as a table takes beyond its slots
+  const size_t slots = t.cap * sizeof(RelSlot), least = (size_t)4 << 20;
+  size_t words = slots + slots / 2 < least ? least - slots : slots / 2;
+  if (words > kRelMaxWords * sizeof(unsigned)) words = kRelMaxWords * sizeof(unsigned);
+  if (n_nodes > 0) words = n_nodes <= kRelMaxWords ? n_nodes * sizeof(unsigned) : 0;
+  if (int rc = ctx_reserve_words(ctx, words, static_cast<cudaStream_t>(stream))) return rc;
+  ctx->words_reserved = true;
   return SHMT_OK;
 }
 
@@ -1269,12 +1271,13 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
 
   // the relabel table for the largest hop, reserved before anything is queued
   RelWords rel_words;
-  rel_words.n = minibatch_words(ctx, cap[n_hops], n_nodes);
+  rel_words.n = minibatch_words(ctx, n_nodes);
   {
     RelTable biggest;
-    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s, rel_words)) return rc;
+    if (int rc = relabel_table(ctx, cap[n_hops], &biggest, s)) return rc;
   }
   if (rel_words.n) {
+    if (int rc = ctx_reserve_words(ctx, (size_t)rel_words.n * sizeof(unsigned), s)) return rc;
     unsigned ids = 0;
     for (int h = 0; h < n_hops; ++h) ids += (unsigned)cap[h + 1];
     if (int rc = ctx_take_tags(ctx, ids, &rel_words.tag, s)) return rc;
@@ -1371,7 +1374,7 @@ static int await_minibatch(shmt_ctx* ctx) {
   if (int rc = ctx_await_post(ctx, ctx->batch.post, static_cast<cudaStream_t>(ctx->batch.stream))) return rc;
   const int64_t st = ctx->h_words[n_hops * 8];
   if (st != DEV_OK) {
-    ctx->table_dirty = true;
+    ctx_table_failed(ctx);
     set_error("shmt_sample_minibatch: device status %lld (%s)", (long long)st,
               st == DEV_TIMEOUT ? "a bounded look-back wait ran out" : "relabel table overflow");
     return st == DEV_TIMEOUT ? SHMT_ERR_TIMEOUT : SHMT_ERR_CAPACITY;

@@ -668,6 +668,7 @@ extern "C" int shmt_debug_lookback_timeout(shmt_ctx* ctx, void* stream) {
   if (ctx->table)  // index 0 in every slot of the relabel table
     SHMT_CUDA_TRY(cudaMemset2DAsync(ctx->table + offsetof(RelSlot, first), sizeof(RelSlot), 0, sizeof(RelSlot::first),
                                     ctx->table_bytes / sizeof(RelSlot), s));
+  if (ctx->words) SHMT_CUDA_TRY(cudaMemsetAsync(ctx->words, 0, ctx->words_bytes, s));
   return ctx_fetch_words(ctx, s, "shmt_debug_lookback_timeout");
 }
 

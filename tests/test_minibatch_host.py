@@ -1,0 +1,57 @@
+"""What the host does with the context of a mini-batch, on a runtime that runs nothing (fake_runtime.py): the memory
+that a context keeps, a mini-batch that nobody waits for, and a stream that is being captured."""
+import ctypes as C
+
+import pytest
+
+import fake_runtime
+from shmtensor_b200 import _lib
+
+N_IDS = 100_000
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return fake_runtime.load(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def ctx(lib):
+    out = C.c_void_p()
+    assert lib.shmt_ctx_create(0, C.byref(out)) == _lib.OK
+    yield out.value
+    lib.fake_capture(0)
+    lib.shmt_ctx_destroy(out.value)
+
+
+def _buffer(nbytes):
+    return (C.c_char * (nbytes + 16))()
+
+
+def _start(lib, ctx, n_nodes, n_seeds=100, k=5):
+    edges = n_seeds * k
+    pools = _buffer(8 * (n_seeds + 1)), _buffer(8 * (3 * edges + 2 * n_seeds + 16)), _buffer(8 * n_seeds)
+    layout = (C.c_int64 * 5)(0, 0, 0, edges, 2 * edges + n_seeds)
+    some = C.addressof(pools[2])
+    return lib.shmt_minibatch_start(ctx, some, _lib.I64, n_nodes, some, _lib.I64, None, None, None, None, None, None, some,
+                                    n_seeds, (C.c_int64 * 1)(k), 1, 0, 1, 1, C.addressof(pools[0]), C.addressof(pools[1]),
+                                    layout, 0, None)
+
+
+def _relabel(lib, ctx, n=N_IDS):
+    ids, unique, local = (_buffer(8 * n) for _ in range(3))
+    return lib.shmt_relabel(ctx, (C.c_void_p * 1)(C.addressof(ids)), (C.c_int64 * 1)(n), 1, _lib.I64,
+                            C.addressof(unique), C.addressof(local), None, None)
+
+
+@pytest.mark.parametrize("n_nodes", [0, 3, 2_000_000, 1 << 25])
+def test_a_minibatch_moves_no_memory_that_a_sized_context_holds(lib, ctx, n_nodes):
+    """A relabel that was captured in a sized context keeps the addresses of its table: a mini-batch within that size may
+    add memory for its words, and gives none back."""
+    assert lib.shmt_ctx_reserve(ctx, 1 << 20, N_IDS, None) == _lib.OK
+    assert _relabel(lib, ctx) == _lib.OK
+    lib.fake_reset()
+    for _ in range(3):
+        assert _start(lib, ctx, n_nodes) == _lib.OK
+        assert _relabel(lib, ctx) == _lib.OK
+    assert lib.fake_frees() == 0
