@@ -342,6 +342,19 @@ enum : int { HOP_FUSED = 0, HOP_SINGLE = 1, HOP_EARLY = 2, HOP_TINY = 3 };
 // and 51.7.
 constexpr int64_t kTinySeeds = 4 * kHopThreads, kTinyHostSeeds = 64;
 
+// Reductions on one address are served one after the other, 1.15 ns each, so the word of a node that many edges lead to
+// must not get one for every edge.  A CTA of a mini-batch's hop keeps the ids whose words it has lowered, the last
+// at each place: an id below 2^25 times an odd number, modulo 2^25, has its place in the upper 10 bits, and the lower 15 tell
+// ids of one place apart; below them, in the entry, the index within the tile.  A neighbour whose id is there with a
+// smaller index leaves the word alone: whoever made the entry lowers it as far, or has left that to a smaller index still.
+// 8,192 seeds 5/10/15 on 10 M nodes, int64 ids: a tenth of all edges to one node 908 us without, 384 so (third hop 809 and 142;
+// hashed slots 560), neighbours by rank^-1.1 249 and 145 (slots 188), drawn evenly 352 both; 1,024 seeds 213 and 129, 108 and 106,
+// 128 and 130.  With 8-byte entries, and lanes that meet looked for in every step, not in the first alone, 344 was 373.
+constexpr int kLoweredTagBits = 15, kLoweredEntries = (int)(kRelMaxWords >> kLoweredTagBits);
+constexpr unsigned kLoweredLocal = (1u << (32 - kLoweredTagBits)) - 1u;
+// What a kernel may take beside its arrays of fixed size, at most 8 KB, without asking for more.
+constexpr size_t kPlainHopSmem = 40 << 10;
+
 template <typename IxT, int G, int MODE>
 __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sample_hop_kernel(const HopJob job) {
   extern __shared__ __align__(16) unsigned char s_dyn[];  // hop_smem_bytes()
@@ -350,8 +363,12 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   __shared__ LookbackShared s_look;
   __shared__ int s_tile;
   __shared__ int64_t s_prefix, s_end;  // HOP_TINY
+  __shared__ unsigned s_lowered[MODE == HOP_FUSED ? kLoweredEntries : 1];
 
-  pdl_prologue();
+  pdl_launch_next();
+  if (MODE == HOP_FUSED)  // the barriers of the pick counts' scan lie before its first use
+    for (int q = (int)threadIdx.x; q < kLoweredEntries; q += kHopThreads) s_lowered[q] = ~0u;
+  pdl_wait();
   const unsigned full = 0xffffffffu;
   const unsigned tid = threadIdx.x, lane = tid & 31;
   const int S = job.seeds_per_tile;
@@ -515,10 +532,35 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const RelRange range{job.rel_slots,
                        kFused ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
                        job.rel_cap};
+  // The word of node `id`, unless this CTA has lowered it as far (s_lowered).  `local`, the index within the tile as
+  // far as it can be held, goes up with `i`.
+  auto lower = [&](unsigned id, unsigned i, unsigned local, bool crowd) {
+    const unsigned mixed = id * 0x9E3779B1u & (kRelMaxWords - 1);
+    volatile unsigned* last = s_lowered + (mixed >> kLoweredTagBits);
+    const unsigned mine = mixed << (32 - kLoweredTagBits) | local;
+    unsigned seen = *last;
+    if (seen < mine && (seen ^ mine) <= kLoweredLocal) return;
+    *last = mine;
+    unsigned* word = job.rel_words + id;
+    if (crowd) {  // nothing is known yet: lanes that meet here leave it to the lowest, which looks first
+      seen = *last;  // of several lanes' stores one
+      if (seen < mine && (seen ^ mine) <= kLoweredLocal) return;
+      const unsigned together = __activemask();
+      if (__any_sync(together, seen != mine)) {
+        const unsigned same = __match_any_sync(together, id);
+        if (__shfl_sync(same, i, __ffs(same) - 1) < i) return;
+        if (same & (same - 1u) && __ldcg(word) <= job.rel_tag + i) return;
+      }
+    }
+    atomicMin(word, job.rel_tag + i);
+  };
   // the id at index i of [seeds | neighbours]: its slot, for the later relabel passes
-  auto enter = [&](int64_t i, IxT id) {
+  auto enter = [&](int64_t i, IxT id, int64_t local, bool crowd) {
     if ((uint64_t)(long long)id < job.rel_n_words) {
-      atomicMin(job.rel_words + id, job.rel_tag + (unsigned)i);
+      if (local < rows && job.n_dev)  // the distinct ids of the hop before
+        atomicMin(job.rel_words + id, job.rel_tag + (unsigned)i);
+      else
+        lower((unsigned)id, (unsigned)i, (unsigned)min(local, (int64_t)kLoweredLocal), crowd);
       return;
     }
     bool maybe_first;
@@ -707,13 +749,13 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
           store_int(job.out_eids, job.indptr64, o, x.at() + s_eshift[x.seed()]);
         }
       }
-      if (kFused) enter(i, v);
+      if (kFused) enter(i, v, e, e < lead + kHopThreads);
     }
     return;
   }
   if (kFused)
     for (int j = (int)tid; j < rows; j += kHopThreads)
-      enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j));
+      enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j), j, true);
 
   // k > 32, or weighted with replacement (G == 32): one warp per seed
   const uint32_t set_slots = job.set_slots;
@@ -734,7 +776,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
       const IxT val = __ldg(in + pos);
       out_all[o] = val;
       if (job.out_eids) store_int(job.out_eids, job.indptr64, o, s_begin[j] + pos + s_eshift[j]);
-      if (kFused) enter(n + o, val);
+      if (kFused) enter(n + o, val, rows + (o - prefix), false);
     };
     if (job.weights && deg > 0 && job.replace) {
       const float* w = (s_hit[j] ? job.gpu_weights : job.weights) + s_begin[j];
@@ -982,7 +1024,7 @@ static cudaError_t launch_hop_as(const HopJob& job, unsigned grid, size_t smem, 
     if (job.k <= 8) return launch_kernel(pdl, sample_hop_kernel<IxT, 8, MODE>, grid, kHopThreads, smem, s, job);
     if (job.k <= 16) return launch_kernel(pdl, sample_hop_kernel<IxT, 16, MODE>, grid, kHopThreads, smem, s, job);
   }
-  if (smem > (48 << 10)) {
+  if (smem > kPlainHopSmem) {
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !configured[dev]) {

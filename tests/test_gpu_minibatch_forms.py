@@ -3,6 +3,7 @@ the row count is known, hashed slots for every id where it is not or where a siz
 words.  All give the same result, bit for bit, and that of the oracle; so they do on graphs with popular neighbours, where many
 lanes lower one word."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -185,3 +186,29 @@ def test_a_sized_context_without_room_for_the_words_works_by_slots(capi):
         wu, (_, wx) = oracle.tensor_relabel([cur, sx.cpu().numpy()])
         assert np.array_equal(front.cpu().numpy(), wu) and np.array_equal(rel.cpu().numpy(), wx)
         cur = wu
+
+
+def test_popular_neighbours_are_no_slower_by_words_than_by_slots(capi, monkeypatch):
+    """A tenth of all edges leads to one node: its word must not be lowered once for every one of them.  By slots, which
+    leave a smaller index alone, a batch takes 440 us; with a reduction for every edge it took 628 by words, 308 without."""
+    n = 2_400_000
+    g = torch.Generator(device="cuda").manual_seed(1)
+    indptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    torch.cumsum(torch.randint(5, 36, (n,), generator=g, device="cuda"), 0, out=indptr[1:])
+    indices = torch.randint(0, n, (int(indptr[-1]),), generator=g, device="cuda")
+    indices[torch.rand(indices.numel(), generator=g, device="cuda") < 0.1] = 17
+    seeds = torch.randint(0, n, (8192,), generator=g, device="cuda")
+
+    def us(call, reps=10):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        for _ in range(reps):
+            call()
+        torch.cuda.synchronize()
+        return (time.perf_counter() - t) / reps * 1e6
+
+    words = lambda: capi.sample_minibatch(indptr, indices, seeds, [5, 10, 15])
+    slots = lambda: _by_slots(capi, monkeypatch, indptr, indices, seeds, [5, 10, 15])
+    us(words), us(slots)
+    best = [min(us(call) for _ in range(5)) for call in (words, slots)]
+    assert best[0] < best[1], best
