@@ -333,8 +333,8 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
  *
  * shmt_minibatch_start returns when everything is queued.  shmt_minibatch_hop waits until the sizes of a hop are
  * known (seeds in, edges sampled, distinct ids out), while the hops behind it may still run; asked for the last
- * hop it also reports an error of any of them, and the mini-batch is over.  No other call uses the context
- * in between.                                                                                */
+ * hop it also reports an error of any of them, and the mini-batch is over.  No other call that waits for a
+ * result or takes scratch uses the context in between: a mini-batch that has not been asked to its end is over with it. */
 int shmt_minibatch_start(shmt_ctx* ctx, const void* indptr, int indptr_dtype, int64_t n_nodes,
                          const void* indices, int indices_dtype, const float* weights,
                          const void* gpu_indptr, const void* gpu_indices, const float* gpu_weights,

@@ -25,7 +25,7 @@ from typing import List, Sequence, Tuple
 import torch
 
 from . import _lib
-from ._lib import I32, I64, check, lib
+from ._lib import ERR_INVALID, I32, I64, ShmtError, check, lib
 
 _INT_CODES = {torch.int32: I32, torch.int64: I64}
 _CODE_DTYPES = {I32: torch.int32, I64: torch.int64}
@@ -768,13 +768,22 @@ def sample_minibatch(indptr: torch.Tensor, indices: torch.Tensor, seeds: torch.T
     # the sizes of a hop arrive while those behind it run, and its views are made meanwhile
     sizes = (C.c_int64 * 3)()
     hops = []
-    for h, (p_at, e_at, x_at, r_at, f_at) in enumerate(where):
-        check(lib.shmt_minibatch_hop(ctx, h, sizes))
-        n_in, nnz, n_out = sizes
-        hop = (p_pool.as_strided((n_in + 1,), _ONE, p_at), i_pool.as_strided((nnz,), _ONE, x_at),
-               i_pool.as_strided((nnz,), _ONE, r_at + n_in),  # behind the seeds' new ids
-               i_pool.as_strided((n_out,), _ONE, f_at))
-        hops.append(hop + (p_pool.as_strided((nnz,), _ONE, e_at),) if return_eids else hop)
+    try:
+        for h, (p_at, e_at, x_at, r_at, f_at) in enumerate(where):
+            check(lib.shmt_minibatch_hop(ctx, h, sizes))
+            n_in, nnz, n_out = sizes
+            hop = (p_pool.as_strided((n_in + 1,), _ONE, p_at), i_pool.as_strided((nnz,), _ONE, x_at),
+                   i_pool.as_strided((nnz,), _ONE, r_at + n_in),  # behind the seeds' new ids
+                   i_pool.as_strided((n_out,), _ONE, f_at))
+            hops.append(hop + (p_pool.as_strided((nnz,), _ONE, e_at),) if return_eids else hop)
+    except ShmtError:
+        raise
+    except BaseException:
+        # The mini-batch ends here as well, and if it failed that is the reason: sizes of a hop come before its status.
+        rc = lib.shmt_minibatch_hop(ctx, n_hops - 1, sizes)
+        if rc != ERR_INVALID:  # it had not ended yet
+            check(rc)
+        raise
     return hops[-1][3], hops
 
 

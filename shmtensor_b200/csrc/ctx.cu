@@ -38,7 +38,23 @@ int device_of_pointer(const void* p) {
   return cur;
 }
 
+// A mini-batch that nobody has waited for is over with the next call.  Its sizes are of no use any more, but if it failed
+// it has left entries behind.
+static int ctx_drop_batch(shmt_ctx* ctx) {
+  const int n_hops = ctx->batch.n_hops;
+  if (n_hops == 0) return SHMT_OK;
+  ctx->batch.n_hops = 0;
+  ctx->tail_pending = false;
+  const cudaError_t e = cudaEventSynchronize(ctx->tail_event);
+  const HostPost& post = ctx->batch.post;
+  const bool known = e == cudaSuccess && post.host && ctx->h_words[post.flag_at] == post.seq;
+  if (!known || ctx->h_words[n_hops * 8] != DEV_OK) ctx_table_failed(ctx);
+  SHMT_CUDA_TRY(e);
+  return SHMT_OK;
+}
+
 HostPost ctx_begin_post(shmt_ctx* ctx, const int64_t* dev_words, int n_words, int64_t* done_word) {
+  ctx_drop_batch(ctx);  // before its status is written over; a call with scratch has reported what this returns
   HostPost p{};
   p.words = dev_words;
   p.n_words = n_words;
@@ -124,12 +140,12 @@ int ctx_mark_tail(shmt_ctx* ctx, cudaStream_t stream) {
 }
 
 int ctx_join_tail(shmt_ctx* ctx, cudaStream_t stream) {
+  if (int rc = ctx_drop_batch(ctx)) return rc;
   if (!ctx->tail_pending) return SHMT_OK;
-  // In the tail's own stream everything is queued behind it.  A mini-batch that nobody has waited for could
-  // still write to the host words, though.
+  // In the tail's own stream everything is queued behind it.
   unsigned long long id = 0;
   SHMT_CUDA_TRY(cudaStreamGetId(stream, &id));
-  if (id == ctx->tail_stream && ctx->batch.n_hops == 0) return SHMT_OK;
+  if (id == ctx->tail_stream) return SHMT_OK;
   ctx->tail_pending = false;
   SHMT_CUDA_TRY(cudaEventSynchronize(ctx->tail_event));
   return SHMT_OK;

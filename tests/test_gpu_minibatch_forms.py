@@ -212,3 +212,36 @@ def test_popular_neighbours_are_no_slower_by_words_than_by_slots(capi, monkeypat
     us(words), us(slots)
     best = [min(us(call) for _ in range(5)) for call in (words, slots)]
     assert best[0] < best[1], best
+
+
+def test_a_minibatch_that_is_interrupted_is_over(capi, monkeypatch):
+    """An exception between the hops leaves no mini-batch behind on the context, and the next one is right."""
+    from shmtensor_b200 import _lib
+    rng = np.random.default_rng(2)
+    indptr_n, indices_n = _graph(rng, 3000, 9, "even", np.int64)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    seeds = torch.arange(200, device="cuda")
+    capi.set_sampling_seed(5)
+    want = capi.sample_minibatch(indptr, indices, seeds, [4, 4, 4])
+
+    class Interrupted:
+        def __init__(self, lib, at):
+            self.lib, self.at = lib, at
+
+        def __getattr__(self, name):
+            return getattr(self.lib, name)
+
+        def shmt_minibatch_hop(self, ctx, hop, sizes):
+            if hop == self.at:
+                self.at = None
+                raise KeyboardInterrupt
+            return self.lib.shmt_minibatch_hop(ctx, hop, sizes)
+
+    for at in (0, 1):
+        with monkeypatch.context() as m:
+            m.setattr(capi, "lib", Interrupted(capi.lib, at))
+            with pytest.raises(KeyboardInterrupt):
+                capi.sample_minibatch(indptr, indices, seeds, [4, 4, 4])
+        assert capi.lib.shmt_minibatch_hop(capi._ctx(seeds.device), 2, (C.c_int64 * 3)()) == _lib.ERR_INVALID
+        capi.set_sampling_seed(5)
+        _same(want, capi.sample_minibatch(indptr, indices, seeds, [4, 4, 4]))

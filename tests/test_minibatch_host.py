@@ -55,3 +55,32 @@ def test_a_minibatch_moves_no_memory_that_a_sized_context_holds(lib, ctx, n_node
         assert _start(lib, ctx, n_nodes) == _lib.OK
         assert _relabel(lib, ctx) == _lib.OK
     assert lib.fake_frees() == 0
+
+
+TIMEOUT = 2
+
+
+@pytest.mark.parametrize("status,fails", [(0, False), (TIMEOUT, True), (1, True), (None, True)])
+@pytest.mark.parametrize("between", [(), (1000,)])
+def test_a_minibatch_that_nobody_waits_for_leaves_no_entries(lib, ctx, status, fails, between):
+    """A mini-batch that failed may have left entries in the table.  If nobody asks for its sizes the next call that uses
+    the table empties it: the status is read when the mini-batch is given up, before a small call's (`between`) results come
+    over it, and a mini-batch that never handed it over counts as failed."""
+    assert lib.shmt_ctx_reserve(ctx, 1 << 20, N_IDS, None) == _lib.OK
+    assert _start(lib, ctx, 2_000_000) == _lib.OK
+    if status is not None:
+        words = lib.fake_host_words()
+        words[1], words[3], words[8], words[127] = 500, 600, status, 1  # edges, distinct ids, status, the first post
+    lib.fake_reset()
+    for n in between:
+        found = C.c_int64()
+        ids, unique, local = (_buffer(8 * n) for _ in range(3))
+        assert lib.shmt_relabel(ctx, (C.c_void_p * 1)(C.addressof(ids)), (C.c_int64 * 1)(n), 1, _lib.I64, C.addressof(unique),
+                                C.addressof(local), C.byref(found), None) == _lib.OK
+    assert _relabel(lib, ctx) == _lib.OK
+    assert (lib.fake_largest_fill(0xFF) >= 16 * N_IDS) == fails
+    sizes = (C.c_int64 * 3)()
+    assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.ERR_INVALID  # it is over
+    lib.fake_reset()
+    assert _start(lib, ctx, 2_000_000) == _lib.OK
+    assert (lib.fake_largest_fill(0xFF) >= 4 * 2_000_000) == fails    # and its words too
