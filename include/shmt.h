@@ -331,7 +331,7 @@ int shmt_sample_minibatch_eids(shmt_ctx* ctx, const void* indptr, int indptr_dty
  * at layout[4 * n_hops + h].  Same results.  A context whose table was sized by shmt_ctx_reserve_minibatch
  * does not grow for the words.
  *
- * shmt_minibatch_start returns when everything is queued.  shmt_minibatch_hop waits until the sizes of a hop are
+ * shmt_minibatch_start returns when everything is queued; a stream that is being captured is refused.  shmt_minibatch_hop waits until the sizes of a hop are
  * known (seeds in, edges sampled, distinct ids out), while the hops behind it may still run; asked for the last
  * hop it also reports an error of any of them, and the mini-batch is over.  No other call that waits for a
  * result or takes scratch uses the context in between: a mini-batch that has not been asked to its end is over with it. */

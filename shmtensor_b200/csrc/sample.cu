@@ -1305,6 +1305,10 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
   const int* spt = plan.spt;
   const size_t *off_hop = plan.off_hop, *off_rel = plan.off_rel;
   const size_t cursor = plan.scratch_bytes;
+  // Every batch has tags of its own, which a replay would use again; and nobody can wait for the sizes.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SHMT_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+  SHMT_REQUIRE(capture == cudaStreamCaptureStatusNone, "shmt_sample_minibatch: the stream is being captured");
   if (int rc = ctx_reserve(ctx, cursor, s)) return rc;
   char* base = ctx->region();
   int64_t* words = reinterpret_cast<int64_t*>(base);

@@ -245,3 +245,29 @@ def test_a_minibatch_that_is_interrupted_is_over(capi, monkeypatch):
         assert capi.lib.shmt_minibatch_hop(capi._ctx(seeds.device), 2, (C.c_int64 * 3)()) == _lib.ERR_INVALID
         capi.set_sampling_seed(5)
         _same(want, capi.sample_minibatch(indptr, indices, seeds, [4, 4, 4]))
+
+
+def test_a_minibatch_is_refused_by_a_stream_that_is_being_captured(capi):
+    """With the capture as it was: what else is captured replays, and the context's next mini-batch is right."""
+    rng = np.random.default_rng(2)
+    indptr_n, indices_n = _graph(rng, 3000, 9, "even", np.int64)
+    indptr, indices = torch.from_numpy(indptr_n).cuda(), torch.from_numpy(indices_n).cuda()
+    seeds, x = torch.arange(200, device="cuda"), torch.zeros(8, device="cuda")
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        capi.set_sampling_seed(5)
+        want = capi.sample_minibatch(indptr, indices, seeds, [4, 4])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        x += 1
+        with pytest.raises(RuntimeError, match="being captured"):
+            capi.sample_minibatch(indptr, indices, seeds, [4, 4])
+    graph.replay()
+    graph.replay()
+    assert (x == 2).all()
+    with torch.cuda.stream(stream):
+        capi.set_sampling_seed(5)
+        _same(want, capi.sample_minibatch(indptr, indices, seeds, [4, 4]))
+    torch.cuda.synchronize()

@@ -84,3 +84,17 @@ def test_a_minibatch_that_nobody_waits_for_leaves_no_entries(lib, ctx, status, f
     lib.fake_reset()
     assert _start(lib, ctx, 2_000_000) == _lib.OK
     assert (lib.fake_largest_fill(0xFF) >= 4 * 2_000_000) == fails    # and its words too
+
+
+def test_a_minibatch_is_not_captured(lib, ctx):
+    """Its words hold numbers that only this call has: a replay would find its own of the time before.  Refused before
+    anything is queued, and the context works on."""
+    assert _start(lib, ctx, 1000) == _lib.OK
+    lib.fake_reset()
+    for n_nodes in (0, 1000):
+        lib.fake_capture(1)
+        assert _start(lib, ctx, n_nodes) == _lib.ERR_INVALID
+        assert b"being captured" in lib.shmt_last_error()
+        assert lib.fake_launches() == 0 and lib.fake_largest_fill(0) == 0
+        lib.fake_capture(0)
+    assert _start(lib, ctx, 1000) == _lib.OK and lib.fake_launches() > 0
