@@ -668,27 +668,35 @@ static int launch_lsu(const RowJob& job, cudaStream_t s) {
 constexpr int kBulkStages = 2;
 constexpr int64_t kBulkStageBytes = 2048;
 // A fetch looks a tile's rows up in one go and waits for it, so few rows a tile means few lookups on their way.
-// Rows of 512 bytes and more therefore come 6 a
-// buffer, as long as these fit.  Popular ids, 0.6 GB fetched: 512 bytes 179 -> 155 us, 640 180 -> 150, 800 196 -> 163, 1,024
-// 159 -> 147, 1,200 238 -> 165, 1,600 184 -> 160, 2,048 150 -> 143, 2,800 166 -> 146; 60,000 rows of 800 bytes 18.3 -> 14.7.
-// Ids drawn evenly from 1.6 GB of rows: 1,024 bytes 225 -> 219 us, 1,200 253 -> 224, 2,048 223 -> 213, but 512 229 -> 238
-// and 576 to 900 bytes 7 to 9 % behind (more scattered reads between the writes than HBM likes), which no cache is
-// filled for.  Sets have their own line: 512 bytes 124 us with 4 rows and 129 with 6, 800 bytes 189 with 2 and 208.
+// Rows of 512 bytes and more therefore come 6 a buffer, as long as these fit.  60,000 rows by popularity / drawn evenly
+// from 1.6 GB: 512 bytes 14.4 -> 11.9 us / 18.1 -> 14.9, 800 20.7 -> 16.9 / 24.6 -> 22.4, 1,200 34 -> 20.4 / 37.0 -> 29.8.
+// An output much smaller than the L2 cache stays there.  A larger one is written to HBM while rows are read, and rows drawn
+// evenly come from HBM too: then six rows of 512 to 930 bytes are slower (512 bytes, six and four rows: 90 MB 38.1 us and 38.8, 120 MB
+// 50.4 and 48.6, 600 MB 236 and 224; 640: 37.1 and 38.3, 48.5 and 47.5, 234 and 212; 896: 35.2 and 37.3, 47.4 and 47.2, 227
+// and 208; from 960 on: 230 and 233, 1,008 233 and 240, 1,200 222 and 255), and so are six of 1,550 to 1,730 (1,664: 210, one row 203,
+// five 196).  By popularity six are faster (512: 600 MB 137 and 167; 1,664: 142, five 148), but whether a call's rows
+// repeat is not known here, and a frontier's are distinct.
+// Sets have their own line: 512 bytes 124 us with 4 rows and 129 with 6, 800 bytes 189 with 2 and 208.
 constexpr int64_t kWideRowBytes = 512, kWideStageBytes = 12800;
 constexpr int kWideRows = 6;
+constexpr int64_t kLargeOutBytes = (int64_t)88 << 20, kLargeOutWideRowBytes = 960, kLargeOutFewRowBytes[2] = {1536, 1760};
+constexpr int kLargeOutFewRows = 5;
 constexpr size_t kBulkSmemMax = 200 * 1024;
 
 // Rows per ring buffer, 0 if the rows are not 16-byte units or do not fit.
-static int bulk_rows_per_stage(int64_t row_bytes, int vec, int R_small, bool set) {
+static int bulk_rows_per_stage(int64_t n, int64_t row_bytes, int vec, int R_small, bool set) {
   if (vec != 16) return 0;
   static const int forced = [] {
     const char* e = getenv("SHMT_BULK_ROWS");
     return e ? atoi(e) : 0;
   }();
   int64_t r = forced > 0 ? forced : kBulkStageBytes / row_bytes;
-  if (forced <= 0 && !set && row_bytes >= kWideRowBytes) {
+  const bool large = n > kLargeOutBytes / row_bytes;
+  if (forced <= 0 && !set && row_bytes >= (large ? kLargeOutWideRowBytes : kWideRowBytes)) {
+    const bool few = large && row_bytes > kLargeOutFewRowBytes[0] && row_bytes < kLargeOutFewRowBytes[1];
+    const int most = few ? kLargeOutFewRows : kWideRows;
     r = kWideStageBytes / row_bytes;
-    if (r > kWideRows) r = kWideRows;
+    if (r > most) r = most;
   }
   if (r < 1) r = 1;
   if (r > 32) r = 32;
@@ -777,7 +785,7 @@ template <bool SET>
 static int launch_row_copy(const RowJob& job, int vec, cudaStream_t s) {
   {
     static const bool no_bulk = getenv("SHMT_NO_BULK") != nullptr;
-    const int R = no_bulk ? 0 : bulk_rows_per_stage(job.row_bytes, vec, job.rows_per_tile, SET);
+    const int R = no_bulk ? 0 : bulk_rows_per_stage(job.n, job.row_bytes, vec, job.rows_per_tile, SET);
     if (R >= 1) return launch_bulk<SET>(job, R, s);
     const int ragged = SET || no_bulk ? 0 : ragged_rows_per_stage(job, vec);
     if (ragged >= 1) return launch_ragged(job, ragged, s);

@@ -401,3 +401,16 @@ def test_rows_of_512_bytes_and_more_several_a_buffer(capi, row_bytes):
         assert torch.equal(out[1:n + 1], torch.where(hit[:, None], got, torch.full_like(got, 7)))
         assert (out[0] == 7).all() and (out[n + 1] == 7).all()
     assert capi.device_fault() == 0
+
+
+@pytest.mark.parametrize("row_bytes", [512, 944, 960, 1536, 1552, 1744, 1760])
+def test_rows_a_buffer_on_both_sides_of_an_output_that_leaves_the_l2_cache(capi, row_bytes):
+    """Outputs of up to 88 MiB and larger ones take different numbers of rows a ring buffer, at most widths."""
+    g = torch.Generator(device="cuda").manual_seed(row_bytes)
+    rows, line = 40_000, (88 << 20) // row_bytes
+    table = torch.randint(0, 256, (rows, row_bytes), generator=g, device="cuda", dtype=torch.uint8)
+    m = capi.CUCOStaticHashmap(torch.arange(rows, device="cuda"), torch.arange(rows, dtype=torch.int32, device="cuda"), 0.5)
+    for n in (line, line + 1):
+        ids = torch.randint(0, rows, (n,), generator=g, device="cuda")
+        assert torch.equal(capi.cache_fetch(None, table, ids, m), table[ids])
+    assert capi.device_fault() == 0
