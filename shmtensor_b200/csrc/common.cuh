@@ -16,6 +16,7 @@ void set_error(const char* fmt, ...);
   do {                                                                         \
     cudaError_t e__ = (call);                                                  \
     if (e__ != cudaSuccess) {                                                  \
+      cudaGetLastError(); /* reported here, so not by the caller's next check */ \
       ::shmt::set_error("%s:%d CUDA call `%s` failed: %s (%d)", __FILE__,      \
                         __LINE__, #call, cudaGetErrorString(e__), (int)e__);   \
       return SHMT_ERR_CUDA;                                                    \

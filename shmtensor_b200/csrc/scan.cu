@@ -483,11 +483,13 @@ static int64_t scan_tiles(int64_t n, int vecs = kScanVecs) {
 }
 
 template <typename T, int VECS = kScanVecs>
-static void run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_t* ticket, int64_t* status,
-                     cudaStream_t s, int64_t* clean = nullptr, const TileDesc* carry = nullptr) {
+static int run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_t* ticket, int64_t* status,
+                    cudaStream_t s, int64_t* clean = nullptr, const TileDesc* carry = nullptr) {
   const int vec_ok = ((uintptr_t)data & 15) == 0;
-  launch_kernel(true, scan_kernel<T, VECS>, (unsigned)scan_tiles<T>(n, VECS), kScanThreads, 0, s,
-                static_cast<T*>(data), n, exclusive, vec_ok, st, ticket, status, clean, carry, LaunchPad<32>{});
+  SHMT_CUDA_TRY(launch_kernel(true, scan_kernel<T, VECS>, (unsigned)scan_tiles<T>(n, VECS), kScanThreads, 0, s,
+                              static_cast<T*>(data), n, exclusive, vec_ok, st, ticket, status, clean, carry,
+                              LaunchPad<32>{}));
+  return SHMT_OK;
 }
 
 // Scans of up to kSmallScanTiles 64 KB tiles: look-back state that every launch leaves at zero, and the
@@ -495,17 +497,15 @@ static void run_scan(void* data, int64_t n, int exclusive, TileStates st, int64_
 // stored by many SMs.  In a row of calls (with a memset and 64 KB tiles -> so): 1,000 int32 6.2 -> 2.5 us, 100,000
 // 8.1 -> 4.1, 1,000,000 8.2 -> 6.1; 2,400,001 int64 11.8 -> 10.6.
 template <typename T>
-static void run_scan_small(shmt_ctx* ctx, void* data, int64_t n, int exclusive, cudaStream_t s) {
+static int run_scan_small(shmt_ctx* ctx, void* data, int64_t n, int exclusive, cudaStream_t s) {
   int64_t* words = ctx->scan_words();
   const TileStates st = carve_tile_states(reinterpret_cast<char*>(words + 2), kSmallScanTiles);
   int64_t* status = ctx->d_words() + W_STATUS;
   const int64_t resident = 2 * (int64_t)sm_count();
   if (scan_tiles<T>(n, 2) <= resident)
-    run_scan<T, 2>(data, n, exclusive, st, words, status, s, words + 1);
-  else if (scan_tiles<T>(n, 4) <= resident)
-    run_scan<T, 4>(data, n, exclusive, st, words, status, s, words + 1);
-  else
-    run_scan<T, 8>(data, n, exclusive, st, words, status, s, words + 1);
+    return run_scan<T, 2>(data, n, exclusive, st, words, status, s, words + 1);
+  if (scan_tiles<T>(n, 4) <= resident) return run_scan<T, 4>(data, n, exclusive, st, words, status, s, words + 1);
+  return run_scan<T, 8>(data, n, exclusive, st, words, status, s, words + 1);
 }
 
 // Large, 16-byte aligned inputs: whole 256 KB super-tiles by the persistent cluster kernel, what
@@ -520,8 +520,8 @@ static int run_scan_large(void* data, int64_t n, int exclusive, char* state_base
   const int64_t rest = n - n_super * per_super;
   if (rest > 0) {
     TileStates tail = carve_tile_states(state_base + tile_state_bytes(n_super), scan_tiles<T>(rest));
-    run_scan<T>(static_cast<T*>(data) + n_super * per_super, rest, exclusive, tail, words + W_TICKET,
-                words + W_STATUS, s, nullptr, st.d + (n_super - 1));
+    return run_scan<T>(static_cast<T*>(data) + n_super * per_super, rest, exclusive, tail, words + W_TICKET,
+                       words + W_STATUS, s, nullptr, st.d + (n_super - 1));
   }
   return SHMT_OK;
 }
@@ -547,10 +547,8 @@ int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
   const bool clusters =
       !no_clusters && ((uintptr_t)data & 15) == 0 && n * int_itemsize(dtype) >= kScanClusterMinBytes;
   if (!clusters && (dtype == SHMT_I64 ? scan_tiles<long long>(n) : scan_tiles<int>(n)) <= kSmallScanTiles) {
-    dtype == SHMT_I64 ? run_scan_small<long long>(ctx, data, n, exclusive, stream)
-                      : run_scan_small<int>(ctx, data, n, exclusive, stream);
-    SHMT_CUDA_TRY(cudaGetLastError());
-    return SHMT_OK;
+    return dtype == SHMT_I64 ? run_scan_small<long long>(ctx, data, n, exclusive, stream)
+                             : run_scan_small<int>(ctx, data, n, exclusive, stream);
   }
   if (int rc = ctx_reserve(ctx, scratch_off + scan_scratch_bytes(n), stream)) return rc;
   TileStates st = carve_tile_states(ctx->region() + scratch_off, n_tiles);
@@ -562,19 +560,15 @@ int launch_scan(shmt_ctx* ctx, void* data, int dtype, int64_t n, int exclusive,
     SHMT_CUDA_TRY(cudaMemsetAsync(ctx->d_words(), 0, 256, stream));
     SHMT_CUDA_TRY(cudaMemsetAsync(st.d, 0, tile_state_bytes(n_tiles), stream));
   }
+  int64_t* w = ctx->d_words();
   if (clusters) {
     // the ticketed kernel's descriptor block is larger than what both kernels need here
     char* base = reinterpret_cast<char*>(st.d);
-    if (int rc = dtype == SHMT_I64 ? run_scan_large<long long>(data, n, exclusive, base, ctx->d_words(), stream)
-                                   : run_scan_large<int>(data, n, exclusive, base, ctx->d_words(), stream))
-      return rc;
-  } else if (dtype == SHMT_I64) {
-    run_scan<long long>(data, n, exclusive, st, ctx->d_words() + W_TICKET, ctx->d_words() + W_STATUS, stream);
-  } else {
-    run_scan<int>(data, n, exclusive, st, ctx->d_words() + W_TICKET, ctx->d_words() + W_STATUS, stream);
+    return dtype == SHMT_I64 ? run_scan_large<long long>(data, n, exclusive, base, w, stream)
+                             : run_scan_large<int>(data, n, exclusive, base, w, stream);
   }
-  SHMT_CUDA_TRY(cudaGetLastError());
-  return SHMT_OK;
+  return dtype == SHMT_I64 ? run_scan<long long>(data, n, exclusive, st, w + W_TICKET, w + W_STATUS, stream)
+                           : run_scan<int>(data, n, exclusive, st, w + W_TICKET, w + W_STATUS, stream);
 }
 
 size_t scan_scratch_bytes(int64_t n) {
@@ -630,12 +624,8 @@ extern "C" int shmt_scan_static(void* data, int dtype, int64_t n, int exclusive,
   // the array still holds the previous call's ticket, status and tile descriptors: zero the
   // words and the descriptors this call will use (they sit right behind the 256-byte header)
   SHMT_CUDA_TRY(cudaMemsetAsync(base, 0, 256 + tile_state_bytes(n_tiles), s));
-  if (dtype == SHMT_I64)
-    run_scan<long long>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s);
-  else
-    run_scan<int>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s);
-  SHMT_CUDA_TRY(cudaGetLastError());
-  return SHMT_OK;
+  return dtype == SHMT_I64 ? run_scan<long long>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s)
+                           : run_scan<int>(data, n, exclusive, st, words + W_TICKET, words + W_STATUS, s);
 }
 
 // What the last shmt_scan_static call on the current device left in its status word.  The word

@@ -20,7 +20,8 @@ std::map<void*, size_t> blocks;
 std::vector<Fill> fills;
 void* host_words;
 long launches, frees;
-int capturing;
+int capturing, failing;
+cudaError_t last_error = cudaSuccess;
 }  // namespace
 
 extern "C" {
@@ -28,13 +29,20 @@ void fake_reset() { fills.clear(); launches = frees = 0; }
 long fake_launches() { return launches; }
 long fake_frees() { return frees; }
 void fake_capture(int on) { capturing = on; }
+void fake_fail_launches(int on) { failing = on; }
+int fake_last_error() { return last_error; }
 void* fake_host_words() { return host_words; }
-// bytes of a device block that were filled with `value` since the reset: its largest fill
+// fills with `value` since the reset: the largest, and how many of at least so many bytes
 long fake_largest_fill(int value) {
   long most = 0;
   for (auto& f : fills)
     if (f.value == value && f.bytes > most) most = f.bytes;
   return most;
+}
+long fake_fills(int value, long least) {
+  long n = 0;
+  for (auto& f : fills) n += f.value == value && f.bytes >= least;
+  return n;
 }
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
@@ -42,7 +50,11 @@ cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = last_error;
+  last_error = cudaSuccess;
+  return e;
+}
 cudaError_t cudaMalloc(void** p, size_t n) { *p = aligned_alloc(256, (n + 255) / 256 * 256); blocks[*p] = n; return cudaSuccess; }
 cudaError_t cudaFree(void* p) { ++frees; blocks.erase(p); free(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { host_words = *p = calloc(1, n); return cudaSuccess; }
@@ -78,7 +90,11 @@ cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return c
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 1; return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) { *n = 1; return cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { ++launches; return cudaSuccess; }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { ++launches; return cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) {
+  ++launches;
+  if (failing) last_error = cudaErrorLaunchOutOfResources;
+  return failing ? cudaErrorLaunchOutOfResources : cudaSuccess;
+}
 cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t*, void*) { return cudaErrorNotSupported; }
 cudaError_t cudaIpcOpenMemHandle(void**, cudaIpcMemHandle_t, unsigned) { return cudaErrorNotSupported; }
 cudaError_t cudaIpcCloseMemHandle(void*) { return cudaErrorNotSupported; }
@@ -114,7 +130,8 @@ def load(tmp_path):
         fn.restype, fn.argtypes = res, args
     for name, res, args in (("fake_launches", C.c_long, []), ("fake_frees", C.c_long, []), ("fake_reset", None, []),
                             ("fake_capture", None, [C.c_int]), ("fake_host_words", C.POINTER(C.c_int64), []),
-                            ("fake_largest_fill", C.c_long, [C.c_int])):
+                            ("fake_fail_launches", None, [C.c_int]), ("fake_last_error", C.c_int, []), ("fake_largest_fill", C.c_long, [C.c_int]),
+                            ("fake_fills", C.c_long, [C.c_int, C.c_long])):
         fn = getattr(out, name)
         fn.restype, fn.argtypes = res, args
     return out

@@ -30,7 +30,7 @@ def _buffer(nbytes):
 
 def _start(lib, ctx, n_nodes, n_seeds=100, k=5):
     edges = n_seeds * k
-    pools = _buffer(8 * (n_seeds + 1)), _buffer(8 * (3 * edges + 2 * n_seeds + 16)), _buffer(8 * n_seeds)
+    pools = _buffer(64), _buffer(64), _buffer(64)  # nothing runs, so nothing is read or written
     layout = (C.c_int64 * 5)(0, 0, 0, edges, 2 * edges + n_seeds)
     some = C.addressof(pools[2])
     return lib.shmt_minibatch_start(ctx, some, _lib.I64, n_nodes, some, _lib.I64, None, None, None, None, None, None, some,
@@ -55,6 +55,20 @@ def test_a_minibatch_moves_no_memory_that_a_sized_context_holds(lib, ctx, n_node
         assert _start(lib, ctx, n_nodes) == _lib.OK
         assert _relabel(lib, ctx) == _lib.OK
     assert lib.fake_frees() == 0
+
+
+def test_words_start_over_when_all_numbers_are_used(lib, ctx):
+    """A hop takes as many numbers as it can have ids, here 2,020,000 of 2^32 - 1: 2,126 batches go by between two fills of
+    the words, in the first lap and in the next."""
+    lib.fake_reset()
+    words, sizes = lib.fake_host_words(), (C.c_int64 * 3)()
+    for batch in range(1, 2 * 2126 + 2):
+        assert _start(lib, ctx, 1_000_000, 20_000, 100) == _lib.OK
+        words[8], words[127] = 0, batch  # handed over, without an error
+        assert lib.shmt_minibatch_hop(ctx, 0, sizes) == _lib.OK
+        if batch % 2126 <= 1:
+            table = lib.fake_fills(0xFF, 16_000_000)
+            assert table == 1 and lib.fake_fills(0xFF, 4_000_000) - table == 1 + (batch - 1) // 2126
 
 
 TIMEOUT = 2
@@ -98,3 +112,38 @@ def test_a_minibatch_is_not_captured(lib, ctx):
         assert lib.fake_launches() == 0 and lib.fake_largest_fill(0) == 0
         lib.fake_capture(0)
     assert _start(lib, ctx, 1000) == _lib.OK and lib.fake_launches() > 0
+
+
+@pytest.mark.parametrize("n", [1000, 1_000_000, 9_000_000, 40_000_000])
+def test_a_scan_whose_launch_fails_says_so_once(lib, ctx, n):
+    """Scans of one tile, of a grid, and of clusters with a rest: the call reports the failure, and the caller's own next
+    check of the runtime's last error does not find it again."""
+    data = _buffer(8 * n)
+    at = (C.addressof(data) + 15) & ~15
+    assert lib.shmt_scan(ctx, at, _lib.I64, n, 0, None) == _lib.OK
+    lib.fake_fail_launches(1)
+    try:
+        for where, m in ((at, n), (at + 8, n - 1)):
+            assert lib.shmt_scan(ctx, where, _lib.I64, m, 0, None) == _lib.ERR_CUDA
+            assert lib.fake_last_error() == 0
+    finally:
+        lib.fake_fail_launches(0)
+    assert lib.shmt_scan(ctx, at, _lib.I64, n, 0, None) == _lib.OK
+
+
+def test_lookups_fetches_and_relabels_report_a_failed_launch_once(lib, ctx):
+    """The same of the other calls that are scheduled while the kernel before them runs."""
+    ids, out, table = _buffer(8 * 64), _buffer(64 * 512), _buffer(64 * 512)
+    at = [(C.addressof(b) + 15) & ~15 for b in (ids, out, table)]
+    hmap = C.c_void_p()
+    assert lib.shmt_map_create(0, 128, 64, _lib.I64, _lib.I32, None, None, C.byref(hmap)) == _lib.OK
+    lib.fake_fail_launches(1)
+    try:
+        assert lib.shmt_map_query(hmap, at[0], _lib.I64, 64, at[1], None) == _lib.ERR_CUDA and lib.fake_last_error() == 0
+        for row in (512, 602, 4):  # a ring of rows, of odd ones, and plain copies
+            assert lib.shmt_fetch(hmap, None, 0, None, at[2], at[0], _lib.I64, 32, row, at[1], None) == _lib.ERR_CUDA
+            assert lib.fake_last_error() == 0
+        assert _relabel(lib, ctx, 100) == _lib.ERR_CUDA and lib.fake_last_error() == 0
+    finally:
+        lib.fake_fail_launches(0)
+        lib.shmt_map_destroy(hmap)
