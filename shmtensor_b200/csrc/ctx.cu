@@ -170,7 +170,6 @@ int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
 }
 
 int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
-  if (int rc = ctx_join_tail(ctx, stream)) return rc;
   if (bytes > ctx->table_bytes) {
     if (ctx->table) SHMT_CUDA_TRY(cudaFree(ctx->table));
     ctx->table = nullptr;
@@ -199,7 +198,6 @@ static int empty_words(shmt_ctx* ctx, cudaStream_t stream) {
 }
 
 int ctx_reserve_words(shmt_ctx* ctx, size_t bytes, cudaStream_t stream) {
-  if (int rc = ctx_join_tail(ctx, stream)) return rc;
   if (bytes > ctx->words_bytes) {
     if (ctx->words) SHMT_CUDA_TRY(cudaFree(ctx->words));
     ctx->words = nullptr;

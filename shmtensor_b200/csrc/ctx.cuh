@@ -73,7 +73,8 @@ enum : int { W_STATUS = 0, W_RESULT = 1, W_TICKET = 2, W_DONE = 3 };
 // Make sure ctx->region() holds at least `bytes` (256-byte aligned base).
 int ctx_reserve(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
 
-// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with).
+// Make sure ctx->table holds at least `bytes`, empty (all ones to begin with).  This and the next one are for callers that
+// have been through ctx_reserve, which waits for the context's use in another stream.
 int ctx_reserve_table(shmt_ctx* ctx, size_t bytes, cudaStream_t stream);
 
 // Make sure ctx->words holds at least `bytes`, every word of them above words_tag - 1.

@@ -1125,11 +1125,11 @@ int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64
     return rc;
   RelTable t;
   if (int rc = relabel_table(ctx, plan.cap[n_hops], &t, static_cast<cudaStream_t>(stream))) return rc;
-  // where the node count is not known: room for the words of a small graph, as much as a table takes beyond its slots
+  // and words, at least of as many nodes as fit in what a table takes beyond its slots: another graph may come
   const size_t slots = t.cap * sizeof(RelSlot), least = (size_t)4 << 20;
   size_t words = slots + slots / 2 < least ? least - slots : slots / 2;
   if (words > kRelMaxWords * sizeof(unsigned)) words = kRelMaxWords * sizeof(unsigned);
-  if (n_nodes > 0) words = n_nodes <= kRelMaxWords ? n_nodes * sizeof(unsigned) : 0;
+  if (n_nodes <= kRelMaxWords && words < n_nodes * sizeof(unsigned)) words = n_nodes * sizeof(unsigned);
   if (int rc = ctx_reserve_words(ctx, words, static_cast<cudaStream_t>(stream))) return rc;
   ctx->words_reserved = true;
   return SHMT_OK;

@@ -22,6 +22,7 @@ void* host_words;
 long launches, frees;
 int capturing, failing;
 cudaError_t last_error = cudaSuccess;
+const void* last_kernel;
 }  // namespace
 
 extern "C" {
@@ -31,6 +32,7 @@ long fake_frees() { return frees; }
 void fake_capture(int on) { capturing = on; }
 void fake_fail_launches(int on) { failing = on; }
 int fake_last_error() { return last_error; }
+const void* fake_last_kernel() { return last_kernel; }
 void* fake_host_words() { return host_words; }
 // fills with `value` since the reset: the largest, and how many of at least so many bytes
 long fake_largest_fill(int value) {
@@ -90,8 +92,9 @@ cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return c
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) { *n = 1; return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) { *n = 1; return cudaSuccess; }
 cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { ++launches; return cudaSuccess; }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* kernel, void**) {
   ++launches;
+  last_kernel = kernel;
   if (failing) last_error = cudaErrorLaunchOutOfResources;
   return failing ? cudaErrorLaunchOutOfResources : cudaSuccess;
 }
@@ -130,7 +133,8 @@ def load(tmp_path):
         fn.restype, fn.argtypes = res, args
     for name, res, args in (("fake_launches", C.c_long, []), ("fake_frees", C.c_long, []), ("fake_reset", None, []),
                             ("fake_capture", None, [C.c_int]), ("fake_host_words", C.POINTER(C.c_int64), []),
-                            ("fake_fail_launches", None, [C.c_int]), ("fake_last_error", C.c_int, []), ("fake_largest_fill", C.c_long, [C.c_int]),
+                            ("fake_fail_launches", None, [C.c_int]), ("fake_last_error", C.c_int, []),
+                            ("fake_last_kernel", C.c_void_p, []), ("fake_largest_fill", C.c_long, [C.c_int]),
                             ("fake_fills", C.c_long, [C.c_int, C.c_long])):
         fn = getattr(out, name)
         fn.restype, fn.argtypes = res, args

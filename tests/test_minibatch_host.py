@@ -57,6 +57,21 @@ def test_a_minibatch_moves_no_memory_that_a_sized_context_holds(lib, ctx, n_node
     assert lib.fake_frees() == 0
 
 
+@pytest.mark.parametrize("reserved_for,sampled,slots", [(0, 900_000, False), (1000, 900_000, False), (1000, 3_000_000, True),
+                                                        (3_000_000, 3_000_000, False), (1 << 26, 900_000, False)])
+def test_a_context_sized_for_one_graph_has_words_for_another_that_is_not_much_larger(lib, ctx, reserved_for, sampled, slots):
+    """At least as many as fit in what a small table's block is short of 4 MB."""
+    fan = (C.c_int64 * 1)(5)
+    assert lib.shmt_ctx_reserve_minibatch_nodes(ctx, 100, fan, 1, reserved_for, None) == _lib.OK
+    held = lib.shmt_ctx_scratch_bytes(ctx)
+    lib.fake_reset()
+    assert _start(lib, ctx, 0) == _lib.OK
+    by_slots = lib.fake_last_kernel()  # numbers the repeats, which are numbered otherwise where there are words
+    assert _start(lib, ctx, sampled) == _lib.OK
+    assert (lib.fake_last_kernel() == by_slots) == slots
+    assert lib.shmt_ctx_scratch_bytes(ctx) == held and lib.fake_frees() == 0
+
+
 def test_words_start_over_when_all_numbers_are_used(lib, ctx):
     """A hop takes as many numbers as it can have ids, here 2,020,000 of 2^32 - 1: 2,126 batches go by between two fills of
     the words, in the first lap and in the next."""
