@@ -1113,7 +1113,7 @@ def sampling_object(steps: int, local_rank: int, full: bool = True) -> dict:
                 "e2e": {"value": round(e2e_edges / (e2e_ms * 1e-3), 1), "unit": "edges/s",
                         "h2d_bytes_per_step": N_SEEDS * 4, "d2h_bytes_per_step": 9 * 8 + 4,
                         "ms_per_step": round(e2e_ms, 5)},
-                "gpu_launches": steps * 7, "api": "capi.sample_minibatch (all hops in one native call)"})
+                "gpu_launches": steps * 7, "api": "capi.sample_minibatch (all hops queued by one native call)"})
 
     # like with like against the reference, which needs indptr and indices of one dtype: int64 / int64
     indices64 = torch.from_numpy(indices_n.astype(np.int64))

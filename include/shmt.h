@@ -57,7 +57,8 @@ int64_t shmt_ctx_scratch_bytes(const shmt_ctx* ctx);
 int shmt_ctx_reserve(shmt_ctx* ctx, int64_t scratch_bytes, int64_t relabel_ids, void* stream);
 int shmt_ctx_reserve_minibatch(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                int n_hops, void* stream);
-/* The same, with room for a word per node of a graph of n_nodes (see shmt_minibatch_start). */
+/* The same, with room for a word per node of a graph of n_nodes (see shmt_minibatch_start).  The context does
+ * not grow for words afterwards: mini-batches on graphs with many more nodes use hashed slots.    */
 int shmt_ctx_reserve_minibatch_nodes(shmt_ctx* ctx, int64_t n_seeds, const int64_t* fanouts,
                                      int n_hops, int64_t n_nodes, void* stream);
 /* Wait for `stream` and report what the last asynchronous op on this context (a scan,

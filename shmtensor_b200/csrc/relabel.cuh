@@ -48,10 +48,11 @@ constexpr unsigned kRelNewId = 0x80000000u;  // indexes and new ids stay below 2
 // one's, and no word is ever put back (but all of them when the tags have come down, every 429 batches of
 // 10 M ids).  An element that finds another's index in its word is a repeat of that element, whose result it takes.
 // Other ids (a last hop may reach nodes that have no row) take slots.
-// Slots against words, 8,192 seeds 5/10/15, int64 ids: 2.4 M nodes 416 us and 292, 10 M 536 and 354, 24 M 579
-// and 438, 50 M 597 and 580, 110 M 606 and 712; 1,024 seeds 161 and 138, 165 and 142, 163 and 149, 164 and 156, 164
-// and 178; 50 seeds 93 and 86 at every size (words that held the new ids too).  The line is where the words
-// are the size of the L2 cache.
+// Slots against words, 5/10/15, 5 to 35 neighbours drawn evenly: 8,192 seeds, 2.4 M nodes 478 us and 317, 10 M 674 and 345,
+// 24 M 731 and 454, 33 M 751 and 481; 1,024 seeds 153 and 123, 158 and 130, 158 and 142, 158 and 146; 50 seeds 74 to 80 and 65
+// to 74.  The line is at 128 MB of words, about the L2 cache, for each stream that samples; beyond it the gain shrinks (3 to
+// 17 neighbours, int32, 8,192 seeds: 50 M nodes 433 and 361, 110 M 436 and 409; 1,024 seeds 128 and 118, 128 and
+// 126) while the memory grows to 200 and 440 MB a stream.
 struct RelTable {
   RelSlot* slots;  // cap entries
   uint32_t cap;

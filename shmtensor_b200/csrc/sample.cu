@@ -1269,8 +1269,8 @@ int shmt_sample_hop_eids(shmt_ctx* ctx, const void* indptr, int indptr_dtype, co
 
 // Multi-hop mini-batch: every hop's sampling kernel and relabel kernels are queued back
 // to back; each reads the size of its input from the device word the previous stage
-// wrote, with grids sized for the largest frontier the fan-outs allow.  The host waits
-// once, at the end, for all the sizes.
+// wrote, with grids sized for the largest frontier the fan-outs allow.  With `notes` the host hears of a
+// hop's sizes as soon as its ids are counted, without them of all sizes at the end.
 static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, const void* indices,
                                  int indices_dtype, const void* gpu_indptr, const void* gpu_indices,
                                  const shmt_map* map, const void* seeds, int64_t n_seeds,
@@ -1386,8 +1386,8 @@ static int queue_minibatch(shmt_ctx* ctx, const void* indptr, int indptr_dtype, 
     ps.start[1] = n_seeds;  // used for hop 0 only, whose seed count the host knows
     ps.dev_n0 = h == 0 ? nullptr : words + (h - 1) * 8 + 3;
     ps.dev_n1 = w + 1;
-    // every size and the status word are final once the last hop's ids are counted: that kernel
-    // hands them to the host, which returns while the last remap kernel is still running
+    // every size and the status word are final once the last hop's ids are counted: that kernel hands them
+    // to the host, which returns while the numbers of the repeats are still being written
     if (h == n_hops - 1)
       post = ctx_begin_post(ctx, words, n_hops * 8 + 8, w + 4);
     else
