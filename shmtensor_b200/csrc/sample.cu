@@ -347,11 +347,16 @@ constexpr int64_t kTinySeeds = 4 * kHopThreads, kTinyHostSeeds = 64;
 // at each place: an id below 2^25 times an odd number, modulo 2^25, has its place in the upper 10 bits, and the lower 15 tell
 // ids of one place apart; below them, in the entry, the index within the tile.  A neighbour whose id is there with a
 // smaller index leaves the word alone: whoever made the entry lowers it as far, or has left that to a smaller index still.
-// 8,192 seeds 5/10/15 on 10 M nodes, int64 ids: a tenth of all edges to one node 908 us without, 384 so (third hop 809 and 142;
-// hashed slots 560), neighbours by rank^-1.1 249 and 145 (slots 188), drawn evenly 352 both; 1,024 seeds 213 and 129, 108 and 106,
-// 128 and 130.  With 8-byte entries, and lanes that meet looked for in every step, not in the first alone, 344 was 373.
+// 8,192 seeds 5/10/15 on 10 M nodes, int64 ids: a tenth of all edges to one node 964 us without, 394 so (third hop 809 and 142;
+// hashed slots 560), neighbours by rank^-1.1 236 and 145 (slots 188), drawn evenly 344 both; 1,024 seeds 221 and 133, 106 and 107,
+// 127 and 129.  With 8-byte entries, and lanes that meet looked for in every step, not in the first alone, 344 was 373.
 constexpr int kLoweredTagBits = 15, kLoweredEntries = (int)(kRelMaxWords >> kLoweredTagBits);
 constexpr unsigned kLoweredLocal = (1u << (32 - kLoweredTagBits)) - 1u;
+// To look for lanes that meet costs a hop 0.5 us, so hops of fewer possible edges do without: with a line at 0, 2^15, 2^16 and
+// 2^17, 50 seeds 64.5, 66.7, 66.0 and 66.0 us (62.2 and 66.0 without any of this, the first on another box), 1,024
+// seeds 125.8, 127, 126.9 and 126.0 (124.3, 124.7), 1,024 of them on 10 M nodes with a tenth of all edges to one 127, 128, 134
+// and 134 (220).
+constexpr int64_t kCrowdedEdges = 1 << 16;
 // What a kernel may take beside its arrays of fixed size, at most 8 KB, without asking for more.
 constexpr size_t kPlainHopSmem = 40 << 10;
 
@@ -532,6 +537,7 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
   const RelRange range{job.rel_slots,
                        kFused ? relabel_near(most, relabel_slots_per_id(most, kHopSlotsPerEdge), job.rel_cap) : 0u,
                        job.rel_cap};
+  const bool crowds = n * k >= kCrowdedEdges;
   // The word of node `id`, unless this CTA has lowered it as far (s_lowered).  `local`, the index within the tile as
   // far as it can be held, goes up with `i`.
   auto lower = [&](unsigned id, unsigned i, unsigned local, bool crowd) {
@@ -749,13 +755,13 @@ __global__ void __launch_bounds__(kHopThreads, G < 32 ? kHopCtasPerSm : 4) sampl
           store_int(job.out_eids, job.indptr64, o, x.at() + s_eshift[x.seed()]);
         }
       }
-      if (kFused) enter(i, v, e, e < lead + kHopThreads);
+      if (kFused) enter(i, v, e, crowds && e < lead + kHopThreads);
     }
     return;
   }
   if (kFused)
     for (int j = (int)tid; j < rows; j += kHopThreads)
-      enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j), j, true);
+      enter(first + j, (IxT)load_int(job.seeds, job.seeds64, first + j), j, crowds);
 
   // k > 32, or weighted with replacement (G == 32): one warp per seed
   const uint32_t set_slots = job.set_slots;
